@@ -1142,10 +1142,10 @@ __global__ void k_leaf_summary(int nleaves, const int *__restrict__ leaf_r, RawO
     }
 }
 
-// leaf centres and each raw point in FP32 relative to its leaf's centre,
-// stored ready for the tile kernel's distance expansion
+// leaf boxes as the tile kernel reads them, and each raw point in FP32
+// relative to its leaf's centre
 __global__ void k_leaf_rel(int nleaves, const int *__restrict__ leaf_r, RawOut o,
-                           const double *__restrict__ box, double *leaf_c, float4 *t4,
+                           const double *__restrict__ box, kd_leaf *leaf, float4 *t4,
                            unsigned long long *hdiag)
 {
     int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -1153,20 +1153,19 @@ __global__ void k_leaf_rel(int nleaves, const int *__restrict__ leaf_r, RawOut o
     const double *b = box + 6 * (size_t)(nleaves + w);
     double cx = 0.5 * (b[0] + b[3]), cy = 0.5 * (b[1] + b[4]), cz = 0.5 * (b[2] + b[5]);
     if (lane == 0) {
-        leaf_c[3 * (size_t)w] = cx;
-        leaf_c[3 * (size_t)w + 1] = cy;
-        leaf_c[3 * (size_t)w + 2] = cz;
-        double hx = 0.5 * (b[3] - b[0]), hy = 0.5 * (b[4] - b[1]), hz = 0.5 * (b[5] - b[2]);
+        const double hx = fmax(b[3] - cx, cx - b[0]), hy = fmax(b[4] - cy, cy - b[1]),
+                     hz = fmax(b[5] - cz, cz - b[2]);
+        kd_leaf l;
+        l.c[0] = cx, l.c[1] = cy, l.c[2] = cz;
+        l.h[0] = __double2float_ru(hx), l.h[1] = __double2float_ru(hy), l.h[2] = __double2float_ru(hz);
+        l.pad_[0] = l.pad_[1] = l.pad_[2] = 0.0f;
+        leaf[w] = l;
         double h = sqrt(hx * hx + hy * hy + hz * hz);
         atomicMax(hdiag, (unsigned long long)__double_as_longlong(h));
     }
-    // (-2 t, |t|^2) of t = fl32(p - centre); |t|^2 is exact in FP64 from the
-    // FP32 components and rounded once
-    for (int i = leaf_r[w] + lane; i < leaf_r[w + 1]; i += 32) {
-        float tx = (float)(o.x[i] - cx), ty = (float)(o.y[i] - cy), tz = (float)(o.z[i] - cz);
-        double tn = (double)tx * tx + (double)ty * ty + (double)tz * tz;
-        t4[i] = make_float4(-2.0f * tx, -2.0f * ty, -2.0f * tz, (float)tn);
-    }
+    for (int i = leaf_r[w] + lane; i < leaf_r[w + 1]; i += 32)
+        t4[i] = make_float4(-2.0f * (float)(o.x[i] - cx), -2.0f * (float)(o.y[i] - cy),
+                            -2.0f * (float)(o.z[i] - cz), 0.0f);
 }
 
 __global__ void k_internal_summary(int lo_h, int hi_h, Summ sm)
@@ -1814,12 +1813,12 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
                                                                              sm);
     for (int d = D - 1; d >= 0; d--)
         k_internal_summary<<<blocks_for(1 << d, TPB), TPB, 0, s>>>(1 << d, 2 << d, sm);
-    double *leaf_c = keep.alloc<double>(3 * (size_t)nleaves);
+    kd_leaf *leaf = keep.alloc<kd_leaf>(nleaves);
     float4 *t4 = keep.alloc<float4>(n);
     unsigned long long *hdiag = pool.alloc<unsigned long long>(1);
     check(cudaMemsetAsync(hdiag, 0, sizeof(unsigned long long), s), "memset");
     k_leaf_rel<<<blocks_for((long long)nleaves * 32, TPB), TPB, 0, s>>>(nleaves, leaf_r, ro, sm.box,
-                                                                         leaf_c, t4, hdiag);
+                                                                         leaf, t4, hdiag);
     double leaf_hdiag = 0;
     {
         unsigned long long hb = read1(hdiag, s);
@@ -1908,7 +1907,7 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
     cat->d_run_tf = keep.keep(run_tf);
     cat->d_run_leaf = keep.keep(run_leaf);
     cat->d_t4 = keep.keep(t4);
-    cat->d_leaf_c = keep.keep(leaf_c);
+    cat->d_leaf = keep.keep(leaf);
     cat->leaf_hdiag = leaf_hdiag;
     cat->nblocks = nblocks;
     cat->d_blk_start = keep.keep(bstart);
@@ -2252,7 +2251,7 @@ extern "C" void kdg_free(kd_catalog *cat)
                     cat->d_box,      cat->d_ncount,      cat->d_ntf,     cat->d_nqf,
                     cat->d_leaf_run, cat->d_leaf_pos,    cat->d_run_start, cat->d_run_len,
                     cat->d_run_tf,
-                    cat->d_run_leaf, cat->d_t4,          cat->d_leaf_c,
+                    cat->d_run_leaf, cat->d_t4,          cat->d_leaf,
                     cat->d_blk_start, cat->d_blk_len,    cat->d_blk_qf,  cat->d_blk_box};
     for (void *p : ptrs)
         if (p) cudaFree(p);

@@ -17,18 +17,18 @@
 //                are accepted as count(block) x count(node), and leaf pairs
 //                become tile records (tree run, active edge range).  Run twice:
 //                once to count the tiles, once to write them.
-//   k_tiles    : one warp per query block, four query points per lane, walks
-//                its tile records.  Each tree run is staged into the warp's
-//                shared memory (the next run's loads already in flight) and
-//                every staged point is compared with the lane's four queries.
-//                Mixed mode: FP32 distances relative to the block centre,
-//                binned against the active edges with a saturating ramp that
-//                is exactly 0 or 1 outside a rigorous error band; a query
-//                with any pair of the run inside the band is recounted in
-//                FP64 with the reference's operation order.  FP64 mode: every
-//                distance in FP64.  Per-query bin counters live in shared
-//                memory and are reduced per (own field) into the global
-//                (bin, qfield, tfield) histogram when the tree field changes.
+//   k_tiles    : one CTA per query block, its queries as eight tiles of 16,
+//                walks the block's tile records.  Each query tile is compared
+//                with a run's points only against the edges that its own box
+//                and the leaf's allow.  Mixed mode: FP32 distances relative to
+//                the block centre from the tensor pipe, binned against those
+//                edges with a saturating ramp that is exactly 0 or 1 outside a
+//                rigorous error band; a query with any pair of the run inside
+//                the band is recounted in FP64 with the reference's operation
+//                order.  FP64 mode: every distance in FP64.  Per-query counters
+//                live in shared memory and are reduced per own field into the
+//                global (bin, qfield, tfield) histogram, tree field by tree
+//                field.
 
 #include <algorithm>
 #include <exception>
@@ -39,6 +39,8 @@
 #include <cmath>
 #include <mutex>
 #include <vector>
+
+#include <cuda_fp16.h>
 
 #include "kd_cuda_util.cuh"
 #include "kd_sort.cuh"
@@ -55,25 +57,7 @@ constexpr int kTravWarps = 4;
 // clustered 1M / 20M batch takes 16.3 ms instead of 19.5.
 constexpr int kStack = 1024;
 static_assert(kStack >= 32 * 24 + 64, "stack bound of a depth-24 counting tree");
-constexpr int kQ = KD_QPL;              // query points per lane
-constexpr int kTileWarpsPerCta = 4;
-constexpr int kMaxDistinctQf = 8;       // own fields reduced per warp at a flush
-constexpr int kPass32 = 4;              // edges per FP32 pass (register budget)
-constexpr int kStageMax = KD_RUN_MAX;  // points staged per pass
-
-constexpr int kCoopMax = 32;            // rechecks of a run done by the whole warp
-constexpr int kShardChunk = 32;         // blocks per interleaved shard chunk
-constexpr int kRunPerLane = KD_RUN_MAX / 32;  // staged run points per lane
-// FP32 tiles only where every staged value and square stays far inside FP32
-// range: tree and query points within kFp32Span of the block centre (their
-// squares and products below 1e30 < FLT_MAX) and squared edges below 1e30.
-// Records beyond that (coordinates or radii of 1e15 and more) are counted
-// by the exact FP64 path, as infinite radii are.
-constexpr double kFp32Span = 1e15;
-constexpr double kFp32MaxR = 1e30;
-// A run's exact counts travel one per byte (recounts) and its FP32 band sums
-// stay small (at most 4 * KD_RUN_MAX terms in [0, 1]): both need short runs.
-static_assert(KD_RUN_MAX % 32 == 0 && KD_RUN_MAX <= 128, "runs of 32..128 points");
+constexpr int kShardChunk = 32;  // blocks per interleaved shard chunk
 
 struct TreeSide {
     const double *box;
@@ -95,8 +79,8 @@ struct JobDesc {
     TreeSide T;
     QuerySide Q;
     const double *tx, *ty, *tz;  // tree points, FP64, counting order
-    const float4 *t4;            // tree points: (-2 t_r, |t_r|^2), t_r relative to leaf centre
-    const double *leaf_c;        // 3 per leaf
+    const float4 *t4;            // tree points: -2 t_r, t_r relative to the leaf's centre
+    const kd_leaf *leaf;         // leaf boxes: centre and half-extents
     double hT;                   // largest leaf half-diagonal, with margin
     unsigned long long *H;       // (ne + 1) x Fqe x Fte bin histogram
     // Symmetric job (tree and query are one catalog whose points all have own
@@ -316,116 +300,94 @@ __global__ void __launch_bounds__(32 * kTravWarps) k_traverse(const JobDesc *__r
     }
 }
 
-// Rigorous half-width E of the uncertain band around edge R.
-// Geometry of a tile: query points within Rq of the block centre o; a tree
-// point t is stored as t_r = fl32(t - c) (c: its leaf's centre, |t - c| <= hT)
-// and staged as t' = fl32(t_r + fl32(c - o)); the query as q' = fl32(q - o);
-//   T = |t'|^2 (FP32 FMA chain),  s = T - 2 q'.t' (FP32 FMA chain),
-//   thr = R - |q'|^2,  c = sat(a - s/4E) with a = fl(A - |q'|^2/4E),
-//   A = fl(1/2 + R/4E).
-// c is exactly 1 when s is more than 2E below thr and 0 when more than 2E
-// above.  Every pair that is counted or lies within E of the edge has
-// d2 <= 2R, so |t - o| <= P = sqrt(2R) + Rq, and for such pairs
-//   |(s - thr) - (d2 - R)| <= u32 [2 (P + Rq)(2P + 2hT + Rq) + 6 P (P + Rq)
-//                                  + 3 (R + Rq^2)]
-// (coordinate rounding 2 sqrt(d2) eta with eta <= u32 (2P + 2hT + Rq), the
-// roundings of T and of the FMA chain for s, and those of the threshold).
-// E adds 25% and a term for the FP64 reference's own rounding, and is rounded
-// up to a power of two so that 1/(4E) is exact in FP32.  Pairs with d2 > 2R
-// sit far above the band: their FP32 error grows only like 10 u32 d2.
-__device__ __forceinline__ double band_halfwidth(double R, double Rq, double hT)
-{
-    const double u32 = 5.9604644775390625e-08;  // 2^-24
-    const double P = sqrt(2.0 * R) + Rq;
-    const double e = 2.0 * (P + Rq) * (2.0 * P + 2.0 * hT + Rq) + 6.0 * P * (P + Rq) +
-                     3.0 * (R + Rq * Rq);
-    const double E = 1.25 * u32 * e + 1e-15 * R + 1e-30;
-    int ex;
-    frexp(E, &ex);
-    return ldexp(1.0, ex);
-}
+// ---------------------------------------------------------------- tiles
+//
+// One CTA of four warps per query block.  Its 128 queries are eight tiles of
+// 16; the warps take the block's tile records (each a run of up to 64 points
+// of one leaf) in chunks of 4 to 32, one tree field after the other, and share
+// the queries' operands and the counters.  For every record each query tile
+// has its own window: the edges that the distances between the tile's box and
+// the leaf's box allow, found by one lane per (query tile, record) for four
+// records at a time.  A query tile without an edge in its window costs one
+// counter; the others run over the run's points in steps of 16 queries x 8
+// points, against the edges of their window only.  With one window per block
+// and leaf, a pair of the clustered 1M / 20M batch is compared with 3.0 edges;
+// with one per 16 queries it is 1.5, and a quarter of the pairs needs none.
+//
+// Mixed mode: the squared distances of a step are one mma.m16n8k16 (F16 in,
+// FP32 out): each coordinate of query and point is split into two halves, so
+// that all four half products of the three coordinates are 12 of the 16 terms,
+// and N = |t|^2 - Rref as two halves times 1 are two more; the accumulator
+// starts at |q|^2 + Rref - R of the window's first edge.  The products are
+// exact, and the result x = d2 - R is small where the decision is made: its
+// error is 0.59 to 1.09 u (sqrt(d2) + Rq)^2 RMS (u = 2^-24) at radii of 2 to 10
+// block radii Rq and 0.25 at half a block radius, where the FP32 FMA chain it
+// replaces has 0.59 to 1.16 and 0.23.
+// FP64 mode: two query tiles at a time, a query per lane, every distance in
+// the reference's operation order.
+//
+// Bound: the FP32 pipe, by the binning (a ramp, a count and a check per pair
+// and edge: 15 clocks per 128 pairs and edge in isolation, 20 here), then the
+// per-pass work around it.  Seven CTAs per SM: what is uniform over a block
+// lives in shared memory so that 72 registers do (four warps per scheduler and
+// 128 registers: 31.5 ms for 3M uniform points and 21 edges, seven: 23.8; the
+// former kernel, a warp per block with four queries per lane and one window:
+// 36.2.  1 edge: 10.8 against 16.4.  FP64 mode: 37.3 against 51.0).  CTA per
+// block instead of warp per block also gives small counts four times the
+// warps: 0.31 against 1.72 ms for DD + DR + RR of 4k / 80k points.
+// Measured and left out: tcgen05 with the batch's distances in TMEM (free
+// distances, but 128 queries in step and the same binning: 45.7 ms); items of
+// one query tile and one edge, four at a time, repeating the MMA (39.3); two
+// query tiles per pass where their windows agree on two edges (24.1).
 
-// saturating FMA: clamp(a*b + c, 0, 1) in one instruction (NaN -> 0)
-__device__ __forceinline__ float fma_sat(float a, float b, float c)
-{
-    float d;
-    asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-    return d;
-}
+constexpr int kMT = 16;                       // queries per tile (MMA rows)
+constexpr int kMTiles = KD_BLOCK_MAX / kMT;   // query tiles per block
+constexpr int kNT = 8;                        // points per step (MMA columns)
+constexpr int kGroup = 32 / kMTiles;          // records whose windows are found together
+constexpr int kTileWarps = 4;
+constexpr int kTileThreads = 32 * kTileWarps;
+constexpr int kTilesPerSm = 7;                // CTAs per SM the registers are held to
+constexpr int kPStride = 136;                 // counters per edge (128 queries + bank shift)
+static_assert(kMTiles == 8 && KD_RUN_MAX == 64 && kTileThreads == KD_BLOCK_MAX, "lane layouts below");
 
-// FP32 pass of a lane's four queries over a staged run and K (<= 4) edges.
-// Each pair gives c = sat(a_k + s * nsl_k): exactly 0 or 1 outside the band,
-// in [1/4, 3/4] inside it.  Per query, sum_k acc_k equals acc2 = sum c^2 bit
-// for bit when every c is 0 or 1; a band pair makes them differ by at least
-// 3/16, far above the FP32 rounding of these short sums (at most
-// 4 * kStageMax <= 512 terms in [0, 1]: each sum is off by at most
-// 512 * 512 * 2^-24 = 1/64).
-// Queries travel in pairs through the packed FP32 pipe (FFMA2/FADD2: two
-// independent round-to-nearest operations per instruction, the same values
-// as the scalar chain); the saturating ramp has no packed form and stays
-// scalar.  A staged point is (X, X, Y, Y), (Z, Z, N, N): each coordinate
-// twice, so one 16-byte shared load feeds both halves of a pair.
-// Returns a bit mask of the queries with a band pair.
-template <int K>
-__device__ __forceinline__ unsigned fp32_run(const float4 *__restrict__ ts, int rl,
-                                             const float2 (&qx)[kQ / 2],
-                                             const float2 (&qy)[kQ / 2],
-                                             const float2 (&qz)[kQ / 2],
-                                             const float (&a)[kQ][kPass32],
-                                             const float (&nsl)[kPass32],
-                                             unsigned (&pc)[kQ / 2][4])
+// FP32 tiles only where every staged value and square stays far inside FP32
+// range: tree and query points within kFp32Span of the block centre (their
+// squares and products below 1e30 < FLT_MAX) and squared edges below 1e30.
+// Records beyond that (coordinates or radii of 1e15 and more) are counted
+// by the exact FP64 path.
+constexpr double kFp32Span = 1e15;
+constexpr double kFp32MaxR = 1e30;
+
+// Half-width E of the band around edge R inside which the MMA's decision is
+// not trusted: a pair whose computed d2 - R is at least E away from zero is
+// on the side that the FP64 reference puts it on.
+// Geometry: query q and tree point t relative to the block centre, |q| <= Rq;
+// t is staged as t' = fl32(fl32(t - c) + fl32(c - o)) (c: its leaf's centre,
+// |t - c| <= hT), both scaled by a power of two S.  The MMA sums
+//   x = C + N - 2 q.t',  N = |t'|^2 - Rref,  C = |q|^2 + Rref - R0,
+// with the cross term's factors and N as two halves each (products exact).
+// The decision is on x - (R - R0).  With u = 2^-24, P = sqrt(1.2 R) + Rq >=
+// |t'| for every pair with d2 <= 1.2 R, and M = P^2 + R:
+//   coordinates  2 (P + Rq) u (2P + 2hT + Rq)   as two roundings of t
+//   N            3u M as an FMA chain, 2u M its two halves
+//   cross term   8u Rq P      (2^-23 relative for each split factor)
+//   C, edges     2u (Rq^2 + R) + 3u R
+//   ramp         4u R         (its offset and slope)
+//   accumulation 17 terms, each cut at no more than u of the largest one
+//                (|N|, |C| <= M, |2 q t'| <= 2 Rq P): 17u max(M, 2 Rq P)
+// plus the halves' absolute floor, 2^-25 of the scaled values, and the
+// rounding of the FP64 reference itself; 25% on top.  (Measured: at most 6u
+// (sqrt(d2) + Rq)^2 in all.)  Pairs with d2 > 1.2 R: their error grows with
+// (sqrt(d2) + Rq)^2 while x - (R - R0) >= d2 / 6, so the sign is right
+// unless d2 is so small beside Rq^2 that E's Rq terms cover the error.
+__device__ __forceinline__ double band_halfwidth(double R, double Rq, double hT, double S)
 {
-    float2 acc[kQ / 2][K], acc2[kQ / 2];
-#pragma unroll
-    for (int h = 0; h < kQ / 2; h++) {
-        acc2[h] = make_float2(0.0f, 0.0f);
-#pragma unroll
-        for (int k = 0; k < K; k++) acc[h][k] = make_float2(0.0f, 0.0f);
-    }
-    auto point = [&](const float4 xy, const float4 zn) {
-        const float2 X = make_float2(xy.x, xy.y), Y = make_float2(xy.z, xy.w);
-        const float2 Z = make_float2(zn.x, zn.y), N = make_float2(zn.z, zn.w);
-#pragma unroll
-        for (int h = 0; h < kQ / 2; h++) {
-            const float2 s = __ffma2_rn(qz[h], Z, __ffma2_rn(qy[h], Y, __ffma2_rn(qx[h], X, N)));
-#pragma unroll
-            for (int k = 0; k < K; k++) {
-                const float2 c = make_float2(fma_sat(s.x, nsl[k], a[2 * h][k]),
-                                             fma_sat(s.y, nsl[k], a[2 * h + 1][k]));
-                acc[h][k] = __fadd2_rn(acc[h][k], c);
-                acc2[h] = __ffma2_rn(c, c, acc2[h]);
-            }
-        }
-    };
-    int j = 0;
-    for (; j + 4 <= rl; j += 4) {
-        const float4 t0 = ts[2 * j], t1 = ts[2 * j + 1], t2 = ts[2 * j + 2], t3 = ts[2 * j + 3];
-        const float4 t4 = ts[2 * j + 4], t5 = ts[2 * j + 5], t6 = ts[2 * j + 6], t7 = ts[2 * j + 7];
-        point(t0, t1);
-        point(t2, t3);
-        point(t4, t5);
-        point(t6, t7);
-    }
-    for (; j < rl; j++) point(ts[2 * j], ts[2 * j + 1]);
-    // Counts without the conversion unit: v + 1.5 * 2^23 lands on the integer
-    // grid of that binade, so the low 16 bits of its pattern are round(v)
-    // (0 <= v <= 256; the bias 0x4B400000 has zero low half).  The two
-    // queries of a pair are packed as (query 2h) | (query 2h + 1) << 16.
-    const float2 bias = make_float2(12582912.0f, 12582912.0f);
-    unsigned band = 0;
-#pragma unroll
-    for (int h = 0; h < kQ / 2; h++) {
-        float2 tot = make_float2(0.0f, 0.0f);
-#pragma unroll
-        for (int k = 0; k < K; k++) {
-            tot = __fadd2_rn(tot, acc[h][k]);
-            const float2 b = __fadd2_rn(acc[h][k], bias);
-            pc[h][k] = __byte_perm(__float_as_uint(b.x), __float_as_uint(b.y), 0x5410);
-        }
-        if (tot.x != acc2[h].x) band |= 1u << (2 * h);
-        if (tot.y != acc2[h].y) band |= 2u << (2 * h);
-    }
-    return band;
+    const double u = 5.9604644775390625e-08;  // 2^-24
+    const double P = sqrt(1.2 * R) + Rq, M = P * P + R;
+    const double e = 2.0 * (P + Rq) * (2.0 * P + 2.0 * hT + Rq) + 5.0 * M + 8.0 * Rq * P +
+                     2.0 * (Rq * Rq + R) + 7.0 * R + 17.0 * fmax(M, 2.0 * Rq * P);
+    const double f = 1.1920928955078125e-07 / S;  // 2^-23 / S
+    return 1.25 * u * e + 1e-15 * R + f * (P + Rq) + f / S;
 }
 
 // reference-order FP64 distance (kdquery.c:39-47 as compiled)
@@ -436,74 +398,6 @@ __device__ __forceinline__ double d2_ref(double tx, double ty, double tz, double
     double s = __dmul_rn(dx, dx);
     s = __fma_rn(dy, dy, s);
     return __fma_rn(dz, dz, s);
-}
-
-// FP64 pass of the four queries over a staged run (FP64 mode): cumulative
-// counts for K (<= 4) edges.
-template <int K>
-__device__ __forceinline__ void fp64_run(const double *__restrict__ tx,
-                                         const double *__restrict__ ty,
-                                         const double *__restrict__ tz, int rl,
-                                         const double (&qx)[kQ], const double (&qy)[kQ],
-                                         const double (&qz)[kQ], const double *R,
-                                         int (&cnt)[kQ][4])
-{
-    double r[K];
-#pragma unroll
-    for (int k = 0; k < K; k++) r[k] = R[k];
-#pragma unroll
-    for (int p = 0; p < kQ; p++)
-#pragma unroll
-        for (int k = 0; k < 4; k++) cnt[p][k] = 0;
-    for (int j = 0; j < rl; j++) {
-        const double x = tx[j], y = ty[j], z = tz[j];
-#pragma unroll
-        for (int p = 0; p < kQ; p++) {
-            const double d2 = d2_ref(x, y, z, qx[p], qy[p], qz[p]);
-#pragma unroll
-            for (int k = 0; k < K; k++) cnt[p][k] += d2 < r[k];
-        }
-    }
-}
-
-// Warp-cooperative exact recount of one query over a run: every lane takes
-// the points j = lane, lane + 32, ... (at most KD_RUN_MAX / 32, so the warp
-// sum of each per-edge count is at most KD_RUN_MAX <= 128: the four
-// byte-packed counts add without carries in one reduction).  Returns the
-// packed counts in all lanes.
-__device__ __noinline__ unsigned exact_pass_warp(const double *__restrict__ tx,
-                                                 const double *__restrict__ ty,
-                                                 const double *__restrict__ tz, int rl,
-                                                 double qx, double qy, double qz,
-                                                 const double *R, int kn, int lane)
-{
-    unsigned part = 0;
-    for (int j = lane; j < rl; j += 32) {
-        const double d2 = d2_ref(__ldg(tx + j), __ldg(ty + j), __ldg(tz + j), qx, qy, qz);
-#pragma unroll
-        for (int k = 0; k < 4; k++)
-            if (k < kn) part += (unsigned)(d2 < R[k]) << (8 * k);
-    }
-    return __reduce_add_sync(0xffffffffu, part);
-}
-
-// Exact recount of one query over a run (global FP64 coordinates), for band
-// rechecks and edges FP32 cannot represent; counts packed one per byte.  Out
-// of line so the FP32 loop stays small.
-__device__ __noinline__ unsigned exact_pass(const double *__restrict__ tx,
-                                            const double *__restrict__ ty,
-                                            const double *__restrict__ tz, int rl, double qx,
-                                            double qy, double qz, const double *R, int kn)
-{
-    int c4[4] = {0, 0, 0, 0};
-    for (int j = 0; j < rl; j++) {
-        const double d2 = d2_ref(__ldg(tx + j), __ldg(ty + j), __ldg(tz + j), qx, qy, qz);
-#pragma unroll
-        for (int k = 0; k < 4; k++)
-            if (k < kn) c4[k] += d2 < R[k];
-    }
-    return (unsigned)c4[0] | ((unsigned)c4[1] << 8) | ((unsigned)c4[2] << 16) |
-           ((unsigned)c4[3] << 24);
 }
 
 struct TileArgs {
@@ -517,424 +411,670 @@ struct TileArgs {
     const long long *off;       // launch-relative tile offsets
     const uint4 *rec;
     int *work;
-    unsigned long long *stats;  // tested, rechecked, accepted, wide, edge-pairs, warp tiles
+    unsigned long long *stats;  // tested, rechecked, accepted, wide, edge-pairs, tiles
 };
 
-// shared memory of one warp
-template <int MODE> struct WarpSmem {
+// saturating FMA: clamp(a*b + c, 0, 1) in one instruction (NaN -> 0)
+__device__ __forceinline__ float fma_sat(float a, float b, float c)
+{
+    float d;
+    asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
+// d = A (16 x 16, row) B (16 x 8, col) + c, rows g = lane / 4 and g + 8 at
+// columns 2 (lane % 4) and + 1 (c0, c1: the rows' start values)
+__device__ __forceinline__ void mma_16x8x16(float (&d)[4], const uint4 &a, uint32_t b, float c0,
+                                            float c1)
+{
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, "
+        "{%4, %5, %6, %7}, {%8, %8}, {%9, %9, %10, %10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b), "f"(c0), "f"(c1));
+}
+
+// v as two halves hi + lo (lo rounds what hi left over)
+__device__ __forceinline__ uint32_t split_halves(float v)
+{
+    const __half hi = __float2half_rn(v);
+    const __half lo = __float2half_rn(v - __half2float(hi));
+    return (uint32_t)__half_as_ushort(hi) | ((uint32_t)__half_as_ushort(lo) << 16);
+}
+
+// FP64 mode: a query's pairs with a staged run (np pairs of points; a missing
+// one is at 1e300) below K (<= 4) edges
+template <int K>
+__device__ __forceinline__ void fp64_run(const double2 *__restrict__ tx,
+                                         const double2 *__restrict__ ty,
+                                         const double2 *__restrict__ tz, int np, double qx, double qy,
+                                         double qz, const double *R, unsigned (&cnt)[4])
+{
+    double r[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) r[k] = R[k];
+#pragma unroll 4
+    for (int j = 0; j < np; j++) {
+        const double2 x = tx[j], y = ty[j], z = tz[j];
+        const double a = d2_ref(x.x, y.x, z.x, qx, qy, qz), b = d2_ref(x.y, y.y, z.y, qx, qy, qz);
+#pragma unroll
+        for (int k = 0; k < K; k++) cnt[k] += (unsigned)(a < r[k]) + (unsigned)(b < r[k]);
+    }
+}
+
+// Shared memory of a CTA (what is the same for all threads of a block lives
+// here rather than in registers: warps in flight are what the kernel needs).
+//   F[e * kMTiles + m]: points of records below edges e, e + 1, ... for every
+//     query of tile m
+//   P[e * kPStride + q], behind it: pairs of query q below edge e, over the
+//     records whose window for q's tile holds e
+struct TileCommon {
     JobDesc job;  // the job of the block being counted
-    float Aw[KD_MAX_EDGES];
-    float nsl[KD_MAX_EDGES];
-    double cmax2;  // squared leaf-centre distance below which FP32 is safe
-    int uq[kMaxDistinctQf];
-    float4 stage[MODE == KD_MODE_MIXED ? 2 * kStageMax : 1];  // (X,X,Y,Y), (Z,Z,N,N)
-    double stage64[MODE == KD_MODE_FP64 ? 3 * KD_RUN_MAX : 1];
+    double R[KD_MAX_EDGES];
+    double o[3];                             // block centre
+    float Rup[KD_MAX_EDGES], Rdn[KD_MAX_EDGES];  // R rounded up / down
+    float qc[kMTiles][3], qh[kMTiles][3];    // the query tiles' boxes: centre, half-extents
+    unsigned F[(KD_MAX_EDGES + 1) * kMTiles];
+    unsigned keys[16];                       // the block's flush keys, a bit each
+    unsigned long long stats[5];             // tested, rechecked, wide, edge-pairs, tiles
+    long long eoff;                          // the block's records: first, number
+    int ecnt, chunk;
+    int qs, qlen;                            // its queries: first, number
+    int next, item, kmin, kmax, kfp;
+    float Rq, hT, S;
 };
+template <int MODE> struct TileSmem;
+template <> struct TileSmem<KD_MODE_MIXED> : TileCommon {
+    alignas(16) uint4 qa[kMTiles][32];       // MMA A fragments of the query tiles
+    float2 qn[kMTiles][kMT / 2];             // |q|^2 S^2 of rows g and g + 8
+    float2 edge[KD_MAX_EDGES];               // R S^2 and 0.4545 / (E S^2)
+    alignas(16) uint32_t bs[kTileWarps][KD_RUN_MAX / kNT * 32];  // MMA B fragments of the staged runs
+};
+template <> struct TileSmem<KD_MODE_FP64> : TileCommon {
+    alignas(16) double pt[kTileWarps][3][KD_RUN_MAX];  // the staged runs
+};
+
+// The MMA operands of the block's queries (relative to the block centre o) and
+// the edge tables, at scale S, by the whole CTA.  Lane (g, t) of a query
+// tile's fragment holds, for t < 3, coordinate t of rows g and g + 8: the
+// halves of v = -2 q_t S as (hi, hi) against the point's (hi, lo), and (lo,
+// lo) against the same; for t = 3, (1, 1) against the halves of N, and (0, 0).
+__device__ __noinline__ void set_scale(TileSmem<KD_MODE_MIXED> &s, int ne, int tid)
+{
+    const double S = (double)s.S, Rq = (double)s.Rq, hT = (double)s.hT;
+    const int qs = s.qs, qlen = s.qlen;
+    for (int i = tid; i < kMTiles * 32; i += kTileThreads) {
+        const int m = i >> 5, g = (i & 31) >> 2, t = i & 3;
+        uint32_t hh[2] = {0x3C003C00u, 0x3C003C00u}, ll[2] = {0u, 0u};
+        if (t < 3) {
+            const double *const src = t == 0 ? s.job.Q.x : (t == 1 ? s.job.Q.y : s.job.Q.z);
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                const int q = kMT * m + g + 8 * r;
+                const double v = q < qlen ? -2.0 * (src[qs + q] - s.o[t]) * S : 0.0;
+                const __half h = __double2half(v), l = __double2half(v - (double)__half2float(h));
+                hh[r] = (uint32_t)__half_as_ushort(h) * 0x10001u;
+                ll[r] = (uint32_t)__half_as_ushort(l) * 0x10001u;
+            }
+        }
+        s.qa[m][i & 31] = make_uint4(hh[0], hh[1], ll[0], ll[1]);
+    }
+    {
+        double n = 0.0;
+        if (tid < qlen) {
+            const double x = (s.job.Q.x[qs + tid] - s.o[0]) * S, y = (s.job.Q.y[qs + tid] - s.o[1]) * S,
+                         z = (s.job.Q.z[qs + tid] - s.o[2]) * S;
+            n = x * x + y * y + z * z;
+        }
+        float2 &q = s.qn[tid / kMT][tid % 8];
+        if (tid % kMT < 8) q.x = (float)n;
+        else q.y = (float)n;
+    }
+    for (int k = tid; k < ne; k += kTileThreads)
+        s.edge[k] = make_float2((float)(s.R[k] * S * S),
+                                (float)(0.5 / 1.1 / (band_halfwidth(s.R[k], Rq, hT, S) * S * S)));
+}
+__device__ __forceinline__ void set_scale(TileSmem<KD_MODE_FP64> &, int, int) {}
+
+// Exact counts of the flagged rows of query tile m (rows: bit per row) over
+// the run [rs, rs + n) for kn (<= 4) edges from kk on, added to their counters
+// less what the lanes (g, t < kn) added before: v, rows g and g + 8.  The
+// run's points stay in registers, two per lane.
+__device__ __noinline__ void recount_rows(TileCommon &s, unsigned *P, unsigned rows, int m, int rs, int n,
+                                          int kk, int kn, unsigned v, int lane)
+{
+    static_assert(KD_RUN_MAX <= 64, "two points per lane");
+    const JobDesc &J = s.job;
+    const int g = lane >> 2, t = lane & 3;
+    rows &= (2u << (min(kMT, s.qlen - kMT * m) - 1)) - 1u;
+    if (lane == 0) atomicAdd(&s.stats[1], (unsigned long long)(__popc(rows) * n));
+    double x[2], y[2], z[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int j = rs + min(lane + 32 * h, n - 1);
+        x[h] = __ldg(J.tx + j);
+        y[h] = __ldg(J.ty + j);
+        z[h] = __ldg(J.tz + j);
+    }
+    while (rows) {
+        const int row = __ffs(rows) - 1;
+        rows &= rows - 1;
+        const int qi = s.qs + kMT * m + row;
+        const double qx = __ldg(J.Q.x + qi), qy = __ldg(J.Q.y + qi), qz = __ldg(J.Q.z + qi);
+        unsigned part = 0;  // counts of four edges, a byte each (n <= 64)
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+            if (lane + 32 * h < n) {
+                const double d2 = d2_ref(x[h], y[h], z[h], qx, qy, qz);
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    if (k < kn) part += (unsigned)(d2 < s.R[kk + k]) << (8 * k);
+            }
+        const unsigned c = (__reduce_add_sync(0xffffffffu, part) >> (8 * t)) & 0xFFu;
+        if (g == (row & 7) && t < kn)
+            atomicAdd(&P[(kk + t) * kPStride + kMT * m + row], c - (row < 8 ? v & 0xFFFFu : v >> 16));
+    }
+}
+
+// M query tiles against a staged run (nt steps of 8 points) and the K edges
+// from kk on (K * M <= 4).  Each pair gives c = sat(a_k - 0.4545 x / E): exactly
+// 0 or 1 where |x| is 10% beyond the band, in [1/22, 21/22] inside it.  Per
+// tile, row and lane, sum_k acc_k equals sq = sum c^2 bit for bit when every c
+// is 0 or 1; a band pair makes them differ by at least 0.04, far above the
+// FP32 rounding of these short sums (at most 4 * 16 terms in [0, 1]).  Rows g
+// and g + 8 travel as a pair through the packed FP32 pipe (FADD2 / FFMA2); the
+// saturating ramp has no packed form.
+template <int K, int M>
+__device__ __forceinline__ void tile_pass(TileSmem<KD_MODE_MIXED> &s, unsigned *P, const int (&mt)[2],
+                                          int kk, int nt, float ref, int rs, int n, int lane,
+                                          const uint32_t *__restrict__ bs)
+{
+    static_assert(K * M <= 4 && M <= 2, "an item per lane of a row");
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int NI = K * M;  // item i: edge kk + i % K of tile mt[i / K]
+    const int g = lane >> 2, t = lane & 3;
+    const float e0 = s.edge[kk].x, nsl = -s.edge[kk + K - 1].y;
+    float a[K];
+    a[0] = 0.5f;
+#pragma unroll
+    for (int k = 1; k < K; k++) a[k] = fmaf(e0 - s.edge[kk + k].x, nsl, 0.5f);
+    uint4 qa[M];
+    float c0[M], c1[M];
+    float2 acc[M][K], sq[M][2];
+#pragma unroll
+    for (int i = 0; i < M; i++) {
+        qa[i] = s.qa[mt[i]][lane];
+        const float2 qn = s.qn[mt[i]][g];
+        c0[i] = qn.x + (ref - e0);
+        c1[i] = qn.y + (ref - e0);
+        sq[i][0] = sq[i][1] = make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int k = 0; k < K; k++) acc[i][k] = make_float2(0.0f, 0.0f);
+    }
+    auto bin = [&](const float (&x)[4], int i) {
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            const float2 c = make_float2(fma_sat(x[0], nsl, a[k]), fma_sat(x[2], nsl, a[k]));
+            const float2 d = make_float2(fma_sat(x[1], nsl, a[k]), fma_sat(x[3], nsl, a[k]));
+            acc[i][k] = __fadd2_rn(acc[i][k], c);
+            sq[i][0] = __ffma2_rn(c, c, sq[i][0]);
+            acc[i][k] = __fadd2_rn(acc[i][k], d);
+            sq[i][1] = __ffma2_rn(d, d, sq[i][1]);
+        }
+    };
+    if constexpr (M == 1) {
+        for (; nt >= 2; nt -= 2, bs += 64) {
+            float x[4], y[4];
+            mma_16x8x16(x, qa[0], bs[0], c0[0], c1[0]);
+            mma_16x8x16(y, qa[0], bs[32], c0[0], c1[0]);
+            bin(x, 0);
+            bin(y, 0);
+        }
+        if (nt) {
+            float x[4];
+            mma_16x8x16(x, qa[0], bs[0], c0[0], c1[0]);
+            bin(x, 0);
+        }
+    } else {
+        for (; nt; nt--, bs += 32) {
+            float x[M][4];
+#pragma unroll
+            for (int i = 0; i < M; i++) mma_16x8x16(x[i], qa[i], bs[0], c0[i], c1[i]);
+#pragma unroll
+            for (int i = 0; i < M; i++) bin(x[i], i);
+        }
+    }
+    // counts without the conversion unit: v + 1.5 * 2^23 has round(v) in the
+    // low bits of its pattern (the bias's low half is zero); rows g | g + 8 << 16
+    unsigned pc[4] = {0u, 0u, 0u, 0u};
+    bool b0[M], b1[M], any = false;
+#pragma unroll
+    for (int i = 0; i < M; i++) {
+        const float2 q = __fadd2_rn(sq[i][0], sq[i][1]);
+        float2 tot = acc[i][0];
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            if (k) tot = __fadd2_rn(tot, acc[i][k]);
+            const float2 b = __fadd2_rn(acc[i][k], make_float2(12582912.0f, 12582912.0f));
+            pc[i * K + k] = __byte_perm(__float_as_uint(b.x), __float_as_uint(b.y), 0x5410);
+        }
+        b0[i] = tot.x != q.x;
+        b1[i] = tot.y != q.y;
+        any = any || b0[i] || b1[i];
+    }
+    // sums over a row's four lanes, item i ending in lane i of the row
+    unsigned v;
+    if constexpr (NI == 1) {
+        v = pc[0] + __shfl_xor_sync(FULL, pc[0], 1);
+        v += __shfl_xor_sync(FULL, v, 2);
+    } else {
+        const bool odd = t & 1, high = t & 2;
+        v = (odd ? pc[1] : pc[0]) + __shfl_xor_sync(FULL, odd ? pc[0] : pc[1], 1);
+        if constexpr (NI == 2) {
+            v += __shfl_xor_sync(FULL, v, 2);
+        } else {
+            const unsigned u = (odd ? pc[3] : pc[2]) + __shfl_xor_sync(FULL, odd ? pc[2] : pc[3], 1);
+            const unsigned give = high ? v : u;
+            v = (high ? u : v) + __shfl_xor_sync(FULL, give, 2);
+        }
+    }
+    const int my = M == 1 ? mt[0] : (t / K == 0 ? mt[0] : mt[1]);
+    unsigned *const at = P + (kk + t % K) * kPStride + kMT * my + g;
+    if (t < NI) {
+        atomicAdd(at, v & 0xFFFFu);
+        atomicAdd(at + 8, v >> 16);
+    }
+    if (__any_sync(FULL, any)) {
+#pragma unroll
+        for (int i = 0; i < M; i++) {
+            const unsigned lo = __ballot_sync(FULL, b0[i]), hi = __ballot_sync(FULL, b1[i]);
+            if (!(lo | hi)) continue;
+            unsigned rows = 0;
+#pragma unroll
+            for (int r = 0; r < 8; r++)
+                rows |= (((lo >> (4 * r)) & 0xFu) ? 1u << r : 0u) | (((hi >> (4 * r)) & 0xFu) ? 256u << r : 0u);
+            const unsigned vi = i == 0 ? v : __shfl_sync(FULL, v, (lane & 28) | ((t + K) & 3));
+            recount_rows(s, P, rows, mt[i], rs, n, kk, K, vi, lane);
+        }
+    }
+}
 
 template <int MODE>
-__global__ void __launch_bounds__(32 * kTileWarpsPerCta, 4) k_tiles(TileArgs A)
+__global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
 {
     extern __shared__ __align__(16) unsigned char smem[];
+    constexpr unsigned FULL = 0xffffffffu;
+    TileSmem<MODE> &s = *(TileSmem<MODE> *)smem;
     const int ne = A.ne;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double *R = (double *)smem;  // ne
-    WarpSmem<MODE> *ws = (WarpSmem<MODE> *)(R + KD_MAX_EDGES) + w;
-    // per-query bin counters, two queries per word, 16 bits each (a flush
-    // empties them before any could pass 65535): P[(e * kQ / 2 + h) * 32 + lane]
-    // holds queries 2h (low half) and 2h + 1 (high half)
-    unsigned *P = (unsigned *)((WarpSmem<MODE> *)(R + KD_MAX_EDGES) + kTileWarpsPerCta) +
-                  (size_t)w * (ne + 1) * (kQ / 2) * 32;
-    for (int k = threadIdx.x; k < ne; k += blockDim.x) R[k] = A.rsq[k];
-    __syncthreads();
-    unsigned long long pairs = 0, rechecked = 0, wide = 0, kpairs = 0, wtiles = 0;
+    unsigned *const P = (unsigned *)(smem + sizeof(TileSmem<MODE>));
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    const int wm = lane & (kMTiles - 1), wr = lane / kMTiles;  // this lane's window: tile, record
+    for (int k = tid; k < ne; k += kTileThreads) {
+        const double r = A.rsq[k];
+        s.R[k] = r;
+        s.Rup[k] = __double2float_ru(r);
+        s.Rdn[k] = __double2float_rd(r);
+    }
+    for (int k = tid; k < ne * kPStride; k += kTileThreads) P[k] = 0;
+    for (int k = tid; k < (KD_MAX_EDGES + 1) * kMTiles; k += kTileThreads) s.F[k] = 0;
+    if (tid < 5) s.stats[tid] = 0;
 
     while (true) {
-        int item = 0;
-        if (lane == 0) item = atomicAdd(A.work, 1);
-        item = __shfl_sync(0xffffffffu, item, 0);
-        const int li = A.g0 + item;
+        __syncthreads();
+        if (tid == 0) s.item = atomicAdd(A.work, 1);
+        if (tid < 16) s.keys[tid] = 0;
+        if (tid == 0) {
+            s.kmin = ne;
+            s.kmax = 0;
+            s.kfp = -1;
+        }
+        __syncthreads();
+        const int li = A.g0 + s.item;
         if (li >= A.g1) break;
-        const int g = A.gmap ? A.gmap[li] : li;
-        const int jb = job_of(A.jblk, A.njobs, g);
         {
+            const long long eoff = A.off[li - A.g0];
+            const int ecnt = (int)(A.off[li - A.g0 + 1] - eoff);
+            if (ecnt == 0) continue;
+            const int g = A.gmap ? A.gmap[li] : li;
+            const int jb = job_of(A.jblk, A.njobs, g);
             const unsigned long long *src = (const unsigned long long *)(A.jobs + jb);
-            unsigned long long *dst = (unsigned long long *)&ws->job;
-            for (int u = lane; u < (int)(sizeof(JobDesc) / 8); u += 32) dst[u] = src[u];
-            __syncwarp();
+            unsigned long long *dst = (unsigned long long *)&s.job;
+            for (int u = tid; u < (int)(sizeof(JobDesc) / 8); u += kTileThreads) dst[u] = src[u];
+            // the records' keys and edges
+            for (int i = tid; i < ecnt; i += kTileThreads) {
+                const uint4 r = __ldg(A.rec + eoff + i);
+                const unsigned key = ((r.z >> 8) & 0xFF) | (r.w << 8);
+                const int k0 = (r.z >> 16) & 0xFF, k1 = k0 + (int)(r.z >> 24);
+                atomicOr(&s.keys[key >> 5], 1u << (key & 31));
+                atomicMin(&s.kmin, k0);
+                atomicMax(&s.kmax, k1);
+                if (k1 > k0 && s.R[k1 - 1] < kFp32MaxR) atomicMax(&s.kfp, k1 - 1);
+            }
+            __syncthreads();
+            const JobDesc &J = s.job;
+            const int b = g - A.jblk[jb];
+            const int qlen = J.Q.blk_len[b], qs = J.Q.blk_start[b];
+            const double *bx = J.Q.blk_box + 6 * (size_t)b;
+            const double ox = 0.5 * (bx[0] + bx[3]), oy = 0.5 * (bx[1] + bx[4]), oz = 0.5 * (bx[2] + bx[5]);
+            const double hx = 0.5 * (bx[3] - bx[0]), hy = 0.5 * (bx[4] - bx[1]), hz = 0.5 * (bx[5] - bx[2]);
+            const float Rq = __double2float_ru(sqrt(hx * hx + hy * hy + hz * hz) * (1.0 + 1e-12));
+            const float hT = __double2float_ru(J.hT);
+            float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+            if (tid < qlen) {
+                lo[0] = hi[0] = (float)(J.Q.x[qs + tid] - ox);
+                lo[1] = hi[1] = (float)(J.Q.y[qs + tid] - oy);
+                lo[2] = hi[2] = (float)(J.Q.z[qs + tid] - oz);
+            }
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+#pragma unroll
+                for (int o = kMT / 2; o; o >>= 1) {
+                    lo[d] = fminf(lo[d], __shfl_xor_sync(FULL, lo[d], o));
+                    hi[d] = fmaxf(hi[d], __shfl_xor_sync(FULL, hi[d], o));
+                }
+                if ((tid & (kMT - 1)) == 0) {
+                    s.qc[tid / kMT][d] = 0.5f * (lo[d] + hi[d]);
+                    s.qh[tid / kMT][d] = 0.5f * (hi[d] - lo[d]);
+                }
+            }
+            // every coordinate and edge root of a record with pairs below edge
+            // kfp stays below Bm: scaled values below 240, squares below 65504
+            float S = 0.0f;
+            const float Bm = (s.kfp >= 0 ? sqrtf(s.Rup[s.kfp]) * 1.0001f : 0.0f) + 2.1f * hT + 4.0f * Rq;
+            if (Bm > 0.0f && Bm < (float)kFp32Span) {
+                int ex;
+                frexpf(Bm, &ex);  // Bm in [2^(ex-1), 2^ex)
+                S = ldexpf(1.0f, max(-60, min(60, 7 - ex)));
+            }
+            if (tid == 0) {
+                s.o[0] = ox;
+                s.o[1] = oy;
+                s.o[2] = oz;
+                s.eoff = eoff;
+                s.ecnt = ecnt;
+                // records a warp takes at a time: a few, where the block has few
+                s.chunk = ecnt >= 1024 ? 32 : (ecnt >= 512 ? 16 : (ecnt >= 128 ? 8 : 4));
+                s.qs = qs;
+                s.qlen = qlen;
+                s.Rq = Rq;
+                s.hT = hT;
+                s.S = S;
+            }
+            __syncthreads();
+            if (MODE == KD_MODE_MIXED && S > 0.0f) set_scale(s, ne, tid);
         }
-        const JobDesc &J = ws->job;
-        const int b = g - A.jblk[jb];
-        const int qlen = J.Q.blk_len[b], qs = J.Q.blk_start[b];
-        const long long eoff = A.off[li - A.g0];
-        const int ecnt = (int)(A.off[li - A.g0 + 1] - eoff);
-        const double *bx = J.Q.blk_box + 6 * (size_t)b;
-        const double ox = 0.5 * (bx[0] + bx[3]), oy = 0.5 * (bx[1] + bx[4]),
-                     oz = 0.5 * (bx[2] + bx[5]);
-        // queries 4*lane .. 4*lane+3 of the block; their FP64 coordinates and
-        // own fields are re-read from global memory when needed (exact
-        // recounts, flushes) instead of being held in registers
-        const int qbase = qs + kQ * lane;
-        float qx[kQ], qy[kQ], qz[kQ], qn[kQ];
-        unsigned vmask = 0;
-#pragma unroll
-        for (int p = 0; p < kQ; p++) {
-            const int j = kQ * lane + p;
-            const bool v = j < qlen;
-            vmask |= (unsigned)v << p;
-            const double xd = v ? J.Q.x[qs + j] : ox, yd = v ? J.Q.y[qs + j] : oy,
-                         zd = v ? J.Q.z[qs + j] : oz;
-            qx[p] = (float)(xd - ox);
-            qy[p] = (float)(yd - oy);
-            qz[p] = (float)(zd - oz);
-            qn[p] = (float)((double)qx[p] * qx[p] + (double)qy[p] * qy[p] + (double)qz[p] * qz[p]);
-        }
-        const int nvalid = __popc(vmask);
-        float2 qx2[kQ / 2], qy2[kQ / 2], qz2[kQ / 2];
-#pragma unroll
-        for (int h = 0; h < kQ / 2; h++) {
-            qx2[h] = make_float2(qx[2 * h], qx[2 * h + 1]);
-            qy2[h] = make_float2(qy[2 * h], qy[2 * h + 1]);
-            qz2[h] = make_float2(qz[2 * h], qz[2 * h + 1]);
-        }
-        // half-word masks of the valid queries of each pair (invalid add 0)
-        unsigned vm[kQ / 2];
-#pragma unroll
-        for (int h = 0; h < kQ / 2; h++)
-            vm[h] = (((vmask >> (2 * h)) & 1) ? 0xFFFFu : 0u) |
-                    (((vmask >> (2 * h + 1)) & 1) ? 0xFFFF0000u : 0u);
-        auto qfield = [&](int p) { return ((vmask >> p) & 1) ? J.Q.qf[qbase + p] : -1; };
-        // the distinct own fields of the block (up to kMaxDistinctQf are
-        // reduced per warp at a flush; beyond that, per-query atomics)
-        int nuq = 0;
-        {
-            unsigned todo = vmask;
-            for (int round = 0; round <= kQ * 32; round++) {
-                int cand = -1;
-#pragma unroll
-                for (int p = 0; p < kQ; p++)
-                    if (cand < 0 && ((todo >> p) & 1)) cand = qfield(p);
-                const unsigned any = __ballot_sync(0xffffffffu, cand >= 0);
-                if (!any) break;
-                const int pick = __shfl_sync(0xffffffffu, cand, __ffs(any) - 1);
-                if (nuq < kMaxDistinctQf && lane == 0) ws->uq[nuq] = pick;
-                nuq++;
-#pragma unroll
-                for (int p = 0; p < kQ; p++)
-                    if (((todo >> p) & 1) && qfield(p) == pick) todo &= ~(1u << p);
-            }
-        }
-        if (MODE == KD_MODE_MIXED) {
-            const double hx = 0.5 * (bx[3] - bx[0]), hy = 0.5 * (bx[4] - bx[1]),
-                         hz = 0.5 * (bx[5] - bx[2]);
-            const double Rq = sqrt(hx * hx + hy * hy + hz * hz) * (1.0 + 1e-12);
-            if (lane == 0) {
-                // |t' - o| <= |c - o| + hT and |q' - o| <= Rq must stay
-                // within kFp32Span (NaN box: never)
-                const double lim = kFp32Span - J.hT - Rq;
-                ws->cmax2 = lim > 0 ? lim * lim : -1.0;
-            }
-            for (int k = lane; k < ne; k += 32) {
-                if (isfinite(R[k])) {
-                    const double inv4e = 0.25 / band_halfwidth(R[k], Rq, J.hT);
-                    ws->nsl[k] = (float)(-inv4e);
-                    ws->Aw[k] = (float)(0.5 + R[k] * inv4e);
-                } else {
-                    ws->nsl[k] = 0.0f;
-                    ws->Aw[k] = 0.0f;
-                }
-            }
-        }
-        for (int e = 0; e <= ne; e++)
-#pragma unroll
-            for (int h = 0; h < kQ / 2; h++) P[(e * (kQ / 2) + h) * 32 + lane] = 0;
-        __syncwarp();
-        int cur_tf = -1;
-        int since = 0;
-        int tlo = ne, thi = -1;  // bins written since the last flush
-
-        // flush key: tree field | 256 for the once-counted part of a symmetric job
-        auto flush = [&](int key) {
-            const int tf = key & 0xFF;
-            unsigned long long *const Hd = (key >> 8) ? J.H2 : J.H;
-            int qf[kQ];
-#pragma unroll
-            for (int p = 0; p < kQ; p++) qf[p] = qfield(p);
-            const int ehi = min(thi, ne - 1);
-            for (int e = tlo; e <= ehi; e++) {
-                int v[kQ];
-#pragma unroll
-                for (int h = 0; h < kQ / 2; h++) {
-                    const unsigned wv = P[(e * (kQ / 2) + h) * 32 + lane];
-                    P[(e * (kQ / 2) + h) * 32 + lane] = 0;
-                    v[2 * h] = (int)(wv & 0xFFFFu);
-                    v[2 * h + 1] = (int)(wv >> 16);
-                }
-                if (nuq <= kMaxDistinctQf) {
-                    for (int u = 0; u < nuq; u++) {
-                        const int uf = ws->uq[u];
-                        int sum = 0;
-#pragma unroll
-                        for (int p = 0; p < kQ; p++) sum += qf[p] == uf ? v[p] : 0;
-                        for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-                        if (lane == 0 && sum)
-                            atomicAdd(&Hd[((size_t)e * J.Fqe + uf) * J.Fte + tf],
-                                      (unsigned long long)sum);
-                    }
-                } else {
-#pragma unroll
-                    for (int p = 0; p < kQ; p++)
-                        if (((vmask >> p) & 1) && v[p])
-                            atomicAdd(&Hd[((size_t)e * J.Fqe + qf[p]) * J.Fte + tf],
-                                      (unsigned long long)v[p]);
-                }
-            }
-            if (thi == ne) {
-#pragma unroll
-                for (int h = 0; h < kQ / 2; h++) P[(ne * (kQ / 2) + h) * 32 + lane] = 0;
-            }
-            tlo = ne;
-            thi = -1;
-        };
-
-        // the next record's loads, held in registers while the current run
-        // is counted
-        uint4 nrec = make_uint4(0, 0, 0, 0);
-        float4 npt[kRunPerLane];
-#pragma unroll
-        for (int h = 0; h < kRunPerLane; h++) npt[h] = make_float4(0, 0, 0, 0);
-        double ncx = 0, ncy = 0, ncz = 0;
-        auto issue = [&](int i) {
-            nrec = A.rec[eoff + i];
-            const int rl = nrec.z & 0xFF, K = nrec.z >> 24;
-            if (K == 0) return;
-            if (MODE == KD_MODE_MIXED) {
-                const unsigned rs = nrec.x, leaf = nrec.y;
-                ncx = J.leaf_c[3 * (size_t)leaf];
-                ncy = J.leaf_c[3 * (size_t)leaf + 1];
-                ncz = J.leaf_c[3 * (size_t)leaf + 2];
-#pragma unroll
-                for (int h = 0; h < kRunPerLane; h++)
-                    if (lane + 32 * h < rl) npt[h] = J.t4[rs + lane + 32 * h];
-            } else {
-                const unsigned rs = nrec.x;
-                if (lane < rl) {
-                    ncx = J.tx[rs + lane];
-                    ncy = J.ty[rs + lane];
-                    ncz = J.tz[rs + lane];
-                }
-            }
-        };
-
-        // stage the prefetched run (mixed mode); returns whether its leaf
-        // lies in FP32 range of the block centre
-        auto stage_run = [&](int rl_) {
-            const double ex = ncx - ox, ey = ncy - oy, ez = ncz - oz;
-            const bool in_range = ex * ex + ey * ey + ez * ez < ws->cmax2;
-            const float dx = (float)ex, dy = (float)ey, dz = (float)ez;
-#pragma unroll
-            for (int h = 0; h < kRunPerLane; h++) {
-                const int j = lane + 32 * h;
-                if (j < rl_) {
-                    // t' = t_r + (c - o); -0.5 * (-2 t_r) is exact
-                    const float lx = fmaf(-0.5f, npt[h].x, dx);
-                    const float ly = fmaf(-0.5f, npt[h].y, dy);
-                    const float lz = fmaf(-0.5f, npt[h].z, dz);
-                    const float X = -2.0f * lx, Y = -2.0f * ly, Z = -2.0f * lz;
-                    const float N = fmaf(lz, lz, fmaf(ly, ly, lx * lx));
-                    ws->stage[2 * j] = make_float4(X, X, Y, Y);
-                    ws->stage[2 * j + 1] = make_float4(Z, Z, N, N);
-                }
-            }
-            return in_range;
-        };
-
-        if (ecnt > 0) issue(0);
-        for (int i = 0; i < ecnt; i++) {
-            const uint4 rec = nrec;
-            const int rs = (int)rec.x, rl1 = rec.z & 0xFF, tf = (rec.z >> 8) & 0xFF;
-            const int k0 = (rec.z >> 16) & 0xFF, K = rec.z >> 24;
-            // commit the staged run
-            bool fp32_range = false;
-            if (K != 0) {
-                if (MODE == KD_MODE_MIXED) {
-                    fp32_range = stage_run(rl1);
-                } else {
-                    const int rl = rl1;
-                    if (lane < rl) {
-                        ws->stage64[lane] = ncx;
-                        ws->stage64[KD_RUN_MAX + lane] = ncy;
-                        ws->stage64[2 * KD_RUN_MAX + lane] = ncz;
-                    }
-                    for (int j = lane + 32; j < rl; j += 32) {
-                        ws->stage64[j] = J.tx[rs + j];
-                        ws->stage64[KD_RUN_MAX + j] = J.ty[rs + j];
-                        ws->stage64[2 * KD_RUN_MAX + j] = J.tz[rs + j];
-                    }
-                }
-            }
-            __syncwarp();
-            if (i + 1 < ecnt) issue(i + 1);
-            const int rl = rl1;
-
-            const int key = tf | (int)(rec.w << 8);
-            if (key != cur_tf || since + rl > 0xFFFF) {
-                if (cur_tf >= 0) flush(cur_tf);
-                cur_tf = key;
-                since = 0;
-            }
-            since += rl;
-            tlo = min(tlo, k0);
-            thi = max(thi, k0 + K);
-            if (K == 0) {
-#pragma unroll
-                for (int h = 0; h < kQ / 2; h++)
-                    P[(k0 * (kQ / 2) + h) * 32 + lane] += (((unsigned)rl | ((unsigned)rl << 16)) & vm[h]);
-                __syncwarp();
+        // ---- one flush key after the other (tree field | 256 for the
+        // once-counted part of a symmetric job)
+        for (int key = 0; key < 512; key++) {
+            const unsigned kw = s.keys[key >> 5] >> (key & 31);
+            if (!kw) {
+                key |= 31;
                 continue;
             }
-            wtiles++;
-            const bool fp32 = MODE == KD_MODE_MIXED && fp32_range && R[k0 + K - 1] < kFp32MaxR;
-            // packed cumulative count of the previous edge, per query pair
-            unsigned prev[kQ / 2];
-#pragma unroll
-            for (int h = 0; h < kQ / 2; h++) prev[h] = 0;
-            const int pw = MODE == KD_MODE_MIXED && fp32 ? kPass32 : 4;
-            for (int kb = 0; kb < K; kb += pw) {
-                const int kn = min(pw, K - kb);
-                unsigned pc[kQ / 2][4];
-#pragma unroll
-                for (int h = 0; h < kQ / 2; h++)
-#pragma unroll
-                    for (int k = 0; k < 4; k++) pc[h][k] = 0;
-                unsigned redo = vmask;
-                if (fp32) {
-                    float a[kQ][kPass32], sl[kPass32];
-#pragma unroll
-                    for (int k = 0; k < kPass32; k++) {
-                        sl[k] = k < kn ? ws->nsl[k0 + kb + k] : 0.0f;
-                        const float Ak = k < kn ? ws->Aw[k0 + kb + k] : 0.0f;
-#pragma unroll
-                        for (int p = 0; p < kQ; p++) a[p][k] = fmaf(qn[p], sl[k], Ak);
-                    }
-                    unsigned band;
-                    switch (kn) {
-                    case 1: band = fp32_run<1>(ws->stage, rl, qx2, qy2, qz2, a, sl, pc); break;
-                    case 2: band = fp32_run<2>(ws->stage, rl, qx2, qy2, qz2, a, sl, pc); break;
-                    case 3: band = fp32_run<3>(ws->stage, rl, qx2, qy2, qz2, a, sl, pc); break;
-                    default: band = fp32_run<4>(ws->stage, rl, qx2, qy2, qz2, a, sl, pc); break;
-                    }
-                    redo = band & vmask;
-                    rechecked += (unsigned long long)__popc(redo) * rl;
-                } else if (MODE == KD_MODE_FP64) {
-                    double qxd[kQ], qyd[kQ], qzd[kQ];
-#pragma unroll
-                    for (int p = 0; p < kQ; p++) {
-                        const bool v = (vmask >> p) & 1;
-                        qxd[p] = v ? J.Q.x[qbase + p] : ox;
-                        qyd[p] = v ? J.Q.y[qbase + p] : oy;
-                        qzd[p] = v ? J.Q.z[qbase + p] : oz;
-                    }
-                    const double *s64 = ws->stage64;
-                    int cnt[kQ][4];
-                    switch (kn) {
-                    case 1: fp64_run<1>(s64, s64 + KD_RUN_MAX, s64 + 2 * KD_RUN_MAX, rl, qxd, qyd, qzd, R + k0 + kb, cnt); break;
-                    case 2: fp64_run<2>(s64, s64 + KD_RUN_MAX, s64 + 2 * KD_RUN_MAX, rl, qxd, qyd, qzd, R + k0 + kb, cnt); break;
-                    case 3: fp64_run<3>(s64, s64 + KD_RUN_MAX, s64 + 2 * KD_RUN_MAX, rl, qxd, qyd, qzd, R + k0 + kb, cnt); break;
-                    default: fp64_run<4>(s64, s64 + KD_RUN_MAX, s64 + 2 * KD_RUN_MAX, rl, qxd, qyd, qzd, R + k0 + kb, cnt); break;
-                    }
-#pragma unroll
-                    for (int h = 0; h < kQ / 2; h++)
-#pragma unroll
-                        for (int k = 0; k < 4; k++)
-                            pc[h][k] = (unsigned)cnt[2 * h][k] | ((unsigned)cnt[2 * h + 1][k] << 16);
-                    redo = 0;
+            key += __ffs(kw) - 1;
+            __syncthreads();  // the last key's counters are clear
+            if (tid == 0) s.next = 0;
+            __syncthreads();
+            while (true) {
+                int c0 = 0;
+                if (lane == 0) c0 = atomicAdd(&s.next, s.chunk);
+                c0 = __shfl_sync(FULL, c0, 0);
+                if (c0 >= s.ecnt) break;
+                const uint4 *const crec = A.rec + s.eoff + c0;
+                unsigned mine;
+                {
+                    uint2 r = make_uint2(0, 0);
+                    const bool in = lane < s.chunk && c0 + lane < s.ecnt;
+                    if (in) r = __ldg(reinterpret_cast<const uint2 *>(crec + lane) + 1);
+                    mine = __ballot_sync(FULL, in && (((r.x >> 8) & 0xFF) | (r.y << 8)) == (unsigned)key);
                 }
-                // exact FP64 recount of the queries FP32 could not decide: a
-                // few of them (band pairs) by the whole warp, one after the
-                // other; many (edges FP32 cannot represent) lane by lane
-                const unsigned nre = __reduce_add_sync(0xffffffffu, (unsigned)__popc(redo));
-                if (nre <= kCoopMax) {
-                    for (unsigned it = 0; it < nre; it++) {
-                        const unsigned has = __ballot_sync(0xffffffffu, redo != 0);
-                        const int src = __ffs(has) - 1;
-                        const int pq = __shfl_sync(0xffffffffu, __ffs(redo) - 1, src);
-                        const int qi = qs + kQ * src + pq;
-                        const unsigned pk =
-                            exact_pass_warp(J.tx + rs, J.ty + rs, J.tz + rs, rl, J.Q.x[qi],
-                                            J.Q.y[qi], J.Q.z[qi], R + k0 + kb, kn, lane);
-                        if (lane == src) {
-                            // replace query pq's half-word (selects, no indexing)
+                while (mine) {
+                    // ---- the next four records: lane (wm, wr) has record wr
+                    const unsigned m1 = mine & (mine - 1), m2 = m1 & (m1 - 1), m3 = m2 & (m2 - 1);
+                    const unsigned sel = wr == 0 ? mine : (wr == 1 ? m1 : (wr == 2 ? m2 : m3));
+                    const bool have = sel != 0;
+                    const int nr = min(kGroup, __popc(mine));
+                    mine = m3 & (m3 - 1);
+                    const int from = have ? __ffs(sel) - 1 : 0;
+                    const uint4 rec = __ldg(crec + from);
+                    const int r_rs = (int)rec.x;
+                    const unsigned r_z = have ? rec.z : 0u;
+                    const int rl = r_z & 0xFF, rk0 = (r_z >> 16) & 0xFF, rK = r_z >> 24;
+                    // ---- windows: edges [k0, k1) may separate pairs of query
+                    // tile wm and the record; every pair lies below the edges
+                    // from k1 on
+                    int k0 = rk0, k1 = rk0 + rK;
+                    bool ok = have && rK != 0;
+                    float dx, dy, dz;
+                    {
+                        const double2 *geo = reinterpret_cast<const double2 *>(s.job.leaf + rec.y);
+                        const double2 ga = __ldg(geo), gb = __ldg(geo + 1);
+                        const float hx = __int_as_float(__double2loint(gb.y)),
+                                    hy = __int_as_float(__double2hiint(gb.y)),
+                                    hz = __ldg(reinterpret_cast<const float *>(geo + 2));
+                        dx = (float)(ga.x - s.o[0]);
+                        dy = (float)(ga.y - s.o[1]);
+                        dz = (float)(gb.x - s.o[2]);
+                        // B >= |t'| of every point of the leaf and sqrt of
+                        // every edge of the record
+                        const float B = sqrtf(dx * dx + dy * dy + dz * dz) * 1.0001f + s.hT + 2.0f * s.Rq;
+                        ok = ok && B < (float)kFp32Span && s.R[k1 - 1] < kFp32MaxR &&
+                             (MODE == KD_MODE_FP64 || (s.S > 0.0f && B * s.S <= 240.0f));
+                        if (ok) {
+                            // rounding of the staged coordinates and of the tile box
+                            const float mg = 4.8e-7f * (fabsf(dx) + fabsf(dy) + fabsf(dz) + hx + hy + hz +
+                                                        2.0f * (s.Rq + s.hT));
+                            const float ax = fabsf(dx - s.qc[wm][0]), ay = fabsf(dy - s.qc[wm][1]),
+                                        az = fabsf(dz - s.qc[wm][2]);
+                            const float ex = hx + s.qh[wm][0] + mg, ey = hy + s.qh[wm][1] + mg,
+                                        ez = hz + s.qh[wm][2] + mg;
+                            const float gx = fmaxf(ax - ex, 0.0f), gy = fmaxf(ay - ey, 0.0f),
+                                        gz = fmaxf(az - ez, 0.0f);
+                            const float sx = ax + ex, sy = ay + ey, sz = az + ez;
+                            const float lo2 = (gx * gx + gy * gy + gz * gz) * (1.0f - 4e-6f);
+                            const float hi2 = (sx * sx + sy * sy + sz * sz) * (1.0f + 4e-6f);
+                            int below = 0, upto = 0;  // edges below / not above the pairs
+                            for (int k = rk0; k < rk0 + rK; k++) {
+                                below += s.Rup[k] <= lo2;
+                                upto += s.Rdn[k] <= hi2;
+                            }
+                            k0 = rk0 + below;
+                            k1 = rk0 + max(below, upto);
+                        }
+                    }
+                    const int mval = max(0, min(kMT, s.qlen - kMT * wm));  // queries of tile wm
+                    if constexpr (MODE == KD_MODE_FP64) {  // one window for two query tiles
+                        const int p0 = __shfl_xor_sync(FULL, k0, 1), p1 = __shfl_xor_sync(FULL, k1, 1);
+                        const bool pv = __shfl_xor_sync(FULL, mval, 1) != 0;
+                        if (pv && (k1 > k0 || p1 > p0)) {
+                            k0 = min(k0, p0);
+                            k1 = max(k1, p1);
+                        }
+                    }
+                    const int K = have && mval ? k1 - k0 : 0;
+                    const unsigned win = (unsigned)k0 | ((unsigned)K << 8);
+                    const unsigned actm = __ballot_sync(FULL, K != 0), okm = __ballot_sync(FULL, ok);
+                    if (have && mval) atomicAdd(&s.F[k1 * kMTiles + wm], (unsigned)rl);
+                    {
+                        const unsigned q = K ? (unsigned)(mval * rl) : 0u;
+                        const unsigned np = __reduce_add_sync(FULL, q), nk = __reduce_add_sync(FULL, q * (unsigned)K),
+                                       nw = __reduce_add_sync(FULL, K > 4 ? q : 0u);
+                        if (lane < 4) {
+                            const unsigned v = lane == 0 ? np : (lane == 1 ? nw : (lane == 2 ? nk : __popc(actm)));
+                            atomicAdd(&s.stats[lane == 0 ? 0 : lane + 1], (unsigned long long)v);
+                        }
+                    }
+                    // ---- record by record
+                    float4 npt[2];
+                    double px[2], py[2], pz[2];
+                    auto load_points = [&](int r) {
+                        const int rs = __shfl_sync(FULL, r_rs, r * kMTiles);
+                        const int n = __shfl_sync(FULL, rl, r * kMTiles);
 #pragma unroll
-                            for (int h = 0; h < kQ / 2; h++) {
-                                const bool lo = pq == 2 * h, hi = pq == 2 * h + 1;
-#pragma unroll
-                                for (int k = 0; k < 4; k++) {
-                                    const unsigned v = (pk >> (8 * k)) & 0xFFu;
-                                    pc[h][k] = lo ? ((pc[h][k] & 0xFFFF0000u) | v)
-                                                  : hi ? ((pc[h][k] & 0xFFFFu) | (v << 16)) : pc[h][k];
+                        for (int h = 0; h < 2; h++)
+                            if (lane + 32 * h < n) {
+                                const int j = rs + lane + 32 * h;
+                                if constexpr (MODE == KD_MODE_MIXED) {
+                                    npt[h] = __ldg(s.job.t4 + j);
+                                } else {
+                                    px[h] = __ldg(s.job.tx + j);
+                                    py[h] = __ldg(s.job.ty + j);
+                                    pz[h] = __ldg(s.job.tz + j);
                                 }
                             }
-                            redo &= ~(1u << pq);
+                    };
+                    load_points(0);
+                    for (int r = 0; r < nr; r++) {
+                        const int src = r * kMTiles;
+                        const int n = __shfl_sync(FULL, rl, src), rs = __shfl_sync(FULL, r_rs, src);
+                        unsigned act = (actm >> src) & 0xFFu;
+                        if constexpr (MODE == KD_MODE_MIXED) {
+                            const bool fast = (okm >> src) & 1;
+                            const float ref = s.edge[(__shfl_sync(FULL, r_z, src) >> 16) & 0xFF].x, S = s.S;
+                            const float Dx = __shfl_sync(FULL, dx, src), Dy = __shfl_sync(FULL, dy, src),
+                                        Dz = __shfl_sync(FULL, dz, src);
+                            // ---- stage the run: lane (g, t) of step j reads
+                            // word t of point 8 j + g
+                            if (act && fast) {
+#pragma unroll
+                                for (int h = 0; h < 2; h++) {
+                                    const int j = lane + 32 * h;
+                                    if (j < ((n + kNT - 1) & ~(kNT - 1))) {
+                                        // t' = t_r + (c - o); -0.5 * (-2 t_r) is exact
+                                        const float x = fmaf(-0.5f, npt[h].x, Dx) * S,
+                                                    y = fmaf(-0.5f, npt[h].y, Dy) * S,
+                                                    zz = fmaf(-0.5f, npt[h].z, Dz) * S;
+                                        const float N = fmaf(zz, zz, fmaf(y, y, fmaf(x, x, -ref)));
+                                        uint4 v = make_uint4(split_halves(x), split_halves(y),
+                                                             split_halves(zz), split_halves(N));
+                                        // columns without a point lie above every edge
+                                        if (j >= n) v = make_uint4(0u, 0u, 0u, 0x7BFF7BFFu);
+                                        *reinterpret_cast<uint4 *>(s.bs[w] + 4 * j) = v;
+                                    }
+                                }
+                            }
+                            if (r + 1 < nr) load_points(r + 1);
+                            __syncwarp();
+                            const int nt = (n + kNT - 1) / kNT;
+                            const uint32_t *const bs = s.bs[w] + lane;
+                            while (act) {
+                                int mt[2];
+                                mt[0] = __ffs(act) - 1;
+                                act &= act - 1;
+                                mt[1] = act ? __ffs(act) - 1 : mt[0];
+                                const unsigned wv = __shfl_sync(FULL, win, src + mt[0]),
+                                               wv2 = __shfl_sync(FULL, win, src + mt[1]);
+                                int kk = wv & 0xFF, left = wv >> 8;
+                                if (fast) {
+                                    // two tiles with one window go together
+                                    if (left == 1 && act && wv2 == wv) {
+                                        act &= act - 1;
+                                        tile_pass<1, 2>(s, P, mt, kk, nt, ref, rs, n, lane, bs);
+                                        continue;
+                                    }
+                                    for (; left > 4; left -= 4, kk += 4)
+                                        tile_pass<4, 1>(s, P, mt, kk, nt, ref, rs, n, lane, bs);
+                                    switch (left) {
+                                    case 1: tile_pass<1, 1>(s, P, mt, kk, nt, ref, rs, n, lane, bs); break;
+                                    case 2: tile_pass<2, 1>(s, P, mt, kk, nt, ref, rs, n, lane, bs); break;
+                                    case 3: tile_pass<3, 1>(s, P, mt, kk, nt, ref, rs, n, lane, bs); break;
+                                    default: tile_pass<4, 1>(s, P, mt, kk, nt, ref, rs, n, lane, bs); break;
+                                    }
+                                } else {  // out of FP32 range: every row exactly
+                                    for (; left > 0; left -= 4, kk += 4)
+                                        recount_rows(s, P, 0xFFFFu, mt[0], rs, n, kk, min(4, left), 0u, lane);
+                                }
+                            }
+                        } else {
+                            if (act) {
+#pragma unroll
+                                for (int h = 0; h < 2; h++) {
+                                    const int j = lane + 32 * h;
+                                    if (j < ((n + 1) & ~1)) {
+                                        s.pt[w][0][j] = j < n ? px[h] : 1e300;
+                                        s.pt[w][1][j] = j < n ? py[h] : 1e300;
+                                        s.pt[w][2][j] = j < n ? pz[h] : 1e300;
+                                    }
+                                }
+                            }
+                            if (r + 1 < nr) load_points(r + 1);
+                            __syncwarp();
+                            const double2 *X = reinterpret_cast<const double2 *>(s.pt[w][0]),
+                                          *Y = reinterpret_cast<const double2 *>(s.pt[w][1]),
+                                          *Z = reinterpret_cast<const double2 *>(s.pt[w][2]);
+                            for (int p = 0; p < kMTiles / 2; p++) {
+                                // (a tile without queries has no window: take the other's)
+                                const unsigned two = (act >> (2 * p)) & 3u;
+                                if (!two) continue;
+                                const unsigned wv = __shfl_sync(FULL, win, src + 2 * p + (two == 2u));
+                                const int q = 32 * p + lane;
+                                const bool v = q < s.qlen;
+                                const double qx = v ? s.job.Q.x[s.qs + q] : s.o[0],
+                                             qy = v ? s.job.Q.y[s.qs + q] : s.o[1],
+                                             qz = v ? s.job.Q.z[s.qs + q] : s.o[2];
+                                for (int kk = wv & 0xFF, left = wv >> 8; left > 0; left -= 4, kk += 4) {
+                                    unsigned cnt[4] = {0u, 0u, 0u, 0u};
+                                    switch (min(left, 4)) {
+                                    case 1: fp64_run<1>(X, Y, Z, (n + 1) / 2, qx, qy, qz, s.R + kk, cnt); break;
+                                    case 2: fp64_run<2>(X, Y, Z, (n + 1) / 2, qx, qy, qz, s.R + kk, cnt); break;
+                                    case 3: fp64_run<3>(X, Y, Z, (n + 1) / 2, qx, qy, qz, s.R + kk, cnt); break;
+                                    default: fp64_run<4>(X, Y, Z, (n + 1) / 2, qx, qy, qz, s.R + kk, cnt); break;
+                                    }
+#pragma unroll
+                                    for (int k = 0; k < 4; k++)
+                                        if (k < left) atomicAdd(&P[(kk + k) * kPStride + q], cnt[k]);
+                                }
+                            }
                         }
+                        __syncwarp();
                     }
                 }
-#pragma unroll
-                for (int p = 0; p < kQ; p++)
-                    if ((redo >> p) & 1) {
-                        const unsigned pk =
-                            exact_pass(J.tx + rs, J.ty + rs, J.tz + rs, rl, J.Q.x[qbase + p],
-                                       J.Q.y[qbase + p], J.Q.z[qbase + p], R + k0 + kb, kn);
-                        const int sh = 16 * (p & 1);
-#pragma unroll
-                        for (int k = 0; k < 4; k++)
-                            pc[p >> 1][k] = (pc[p >> 1][k] & ~(0xFFFFu << sh)) |
-                                            (((pk >> (8 * k)) & 0xFFu) << sh);
-                    }
-                // bin increments: packed cumulative counts minus the previous
-                // edge's (no borrow between the halves: counts grow with k)
-#pragma unroll
-                for (int h = 0; h < kQ / 2; h++)
-#pragma unroll
-                    for (int k = 0; k < 4; k++)
-                        if (k < kn) {
-                            P[((k0 + kb + k) * (kQ / 2) + h) * 32 + lane] += (pc[h][k] - prev[h]) & vm[h];
-                            prev[h] = pc[h][k];
-                        }
             }
-            const unsigned rl2 = (unsigned)rl | ((unsigned)rl << 16);
-#pragma unroll
-            for (int h = 0; h < kQ / 2; h++)
-                P[((k0 + K) * (kQ / 2) + h) * 32 + lane] += (rl2 - prev[h]) & vm[h];
-            const unsigned long long tp = (unsigned long long)nvalid * rl;
-            pairs += tp;
-            kpairs += tp * K;
-            if (K > 4) wide += tp;
-            __syncwarp();
+            __syncthreads();
+            // ---- the key's counters to the global histogram: thread = query
+            {
+                const JobDesc &J = s.job;
+                unsigned long long *const Hd = (key >> 8) ? J.H2 : J.H;
+                const int tf = key & 0xFF, kmin = s.kmin, kmax = s.kmax;
+                const int qf = tid < s.qlen ? J.Q.qf[s.qs + tid] : -1;
+                unsigned run = 0, before = 0;
+                const unsigned vm = __ballot_sync(FULL, qf >= 0);
+                for (int e = kmin; e < min(kmax + 1, ne); e++) {
+                    run += s.F[e * kMTiles + tid / kMT];
+                    const unsigned cum = run + P[e * kPStride + tid];
+                    P[e * kPStride + tid] = 0;
+                    const unsigned v = cum - before;
+                    before = cum;
+                    unsigned rem = vm;
+                    while (rem) {  // one round per distinct own field of the warp
+                        const int from = __ffs(rem) - 1;
+                        const int f = __shfl_sync(FULL, qf, from);
+                        const bool same = qf == f;
+                        const unsigned sum = __reduce_add_sync(FULL, same ? v : 0u);
+                        if (lane == from && sum)
+                            atomicAdd(&Hd[((size_t)e * J.Fqe + f) * J.Fte + tf], (unsigned long long)sum);
+                        rem &= ~__ballot_sync(FULL, same);
+                    }
+                }
+                __syncthreads();
+                for (int i = kmin * kMTiles + tid; i < (kmax + 1) * kMTiles; i += kTileThreads) s.F[i] = 0;
+            }
         }
-        if (cur_tf >= 0) flush(cur_tf);
-        __syncwarp();
     }
-    for (int o = 16; o; o >>= 1) {
-        pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
-        rechecked += __shfl_xor_sync(0xffffffffu, rechecked, o);
-        wide += __shfl_xor_sync(0xffffffffu, wide, o);
-        kpairs += __shfl_xor_sync(0xffffffffu, kpairs, o);
-    }
-    if (lane == 0) {
-        if (pairs) atomicAdd(&A.stats[0], pairs);
-        if (rechecked) atomicAdd(&A.stats[1], rechecked);
-        if (wide) atomicAdd(&A.stats[3], wide);
-        if (kpairs) atomicAdd(&A.stats[4], kpairs);
-        if (wtiles) atomicAdd(&A.stats[5], wtiles);
+    // (the loop ends behind a barrier)
+    if (tid == 0) {
+        if (s.stats[0]) atomicAdd(&A.stats[0], s.stats[0]);
+        if (s.stats[1]) atomicAdd(&A.stats[1], s.stats[1]);
+        if (s.stats[2]) atomicAdd(&A.stats[3], s.stats[2]);
+        if (s.stats[3]) atomicAdd(&A.stats[4], s.stats[3]);
+        if (s.stats[4]) atomicAdd(&A.stats[5], s.stats[4]);
     }
 }
 
 static size_t tile_smem(int ne, int mode)
 {
-    const size_t ws = mode == KD_MODE_MIXED ? sizeof(WarpSmem<KD_MODE_MIXED>)
-                                            : sizeof(WarpSmem<KD_MODE_FP64>);
-    return sizeof(double) * KD_MAX_EDGES + ws * kTileWarpsPerCta +
-           sizeof(unsigned) * (size_t)(ne + 1) * (kQ / 2) * 32 * kTileWarpsPerCta;
+    const size_t fixed = mode == KD_MODE_MIXED ? sizeof(TileSmem<KD_MODE_MIXED>)
+                                               : sizeof(TileSmem<KD_MODE_FP64>);
+    return fixed + sizeof(unsigned) * (size_t)ne * kPStride;
 }
 
 struct Events {
@@ -983,7 +1123,7 @@ static JobDesc job_desc(const kd_catalog *tc, const kd_catalog *qc, unsigned lon
     d.ty = tc->d_y;
     d.tz = tc->d_z;
     d.t4 = (const float4 *)tc->d_t4;
-    d.leaf_c = tc->d_leaf_c;
+    d.leaf = tc->d_leaf;
     d.hT = tc->leaf_hdiag * (1.0 + 1e-12);
     d.H = H;
     d.H2 = nullptr;
@@ -1144,7 +1284,7 @@ static void count_batch_impl(const kd_catalog *const *tcs, const kd_catalog *con
           "smem attribute");
     int nsm = 148, occ = 1;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
-    check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32 * kTileWarpsPerCta, smem),
+    check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kTileThreads, smem),
           "occupancy");
     occ = std::max(occ, 1);
 
@@ -1185,9 +1325,8 @@ static void count_batch_impl(const kd_catalog *const *tcs, const kd_catalog *con
         ta.work = work;
         ta.stats = dstats;
         check(cudaMemsetAsync(work, 0, sizeof(int), s), "memset");
-        const int grid = (int)std::min<long long>(
-            ((long long)(b1 - b0) + kTileWarpsPerCta - 1) / kTileWarpsPerCta, (long long)nsm * occ);
-        kern<<<grid, 32 * kTileWarpsPerCta, smem, s>>>(ta);
+        const int grid = (int)std::min<long long>(b1 - b0, (long long)nsm * occ);
+        kern<<<grid, kTileThreads, smem, s>>>(ta);
         launches++;
         tile_launches++;
         KD_LAUNCH_CHECK("k_tiles");
@@ -1400,7 +1539,7 @@ static void count_static_impl(const kd_catalog *tc, int Ft, const kd_catalog *qc
           "smem attribute");
     int nsm = 148, occ = 1;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, tc->device);
-    check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, 32 * kTileWarpsPerCta, smem),
+    check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kTileThreads, smem),
           "occupancy");
     occ = std::max(occ, 1);
     int b0 = 0;
@@ -1432,9 +1571,8 @@ static void count_static_impl(const kd_catalog *tc, int Ft, const kd_catalog *qc
         ta.work = err + 1;
         ta.stats = misc;
         check(cudaMemsetAsync(err + 1, 0, sizeof(int), s), "memset");
-        const int grid = (int)std::min<long long>(
-            ((long long)(b1 - b0) + kTileWarpsPerCta - 1) / kTileWarpsPerCta, (long long)nsm * occ);
-        kern<<<grid, 32 * kTileWarpsPerCta, smem, s>>>(ta);
+        const int grid = (int)std::min<long long>(b1 - b0, (long long)nsm * occ);
+        kern<<<grid, kTileThreads, smem, s>>>(ta);
         KD_LAUNCH_CHECK("k_tiles");
         b0 = b1;
     }

@@ -32,13 +32,19 @@ extern "C" {
 #endif
 
 #define KD_RUN_MAX 64      /* points per tree-side run (shared-memory tile) */
-#define KD_BLOCK_MAX 128   /* query points per block (one warp, 4 per lane) */
-#define KD_QPL 4           /* query points per lane */
+#define KD_BLOCK_MAX 128   /* query points per block (one warp) */
 #define KD_LEAF_TARGET 64  /* unique points per counting leaf, upper bound */
 #define KD_MAX_EDGES 64    /* distinct finite squared edges per count job */
 
 /* the status codes (KD_OK, KD_EINVAL, ...) and KD_MAX_POINTS are public:
  * include/kdtree.h; the device error words use the same codes */
+
+/* box of a counting leaf; the half-extents cover its points, rounded up */
+typedef struct kd_leaf {
+    double c[3];
+    float h[3];
+    float pad_[3];
+} kd_leaf;
 
 typedef struct kd_catalog {
     int device;
@@ -75,9 +81,9 @@ typedef struct kd_catalog {
     int *d_run_start, *d_run_len, *d_run_tf, *d_run_leaf;
 
     /* tree side in FP32: t = fl32(point - leaf box centre), stored as
-     * float4 (-2 t.x, -2 t.y, -2 t.z, fl32(|t|^2)) */
+     * float4 (-2 t.x, -2 t.y, -2 t.z, 0) */
     void *d_t4;
-    double *d_leaf_c;  /* 3 per leaf: box centre */
+    kd_leaf *d_leaf;
     double leaf_hdiag; /* largest leaf box half-diagonal */
 
     int nblocks;

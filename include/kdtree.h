@@ -112,13 +112,14 @@ void destroy(kdtree_t tree);
 #define KD_MAX_POINTS 1073741823
 
 typedef struct kd_count_stats {
-    long long pairs_tested;    /* distances evaluated in tiles */
+    long long pairs_tested;    /* distances evaluated in tiles and binned: (16 queries, tree
+                                * run) tiles that some edge may separate */
     long long pairs_rechecked; /* pairs recomputed in FP64 after an FP32 band hit */
     long long pairs_accepted;  /* pairs binned by whole node pairs, no distance */
     long long pairs_wide;      /* pairs of tiles spanning more than 4 edges */
     long long edge_pairs;      /* sum over tested pairs of the edges each was binned against */
-    long long warp_tiles;      /* (query block, tree run) tiles with distances computed */
-    long long entries;         /* (query block, tree run) tiles listed */
+    long long warp_tiles;      /* (16 queries, tree run) tiles with distances binned */
+    long long entries;         /* (query block, tree run) records listed */
     double ms_traverse;        /* device time: node-pair traversal */
     double ms_tiles;           /* device time: tile kernels */
     double ms_total;           /* device time: whole count */
