@@ -392,16 +392,14 @@ __device__ __forceinline__ double gam(double m)
     return m * u / (1.0 - m * u);
 }
 
-// Decide the split dimension of a big segment from rigorous intervals around
-// the reference's rounded variances, or mark it for the sequential fallback.
-__global__ void k_var_decide(Segs sg, int ub, LevelBufs lb)
+// The split dimension of a segment of n points from rigorous intervals around
+// the reference's rounded variances, or -1 when they overlap.  a: sums of v,
+// |v| and (v - mean)^2 per dimension, in any order of summation.
+__device__ __forceinline__ int decide_dim(double n, const double *a)
 {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= ub || s >= *sg.count || !lb.big[s]) return;
     const double u = 1.1102230246251565e-16;
-    double n = (double)(sg.r[s] - sg.l[s] + 1);
-    const double *a = lb.acc + 9 * (size_t)s;
     double lo[3], hi[3];
+#pragma unroll
     for (int j = 0; j < 3; j++) {
         double A = a[3 + j] * (1.0 + gam(n));
         double dmu = (gam(n - 1) * (1.0 + u) + u) * A / n * (1.0 + 4 * u);
@@ -417,9 +415,20 @@ __global__ void k_var_decide(Segs sg, int ub, LevelBufs lb)
     if (a[7] > a[6 + c]) c = 1;
     if (a[8] > a[6 + c]) c = 2;
     bool ok = true;
+#pragma unroll
     for (int j = 0; j < 3; j++)
         if (j != c && !(lo[c] > hi[j])) ok = false;
-    if (ok) lb.tdim[s] = c;
+    return ok ? c : -1;
+}
+
+// Decide the split dimension of a big segment, or mark it for the sequential
+// fallback.
+__global__ void k_var_decide(Segs sg, int ub, LevelBufs lb)
+{
+    int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= ub || s >= *sg.count || !lb.big[s]) return;
+    const int c = decide_dim((double)(sg.r[s] - sg.l[s] + 1), lb.acc + 9 * (size_t)s);
+    if (c >= 0) lb.tdim[s] = c;
     else lb.fallback[s] = 1;
 }
 
@@ -921,6 +930,247 @@ __global__ void k_inorder_rep(int n_u, const int *__restrict__ inorder_u,
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_u; i += gridDim.x * blockDim.x)
         out[i] = urep[inorder_u[i]];
+}
+
+// ------------------------------------------------------------ subtrees
+
+// Whole subtrees of up to kSubCap points, one CTA each, from the level where
+// every segment fits: the level loop's steps (split dimension, node, stable
+// partition of the three orders) in shared memory, all subtrees of one depth
+// together, with the points as 16-bit places in the segment's order 0.  Every
+// point is read once and every node written once, where the level loop reads
+// and writes ~180 bytes per point and level in twelve launches: the last ten
+// levels of a 5M-point build took 3.7 ms there and take 1.8 ms here, all levels
+// of a 4000-point build 0.93 and 0.39 ms.  What bounds it is the latency of its
+// shared-memory gathers and the barriers between its steps (a third of the
+// issue slots are used, with four blocks per SM).  1024 points: a larger cap
+// would halve the blocks per SM, a smaller one would leave levels to the loop.
+constexpr int kSubCap = 1024;
+constexpr int kSubThreads = 256;
+constexpr int kSubSeq = 48;  // segments up to this size: one thread, sequentially
+
+struct SubSmem {
+    double v[3][kSubCap];               // coordinates by place
+    int gid[kSubCap];                   // unique-point ids by place
+    unsigned short o[2][3][kSubCap];    // the three orders: places by position
+    short seg[2][kSubCap];              // position -> segment of the level, -1: none
+    short l[2][kSubCap / 2 + 1], r[2][kSubCap / 2 + 1];  // segments: positions [l, r]
+    unsigned mask[3][2][kSubCap / 32];  // positions going left / right, a bit each
+    unsigned short pre[3][2][kSubCap / 32];
+    unsigned char side[kSubCap];        // by place: 0 left, 1 right, 2 median
+    unsigned char tdim[kSubCap / 2 + 1];
+};
+
+// max_variance_dim exactly as the reference evaluates it (kdbuild.c:308-351)
+__device__ __forceinline__ int sub_var_seq(const SubSmem &s, const unsigned short (&o)[3][kSubCap], int l,
+                                           int r)
+{
+    double m[3] = {0.0, 0.0, 0.0}, q[3] = {0.0, 0.0, 0.0};
+    for (int i = l; i <= r; i++)
+#pragma unroll
+        for (int d = 0; d < 3; d++) m[d] = __dadd_rn(m[d], s.v[d][o[d][i]]);
+    const double nn = (double)(r - l + 1);
+#pragma unroll
+    for (int d = 0; d < 3; d++) m[d] = __ddiv_rn(m[d], nn);
+    for (int i = l; i <= r; i++)
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            const double e = __dsub_rn(s.v[d][o[d][i]], m[d]);
+            q[d] = __fma_rn(e, e, q[d]);
+        }
+    int dim = 0;
+    double mx = q[0];
+    if (q[1] > mx) {
+        mx = q[1];
+        dim = 1;
+    }
+    if (q[2] > mx) dim = 2;
+    return dim;
+}
+
+__global__ void __launch_bounds__(kSubThreads) k_subtrees(Segs sg, const int *__restrict__ a0,
+                                                         const int *__restrict__ a1,
+                                                         const int *__restrict__ a2, UniqueArrays u,
+                                                         TreeOut t, int *place, int *err)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    SubSmem &s = *reinterpret_cast<SubSmem *>(smem);
+    constexpr unsigned FULL = 0xffffffffu;
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, b = blockIdx.x;
+    if (b >= *sg.count) return;
+    const int base = sg.l[b], m = sg.r[b] - base + 1;
+    const long long root = sg.p[b];
+    if (m < 1) return;
+    if (m > kSubCap) {
+        if (tid == 0) set_err(err, KD_EINTERNAL);
+        return;
+    }
+    // places: positions in order 0; the other orders through the point's place
+    for (int i = tid; i < m; i += kSubThreads) {
+        const int pt = a0[base + i];
+        s.gid[i] = pt;
+        s.o[0][0][i] = (unsigned short)i;
+        place[pt] = i;
+        s.v[0][i] = u.ux[pt];
+        s.v[1][i] = u.uy[pt];
+        s.v[2][i] = u.uz[pt];
+        s.seg[0][i] = 0;
+    }
+    if (tid == 0) {
+        s.l[0][0] = 0;
+        s.r[0][0] = (short)(m - 1);
+    }
+    __syncthreads();  // (place[] of this segment's points is written by this CTA alone)
+    for (int i = tid; i < m; i += kSubThreads) {
+        const int p1 = place[a1[base + i]], p2 = place[a2[base + i]];
+        if ((unsigned)p1 >= (unsigned)m || (unsigned)p2 >= (unsigned)m) set_err(err, KD_EINTERNAL);
+        s.o[0][1][i] = (unsigned short)min(max(p1, 0), m - 1);
+        s.o[0][2][i] = (unsigned short)min(max(p2, 0), m - 1);
+    }
+    __syncthreads();
+    const int words = (m + 31) / 32;
+    int cur = 0;
+    for (int lev = 0;; lev++) {
+        const int nseg = 1 << lev;
+        const short *const L = s.l[cur], *const R = s.r[cur];
+        auto &o = s.o[cur];
+        auto &o2 = s.o[cur ^ 1];
+        // ---- split dimensions: a warp per large segment, a thread per small one
+        if ((m >> lev) > kSubSeq) {
+            for (int g = w; g < nseg; g += kSubThreads / 32) {
+                const int l = L[g], r = R[g], n = r - l + 1;
+                if (n <= kSubSeq) continue;
+                double a[9];
+#pragma unroll
+                for (int k = 0; k < 9; k++) a[k] = 0.0;
+                for (int i = l + lane; i <= r; i += 32)
+#pragma unroll
+                    for (int d = 0; d < 3; d++) {
+                        const double v = s.v[d][o[0][i]];  // (the sums' order is free)
+                        a[d] += v;
+                        a[3 + d] += fabs(v);
+                    }
+#pragma unroll
+                for (int k = 0; k < 6; k++)
+#pragma unroll
+                    for (int f = 16; f; f >>= 1) a[k] += __shfl_xor_sync(FULL, a[k], f);
+                const double mu[3] = {a[0] / (double)n, a[1] / (double)n, a[2] / (double)n};
+                for (int i = l + lane; i <= r; i += 32)
+#pragma unroll
+                    for (int d = 0; d < 3; d++) {
+                        const double e = s.v[d][o[0][i]] - mu[d];
+                        a[6 + d] += e * e;
+                    }
+#pragma unroll
+                for (int k = 6; k < 9; k++)
+#pragma unroll
+                    for (int f = 16; f; f >>= 1) a[k] += __shfl_xor_sync(FULL, a[k], f);
+                int c = decide_dim((double)n, a);
+                if (c < 0 && lane == 0) c = sub_var_seq(s, o, l, r);
+                if (lane == 0) s.tdim[g] = (unsigned char)c;
+            }
+        }
+        for (int g = tid; g < nseg; g += kSubThreads) {
+            const int l = L[g], r = R[g], n = r - l + 1;
+            if (n >= 4 && n <= kSubSeq) s.tdim[g] = (unsigned char)sub_var_seq(s, o, l, r);
+        }
+        __syncthreads();
+        // ---- the level's nodes (k_level_nodes)
+        for (int g = tid; g < nseg; g += kSubThreads) {
+            const int l = L[g], r = R[g], n = r - l + 1;
+            const int p = (int)((root << lev) + g);
+            if (n >= 4) {
+                const int med = (l + r + 1) / 2, d = s.tdim[g];
+                put_node(t, u, p, s.gid[o[d][med]], d, 1, 1, base + med, err);
+            } else if (n == 3) {
+                put_node(t, u, p, s.gid[o[0][l + 1]], 0, 1, 1, base + l + 1, err);
+                put_node(t, u, 2 * p, s.gid[o[0][l]], 0, 0, 0, base + l, err);
+                put_node(t, u, 2 * p + 1, s.gid[o[0][r]], 0, 0, 0, base + r, err);
+            } else if (n == 2) {
+                put_node(t, u, p, s.gid[o[0][r]], 0, 1, 0, base + r, err);
+                put_node(t, u, 2 * p, s.gid[o[0][l]], 0, 0, 0, base + l, err);
+            } else if (n == 1) {
+                put_node(t, u, p, s.gid[o[0][l]], 0, 0, 0, base + l, err);
+            }
+        }
+        if ((m >> lev) < 4) break;  // every segment was a base case
+        // ---- sides of the points of splitting segments
+        for (int i = tid; i < m; i += kSubThreads) {
+            const int g = s.seg[cur][i];
+            if (g < 0) continue;
+            const int l = L[g], r = R[g];
+            if (r - l + 1 < 4) continue;
+            const int med = (l + r + 1) / 2;
+            s.side[o[s.tdim[g]][i]] = i < med ? 0 : (i == med ? 2 : 1);
+        }
+        __syncthreads();
+        // ---- stable partition: prefix counts of left and right points along
+        // each order, then the move
+        for (int x = w; x < 3 * words; x += kSubThreads / 32) {
+            const int d = x / words, wd = x % words, i = 32 * wd + lane;
+            int sd = 3;
+            if (i < m) {
+                const int g = s.seg[cur][i];
+                if (g >= 0 && R[g] - L[g] + 1 >= 4) sd = s.side[o[d][i]];
+            }
+            const unsigned ml = __ballot_sync(FULL, sd == 0), mr = __ballot_sync(FULL, sd == 1);
+            if (lane == 0) {
+                s.mask[d][0][wd] = ml;
+                s.mask[d][1][wd] = mr;
+            }
+        }
+        __syncthreads();
+        if (w < 6) {
+            static_assert(kSubCap / 32 <= 32, "one lane per word");
+            const int c = lane < words ? __popc(s.mask[w / 2][w % 2][lane]) : 0;
+            int inc = c;
+#pragma unroll
+            for (int f = 1; f < 32; f <<= 1) {
+                const int v = __shfl_up_sync(FULL, inc, f);
+                if (lane >= f) inc += v;
+            }
+            if (lane < words) s.pre[w / 2][w % 2][lane] = (unsigned short)(inc - c);
+        }
+        __syncthreads();
+        for (int i = tid; i < m; i += kSubThreads) {
+            const int g = s.seg[cur][i];
+            int ng = -1;
+            if (g >= 0) {
+                const int l = L[g], r = R[g], med = (l + r + 1) / 2;
+                if (r - l + 1 >= 4) {
+#pragma unroll
+                    for (int d = 0; d < 3; d++) {
+                        const int pl = o[d][i], sd = s.side[pl];
+                        int dst = med;
+                        if (sd != 2) {
+                            const unsigned *mk = s.mask[d][sd];
+                            const unsigned short *pr = s.pre[d][sd];
+                            const int at = pr[i >> 5] + __popc(mk[i >> 5] & ((1u << (i & 31)) - 1u)),
+                                      from = pr[l >> 5] + __popc(mk[l >> 5] & ((1u << (l & 31)) - 1u));
+                            dst = (sd == 0 ? l : med + 1) + at - from;
+                        }
+                        if (dst < l || dst > r) {
+                            set_err(err, KD_EINTERNAL);
+                            dst = i;
+                        }
+                        o2[d][dst] = (unsigned short)pl;
+                    }
+                    if (i != med) ng = 2 * g + (i > med);
+                }
+            }
+            s.seg[cur ^ 1][i] = (short)ng;
+        }
+        for (int g = tid; g < nseg; g += kSubThreads) {
+            const int l = L[g], r = R[g], med = (l + r + 1) / 2;
+            const bool split = r - l + 1 >= 4;
+            s.l[cur ^ 1][2 * g] = (short)(split ? l : 0);
+            s.r[cur ^ 1][2 * g] = (short)(split ? med - 1 : -1);
+            s.l[cur ^ 1][2 * g + 1] = (short)(split ? med + 1 : 0);
+            s.r[cur ^ 1][2 * g + 1] = (short)(split ? r : -1);
+        }
+        __syncthreads();
+        cur ^= 1;
+    }
 }
 
 // ------------------------------------------------------------ counting layout
@@ -1646,6 +1896,8 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
             if ((reinterpret_cast<uintptr_t>(p) & 15) != 0)
                 raise(KD_EINTERNAL, "build array not 16-byte aligned");
     }
+    check(cudaFuncSetAttribute(k_subtrees, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)sizeof(SubSmem)), "smem attribute");
     int cur = 0, nlevels = 0;
     for (int lev = 0; (1LL << lev) <= (long long)n_u; lev++) {
         nlevels = lev + 1;
@@ -1653,8 +1905,15 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
         int ub = (int)ub64;
         unsigned gs = blocks_for(ub, TPB);
         Segs S = sg[cur], N = sg[cur ^ 1];
-        k_seg_setup<<<gs, TPB, 0, s>>>(S, ub, lb);
         long long maxsize = (long long)n_u >> lev;
+        if (maxsize <= kSubCap) {  // the rest of the tree, a CTA per segment
+            while ((n_u >> (nlevels - 1)) >= 4) nlevels++;
+            k_subtrees<<<ub, kSubThreads, sizeof(SubSmem), s>>>(S, A[0], A[1], A[2], u, to,
+                                                                reinterpret_cast<int *>(sd_pos), err);
+            KD_LAUNCH_CHECK("k_subtrees");
+            break;
+        }
+        k_seg_setup<<<gs, TPB, 0, s>>>(S, ub, lb);
         if (maxsize > kSmallSeg) {
             unsigned gv = blocks_for(n_u, kVarChunk);
             k_var_par<0><<<gv, kVarThreads, 0, s>>>(n_u, pos[cur], S, lb, C[0], C[1], C[2]);
@@ -1664,7 +1923,6 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
         k_var_seq<<<blocks_for(ub, 64), 64, 0, s>>>(S, ub, lb, C[0], C[1], C[2]);
         k_level_nodes<<<gs, TPB, 0, s>>>(S, ub, lb, A[0], A[1], A[2], u, to, err);
         KD_LAUNCH_CHECK("level kernels");
-        if (maxsize < 4) break;  // every segment of this level was a base case
         // levels 0 .. lev are final: copy their slots once they are large
         // enough to be worth a copy of their own
         {
