@@ -4,14 +4,17 @@
 // the counting layout.
 //
 // Scan: reduce-then-scan over tiles of kScanTile elements (tile totals, one
-// block scans the totals, every tile scans itself from its offset).
+// block scans the totals, every tile scans itself from its offset).  Up to
+// kScanOneMax elements one block does it all.
 // Sort: one pass per digit of up to 8 bits; per pass each tile counts its
 // digits, a scan of the digit-major count table (digit 0 of every tile, then
 // digit 1, ...) gives every (digit, tile) its output offset, and each tile
 // scatters its keys in order: each warp owns a contiguous run of the tile's
 // keys, the warps' digit counts are scanned in warp order, and within a
 // round of 32 keys equal digits are ranked by lane, so equal keys keep their
-// input order (stable).
+// input order (stable).  Bound by memory latency and the scattered stores; a
+// key's rank is kept in a register from the counting phase (found again by a
+// second match, a pass over 5M keys took 79 us, and takes 56).
 //
 // Temporary storage is the caller's (a Pool or a carved scratch array): the
 // *_temp_bytes functions give its size.
@@ -143,6 +146,37 @@ __global__ void __launch_bounds__(kScanThreads) k_tile_scan(const T *in, T *out,
     }
 }
 
+// The whole scan by one block, for arrays small enough that three launches
+// cost more: every thread owns kScanOneItems consecutive elements of a chunk.
+constexpr int kScanOneThreads = 1024;
+constexpr int kScanOneItems = 8;
+constexpr long long kScanOneMax = 4LL * kScanOneThreads * kScanOneItems;
+template <class T, class Op, bool INCLUSIVE>
+__global__ void __launch_bounds__(kScanOneThreads) k_scan_one(const T *in, T *out, int n, Op op)
+{
+    __shared__ T sw[32];
+    T carry = Op::template identity<T>();
+    for (int c = 0; c < n; c += kScanOneThreads * kScanOneItems) {
+        const int base = c + threadIdx.x * kScanOneItems;
+        T v[kScanOneItems];
+        T acc = Op::template identity<T>();
+#pragma unroll
+        for (int i = 0; i < kScanOneItems; i++) {
+            v[i] = base + i < n ? in[base + i] : Op::template identity<T>();
+            acc = op(acc, v[i]);
+        }
+        T total;
+        T run = op(carry, block_excl_scan<T>(acc, op, sw, &total));
+#pragma unroll
+        for (int i = 0; i < kScanOneItems; i++) {
+            const T next = op(run, v[i]);
+            if (base + i < n) out[base + i] = INCLUSIVE ? next : run;
+            run = next;
+        }
+        carry = op(carry, total);
+    }
+}
+
 inline long long scan_tiles(long long n) { return n > 0 ? (n + kScanTile - 1) / kScanTile : 1; }
 
 template <class T> inline size_t scan_temp_bytes(long long n)
@@ -156,6 +190,10 @@ template <class T, class Op, bool INCLUSIVE>
 inline cudaError_t scan(void *temp, const T *in, T *out, long long n, Op op, cudaStream_t s)
 {
     if (n <= 0) return cudaSuccess;
+    if (n <= kScanOneMax) {
+        k_scan_one<T, Op, INCLUSIVE><<<1, kScanOneThreads, 0, s>>>(in, out, (int)n, op);
+        return cudaGetLastError();
+    }
     const long long nt = scan_tiles(n);
     T *tot = (T *)temp;
     k_tile_reduce<T, Op><<<(unsigned)nt, kScanThreads, 0, s>>>(in, n, tot, op);
@@ -221,20 +259,32 @@ __global__ void __launch_bounds__(kSortThreads) k_digit_scatter(const K *kin, K 
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int i = threadIdx.x; i < kSortWarps * kBins; i += blockDim.x) (&wc[0][0])[i] = 0;
     __syncthreads();
-    // warp w owns keys [w * 32 * kSortRounds, (w + 1) * 32 * kSortRounds) of the tile
+    // warp w owns keys [w * 32 * kSortRounds, (w + 1) * 32 * kSortRounds) of
+    // the tile; a key's rank among the warp's keys of its digit is the count so
+    // far plus the lower lanes of this round that hold the same digit
     const long long tbase = (long long)blockIdx.x * kSortTile;
     const long long base = tbase + (long long)w * 32 * kSortRounds;
+    K key[kSortRounds];
+    V val[kSortRounds];
     int dg[kSortRounds];
+    unsigned rank[kSortRounds];
 #pragma unroll
     for (int r = 0; r < kSortRounds; r++) {
         const long long j = base + r * 32 + lane;
-        const bool v = j < n;
-        dg[r] = v ? digit_of(kin[j], shift, mask) : -1;
-        const unsigned act = __ballot_sync(0xffffffffu, v);
-        if (v) {
-            const unsigned peers = __match_any_sync(act, dg[r]);
-            if (lane == __ffs(peers) - 1) wc[w][dg[r]] += __popc(peers);
+        dg[r] = -1;
+        if (j < n) {
+            key[r] = kin[j];
+            val[r] = vin[j];
+            dg[r] = digit_of(key[r], shift, mask);
         }
+    }
+#pragma unroll
+    for (int r = 0; r < kSortRounds; r++) {
+        const unsigned peers = __match_any_sync(0xffffffffu, dg[r]);
+        const unsigned before = dg[r] >= 0 ? wc[w][dg[r]] : 0u;
+        rank[r] = before + __popc(peers & ((1u << lane) - 1u));
+        __syncwarp();
+        if (dg[r] >= 0 && lane == __ffs(peers) - 1) wc[w][dg[r]] = before + __popc(peers);
         __syncwarp();
     }
     __syncthreads();
@@ -269,20 +319,12 @@ __global__ void __launch_bounds__(kSortThreads) k_digit_scatter(const K *kin, K 
     __syncthreads();
     // the tile in digit order, in shared memory
 #pragma unroll
-    for (int r = 0; r < kSortRounds; r++) {
-        const long long j = base + r * 32 + lane;
-        const bool v = dg[r] >= 0;
-        const unsigned act = __ballot_sync(0xffffffffu, v);
-        if (v) {
-            const unsigned peers = __match_any_sync(act, dg[r]);
-            const unsigned pos = wc[w][dg[r]] + __popc(peers & ((1u << lane) - 1u));
-            skey[pos] = kin[j];
-            sval[pos] = vin[j];
-            __syncwarp(act);
-            if (lane == __ffs(peers) - 1) wc[w][dg[r]] += __popc(peers);
+    for (int r = 0; r < kSortRounds; r++)
+        if (dg[r] >= 0) {
+            const unsigned pos = wc[w][dg[r]] + rank[r];
+            skey[pos] = key[r];
+            sval[pos] = val[r];
         }
-        __syncwarp();
-    }
     __syncthreads();
     // written out in that order: consecutive positions of a digit go to
     // consecutive output addresses
@@ -294,6 +336,99 @@ __global__ void __launch_bounds__(kSortThreads) k_digit_scatter(const K *kin, K 
         const unsigned dst = gofs[d] + ((unsigned)i - tstart[d]);
         kout[dst] = k;
         vout[dst] = sval[i];
+    }
+}
+
+// The whole sort by one block, all digits in shared memory, for arrays small
+// enough that three launches per digit cost more (the orders of 4000 points:
+// 0.36 ms by three launches per digit, 0.15 ms so).
+constexpr int kSmallThreads = 512;
+constexpr int kSmallWarps = kSmallThreads / 32;
+constexpr int kSmallRounds = 8;
+constexpr int kSmallMax = kSmallThreads * kSmallRounds;
+template <class K, class V> struct SmallSmem {
+    K key[kSmallMax];
+    V val[kSmallMax];
+    unsigned short wc[kSmallWarps][kBins];
+    unsigned wsum[kBins / 32];
+};
+template <class K, class V>
+__global__ void __launch_bounds__(kSmallThreads) k_sort_small(const K *kin, K *kout, const V *vin, V *vout,
+                                                              int n, int b0, int b1)
+{
+    extern __shared__ __align__(16) unsigned char sort_smem[];
+    SmallSmem<K, V> &s = *reinterpret_cast<SmallSmem<K, V> *>(sort_smem);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    // warp w owns rounds * 32 consecutive keys
+    const int rounds = (n + kSmallThreads - 1) / kSmallThreads, base = w * rounds * 32;
+    for (int i = threadIdx.x; i < n; i += kSmallThreads) {
+        s.key[i] = kin[i];
+        s.val[i] = vin[i];
+    }
+    for (int shift = b0; shift < b1; shift += kRadixBits) {
+        const int mask = (1 << (b1 - shift < kRadixBits ? b1 - shift : kRadixBits)) - 1;
+        for (int i = threadIdx.x; i < kSmallWarps * kBins; i += kSmallThreads) (&s.wc[0][0])[i] = 0;
+        __syncthreads();
+        K key[kSmallRounds];
+        V val[kSmallRounds];
+        int dg[kSmallRounds];
+        unsigned rank[kSmallRounds];
+#pragma unroll
+        for (int r = 0; r < kSmallRounds; r++)
+            if (r < rounds) {
+                const int j = base + r * 32 + lane;
+                dg[r] = -1;
+                if (j < n) {
+                    key[r] = s.key[j];
+                    val[r] = s.val[j];
+                    dg[r] = digit_of(key[r], shift, mask);
+                }
+                const unsigned peers = __match_any_sync(0xffffffffu, dg[r]);
+                const unsigned before = dg[r] >= 0 ? s.wc[w][dg[r]] : 0u;
+                rank[r] = before + __popc(peers & ((1u << lane) - 1u));
+                __syncwarp();
+                if (dg[r] >= 0 && lane == __ffs(peers) - 1)
+                    s.wc[w][dg[r]] = (unsigned short)(before + __popc(peers));
+                __syncwarp();
+            }
+        __syncthreads();
+        // first position of every (digit, warp): digits in order, a thread each
+        unsigned tot = 0, inc = 0;
+        if (threadIdx.x < kBins) {
+#pragma unroll
+            for (int k = 0; k < kSmallWarps; k++) tot += s.wc[k][threadIdx.x];
+            inc = tot;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned y = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += y;
+            }
+            if (lane == 31) s.wsum[w] = inc;
+        }
+        __syncthreads();
+        if (threadIdx.x < kBins) {
+            unsigned run = inc - tot;
+            for (int k = 0; k < w; k++) run += s.wsum[k];
+#pragma unroll
+            for (int k = 0; k < kSmallWarps; k++) {
+                const unsigned c = s.wc[k][threadIdx.x];
+                s.wc[k][threadIdx.x] = (unsigned short)run;
+                run += c;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kSmallRounds; r++)
+            if (r < rounds && dg[r] >= 0) {
+                const unsigned pos = s.wc[w][dg[r]] + rank[r];
+                s.key[pos] = key[r];
+                s.val[pos] = val[r];
+            }
+        __syncthreads();
+    }
+    for (int i = threadIdx.x; i < n; i += kSmallThreads) {
+        kout[i] = s.key[i];
+        vout[i] = s.val[i];
     }
 }
 
@@ -330,6 +465,14 @@ inline cudaError_t sort_pairs(void *temp, const K *kin, K *kout, const V *vin, V
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(vout, vin, sizeof(V) * (size_t)n, cudaMemcpyDeviceToDevice, s);
         return e;
+    }
+    if (n <= kSmallMax) {
+        const size_t smem = sizeof(SmallSmem<K, V>);
+        cudaError_t e = cudaFuncSetAttribute(k_sort_small<K, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)smem);
+        if (e != cudaSuccess) return e;
+        k_sort_small<K, V><<<1, kSmallThreads, smem, s>>>(kin, kout, vin, vout, (int)n, b0, b1);
+        return cudaGetLastError();
     }
     // ping-pong so that the last pass writes kout/vout
     const K *ks = kin;

@@ -36,3 +36,41 @@ def test_subtree_sizes(n, kind):
     elif kind == "duplicates":
         p = p[rs.randint(0, (n + 1) // 2, n)]
     _check(p, rs.randint(0, 3, len(p)).astype(np.int32), 3)
+
+
+def _wide(kind, n, rs):
+    p = rs.rand(n, 3)
+    if kind == "scales":  # twelve decades, both signs: many points on a key
+        p = 10.0 ** (-12 * p) * np.where(rs.rand(n, 3) < 0.5, -1, 1)
+    elif kind == "outlier":  # all others on one key
+        p[n // 3] = [1e300, -1e300, 1e300]
+    elif kind == "overflow":
+        p[n // 3], p[n // 2] = 1.7e308, -1.7e308
+    elif kind == "infinite":
+        p[n // 3, 0], p[n // 2, 1], p[n // 5, 2] = np.inf, -np.inf, np.inf
+    elif kind == "float32":  # ties along one axis, few and short
+        p = p.astype(np.float32).astype(np.float64)
+    elif kind == "columns":  # runs of equal x, longer than those put right in place
+        p[:, 0] = p[rs.randint(0, n // 60, n), 0]
+    elif kind == "pairs":  # runs of equal x, of two and three points, then equal y
+        p[:, 0] = p[rs.randint(0, n // 2, n), 0]
+        p[:, 1] = np.where(rs.rand(n) < 0.5, p[:, 0], p[:, 1])
+    elif kind == "zeros":
+        p[rs.rand(n) < 0.01] = 0.0
+        p[rs.rand(n, 3) < 0.01] = -0.0
+    return p[rs.permutation(n)]
+
+
+@pytest.mark.parametrize("kind", ["scales", "outlier", "overflow", "infinite", "float32", "columns",
+                                  "pairs", "zeros"])
+@pytest.mark.parametrize("n", [200, 4096, 4097, 70001])
+def test_orders_of_wide_keys(n, kind):
+    """The three orders by 32-bit keys, at both sorts and with every rule for a
+    key's bits; the general path is the oracle's comparison of all 64."""
+    rs = np.random.RandomState(n)
+    p = _wide(kind, n, rs)
+    f = np.zeros(n, np.int32)
+    if kind == "zeros":  # at most 255 copies of a point are a valid tree
+        _, first = np.unique(p, axis=0, return_index=True)
+        p, f = p[np.sort(first)], f[:len(first)]
+    _check(p, f, 1)
