@@ -425,41 +425,35 @@ static int query_catalog(const double *xyz, const int *fields, int n, int Fq, kd
                          int *empty)
 {
     int i, m = 0, rc;
-    double *px = NULL;
-    int *pf = NULL;
-    const double *use_x = xyz;
-    const int *use_f = fields;
+    double *px;
+    int *pf;
     *empty = 0;
-    for (i = 0; i < n; i++)
-        if (isnan(xyz[3 * (size_t)i]) || isnan(xyz[3 * (size_t)i + 1]) || isnan(xyz[3 * (size_t)i + 2]))
-            break;
-    if (i < n) {
-        px = (double *)malloc(sizeof(double) * 3 * (size_t)n);
-        pf = fields ? (int *)malloc(sizeof(int) * (size_t)n) : NULL;
-        if (!px || (fields && !pf)) {
-            free(px);
-            free(pf);
-            kd_set_error(KD_ENOMEM, "out of host memory");
-            return KD_ENOMEM;
-        }
-        for (i = 0; i < n; i++) {
-            const double *p = xyz + 3 * (size_t)i;
-            if (isnan(p[0]) || isnan(p[1]) || isnan(p[2])) continue;
-            memcpy(px + 3 * (size_t)m, p, 3 * sizeof(double));
-            if (pf) pf[m] = fields[i];
-            m++;
-        }
-        use_x = px;
-        use_f = pf;
-        n = m;
+    /* the build reports a NaN; only then are the points looked through here */
+    rc = kdg_build(xyz, fields, n, Fq, 1, qc);
+    if (rc != KD_ENAN) return rc;
+    clear_error();
+    px = (double *)malloc(sizeof(double) * 3 * (size_t)n);
+    pf = fields ? (int *)malloc(sizeof(int) * (size_t)n) : NULL;
+    if (!px || (fields && !pf)) {
+        free(px);
+        free(pf);
+        kd_set_error(KD_ENOMEM, "out of host memory");
+        return KD_ENOMEM;
     }
-    if (n == 0) {
+    for (i = 0; i < n; i++) {
+        const double *p = xyz + 3 * (size_t)i;
+        if (isnan(p[0]) || isnan(p[1]) || isnan(p[2])) continue;
+        memcpy(px + 3 * (size_t)m, p, 3 * sizeof(double));
+        if (pf) pf[m] = fields[i];
+        m++;
+    }
+    if (m == 0) {
         *empty = 1;
         free(px);
         free(pf);
         return KD_OK;
     }
-    rc = kdg_build(use_x, use_f, n, Fq, 1, qc);
+    rc = kdg_build(px, pf, m, Fq, 1, qc);
     free(px);
     free(pf);
     return rc;

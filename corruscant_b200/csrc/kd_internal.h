@@ -99,7 +99,9 @@ typedef struct kd_catalog {
 /* Build a catalog from host arrays (xyz interleaved (n,3), fields may be
  * NULL) to serve as the query side of counts only: a point may repeat 256 or
  * more times (only tree nodes store an 8-bit weight) and no node array is
- * returned.  Returns KD_OK or a negative status; on failure nothing is held. */
+ * returned.  With query_only the catalog may hold the query side alone (points
+ * in counting order and blocks).  Returns KD_OK or a negative status; on
+ * failure nothing is held. */
 int kdg_build(const double *h_xyz, const int *h_fields, int n, int num_fields,
               int query_only, kd_catalog *cat);
 

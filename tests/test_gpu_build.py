@@ -74,3 +74,42 @@ def test_orders_of_wide_keys(n, kind):
         _, first = np.unique(p, axis=0, return_index=True)
         p, f = p[np.sort(first)], f[:len(first)]
     _check(p, f, 1)
+
+
+@pytest.mark.parametrize("kind", ["uniform", "scales", "outlier", "overflow", "infinite", "columns",
+                                  "zeros", "copies", "tight", "line"])
+@pytest.mark.parametrize("n", [1, 2, 127, 128, 129, 200, 4096, 4097, 20001])
+def test_query_points(n, kind):
+    """Points ordered along a curve against the oracle's exhaustive counts (up
+    to 4097 points) and against the counts of a tree of the same points."""
+    rs = np.random.RandomState(n)
+    m = max(n, 60)
+    if kind == "copies":  # more than a tree accepts
+        q = rs.rand(1 + m // 300, 3)[rs.randint(0, 1 + m // 300, m)][:n]
+    elif kind == "tight":  # below the curve's cells
+        q = (rs.rand(8, 3)[rs.randint(0, 8, m)] + 1e-9 * rs.rand(m, 3))[:n]
+    elif kind == "line":
+        q = (rs.rand(m, 1) * [[1.0, 0.0, -2.0]] + [[0.0, 3.0, 0.0]])[:n]
+    else:
+        q = _wide(kind, m, rs)[:n]
+    f = rs.randint(0, 3, n).astype(np.int32)
+    scale = {"overflow": 1e308, "outlier": 1.0, "tight": 1e-9}.get(kind, 0.3)
+    radii = np.array([0.1, 0.3, 1.0, 4.0]) * scale
+    tp = np.concatenate([q[: n // 2 + 1], rs.rand(300, 3)])
+    tp = tp[np.unique(tp, axis=0, return_index=True)[1]]
+    tf = rs.randint(0, 3, len(tp)).astype(np.int32)
+    t = N.build_tree(tp, tf, 3)
+    try:
+        for mode in (N.KD_MODE_MIXED, N.KD_MODE_FP64):
+            got = N.count_points(t, q, f, 3, radii, mode=mode)
+            if n <= 4097:
+                want = O.OracleTree(tp, tf, 3).brute_counts(q, f, 3, radii, nthreads=4)
+                assert np.array_equal(got, want), mode
+            elif kind not in ("copies", "zeros"):
+                tq = N.build_tree(q, f, 3)
+                try:
+                    assert np.array_equal(got, N.count_radii(t, tq, radii, mode=mode)), mode
+                finally:
+                    N.destroy(tq)
+    finally:
+        N.destroy(t)
