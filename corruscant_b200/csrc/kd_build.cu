@@ -295,13 +295,13 @@ struct FieldInfo {
 
 __global__ void k_weights(UniqueArrays u, int n_u, const int *__restrict__ p,
                           const int *__restrict__ cls, const int *__restrict__ fin, int n,
-                          int heavy_ok, int *err, FieldInfo *fi)
+                          int *err, FieldInfo *fi)
 {
     int maxtf = 0;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n_u; c += gridDim.x * blockDim.x) {
         int w = u.uhead[c + 1] - u.uhead[c];
         u.uw[c] = w;
-        if (w > 255 && !heavy_ok) set_err(err, KD_EDUP);
+        if (w > 255) set_err(err, KD_EDUP);
         maxtf = max(maxtf, u.ufield[c]);
     }
     int minq = 0x7fffffff, maxq = -0x7fffffff, split = 0;
@@ -605,9 +605,7 @@ __global__ void k_var_seq(Segs sg, int ub, LevelBufs lb, const double *__restric
 
 struct TreeOut {
     NodeRec *nodes;
-    int *npoint;
-    unsigned char *ndim;
-    int *inorder_u;
+    int *inorder_rep;  // input index of the point at every in-order position
     int memsize;
 };
 
@@ -627,9 +625,7 @@ __device__ __forceinline__ void put_node(TreeOut t, const UniqueArrays &u, int h
     rec.flags = (uint32_t)hl | ((uint32_t)hr << 1) | ((uint32_t)dim << 2);
     rec.pad1 = 0;
     t.nodes[hp] = rec;
-    t.npoint[hp] = pt;
-    t.ndim[hp] = (unsigned char)dim;
-    t.inorder_u[pos] = pt;
+    t.inorder_rep[pos] = u.urep[pt];
 }
 
 __global__ void k_level_nodes(Segs sg, int ub, LevelBufs lb, const int *__restrict__ a0,
@@ -1021,13 +1017,6 @@ __global__ void k_next_pos(int n_u, const int *__restrict__ pos_seg, Segs sg, Le
     }
 }
 
-__global__ void k_inorder_rep(int n_u, const int *__restrict__ inorder_u,
-                              const int *__restrict__ urep, int *out)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_u; i += gridDim.x * blockDim.x)
-        out[i] = urep[inorder_u[i]];
-}
-
 // ------------------------------------------------------------ subtrees
 
 // Whole subtrees of up to kSubCap points, one CTA each, from the level where
@@ -1271,133 +1260,23 @@ __global__ void __launch_bounds__(kSubThreads) k_subtrees(Segs sg, const int *__
 
 // ------------------------------------------------------------ counting layout
 
-// in-order range of heap id h at depth D (the range recursion is data
-// independent: med = (l+r+1)/2, children (l, med-1) and (med+1, r))
-__device__ __forceinline__ void heap_range(int n_u, int h, int D, int &l, int &r)
-{
-    l = 0;
-    r = n_u - 1;
-    for (int b = D - 1; b >= 0; b--) {
-        int med = (l + r + 1) / 2;
-        if ((h >> b) & 1) l = med + 1;
-        else r = med - 1;
-    }
-}
-
-__device__ __forceinline__ int superkey_cmp(const UniqueArrays &u, int a, int b, int msd)
-{
-    for (int k = 0; k < 3; k++) {
-        int d = (msd + k) % 3;
-        uint64_t ka = d == 0 ? u.ukx[a] : (d == 1 ? u.uky[a] : u.ukz[a]);
-        uint64_t kb = d == 0 ? u.ukx[b] : (d == 1 ? u.uky[b] : u.ukz[b]);
-        if (ka != kb) return ka < kb ? -1 : 1;
-    }
-    return 0;
-}
-
-// Each node above the counting leaves holds one point; it is placed in the
-// leaf (below its left child, on whose side of the split plane it lies) whose
-// cell contains it, following the splits of the nodes below.
-__global__ void k_anc_leaf(int nleaves, const int *__restrict__ npoint,
-                           const unsigned char *__restrict__ ndim, UniqueArrays u, int *anc_leaf,
-                           int *extra_cnt)
-{
-    int h = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    if (h >= nleaves) return;
-    int pt = npoint[h];
-    int c = 2 * h;
-    while (c < nleaves) c = 2 * c + (superkey_cmp(u, pt, npoint[c], ndim[c]) > 0);
-    int leaf = c - nleaves;
-    anc_leaf[h - 1] = leaf;
-    atomicAdd(&extra_cnt[leaf], 1);
-}
-
-__global__ void k_leaf_ucount(int n_u, int D, int nleaves, const int *__restrict__ extra_cnt,
-                              int *ucount)
-{
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= nleaves) return;
-    int l, r;
-    heap_range(n_u, nleaves + j, D, l, r);
-    ucount[j] = (r - l + 1) + (extra_cnt ? extra_cnt[j] : 0);
-}
-
-__global__ void k_cpos_sub(int n_u, int D, int nleaves, const int *__restrict__ ustart,
-                           const int *__restrict__ inorder_u, int *cpos)
-{
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= nleaves) return;
-    int l, r;
-    heap_range(n_u, nleaves + j, D, l, r);
-    int base = ustart[j];
-    for (int i = l; i <= r; i++) cpos[inorder_u[i]] = base + (i - l);
-}
-
-// sorted (leaf, ancestor) pairs -> counting positions of ancestor points
-__global__ void k_cpos_extra(int nanc, int n_u, int D, int nleaves,
-                             const int *__restrict__ sleaf, const int *__restrict__ sanc,
-                             const int *__restrict__ extra_start, const int *__restrict__ ustart,
-                             const int *__restrict__ npoint, int *cpos)
-{
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nanc) return;
-    int j = sleaf[k];
-    int l, r;
-    heap_range(n_u, nleaves + j, D, l, r);
-    cpos[npoint[sanc[k]]] = ustart[j] + (r - l + 1) + (k - extra_start[j]);
-}
-
-__global__ void k_scatter_w(int n_u, const int *__restrict__ cpos, const int *__restrict__ uw,
-                            int *wc)
-{
-    for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < n_u; u += gridDim.x * blockDim.x)
-        wc[cpos[u]] = uw[u];
-}
-
-struct RawOut {
-    double *x, *y, *z;
-    int *qf, *tf;
-};
-
-__global__ void k_raw_scatter(int n, const int *__restrict__ p, const int *__restrict__ cls,
-                              const int *__restrict__ uhead, const int *__restrict__ cpos,
-                              const int *__restrict__ rstart, const double *__restrict__ xyz,
-                              const int *__restrict__ fin, const int *__restrict__ ufield,
-                              RawOut o, int split)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        int r = p[i], c = cls[i] - 1;
-        int pos = rstart[cpos[c]] + (i - uhead[c]);
-        o.x[pos] = xyz[3 * (size_t)r];
-        o.y[pos] = xyz[3 * (size_t)r + 1];
-        o.z[pos] = xyz[3 * (size_t)r + 2];
-        o.qf[pos] = fin ? fin[r] : 0;
-        if (split) o.tf[pos] = ufield[c];
-    }
-}
-
-__global__ void k_leaf_rstart(int nleaves, const int *__restrict__ ustart,
-                              const int *__restrict__ rstart, int *leaf_r)
-{
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j > nleaves) return;
-    leaf_r[j] = rstart[ustart[j]];
-}
-
-// key (leaf, tree field) per raw position; flag when a leaf is out of order
-__global__ void k_leaf_keys(int nleaves, const int *__restrict__ leaf_r,
-                            const int *__restrict__ tf, unsigned *key, int *unsorted)
-{
-    int j = blockIdx.x;
-    if (j >= nleaves) return;
-    int a = leaf_r[j], b = leaf_r[j + 1];
-    int bad = 0;
-    for (int i = a + threadIdx.x; i < b; i += blockDim.x) {
-        key[i] = ((unsigned)j << 8) | (unsigned)tf[i];
-        if (i > a && tf[i] < tf[i - 1]) bad = 1;
-    }
-    if (bad) atomicOr(unsorted, 1);
-}
+// The counting order.  Raw points go by cells of at most kChunk points: of a
+// tree's, the cells of its own splits at the depth where they have become that
+// small (they are boxes that tile the points' cloud, whatever its shape); of
+// query points that have no tree, stretches of a Hilbert curve.  Within a cell
+// they are split in the middle again and again (k_refine).  A cell's points are
+// then cut every KD_RUN_MAX into leaves (each grouped by tree field into runs)
+// and every KD_BLOCK_MAX into query blocks, so that a block is two leaves and a
+// symmetric count's runs never straddle one; only a cell's last leaf and block
+// are partly filled.
+// Against leaves by the tree's own depth (32 to 64 points each, and blocks cut
+// across them at the ends of 16-leaf subtrees), in the tile kernel: 3M uniform
+// points with themselves in 21 edges 7.6 -> 5.8 ms, 5M on the sky in 16 edges
+// 13.9 -> 11.2, 1M + 1M on a grid in 30 edges 25.9 -> 21.9; the layout of 5M
+// points 2.8 -> 1.9 ms.  Curves instead of the tree's cells, without splits and
+// with: 7.4 and 6.2 ms, 18.4 and 15.0, 25.8 and 23.1 (a curve leaves and enters
+// a surface again, far away).  Leaves of 32 points: 6.5 ms for the first, but
+// 647 instead of 572 ms for 1M / 20M points in edges spread over two decades.
 
 template <class T>
 __global__ void k_gather(const T *__restrict__ src, const int *__restrict__ idx, int n, T *dst)
@@ -1406,152 +1285,571 @@ __global__ void k_gather(const T *__restrict__ src, const int *__restrict__ idx,
         dst[i] = src[idx[i]];
 }
 
-// group heads (leaf or tree-field change) carry their own index, others 0;
-// an inclusive max-scan then gives every position its group start
-__global__ void k_group_heads(int n, const unsigned *__restrict__ key, int *gh)
+// The bits of v (21 of them) three apart.
+__device__ __forceinline__ uint64_t spread3(uint64_t v)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        gh[i] = (i == 0 || key[i] != key[i - 1]) ? i : 0;
+    v = (v | (v << 32)) & 0x001f00000000ffffull;
+    v = (v | (v << 16)) & 0x001f0000ff0000ffull;
+    v = (v | (v << 8)) & 0x100f00f00f00f00full;
+    v = (v | (v << 4)) & 0x10c30c30c30c30c3ull;
+    return (v | (v << 2)) & 0x1249249249249249ull;
 }
 
-// a run starts at every KD_RUN_MAX-th point of a group
-__global__ void k_run_heads(int n, const int *__restrict__ gs, int *head)
+// Position along the Hilbert curve of 2^21 cells per side, three bits a level,
+// by the transform of Skilling (AIP Conf. Proc. 707, 381, 2004): from the
+// coarsest level down, each axis exchanges or inverts the finer bits of the
+// first one, and a Gray code orders the eight cells of a level.
+__device__ __forceinline__ uint64_t hilbert(unsigned (&c)[3])
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        head[i] = ((i - gs[i]) % KD_RUN_MAX) == 0;
+#pragma unroll 1
+    for (unsigned bit = 1u << 20; bit > 1; bit >>= 1) {
+        const unsigned finer = bit - 1;
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            const unsigned swap = (c[d] & bit) ? 0u : (c[0] ^ c[d]) & finer;
+            c[0] ^= (c[d] & bit) ? finer : swap;
+            if (d) c[d] ^= swap;
+        }
+    }
+    c[1] ^= c[0];
+    c[2] ^= c[1];
+    unsigned flip = c[2] >> 1;  // bit b: parity of the bits of c[2] above b
+    flip ^= flip >> 1;
+    flip ^= flip >> 2;
+    flip ^= flip >> 4;
+    flip ^= flip >> 8;
+    flip ^= flip >> 16;
+    return spread3(c[0] ^ flip) << 2 | spread3(c[1] ^ flip) << 1 | spread3(c[2] ^ flip);
 }
 
-__global__ void k_runs(int n, const unsigned *__restrict__ key, const int *__restrict__ head,
-                       const int *__restrict__ rid, int nleaves, int *run_start, int *run_tf,
-                       int *run_leaf, int *leaf_run)
+// Position of each point along the curve through the points' cube (key), or
+// its 32 highest bits (key32), and, with fi, the range of the own fields.
+__global__ void __launch_bounds__(TPB) k_curve(const double *__restrict__ xyz, const int *__restrict__ fin,
+                                               int n, const KeySpan *span, uint64_t *key, unsigned *key32,
+                                               int *iota, FieldInfo *fi)
 {
+    double lo[3], ext = 0.0;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        lo[d] = okey_value(~span->inv_lo[d]);
+        ext = fmax(ext, okey_value(span->hi[d]) - lo[d]);
+    }
+    const double top = 2097151.0, scale = ext > 0.0 ? top / ext : 0.0;
+    int minq = 0x7fffffff, maxq = -0x7fffffff;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        if (!head[i]) continue;
-        int r = rid[i] - 1;
-        run_start[r] = i;
-        run_tf[r] = (int)(key[i] & 0xFF);
-        unsigned leaf = key[i] >> 8;
-        run_leaf[r] = (int)leaf;
-        if (i == 0 || (key[i - 1] >> 8) != leaf) leaf_run[leaf] = r;
+        unsigned c[3];
+#pragma unroll
+        for (int d = 0; d < 3; d++)  // (NaN, from an infinite range: the last cell)
+            c[d] = __double2uint_rd(fmin((xyz[3 * (size_t)i + d] - lo[d]) * scale, top));
+        const uint64_t k = hilbert(c);
+        if (key) key[i] = k;
+        else key32[i] = (unsigned)(k >> 31);
+        iota[i] = i;
+        const int qf = fin ? fin[i] : 0;
+        minq = min(minq, qf);
+        maxq = max(maxq, qf);
+    }
+    if (!fi) return;
+    minq = __reduce_min_sync(0xffffffffu, minq);
+    maxq = __reduce_max_sync(0xffffffffu, maxq);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMin(&fi->min_qf, minq);
+        atomicMax(&fi->max_qf, maxq);
     }
 }
 
-__global__ void k_run_len(int nruns, int n, int nleaves, const int *__restrict__ run_start,
-                          int *run_len, int *leaf_run)
+// Points of a run of more than kCellMax equal keys whose places differ.
+constexpr int kCellMax = 512;
+template <class K>
+__global__ void k_full_cells(const K *__restrict__ srt, const int *__restrict__ perm,
+                             const double *__restrict__ xyz, int n, int *full)
 {
-    int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r == 0) leaf_run[nleaves] = nruns;
-    if (r >= nruns) return;
-    int e = r + 1 < nruns ? run_start[r + 1] : n;
-    run_len[r] = e - run_start[r];
+    int c = 0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x + kCellMax; i < n; i += gridDim.x * blockDim.x) {
+        if (srt[i] != srt[i - kCellMax]) continue;
+        const size_t a = perm[i], b = perm[i - kCellMax];
+        c += xyz[3 * a] != xyz[3 * b] || xyz[3 * a + 1] != xyz[3 * b + 1] || xyz[3 * a + 2] != xyz[3 * b + 2];
+    }
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (c && (threadIdx.x & 31) == 0) atomicAdd(full, c);
 }
+
+// A tree's cells: cell c holds places [start[c], start[c + 1]) of the order and
+// owns 2^leaf_bits leaves, the last of them empty.
+struct Cells {
+    const int *start;
+    int bits, leaf_bits;  // 2^bits cells
+};
+
+// The order within a cell, every kChunk points at a time: split in the middle
+// along the longest side of their box, and so on down to kCut points, so that
+// leaves, query tiles and halves of each are boxes that hardly overlap.  One
+// CTA per chunk: keys of 20 bits of the coordinate within the segment's box
+// and the point's place, sorted in every segment at once by a bitonic network
+// (registers, then lanes, then shared memory); positions behind the last point
+// sort last.  Bound by the latency of the network's steps and barriers.
+constexpr int kChunk = 2048;
+constexpr int kCut = 16;
+constexpr int kRefThreads = kChunk / 4;  // thread t: positions 4 t .. 4 t + 3
+constexpr int kRefWarps = kRefThreads / 32;
+struct RefineSmem {
+    double v[3][kChunk];
+    double box[kRefWarps][6];
+    unsigned key[kChunk];
+};
+__global__ void __launch_bounds__(kRefThreads) k_refine(int n, const double *__restrict__ xyz, Cells cells,
+                                                        const int *__restrict__ in, int *__restrict__ out)
+{
+    extern __shared__ __align__(16) unsigned char ref_smem[];
+    RefineSmem &s = *reinterpret_cast<RefineSmem *>(ref_smem);
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int kIdBits = 12, kIdMask = (1 << kIdBits) - 1;
+    static_assert(kChunk <= 1 << kIdBits && kRefWarps <= 32, "ids in a key, a lane per warp's box");
+    const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+    long long base = (long long)blockIdx.x * kChunk, end = n;
+    if (cells.start) {
+        const int per = max(1, (KD_RUN_MAX << cells.leaf_bits) / kChunk);  // chunks per cell
+        base = cells.start[blockIdx.x / per] + (long long)(blockIdx.x % per) * kChunk;
+        end = cells.start[blockIdx.x / per + 1];
+    }
+    const int m = (int)min((long long)kChunk, end - base);
+    if (m <= 0) return;
+    for (int i = t; i < m; i += kRefThreads) {
+        const size_t p = in[base + i];
+#pragma unroll
+        for (int d = 0; d < 3; d++) s.v[d][i] = xyz[3 * p + d];
+    }
+    unsigned key[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) key[k] = 4 * t + k;
+    int first = kChunk;
+    while (first > kCut && first / 2 >= m) first /= 2;
+    __syncthreads();
+    for (int seg = first; seg > kCut; seg >>= 1) {
+        // ---- the segments' boxes
+        double lo[3], hi[3];
+#pragma unroll
+        for (int d = 0; d < 3; d++) lo[d] = INFINITY, hi[d] = -INFINITY;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int id = key[k] & kIdMask;
+            if (id < m)
+#pragma unroll
+                for (int d = 0; d < 3; d++) {
+                    lo[d] = fmin(lo[d], s.v[d][id]);
+                    hi[d] = fmax(hi[d], s.v[d][id]);
+                }
+        }
+        for (int f = 1; f < min(32, seg / 4); f <<= 1)
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                lo[d] = fmin(lo[d], __shfl_xor_sync(FULL, lo[d], f));
+                hi[d] = fmax(hi[d], __shfl_xor_sync(FULL, hi[d], f));
+            }
+        if (seg > 128) {  // several warps per segment
+            if (lane == 0)
+#pragma unroll
+                for (int d = 0; d < 3; d++) s.box[w][d] = lo[d], s.box[w][3 + d] = hi[d];
+            __syncthreads();
+            const int nw = seg / 128, w0 = w & ~(nw - 1);
+            const double *const b = s.box[w0 + (lane & (nw - 1))];
+#pragma unroll
+            for (int d = 0; d < 3; d++) lo[d] = b[d], hi[d] = b[3 + d];
+            for (int f = 1; f < nw; f <<= 1)
+#pragma unroll
+                for (int d = 0; d < 3; d++) {
+                    lo[d] = fmin(lo[d], __shfl_xor_sync(FULL, lo[d], f));
+                    hi[d] = fmax(hi[d], __shfl_xor_sync(FULL, hi[d], f));
+                }
+        }
+        // ---- keys along the longest side (a side of infinite length first)
+        const double ex = hi[0] - lo[0], ey = hi[1] - lo[1], ez = hi[2] - lo[2];
+        const int dim = ex >= ey && ex >= ez ? 0 : (ey >= ez ? 1 : 2);
+        const double ext = dim == 0 ? ex : (dim == 1 ? ey : ez), low = dim == 0 ? lo[0] : (dim == 1 ? lo[1] : lo[2]);
+        const double top = (double)((1 << (32 - kIdBits)) - 2), scale = ext > 0.0 ? top / ext : 0.0;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int id = key[k] & kIdMask;
+            unsigned q = (1u << (32 - kIdBits)) - 1u;
+            if (id < m) q = __double2uint_rd(fmin((s.v[dim][id] - low) * scale, top));
+            key[k] = q << kIdBits | (unsigned)id;
+        }
+        // ---- sort every segment
+        auto swap_if = [&](unsigned &a, unsigned &b, bool up) {  // a before b
+            const unsigned x = min(a, b), y = max(a, b);
+            a = up ? x : y;
+            b = up ? y : x;
+        };
+        for (int k = 2; k <= seg; k <<= 1) {
+            // direction of this thread's elements (k >= 4: one for all four)
+            const bool up = k == seg || !((4 * t) & k);
+            int j = k >> 1;
+            for (; j >= 128; j >>= 1) {
+                __syncthreads();
+                *reinterpret_cast<uint4 *>(s.key + 4 * t) = make_uint4(key[0], key[1], key[2], key[3]);
+                __syncthreads();
+                const uint4 o = *reinterpret_cast<const uint4 *>(s.key + ((4 * t) ^ j));
+                const bool low_half = !((4 * t) & j), take_min = low_half == up;
+                key[0] = take_min ? min(key[0], o.x) : max(key[0], o.x);
+                key[1] = take_min ? min(key[1], o.y) : max(key[1], o.y);
+                key[2] = take_min ? min(key[2], o.z) : max(key[2], o.z);
+                key[3] = take_min ? min(key[3], o.w) : max(key[3], o.w);
+            }
+            for (; j >= 4; j >>= 1) {
+                const bool low_half = !((4 * t) & j), take_min = low_half == up;
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const unsigned o = __shfl_xor_sync(FULL, key[e], j >> 2);
+                    key[e] = take_min ? min(key[e], o) : max(key[e], o);
+                }
+            }
+            if (j == 2) {
+                swap_if(key[0], key[2], up);
+                swap_if(key[1], key[3], up);
+                j = 1;
+            }
+            if (k == 2) {
+                swap_if(key[0], key[1], true);
+                swap_if(key[2], key[3], false);
+            } else {
+                swap_if(key[0], key[1], up);
+                swap_if(key[2], key[3], up);
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (4 * t + k < m) out[base + 4 * t + k] = in[base + (key[k] & kIdMask)];
+}
+
+// For points that the curve's cells do not resolve: the rank of each point's
+// coordinates among their values, in place of the coordinates.
+__global__ void k_value_heads(const uint64_t *__restrict__ key, const int *__restrict__ ord, int n, int *head)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        head[i] = i == 0 || key[ord[i]] != key[ord[i - 1]];
+}
+
+__global__ void k_scatter_rank(const int *__restrict__ cls, const int *__restrict__ ord, int n, int *rank)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        rank[ord[i]] = cls[i] - 1;
+}
+
+__global__ void k_curve_ranks(const int *__restrict__ rx, const int *__restrict__ ry,
+                              const int *__restrict__ rz, int n, uint64_t *key)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int r[3] = {rx[i], ry[i], rz[i]};
+        unsigned c[3];
+#pragma unroll
+        for (int d = 0; d < 3; d++) c[d] = (unsigned)(((unsigned long long)r[d] << 21) / (unsigned)n);
+        key[i] = hilbert(c);
+    }
+}
+
+// The cell (node of depth `bits`) of the point at every in-order position, by
+// its input index.  A point above the cells lies on a split plane: it goes by
+// the splits below its left child.
+__global__ void k_cell_of(int n_u, int bits, const NodeRec *__restrict__ nodes,
+                          const int *__restrict__ inorder_rep, int *cell)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_u; i += gridDim.x * blockDim.x) {
+        int l = 0, r = n_u - 1, h = 1;
+        for (int b = 0; b < bits; b++) {
+            const int med = (l + r + 1) / 2;  // (the ranges do not depend on the data)
+            if (i == med) {
+                const double v[3] = {nodes[h].v[0], nodes[h].v[1], nodes[h].v[2]};
+                for (h *= 2; ++b < bits;) {
+                    const int d = (nodes[h].flags >> 2) & 3;
+                    h = 2 * h + ((d == 0 ? v[0] : (d == 1 ? v[1] : v[2])) > nodes[h].v[d]);
+                }
+                break;
+            }
+            h = 2 * h + (i > med);
+            if (i > med) l = med + 1;
+            else r = med - 1;
+        }
+        cell[inorder_rep[i]] = h - (1 << bits);
+    }
+}
+
+__global__ void k_cell_keys(int n, const int *__restrict__ p, const int *__restrict__ cls,
+                            const int *__restrict__ urep, const int *__restrict__ cell, unsigned *key)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        key[i] = (unsigned)cell[urep[cls[i] - 1]];
+}
+
+// cells' first places (no cell is empty); key: sorted cells, null for one cell
+__global__ void k_cell_starts(int n, int ncells, const unsigned *__restrict__ key, int *start)
+{
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        start[0] = 0;
+        start[ncells] = n;
+    }
+    if (!key) return;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i < n; i += gridDim.x * blockDim.x)
+        if (key[i] != key[i - 1]) start[key[i]] = i;
+}
+
+__global__ void k_cell_max(int ncells, const int *__restrict__ start, int *largest)
+{
+    int m = 0;
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncells; c += gridDim.x * blockDim.x)
+        m = max(m, start[c + 1] - start[c]);
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0) atomicMax(largest, m);
+}
+
+// cells of kChunk places each, empty ones behind the last point
+__global__ void k_even_cells(int n, int ncells, int *start)
+{
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c <= ncells) start[c] = (int)min((long long)n, (long long)c * kChunk);
+}
+
+struct RawOut {
+    double *x, *y, *z;
+    int *qf, *tf;
+};
 
 struct Summ {
     double *box;
-    int *count, *tf, *qf;
+    int *count, *tf;
 };
 
-// one warp per leaf
-__global__ void k_leaf_summary(int nleaves, const int *__restrict__ leaf_r, RawOut o, Summ sm)
-{
-    int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (w >= nleaves) return;
-    int a = leaf_r[w], b = leaf_r[w + 1];
-    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    int tf0 = o.tf[a], qf0 = o.qf[a];
-    int tfm = 0, qfm = 0;
-    for (int i = a + lane; i < b; i += 32) {
-        double v[3] = {o.x[i], o.y[i], o.z[i]};
-        for (int d = 0; d < 3; d++) {
-            lo[d] = fmin(lo[d], v[d]);
-            hi[d] = fmax(hi[d], v[d]);
-        }
-        tfm |= o.tf[i] != tf0;
-        qfm |= o.qf[i] != qf0;
-    }
-    for (int off = 16; off; off >>= 1)
-        for (int d = 0; d < 3; d++) {
-            lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], off));
-            hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], off));
-        }
-    tfm = __any_sync(0xffffffffu, tfm);
-    qfm = __any_sync(0xffffffffu, qfm);
-    if (lane == 0) {
-        int h = nleaves + w;
-        for (int d = 0; d < 3; d++) {
-            sm.box[6 * (size_t)h + d] = lo[d];
-            sm.box[6 * (size_t)h + 3 + d] = hi[d];
-        }
-        sm.count[h] = b - a;
-        sm.tf[h] = tfm ? -1 : tf0;
-        sm.qf[h] = qfm ? -1 : qf0;
-    }
-}
+struct LeafOut {
+    RawOut o;
+    Summ sm;
+    int *qf;        // single own field of the leaf, -1 when mixed
+    kd_leaf *leaf;  // leaf boxes as the tile kernel reads them
+    float4 *t4;     // each point in FP32 relative to its leaf's centre
+    int *pos, *nruns, *blocks;  // blocks: query blocks per pair of leaves
+    unsigned long long *hdiag;
+};
 
-// leaf boxes as the tile kernel reads them, and each raw point in FP32
-// relative to its leaf's centre
-__global__ void k_leaf_rel(int nleaves, const int *__restrict__ leaf_r, RawOut o,
-                           const double *__restrict__ box, kd_leaf *leaf, float4 *t4,
-                           unsigned long long *hdiag)
+constexpr int kBlockLeaves = KD_BLOCK_MAX / KD_RUN_MAX;
+static_assert(KD_BLOCK_MAX == kBlockLeaves * KD_RUN_MAX, "blocks are whole leaves");
+
+// One warp per leaf: its points, gathered and grouped by tree field, its box
+// and summary.  tf: tree field per input point, null where it is the own field.
+__global__ void __launch_bounds__(TPB) k_leaves(int n, int nleaves, Cells cells, const int *__restrict__ perm,
+                                                const double *__restrict__ xyz, const int *__restrict__ fin,
+                                                const int *__restrict__ tfin, LeafOut out)
 {
-    int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (w >= nleaves) return;
-    const double *b = box + 6 * (size_t)(nleaves + w);
-    double cx = 0.5 * (b[0] + b[3]), cy = 0.5 * (b[1] + b[4]), cz = 0.5 * (b[2] + b[5]);
+    constexpr int PL = KD_RUN_MAX / 32;  // points per lane
+    constexpr unsigned FULL = 0xffffffffu;
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (w > nleaves) return;
+    int a = n, len = 0;
+    if (w < nleaves) {
+        const int c = w >> cells.leaf_bits, end = cells.start[c + 1];
+        a = min(end, cells.start[c] + (w - (c << cells.leaf_bits)) * KD_RUN_MAX);
+        len = min(end - a, KD_RUN_MAX);
+    }
     if (lane == 0) {
-        const double hx = fmax(b[3] - cx, cx - b[0]), hy = fmax(b[4] - cy, cy - b[1]),
-                     hz = fmax(b[5] - cz, cz - b[2]);
+        out.pos[w] = a;
+        if (w % kBlockLeaves == 0 || w == nleaves) out.blocks[(w + kBlockLeaves - 1) / kBlockLeaves] = len > 0;
+        if (w == nleaves) out.nruns[w] = 0;
+    }
+    if (w == nleaves) return;
+    double v[PL][3], lo[3], hi[3];
+    int qf[PL], tf[PL], rank[PL];
+#pragma unroll
+    for (int d = 0; d < 3; d++) lo[d] = INFINITY, hi[d] = -INFINITY;
+#pragma unroll
+    for (int k = 0; k < PL; k++) {
+        qf[k] = tf[k] = 0;
+        rank[k] = lane + 32 * k;
+        if (lane + 32 * k < len) {
+            const size_t p = perm[a + lane + 32 * k];
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                v[k][d] = xyz[3 * p + d];
+                lo[d] = fmin(lo[d], v[k][d]);
+                hi[d] = fmax(hi[d], v[k][d]);
+            }
+            if (fin) qf[k] = fin[p];
+            tf[k] = tfin ? tfin[p] : qf[k];
+        }
+    }
+    const int tf0 = __shfl_sync(FULL, tf[0], 0), qf0 = __shfl_sync(FULL, qf[0], 0);
+    bool tmix = false, qmix = false;
+#pragma unroll
+    for (int k = 0; k < PL; k++)
+        if (lane + 32 * k < len) {
+            tmix = tmix || tf[k] != tf0;
+            qmix = qmix || qf[k] != qf0;
+        }
+    tmix = __any_sync(FULL, tmix);
+    qmix = __any_sync(FULL, qmix);
+    int runs = len > 0 ? 1 : 0;
+    if (tmix) {  // stable order by tree field, and the number of fields
+        bool first[PL];
+#pragma unroll
+        for (int k = 0; k < PL; k++) {
+            first[k] = lane + 32 * k < len;
+            rank[k] = 0;
+        }
+#pragma unroll
+        for (int m = 0; m < PL; m++)
+            for (int j = 0; j < 32; j++) {
+                const int at = 32 * m + j, other = __shfl_sync(FULL, tf[m], j);
+                if (at >= len) break;
+#pragma unroll
+                for (int k = 0; k < PL; k++) {
+                    const bool before = at < lane + 32 * k;
+                    rank[k] += other < tf[k] || (other == tf[k] && before);
+                    first[k] = first[k] && !(other == tf[k] && before);
+                }
+            }
+        runs = 0;
+#pragma unroll
+        for (int k = 0; k < PL; k++) runs += __popc(__ballot_sync(FULL, first[k]));
+    }
+#pragma unroll
+    for (int f = 16; f; f >>= 1)
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            lo[d] = fmin(lo[d], __shfl_xor_sync(FULL, lo[d], f));
+            hi[d] = fmax(hi[d], __shfl_xor_sync(FULL, hi[d], f));
+        }
+    double c[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) c[d] = 0.5 * (lo[d] + hi[d]);
+#pragma unroll
+    for (int k = 0; k < PL; k++)
+        if (lane + 32 * k < len) {
+            const size_t i = (size_t)a + rank[k];
+            out.o.x[i] = v[k][0];
+            out.o.y[i] = v[k][1];
+            out.o.z[i] = v[k][2];
+            out.o.qf[i] = qf[k];
+            if (tfin) out.o.tf[i] = tf[k];
+            out.t4[i] = make_float4(-2.0f * (float)(v[k][0] - c[0]), -2.0f * (float)(v[k][1] - c[1]),
+                                    -2.0f * (float)(v[k][2] - c[2]), 0.0f);
+        }
+    if (lane == 0) {
+        const size_t h = (size_t)nleaves + w;
+        double hx[3];
         kd_leaf l;
-        l.c[0] = cx, l.c[1] = cy, l.c[2] = cz;
-        l.h[0] = __double2float_ru(hx), l.h[1] = __double2float_ru(hy), l.h[2] = __double2float_ru(hz);
-        l.pad_[0] = l.pad_[1] = l.pad_[2] = 0.0f;
-        leaf[w] = l;
-        double h = sqrt(hx * hx + hy * hy + hz * hz);
-        atomicMax(hdiag, (unsigned long long)__double_as_longlong(h));
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            out.sm.box[6 * h + d] = lo[d];
+            out.sm.box[6 * h + 3 + d] = hi[d];
+            hx[d] = fmax(hi[d] - c[d], c[d] - lo[d]);
+            l.c[d] = c[d];
+            l.h[d] = __double2float_ru(hx[d]);
+            l.pad_[d] = 0.0f;
+        }
+        out.leaf[w] = l;
+        out.sm.count[h] = len > 0 ? len : 0;
+        out.sm.tf[h] = tmix ? -1 : tf0;
+        out.qf[w] = qmix ? -1 : qf0;
+        out.nruns[w] = runs;
+        if (len > 0)
+            atomicMax(out.hdiag, (unsigned long long)__double_as_longlong(
+                                     sqrt(hx[0] * hx[0] + hx[1] * hx[1] + hx[2] * hx[2])));
     }
-    for (int i = leaf_r[w] + lane; i < leaf_r[w + 1]; i += 32)
-        t4[i] = make_float4(-2.0f * (float)(o.x[i] - cx), -2.0f * (float)(o.y[i] - cy),
-                            -2.0f * (float)(o.z[i] - cz), 0.0f);
 }
 
-__global__ void k_internal_summary(int lo_h, int hi_h, Summ sm)
+// one warp per leaf: its runs, one per tree field
+__global__ void __launch_bounds__(TPB) k_leaf_runs(int nleaves, const int *__restrict__ pos,
+                                                   const int *__restrict__ tf,
+                                                   const int *__restrict__ leaf_run, int *run_start,
+                                                   int *run_len, int *run_tf)
 {
-    int h = lo_h + blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= hi_h) return;
-    int a = 2 * h, b = 2 * h + 1;
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (w >= nleaves) return;
+    const int a = pos[w], len = pos[w + 1] - a;
+    constexpr int PL = KD_RUN_MAX / 32;
+    unsigned long long all = 0;
+    int f[PL];
+#pragma unroll
+    for (int k = 0; k < PL; k++) {
+        const int i = lane + 32 * k;
+        bool hd = false;
+        f[k] = 0;
+        if (i < len) {
+            f[k] = tf[a + i];
+            hd = i == 0 || f[k] != tf[a + i - 1];
+        }
+        all |= (unsigned long long)__ballot_sync(0xffffffffu, hd) << (32 * k);
+    }
+#pragma unroll
+    for (int k = 0; k < PL; k++) {
+        const int i = lane + 32 * k;
+        if (!((all >> i) & 1)) continue;
+        const int r = leaf_run[w] + __popcll(all & ((1ull << i) - 1));
+        const unsigned long long later = i < 63 ? all >> (i + 1) : 0;
+        run_start[r] = a + i;
+        run_len[r] = later ? __ffsll((long long)later) : len - i;
+        run_tf[r] = f[k];
+    }
+}
+
+// Summaries of the levels [max(0, d0 - 8), d0), one CTA per subtree of the
+// lowest of them.  Empty leaves (at the end) leave their parent to its sibling.
+__global__ void __launch_bounds__(TPB) k_internal_summary(int d0, Summ sm)
+{
+    const int top = max(0, d0 - 8);
+    static_assert(TPB >= 128, "a thread per node of the first level");
+    for (int d = d0 - 1; d >= top; d--) {
+        const int cnt = 1 << (d - top);
+        if ((int)threadIdx.x < cnt) {
+            const size_t h = ((size_t)1 << d) + (size_t)blockIdx.x * cnt + threadIdx.x, a = 2 * h, b = 2 * h + 1;
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                sm.box[6 * h + k] = fmin(sm.box[6 * a + k], sm.box[6 * b + k]);
+                sm.box[6 * h + 3 + k] = fmax(sm.box[6 * a + 3 + k], sm.box[6 * b + 3 + k]);
+            }
+            const int nb = sm.count[b];
+            sm.count[h] = sm.count[a] + nb;
+            sm.tf[h] = nb == 0 || sm.tf[a] == sm.tf[b] ? sm.tf[a] : (sm.count[a] == 0 ? sm.tf[b] : -1);
+        }
+        __syncthreads();
+    }
+}
+
+// query blocks of a tree: kBlockLeaves leaves each, where they hold a point
+__global__ void k_tree_blocks(int groups, int nleaves, const int *__restrict__ pos,
+                              const int *__restrict__ off, const double *__restrict__ box,
+                              const int *__restrict__ leaf_qf, int *bstart, int *blen, double *bbox, int *bqf)
+{
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= groups) return;
+    const int l0 = kBlockLeaves * p, l1 = min(nleaves, l0 + kBlockLeaves);
+    const int start = pos[l0], len = pos[l1] - start, b = off[p];
+    if (len <= 0) return;
+    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    int q = leaf_qf[l0];
+    for (int l = l0; l < l1 && pos[l] < pos[l + 1]; l++) {
+        const double *x = box + 6 * ((size_t)nleaves + l);
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            lo[d] = fmin(lo[d], x[d]);
+            hi[d] = fmax(hi[d], x[3 + d]);
+        }
+        if (leaf_qf[l] != q) q = -1;
+    }
+#pragma unroll
     for (int d = 0; d < 3; d++) {
-        sm.box[6 * (size_t)h + d] = fmin(sm.box[6 * (size_t)a + d], sm.box[6 * (size_t)b + d]);
-        sm.box[6 * (size_t)h + 3 + d] =
-            fmax(sm.box[6 * (size_t)a + 3 + d], sm.box[6 * (size_t)b + 3 + d]);
+        bbox[6 * (size_t)b + d] = lo[d];
+        bbox[6 * (size_t)b + 3 + d] = hi[d];
     }
-    sm.count[h] = sm.count[a] + sm.count[b];
-    sm.tf[h] = (sm.tf[a] >= 0 && sm.tf[a] == sm.tf[b]) ? sm.tf[a] : -1;
-    sm.qf[h] = (sm.qf[a] >= 0 && sm.qf[a] == sm.qf[b]) ? sm.qf[a] : -1;
+    bstart[b] = start;
+    blen[b] = len;
+    bqf[b] = q;
 }
 
-// query blocks: each depth-DB subtree's raw range split into equal parts of
-// at most KD_BLOCK_MAX points
-__global__ void k_block_count(int nb_nodes, int span, const int *__restrict__ leaf_r, int *nblk)
+// tree field of every input point: its coordinates' first occurrence's
+__global__ void k_tree_fields(int n, const int *__restrict__ p, const int *__restrict__ cls,
+                              const int *__restrict__ ufield, int *tf)
 {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nb_nodes) return;
-    int len = leaf_r[(k + 1) * span] - leaf_r[k * span];
-    nblk[k] = (len + KD_BLOCK_MAX - 1) / KD_BLOCK_MAX;
-}
-
-__global__ void k_block_fill(int nb_nodes, int span, const int *__restrict__ leaf_r,
-                             const int *__restrict__ nblk, const int *__restrict__ boff,
-                             int *bstart, int *blen)
-{
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nb_nodes) return;
-    int a = leaf_r[k * span], len = leaf_r[(k + 1) * span] - a;
-    int nb = nblk[k];
-    for (int j = 0; j < nb; j++) {
-        int s = a + (int)((long long)len * j / nb), e = a + (int)((long long)len * (j + 1) / nb);
-        bstart[boff[k] + j] = s;
-        blen[boff[k] + j] = e - s;
-    }
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        tf[p[i]] = ufield[cls[i] - 1];
 }
 
 // one CTA of KD_BLOCK_MAX threads per query block: box and single own field
@@ -1635,13 +1933,6 @@ static void incl_sum(Pool &pool, cudaStream_t s, const T *in, T *out, int n)
 {
     char *tmp = pool.alloc<char>(sort::scan_temp_bytes<T>(n));
     check(sort::scan<T, sort::SumOp, true>(tmp, in, out, n, sort::SumOp(), s), "scan");
-}
-
-template <class T>
-static void incl_max(Pool &pool, cudaStream_t s, const T *in, T *out, int n)
-{
-    char *tmp = pool.alloc<char>(sort::scan_temp_bytes<T>(n));
-    check(sort::scan<T, sort::MaxOp, true>(tmp, in, out, n, sort::MaxOp(), s), "max scan");
 }
 
 static int bit_hi(unsigned long long v) { return v ? 64 - __builtin_clzll(v) : 0; }
@@ -1733,6 +2024,76 @@ struct CoordSort {
     }
 };
 
+// Points in counting order, in two halves: launch() queues the order along the
+// curve, and finish(), given the flag that it left (read by the caller, after
+// its next synchronisation), settles cells of more points than a chunk puts in
+// order: by all 63 bits, and where one point in eight is still in such a cell
+// (an outlier far away, an infinite coordinate, detail below 2^-21 of the
+// extent) along the curve through the ranks of the coordinates, which follows
+// the points at any scale but takes three more sorts (a whole call with 5M
+// points: 11.7 ms instead of 7.3).  Then it puts the chunks in order.
+struct Curve {
+    Pool &pool;
+    cudaStream_t s;
+    const double *xyz;
+    int n;
+    int *full;  // device, zeroed here
+    const KeySpan *span;
+    int *iota = nullptr, *perm = nullptr, *tmp = nullptr;
+
+    void launch(const int *fin, FieldInfo *fi)
+    {
+        if (!iota) iota = pool.alloc<int>(n);
+        perm = pool.alloc<int>(n);
+        tmp = pool.alloc<int>(n);
+        unsigned *key32 = pool.alloc<unsigned>(n), *srt = pool.alloc<unsigned>(n);
+        check(cudaMemsetAsync(full, 0, sizeof *full, s), "memset");
+        k_curve<<<grid_for(n), TPB, 0, s>>>(xyz, fin, n, span, nullptr, key32, iota, fi);
+        KD_LAUNCH_CHECK("k_curve");
+        sort_pairs(pool, s, (const unsigned *)key32, srt, (const int *)iota, tmp, n, 0, 32);
+        k_full_cells<<<grid_for(n), TPB, 0, s>>>((const unsigned *)srt, tmp, xyz, n, full);
+        KD_LAUNCH_CHECK("k_full_cells");
+    }
+    void finish(int nfull)
+    {
+        if (nfull) exact(nfull);
+        check(cudaFuncSetAttribute(k_refine, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)sizeof(RefineSmem)), "smem attribute");
+        k_refine<<<blocks_for(n, kChunk), kRefThreads, sizeof(RefineSmem), s>>>(n, xyz, Cells{nullptr, 0, 0},
+                                                                                tmp, perm);
+        KD_LAUNCH_CHECK("k_refine");
+    }
+    void exact(int nfull)
+    {
+        uint64_t *key = pool.alloc<uint64_t>(n), *srt = pool.alloc<uint64_t>(n);
+        k_curve<<<grid_for(n), TPB, 0, s>>>(xyz, nullptr, n, span, key, nullptr, iota, nullptr);
+        sort_pairs(pool, s, (const uint64_t *)key, srt, (const int *)iota, tmp, n, 0, 63);
+        check(cudaMemsetAsync(full, 0, sizeof *full, s), "memset");
+        k_full_cells<<<grid_for(n), TPB, 0, s>>>((const uint64_t *)srt, tmp, xyz, n, full);
+        KD_LAUNCH_CHECK("k_full_cells");
+        if (read1(full, s) <= n / 8) return;
+        uint64_t *k[3];
+        int *rank[3], *head = pool.alloc<int>(n), *cls = pool.alloc<int>(n), *err = pool.alloc<int>(1);
+        KeySpan *sp = pool.alloc<KeySpan>(1);
+        for (int d = 0; d < 3; d++) {
+            k[d] = pool.alloc<uint64_t>(n);
+            rank[d] = pool.alloc<int>(n);
+        }
+        check(cudaMemsetAsync(err, 0, sizeof(int), s), "memset");
+        check(cudaMemsetAsync(sp, 0, sizeof *sp, s), "memset");
+        k_prep<true><<<grid_for(n), TPB, 0, s>>>(xyz, n, k[0], k[1], k[2], iota, err, sp);
+        for (int d = 0; d < 3; d++) {
+            sort_pairs(pool, s, (const uint64_t *)k[d], srt, (const int *)iota, tmp, n, 0, 64);
+            k_value_heads<<<grid_for(n), TPB, 0, s>>>(k[d], tmp, n, head);
+            incl_sum(pool, s, head, cls, n);
+            k_scatter_rank<<<grid_for(n), TPB, 0, s>>>(cls, tmp, n, rank[d]);
+        }
+        k_curve_ranks<<<grid_for(n), TPB, 0, s>>>(rank[0], rank[1], rank[2], n, key);
+        KD_LAUNCH_CHECK("k_curve_ranks");
+        sort_pairs(pool, s, (const uint64_t *)key, srt, (const int *)iota, tmp, n, 0, 63);
+    }
+};
+
 static void copy_to_pageable(void *dst, const void *src, size_t bytes);
 static void copy_from_host(void *dst, const void *src, size_t bytes, cudaStream_t s);
 
@@ -1813,7 +2174,7 @@ struct NodeCopy {
 };
 
 static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_fields,
-                       int query_only, kd_node_sink *sink, int deferred, kd_catalog *cat)
+                       kd_node_sink *sink, int deferred, kd_catalog *cat)
 {
     init_device();
     Stream st;
@@ -1912,7 +2273,7 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
     FieldInfo *fi = pool.alloc<FieldInfo>(1);
     FieldInfo fi0 = {0x7fffffff, -0x7fffffff, 0, 0};
     check(cudaMemcpyAsync(fi, &fi0, sizeof fi0, cudaMemcpyHostToDevice, s), "H2D");
-    k_weights<<<grid_for(std::max(n, n_u)), TPB, 0, s>>>(u, n_u, p3, cls, fin, n, query_only, err, fi);
+    k_weights<<<grid_for(std::max(n, n_u)), TPB, 0, s>>>(u, n_u, p3, cls, fin, n, err, fi);
     KD_LAUNCH_CHECK("k_weights");
     FieldInfo hfi;
     check(cudaMemcpyAsync(&hfi, fi, sizeof hfi, cudaMemcpyDeviceToHost, s), "D2H");
@@ -1963,13 +2324,9 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
     }
     TreeOut to;
     to.memsize = memsize;
-    to.nodes = sink ? keep.alloc_from<NodeRec>(side_pool(kPoolNodes), memsize) : keep.alloc<NodeRec>(memsize);
-    to.npoint = pool.alloc<int>(memsize);
-    to.ndim = pool.alloc<unsigned char>(memsize);
-    to.inorder_u = pool.alloc<int>(n_u);
+    to.nodes = keep.alloc_from<NodeRec>(side_pool(kPoolNodes), memsize);
+    to.inorder_rep = keep.alloc<int>(n_u);
     check(cudaMemsetAsync(to.nodes, 0, sizeof(NodeRec) * (size_t)memsize, s), "memset");
-    check(cudaMemsetAsync(to.npoint, 0xff, sizeof(int) * (size_t)memsize, s), "memset");
-    check(cudaMemsetAsync(to.ndim, 0, (size_t)memsize, s), "memset");
 
     int cap = n_u / 2 + 16;
     Segs sg[2];
@@ -2015,7 +2372,7 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
     size_t node_queued = sizeof(NodeRec);  // slot 0 is never written: it stays zero
     // queue the node slots [node_queued, upto) once the stream reaches here
     auto queue_nodes = [&](size_t upto) {
-        if (!sink || upto <= node_queued) return;
+        if (upto <= node_queued) return;
         cudaEvent_t ev = nullptr;
         check(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "cudaEventCreate");
         nc.events.push_back(ev);
@@ -2139,151 +2496,117 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
     // the counting layout is built
     queue_nodes(node_bytes);
     nc.close();
-    if (sink && !nc.th.joinable()) {  // no copier thread: copy here
+    if (!nc.th.joinable()) {  // no copier thread: copy here
         for (auto &it : nc.items) {
             check(cudaEventSynchronize(it.ev), "node copy wait");
             copy_to_pageable((char *)nc.host + it.off, (const char *)to.nodes + it.off, it.len);
         }
     }
-    int *inorder_rep = keep.alloc<int>(n_u);
-    k_inorder_rep<<<grid_for(n_u), TPB, 0, s>>>(n_u, to.inorder_u, u.urep, inorder_rep);
-    check(cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, s), "D2H");
-    st.sync();
-    if (herr) raise(herr, "tree build exceeded an internal bound");
-
-    check(cudaEventRecord(ph[4], s), "event");
     // ---- counting layout
-    int D = 0;
-    while ((long long)KD_LEAF_TARGET << D < (long long)n_u) D++;
-    if (D > 24) raise(KD_EINVAL, "tree too large for the counting layout (more than 2^29 points)");
-    int nleaves = 1 << D;
-    int *extra_cnt = pool.alloc<int>(nleaves);
-    check(cudaMemsetAsync(extra_cnt, 0, sizeof(int) * (size_t)nleaves, s), "memset");
-    int nanc = nleaves - 1;
-    int *anc_leaf = pool.alloc<int>(std::max(nanc, 1)), *anc_id = pool.alloc<int>(std::max(nanc, 1));
-    int *sleaf = pool.alloc<int>(std::max(nanc, 1)), *sanc = pool.alloc<int>(std::max(nanc, 1));
-    int *extra_start = pool.alloc<int>(nleaves);
-    if (nanc > 0) {
-        k_anc_leaf<<<blocks_for(nanc, TPB), TPB, 0, s>>>(nleaves, to.npoint, to.ndim, u, anc_leaf,
-                                                          extra_cnt);
-        // ancestor ids 1..nanc in order; a stable sort by leaf keeps that order
-        k_gather<int><<<grid_for(nanc), TPB, 0, s>>>(iota + 1, iota, nanc, anc_id);
-        sort_pairs(pool, s, (const int *)anc_leaf, sleaf, (const int *)anc_id, sanc, nanc, 0,
-                   std::max(1, D));
-        excl_sum(pool, s, extra_cnt, extra_start, nleaves);
+    check(cudaEventRecord(ph[4], s), "event");
+    Cells cells = {nullptr, 0, 0};
+    // (points above the cells, one per cell on average, and duplicates join them)
+    while ((n >> cells.bits) > kChunk - 128 && (n_u >> cells.bits) >= 128) cells.bits++;
+    int *start = pool.alloc<int>(((size_t)1 << cells.bits) + 1), *perm = pool.alloc<int>(n);
+    const int *order = p3;
+    cells.start = start;
+    int *flags = pool.alloc<int>(2), hflags[2];  // largest cell, error
+    check(cudaMemsetAsync(flags, 0, sizeof(int), s), "memset");
+    if (cells.bits) {
+        int *cell = pool.alloc<int>(n), *ord = pool.alloc<int>(n);
+        unsigned *key = pool.alloc<unsigned>(n), *skey = pool.alloc<unsigned>(n);
+        k_cell_of<<<grid_for(n_u), TPB, 0, s>>>(n_u, cells.bits, to.nodes, to.inorder_rep, cell);
+        k_cell_keys<<<grid_for(n), TPB, 0, s>>>(n, p3, cls, u.urep, cell, key);
+        sort_pairs(pool, s, (const unsigned *)key, skey, (const int *)p3, ord, n, 0, cells.bits);
+        k_cell_starts<<<grid_for(n), TPB, 0, s>>>(n, 1 << cells.bits, skey, start);
+        order = ord;
+    } else {
+        k_cell_starts<<<1, 32, 0, s>>>(n, 1, nullptr, start);
     }
-    int *ucount = pool.alloc<int>(nleaves + 1), *ustart = pool.alloc<int>(nleaves + 1);
-    k_leaf_ucount<<<blocks_for(nleaves, TPB), TPB, 0, s>>>(n_u, D, nleaves,
-                                                           nanc > 0 ? extra_cnt : nullptr, ucount);
-    check(cudaMemsetAsync(ucount + nleaves, 0, sizeof(int), s), "memset");
-    excl_sum(pool, s, ucount, ustart, nleaves + 1);
-    int *cpos = pool.alloc<int>(n_u);
-    k_cpos_sub<<<blocks_for(nleaves, TPB), TPB, 0, s>>>(n_u, D, nleaves, ustart, to.inorder_u,
-                                                        cpos);
-    if (nanc > 0)
-        k_cpos_extra<<<blocks_for(nanc, TPB), TPB, 0, s>>>(nanc, n_u, D, nleaves, sleaf, sanc,
-                                                           extra_start, ustart, to.npoint, cpos);
-    int *wc = pool.alloc<int>(n_u + 1), *rstart = pool.alloc<int>(n_u + 1);
-    k_scatter_w<<<grid_for(n_u), TPB, 0, s>>>(n_u, cpos, u.uw, wc);
-    check(cudaMemsetAsync(wc + n_u, 0, sizeof(int), s), "memset");
-    excl_sum(pool, s, wc, rstart, n_u + 1);
+    k_cell_max<<<grid_for(1 << cells.bits), TPB, 0, s>>>(1 << cells.bits, start, flags);
+    KD_LAUNCH_CHECK("cell kernels");
+    check(cudaMemcpyAsync(flags + 1, err, sizeof(int), cudaMemcpyDeviceToDevice, s), "copy");
+    check(cudaMemcpyAsync(hflags, flags, sizeof hflags, cudaMemcpyDeviceToHost, s), "D2H");
+    st.sync();
+    if (hflags[1]) raise(hflags[1], "tree build exceeded an internal bound");
+    if (hflags[0] <= 4 * kChunk) {
+        while (KD_RUN_MAX << cells.leaf_bits < hflags[0]) cells.leaf_bits++;
+        check(cudaFuncSetAttribute(k_refine, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)sizeof(RefineSmem)), "smem attribute");
+        const int per = std::max(1, (KD_RUN_MAX << cells.leaf_bits) / kChunk);
+        k_refine<<<per << cells.bits, kRefThreads, sizeof(RefineSmem), s>>>(n, xyz, cells, order, perm);
+        KD_LAUNCH_CHECK("k_refine");
+    } else {
+        // points repeated so often that the tree's cells are very uneven: every
+        // cell would own the largest one's leaves.  Even ones, along the curve.
+        Curve cv{pool, s, xyz, n, flags, dks, iota};
+        cv.launch(nullptr, nullptr);
+        cv.finish(read1(flags, s));
+        perm = cv.perm;
+        cells.bits = 0;
+        while (((long long)kChunk << cells.bits) < n) cells.bits++;
+        while (KD_RUN_MAX << cells.leaf_bits < kChunk) cells.leaf_bits++;
+        start = pool.alloc<int>(((size_t)1 << cells.bits) + 1);
+        k_even_cells<<<blocks_for((1ll << cells.bits) + 1, TPB), TPB, 0, s>>>(n, 1 << cells.bits, start);
+        KD_LAUNCH_CHECK("k_even_cells");
+        cells.start = start;
+    }
 
-    int split = hfi.split ? 1 : 0;
-    RawOut ro;
+    const int split = hfi.split ? 1 : 0;
+    int *tfin = nullptr;
+    if (split) {
+        tfin = pool.alloc<int>(n);
+        k_tree_fields<<<grid_for(n), TPB, 0, s>>>(n, p3, cls, u.ufield, tfin);
+    }
+    const int D = cells.bits + cells.leaf_bits, nleaves = 1 << D;
+    const int groups = std::max(1, nleaves / kBlockLeaves);
+    LeafOut lf;
+    RawOut &ro = lf.o;
+    Summ &sm = lf.sm;
     ro.x = keep.alloc<double>(n);
     ro.y = keep.alloc<double>(n);
     ro.z = keep.alloc<double>(n);
     ro.qf = keep.alloc<int>(n);
     ro.tf = split ? keep.alloc<int>(n) : ro.qf;
-    k_raw_scatter<<<grid_for(n), TPB, 0, s>>>(n, p3, cls, u.uhead, cpos, rstart, xyz, fin,
-                                              u.ufield, ro, split);
-    int *leaf_r = keep.alloc<int>(nleaves + 1);
-    k_leaf_rstart<<<blocks_for(nleaves + 1, TPB), TPB, 0, s>>>(nleaves, ustart, rstart, leaf_r);
+    sm.box = keep.alloc<double>(6 * 2 * (size_t)nleaves);
+    sm.count = keep.alloc<int>(2 * (size_t)nleaves);
+    sm.tf = keep.alloc<int>(2 * (size_t)nleaves);
+    lf.qf = pool.alloc<int>(nleaves);
+    lf.leaf = keep.alloc<kd_leaf>(nleaves);
+    lf.t4 = keep.alloc<float4>(n);
+    lf.pos = keep.alloc<int>((size_t)nleaves + 1);
+    lf.nruns = pool.alloc<int>((size_t)nleaves + 1);
+    lf.blocks = pool.alloc<int>((size_t)groups + 1);
+    lf.hdiag = pool.alloc<unsigned long long>(1);
+    check(cudaMemsetAsync(lf.hdiag, 0, sizeof(unsigned long long), s), "memset");
+    const unsigned gl = blocks_for(32 * ((long long)nleaves + 1), TPB);
+    k_leaves<<<gl, TPB, 0, s>>>(n, nleaves, cells, perm, xyz, fin, tfin, lf);
+    for (int d = D; d > 0; d = std::max(0, d - 8))
+        k_internal_summary<<<1u << std::max(0, d - 8), TPB, 0, s>>>(d, sm);
+    int *leaf_run = keep.alloc<int>((size_t)nleaves + 1);
+    excl_sum(pool, s, lf.nruns, leaf_run, nleaves + 1);
+    int *boff = pool.alloc<int>((size_t)groups + 1);
+    excl_sum(pool, s, lf.blocks, boff, groups + 1);
     KD_LAUNCH_CHECK("layout kernels");
-
-    // group each leaf's points by tree field (stable), then cut runs
-    unsigned *key = pool.alloc<unsigned>(n), *key2 = pool.alloc<unsigned>(n);
-    int *unsorted = pool.alloc<int>(1);
-    check(cudaMemsetAsync(unsorted, 0, sizeof(int), s), "memset");
-    k_leaf_keys<<<nleaves, 64, 0, s>>>(nleaves, leaf_r, ro.tf, key, unsorted);
-    if (read1(unsorted, s)) {
-        int *perm = pool.alloc<int>(n);
-        sort_pairs(pool, s, (const unsigned *)key, key2, (const int *)iota, perm, n, 0, D + 8);
-        std::swap(key, key2);
-        double *tmpd = pool.alloc<double>(n);
-        int *tmpi = pool.alloc<int>(n);
-        double *dd[3] = {ro.x, ro.y, ro.z};
-        for (int d = 0; d < 3; d++) {
-            k_gather<double><<<grid_for(n), TPB, 0, s>>>(dd[d], perm, n, tmpd);
-            check(cudaMemcpyAsync(dd[d], tmpd, sizeof(double) * (size_t)n,
-                                  cudaMemcpyDeviceToDevice, s), "copy");
-        }
-        int *ii[2] = {ro.qf, ro.tf};
-        for (int k = 0; k < (split ? 2 : 1); k++) {
-            k_gather<int><<<grid_for(n), TPB, 0, s>>>(ii[k], perm, n, tmpi);
-            check(cudaMemcpyAsync(ii[k], tmpi, sizeof(int) * (size_t)n, cudaMemcpyDeviceToDevice,
-                                  s), "copy");
-        }
-    }
-    int *rhead = pool.alloc<int>(n), *rid = pool.alloc<int>(n);
-    {
-        int *gh = pool.alloc<int>(n), *gs = pool.alloc<int>(n);
-        k_group_heads<<<grid_for(n), TPB, 0, s>>>(n, key, gh);
-        incl_max(pool, s, (const int *)gh, gs, n);
-        k_run_heads<<<grid_for(n), TPB, 0, s>>>(n, gs, rhead);
-    }
-    incl_sum(pool, s, rhead, rid, n);
-    int nruns = read1(rid + (n - 1), s);
+    double leaf_hdiag;
+    int nblocks;
+    check(cudaMemcpyAsync(&leaf_hdiag, lf.hdiag, sizeof(double), cudaMemcpyDeviceToHost, s), "D2H");
+    check(cudaMemcpyAsync(&nblocks, boff + groups, sizeof(int), cudaMemcpyDeviceToHost, s), "D2H");
+    const int nruns = read1(leaf_run + nleaves, s);
     int *run_start = keep.alloc<int>(nruns), *run_len = keep.alloc<int>(nruns),
-        *run_tf = keep.alloc<int>(nruns), *run_leaf = keep.alloc<int>(nruns),
-        *leaf_run = keep.alloc<int>(nleaves + 1);
-    k_runs<<<grid_for(n), TPB, 0, s>>>(n, key, rhead, rid, nleaves, run_start, run_tf, run_leaf,
-                                       leaf_run);
-    k_run_len<<<blocks_for(nruns + 1, TPB), TPB, 0, s>>>(nruns, n, nleaves, run_start, run_len,
-                                                          leaf_run);
-
-    // counting-tree summaries
-    int nnodes = 2 * nleaves;
-    Summ sm;
-    sm.box = keep.alloc<double>(6 * (size_t)nnodes);
-    sm.count = keep.alloc<int>(nnodes);
-    sm.tf = keep.alloc<int>(nnodes);
-    sm.qf = keep.alloc<int>(nnodes);
-    k_leaf_summary<<<blocks_for((long long)nleaves * 32, TPB), TPB, 0, s>>>(nleaves, leaf_r, ro,
-                                                                             sm);
-    for (int d = D - 1; d >= 0; d--)
-        k_internal_summary<<<blocks_for(1 << d, TPB), TPB, 0, s>>>(1 << d, 2 << d, sm);
-    kd_leaf *leaf = keep.alloc<kd_leaf>(nleaves);
-    float4 *t4 = keep.alloc<float4>(n);
-    unsigned long long *hdiag = pool.alloc<unsigned long long>(1);
-    check(cudaMemsetAsync(hdiag, 0, sizeof(unsigned long long), s), "memset");
-    k_leaf_rel<<<blocks_for((long long)nleaves * 32, TPB), TPB, 0, s>>>(nleaves, leaf_r, ro, sm.box,
-                                                                         leaf, t4, hdiag);
-    double leaf_hdiag = 0;
-    {
-        unsigned long long hb = read1(hdiag, s);
-        memcpy(&leaf_hdiag, &hb, sizeof leaf_hdiag);
-    }
-
-    // query blocks: each 16-leaf subtree cut into equal chunks of <= 128
-    int DB = std::max(0, D - 4);
-    int nbn = 1 << DB, span = nleaves / nbn;
-    int *nblk = pool.alloc<int>(nbn + 1), *boff = pool.alloc<int>(nbn + 1);
-    k_block_count<<<blocks_for(nbn, TPB), TPB, 0, s>>>(nbn, span, leaf_r, nblk);
-    check(cudaMemsetAsync(nblk + nbn, 0, sizeof(int), s), "memset");
-    excl_sum(pool, s, nblk, boff, nbn + 1);
-    int nblocks = read1(boff + nbn, s);
+        *run_tf = keep.alloc<int>(nruns);
     int *bstart = keep.alloc<int>(nblocks), *blen = keep.alloc<int>(nblocks),
         *bqf = keep.alloc<int>(nblocks);
     double *bbox = keep.alloc<double>(6 * (size_t)nblocks);
-    k_block_fill<<<blocks_for(nbn, TPB), TPB, 0, s>>>(nbn, span, leaf_r, nblk, boff, bstart, blen);
-    k_block_boxes<<<nblocks, KD_BLOCK_MAX, 0, s>>>(nblocks, bstart, blen, ro, bbox, bqf);
+    k_tree_blocks<<<blocks_for(groups, TPB), TPB, 0, s>>>(groups, nleaves, lf.pos, boff, sm.box, lf.qf, bstart,
+                                                          blen, bbox, bqf);
+    k_leaf_runs<<<gl, TPB, 0, s>>>(nleaves, lf.pos, ro.tf, leaf_run, run_start, run_len, run_tf);
     KD_LAUNCH_CHECK("summary kernels");
     check(cudaEventRecord(ph[5], s), "event");
     st.sync();
     kd_build_stats bs;
     memset(&bs, 0, sizeof bs);
-    if (!deferred || !sink) {
+    if (!deferred) {
         const double wait0 = wall_ms();
         if (nc.th.joinable()) nc.th.join();
         const double waited = wall_ms() - wait0;
@@ -2317,17 +2640,12 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
     cat->max_tf = hfi.max_tf;
     cat->fields_split = split;
     cat->max_abs = maxabs;
-    if (sink) {
-        // the host holds the node array; the device copy is freed with the
-        // pool, or, while a deferred copy still reads it, once that is done
-        sink->nodes = nc.host;
-        nc.handed = true;
-        nc.sink = nullptr;
-        cat->d_nodes = nullptr;
-    } else {
-        cat->d_nodes = keep.keep(to.nodes);
-    }
-    cat->d_inorder_rep = keep.keep(inorder_rep);
+    // the host holds the node array; the device copy is freed with the pool,
+    // or, while a deferred copy still reads it, once that is done
+    sink->nodes = nc.host;
+    nc.handed = true;
+    nc.sink = nullptr;
+    cat->d_inorder_rep = keep.keep(to.inorder_rep);
     cat->d_x = keep.keep(ro.x);
     cat->d_y = keep.keep(ro.y);
     cat->d_z = keep.keep(ro.z);
@@ -2338,16 +2656,14 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
     cat->d_box = keep.keep(sm.box);
     cat->d_ncount = keep.keep(sm.count);
     cat->d_ntf = keep.keep(sm.tf);
-    cat->d_nqf = keep.keep(sm.qf);
     cat->d_leaf_run = keep.keep(leaf_run);
-    cat->d_leaf_pos = keep.keep(leaf_r);
+    cat->d_leaf_pos = keep.keep(lf.pos);
     cat->nruns = nruns;
     cat->d_run_start = keep.keep(run_start);
     cat->d_run_len = keep.keep(run_len);
     cat->d_run_tf = keep.keep(run_tf);
-    cat->d_run_leaf = keep.keep(run_leaf);
-    cat->d_t4 = keep.keep(t4);
-    cat->d_leaf = keep.keep(leaf);
+    cat->d_t4 = keep.keep(lf.t4);
+    cat->d_leaf = keep.keep(lf.leaf);
     cat->leaf_hdiag = leaf_hdiag;
     cat->nblocks = nblocks;
     cat->d_blk_start = keep.keep(bstart);
@@ -2356,99 +2672,13 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
     cat->d_blk_box = keep.keep(bbox);
     cat->device_bytes = keep.bytes;
     cat->bstats = bs;
-    if (sink && deferred) {
+    if (deferred) {
         nc.dnodes = keep.keep(to.nodes);
         cat->pending = ncu.release();
     }
 }
 
 // ------------------------------------------------------------ query points
-
-// The bits of v (21 of them) three apart.
-__device__ __forceinline__ uint64_t spread3(uint64_t v)
-{
-    v = (v | (v << 32)) & 0x001f00000000ffffull;
-    v = (v | (v << 16)) & 0x001f0000ff0000ffull;
-    v = (v | (v << 8)) & 0x100f00f00f00f00full;
-    v = (v | (v << 4)) & 0x10c30c30c30c30c3ull;
-    return (v | (v << 2)) & 0x1249249249249249ull;
-}
-
-// Position along the Hilbert curve of 2^21 cells per side, three bits a level,
-// by the transform of Skilling (AIP Conf. Proc. 707, 381, 2004): from the
-// coarsest level down, each axis exchanges or inverts the finer bits of the
-// first one, and a Gray code orders the eight cells of a level.
-__device__ __forceinline__ uint64_t hilbert(unsigned (&c)[3])
-{
-#pragma unroll 1
-    for (unsigned bit = 1u << 20; bit > 1; bit >>= 1) {
-        const unsigned finer = bit - 1;
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            const unsigned swap = (c[d] & bit) ? 0u : (c[0] ^ c[d]) & finer;
-            c[0] ^= (c[d] & bit) ? finer : swap;
-            if (d) c[d] ^= swap;
-        }
-    }
-    c[1] ^= c[0];
-    c[2] ^= c[1];
-    unsigned flip = c[2] >> 1;  // bit b: parity of the bits of c[2] above b
-    flip ^= flip >> 1;
-    flip ^= flip >> 2;
-    flip ^= flip >> 4;
-    flip ^= flip >> 8;
-    flip ^= flip >> 16;
-    return spread3(c[0] ^ flip) << 2 | spread3(c[1] ^ flip) << 1 | spread3(c[2] ^ flip);
-}
-
-// Position of each point along the curve through the points' cube, its 32
-// highest bits, and the range of the own fields.
-__global__ void __launch_bounds__(TPB) k_curve(const double *__restrict__ xyz, const int *__restrict__ fin,
-                                               int n, const KeySpan *span, uint64_t *key, unsigned *key32,
-                                               int *iota, FieldInfo *fi)
-{
-    double lo[3], ext = 0.0;
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-        lo[d] = okey_value(~span->inv_lo[d]);
-        ext = fmax(ext, okey_value(span->hi[d]) - lo[d]);
-    }
-    const double top = 2097151.0, scale = ext > 0.0 ? top / ext : 0.0;
-    int minq = 0x7fffffff, maxq = -0x7fffffff;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        unsigned c[3];
-#pragma unroll
-        for (int d = 0; d < 3; d++)  // (NaN, from an infinite range: the last cell)
-            c[d] = __double2uint_rd(fmin((xyz[3 * (size_t)i + d] - lo[d]) * scale, top));
-        const uint64_t k = hilbert(c);
-        key[i] = k;
-        key32[i] = (unsigned)(k >> 31);
-        iota[i] = i;
-        const int qf = fin ? fin[i] : 0;
-        minq = min(minq, qf);
-        maxq = max(maxq, qf);
-    }
-    minq = __reduce_min_sync(0xffffffffu, minq);
-    maxq = __reduce_max_sync(0xffffffffu, maxq);
-    if ((threadIdx.x & 31) == 0) {
-        atomicMin(&fi->min_qf, minq);
-        atomicMax(&fi->max_qf, maxq);
-    }
-}
-
-// neighbours along the curve in one cell, but not at one place
-__global__ void k_shared_cells(const uint64_t *__restrict__ key, const int *__restrict__ perm,
-                               const double *__restrict__ xyz, int n, int *shared)
-{
-    int c = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x + 1; i < n; i += gridDim.x * blockDim.x) {
-        const size_t a = perm[i], b = perm[i - 1];
-        if (key[a] != key[b]) continue;
-        c += xyz[3 * a] != xyz[3 * b] || xyz[3 * a + 1] != xyz[3 * b + 1] || xyz[3 * a + 2] != xyz[3 * b + 2];
-    }
-    c = __reduce_add_sync(0xffffffffu, c);
-    if (c && (threadIdx.x & 31) == 0) atomicAdd(shared, c);
-}
 
 // the points in curve order, and the query blocks' ranges
 __global__ void k_query_points(const double *__restrict__ xyz, const int *__restrict__ fin,
@@ -2480,7 +2710,7 @@ __global__ void k_query_points(const double *__restrict__ xyz, const int *__rest
 // nothing kept, where the cells are too coarse for the points (one in eight
 // shares a cell with another: an outlier far away, or an infinite coordinate):
 // the tree's cuts follow the points at any scale.
-static bool build_query(const double *h_xyz, const int *h_fields, int n, int num_fields, kd_catalog *cat)
+static void build_query(const double *h_xyz, const int *h_fields, int n, int num_fields, kd_catalog *cat)
 {
     init_device();
     Stream st;
@@ -2496,34 +2726,18 @@ static bool build_query(const double *h_xyz, const int *h_fields, int n, int num
     struct State {
         KeySpan span;
         FieldInfo fi;
-        int err, too_long, shared, pad;
-    } init, *dst = pool.alloc<State>(1);
-    memset(&init, 0, sizeof init);
-    init.fi = {0x7fffffff, -0x7fffffff, 0, 0};
-    check(cudaMemcpyAsync(dst, &init, sizeof init, cudaMemcpyHostToDevice, s), "H2D");
-    k_prep<false><<<grid_for(n), TPB, 0, s>>>(xyz, n, nullptr, nullptr, nullptr, nullptr, &dst->err,
-                                              &dst->span);
-    uint64_t *key = pool.alloc<uint64_t>(n);
-    unsigned *key32 = pool.alloc<unsigned>(n), *srt = pool.alloc<unsigned>(n);
-    int *iota = pool.alloc<int>(n), *tmp = pool.alloc<int>(n), *perm = pool.alloc<int>(n);
-    k_curve<<<grid_for(n), TPB, 0, s>>>(xyz, fin, n, &dst->span, key, key32, iota, &dst->fi);
-    KD_LAUNCH_CHECK("k_curve");
-    sort_pairs(pool, s, (const unsigned *)key32, srt, (const int *)iota, tmp, n, 0, 32);
-    copy_perm(perm, tmp, n, s);
-    k_fix_runs<1><<<grid_for(n), TPB, 0, s>>>(srt, n, Keys3{{key, key, key}}, tmp, perm, &dst->too_long);
-    k_shared_cells<<<grid_for(n), TPB, 0, s>>>(key, perm, xyz, n, &dst->shared);
-    KD_LAUNCH_CHECK("k_fix_runs");
-    State h = read1(dst, s);
+        int full, err;
+    } h, *dstate = pool.alloc<State>(1);
+    memset(&h, 0, sizeof h);
+    h.fi = {0x7fffffff, -0x7fffffff, 0, 0};
+    check(cudaMemcpyAsync(dstate, &h, sizeof h, cudaMemcpyHostToDevice, s), "H2D");
+    k_prep<false><<<grid_for(n), TPB, 0, s>>>(xyz, n, nullptr, nullptr, nullptr, nullptr, &dstate->err,
+                                              &dstate->span);
+    Curve cv{pool, s, xyz, n, &dstate->full, &dstate->span};
+    cv.launch(fin, &dstate->fi);
+    h = read1(dstate, s);
     if (h.err) raise(h.err, "NaN coordinate in query points");
-    if (h.too_long) {  // (many points per 32-bit cell: all bits)
-        uint64_t *srt64 = pool.alloc<uint64_t>(n);
-        sort_pairs(pool, s, (const uint64_t *)key, srt64, (const int *)iota, perm, n, 0, 63);
-        check(cudaMemsetAsync(&dst->shared, 0, sizeof(int), s), "memset");
-        k_shared_cells<<<grid_for(n), TPB, 0, s>>>(key, perm, xyz, n, &dst->shared);
-        KD_LAUNCH_CHECK("k_shared_cells");
-        h.shared = read1(&dst->shared, s);
-    }
-    if (h.shared > n / 8) return false;
+    cv.finish(h.full);
 
     const int nblocks = (int)blocks_for(n, KD_BLOCK_MAX);
     RawOut ro;
@@ -2534,7 +2748,7 @@ static bool build_query(const double *h_xyz, const int *h_fields, int n, int num
     int *bstart = keep.alloc<int>(nblocks), *blen = keep.alloc<int>(nblocks),
         *bqf = keep.alloc<int>(nblocks);
     double *bbox = keep.alloc<double>(6 * (size_t)nblocks);
-    k_query_points<<<grid_for(n), TPB, 0, s>>>(xyz, fin, perm, n, ro, nblocks, bstart, blen);
+    k_query_points<<<grid_for(n), TPB, 0, s>>>(xyz, fin, cv.perm, n, ro, nblocks, bstart, blen);
     k_block_boxes<<<nblocks, KD_BLOCK_MAX, 0, s>>>(nblocks, bstart, blen, ro, bbox, bqf);
     KD_LAUNCH_CHECK("k_query_points");
     st.sync();
@@ -2558,21 +2772,20 @@ static bool build_query(const double *h_xyz, const int *h_fields, int n, int num
     cat->d_blk_qf = keep.keep(bqf);
     cat->d_blk_box = keep.keep(bbox);
     cat->device_bytes = keep.bytes;
-    return true;
 }
 
 }  // namespace kd
 
 static int build_entry(const double *h_xyz, const int *h_fields, int n, int num_fields,
-                       int query_only, kd_node_sink *sink, int deferred, kd_catalog *cat)
+                       kd_node_sink *sink, int deferred, kd_catalog *cat)
 {
     if (n < 1) {
         kd_set_error(KD_EINVAL, "a tree needs at least one point");
         return KD_EINVAL;
     }
     try {
-        if (!query_only || !kd::build_query(h_xyz, h_fields, n, num_fields, cat))
-            kd::build_impl(h_xyz, h_fields, n, num_fields, query_only, sink, deferred, cat);
+        if (!sink) kd::build_query(h_xyz, h_fields, n, num_fields, cat);
+        else kd::build_impl(h_xyz, h_fields, n, num_fields, sink, deferred, cat);
         return KD_OK;
     } catch (const kd::Error &e) {
         kd_set_error(e.code, "%s", e.msg);
@@ -2589,7 +2802,11 @@ static int build_entry(const double *h_xyz, const int *h_fields, int n, int num_
 extern "C" int kdg_build(const double *h_xyz, const int *h_fields, int n, int num_fields,
                          int query_only, kd_catalog *cat)
 {
-    return build_entry(h_xyz, h_fields, n, num_fields, query_only, nullptr, 0, cat);
+    if (!query_only) {
+        kd_set_error(KD_EINVAL, "kdg_build: a tree is built by kdg_build_tree");
+        return KD_EINVAL;
+    }
+    return build_entry(h_xyz, h_fields, n, num_fields, nullptr, 0, cat);
 }
 
 extern "C" int kdg_build_tree(const double *h_xyz, const int *h_fields, int n, int num_fields,
@@ -2600,7 +2817,7 @@ extern "C" int kdg_build_tree(const double *h_xyz, const int *h_fields, int n, i
         return KD_EINVAL;
     }
     sink->nodes = nullptr;
-    return build_entry(h_xyz, h_fields, n, num_fields, 0, sink, deferred, cat);
+    return build_entry(h_xyz, h_fields, n, num_fields, sink, deferred, cat);
 }
 
 // Runs a catalog operation on the catalog's device, then restores the
@@ -2886,12 +3103,11 @@ extern "C" void kdg_free(kd_catalog *cat)
         cat->pending = nullptr;
     }
     OnDevice on(cat->device);
-    void *ptrs[] = {cat->d_nodes,    cat->d_inorder_rep, cat->d_x,       cat->d_y,
+    void *ptrs[] = {cat->d_inorder_rep, cat->d_x,    cat->d_y,
                     cat->d_z,        cat->d_qf,          cat->fields_split ? cat->d_tf : nullptr,
-                    cat->d_box,      cat->d_ncount,      cat->d_ntf,     cat->d_nqf,
+                    cat->d_box,      cat->d_ncount,      cat->d_ntf,
                     cat->d_leaf_run, cat->d_leaf_pos,    cat->d_run_start, cat->d_run_len,
-                    cat->d_run_tf,
-                    cat->d_run_leaf, cat->d_t4,          cat->d_leaf,
+                    cat->d_run_tf,   cat->d_t4,          cat->d_leaf,
                     cat->d_blk_start, cat->d_blk_len,    cat->d_blk_qf,  cat->d_blk_box};
     for (void *p : ptrs)
         if (p) cudaFree(p);

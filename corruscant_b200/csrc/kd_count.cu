@@ -51,12 +51,12 @@ constexpr int kTravWarps = 4;
 // Node-pair stack per traversal warp.  A round pops the top min(sp, 32)
 // entries and pushes at most two children for each, so the stack grows by at
 // most 32 entries per tree level: at most 32 * D + 64 entries for a counting
-// tree of depth D <= 24 (832).  A push past the end stops the count with
+// tree of depth D <= 27 (928).  A push past the end stops the count with
 // KD_EINTERNAL instead of writing out of bounds.  4 KB per warp (rather
 // than 8) lets the count pass run more warps per SM: the traversal of the
 // clustered 1M / 20M batch takes 16.3 ms instead of 19.5.
 constexpr int kStack = 1024;
-static_assert(kStack >= 32 * 24 + 64, "stack bound of a depth-24 counting tree");
+static_assert(kStack >= 32 * 27 + 64, "stack bound of a depth-27 counting tree");
 constexpr int kShardChunk = 32;  // blocks per interleaved shard chunk
 
 struct TreeSide {
@@ -348,7 +348,7 @@ constexpr int kTileWarps = 4;
 constexpr int kTileThreads = 32 * kTileWarps;
 constexpr int kTilesPerSm = 7;                // CTAs per SM the registers are held to
 constexpr int kPStride = 136;                 // counters per edge (128 queries + bank shift)
-static_assert(kMTiles == 8 && KD_RUN_MAX == 64 && kTileThreads == KD_BLOCK_MAX, "lane layouts below");
+static_assert(kMTiles == 8 && kTileThreads == KD_BLOCK_MAX, "lane layouts below");
 
 // FP32 tiles only where every staged value and square stays far inside FP32
 // range: tree and query points within kFp32Span of the block centre (their

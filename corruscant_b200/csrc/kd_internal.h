@@ -6,11 +6,9 @@
  *   - the reference-exact k-d tree (node_t array, heap order, root at 1) that
  *     kdbuild.c:451-537 would produce, plus its in-order permutation;
  *   - a counting layout of the RAW input points (duplicates kept, one entry
- *     each) ordered leaf by leaf along the top D levels of that same tree, with
- *     per-node bounding boxes, raw counts and single-field summaries, split
- *     into "runs" (<= KD_RUN_MAX consecutive points of one tree-side field) and
- *     "blocks" (<= KD_BLOCK_MAX consecutive points of one 16-leaf subtree,
- *     the query side of a tile).
+ *     each) along a Hilbert curve, cut into leaves of KD_RUN_MAX points (grouped
+ *     by tree-side field into "runs") and query blocks of KD_BLOCK_MAX, under a
+ *     binary tree of bounding boxes, raw counts and single-field summaries.
  *
  * Every raw point carries two field ids: qf, its own field (what the
  * reference's query side reads, kdquery.c:67-70), and tf, the low 8 bits of
@@ -31,9 +29,8 @@
 extern "C" {
 #endif
 
-#define KD_RUN_MAX 64      /* points per tree-side run (shared-memory tile) */
+#define KD_RUN_MAX 64      /* points per leaf of the counting tree, so at most per run */
 #define KD_BLOCK_MAX 128   /* query points per block (one warp) */
-#define KD_LEAF_TARGET 64  /* unique points per counting leaf, upper bound */
 #define KD_MAX_EDGES 64    /* distinct finite squared edges per count job */
 
 /* the status codes (KD_OK, KD_EINVAL, ...) and KD_MAX_POINTS are public:
@@ -59,7 +56,7 @@ typedef struct kd_catalog {
     double max_abs;   /* largest |coordinate| */
 
     /* reference-exact tree */
-    void *d_nodes;    /* memsize node_t records (40 B), zero where empty */
+    void *d_nodes;    /* node array, where this side keeps one (a build on the device does not) */
     int *d_inorder_rep; /* n_u: input index of the point at in-order position */
 
     /* counting layout, n_raw entries each, in counting order */
@@ -73,12 +70,11 @@ typedef struct kd_catalog {
     double *d_box;    /* 6 per heap id: lo x,y,z, hi x,y,z */
     int *d_ncount;    /* raw points per heap id */
     int *d_ntf;       /* single tree field of the node, -1 when mixed */
-    int *d_nqf;       /* single own field of the node, -1 when mixed */
     int *d_leaf_run;  /* nleaves+1: first run of each leaf */
     int *d_leaf_pos;  /* nleaves+1: first raw position (counting order) of each leaf */
 
     int nruns;
-    int *d_run_start, *d_run_len, *d_run_tf, *d_run_leaf;
+    int *d_run_start, *d_run_len, *d_run_tf;
 
     /* tree side in FP32: t = fl32(point - leaf box centre), stored as
      * float4 (-2 t.x, -2 t.y, -2 t.z, 0) */
@@ -97,11 +93,11 @@ typedef struct kd_catalog {
 } kd_catalog;
 
 /* Build a catalog from host arrays (xyz interleaved (n,3), fields may be
- * NULL) to serve as the query side of counts only: a point may repeat 256 or
- * more times (only tree nodes store an 8-bit weight) and no node array is
- * returned.  With query_only the catalog may hold the query side alone (points
- * in counting order and blocks).  Returns KD_OK or a negative status; on
- * failure nothing is held. */
+ * NULL) to serve as the query side of counts only: it holds the points in
+ * counting order and the blocks, no tree (a point may repeat 256 or more
+ * times: only tree nodes store an 8-bit weight).  query_only is 1 (a tree is
+ * built by kdg_build_tree).  Returns KD_OK or a negative status; on failure
+ * nothing is held. */
 int kdg_build(const double *h_xyz, const int *h_fields, int n, int num_fields,
               int query_only, kd_catalog *cat);
 

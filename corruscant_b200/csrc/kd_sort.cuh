@@ -23,8 +23,6 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <type_traits>
-
 namespace kd {
 namespace sort {
 
@@ -36,14 +34,6 @@ struct SumOp {
     template <class T> __device__ __forceinline__ T operator()(T a, T b) const { return a + b; }
     template <class T> __host__ __device__ static T identity() { return T(0); }
 };
-struct MaxOp {
-    template <class T> __device__ __forceinline__ T operator()(T a, T b) const { return a > b ? a : b; }
-    template <class T> __host__ __device__ static T identity()
-    {
-        return std::is_signed<T>::value ? (T)((unsigned long long)1 << (8 * sizeof(T) - 1)) : T(0);
-    }
-};
-
 // Inclusive scan of one value per thread over the block (warp shuffles,
 // then the scanned warp totals in sw); *total = the block's total.  sw stays
 // valid until the next call.

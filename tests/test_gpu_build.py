@@ -113,3 +113,46 @@ def test_query_points(n, kind):
                     N.destroy(tq)
     finally:
         N.destroy(t)
+
+
+@pytest.mark.parametrize("kind", ["uniform", "sky", "scales", "outlier", "infinite", "lattice", "copies",
+                                  "uneven"])
+@pytest.mark.parametrize("n", [63, 65, 129, 1920, 1921, 2049, 3841, 6000, 9001])
+def test_counting_order(n, kind):
+    """Trees of one and of several cells, with cells made uneven by copies up
+    to the number at which they are no longer the tree's own, against the
+    oracle's exhaustive counts: crossed, and symmetric where no point has
+    copies of other fields."""
+    rs = np.random.RandomState(n)
+    if kind == "sky":
+        p = rs.randn(n, 3)
+        p /= np.sqrt((p * p).sum(1))[:, None]
+    elif kind == "lattice":
+        p = rs.randint(0, 12, (n, 3)) / 12.0
+    elif kind == "copies":  # 250 of each
+        p = np.repeat(rs.rand((n + 249) // 250, 3), 250, axis=0)[:n]
+    elif kind == "uneven":  # 100 of the points in one corner, as many as fit
+        p = rs.rand(n, 3)
+        k = min(100, n // 50)
+        p[: 40 * k] = np.repeat(0.05 * rs.rand(k, 3), 40, axis=0)
+    else:
+        p = _wide(kind, n, rs)
+    p = p[rs.permutation(n)]
+    radii = np.array([0.02, 0.1, 0.3, 0.9])
+    fields = np.minimum((np.abs(p[:, 0]) * 3), 2).astype(np.int32)
+    mixed = rs.randint(0, 3, n).astype(np.int32)
+    for f in (fields, mixed):
+        t = N.build_tree(p, f, 3)
+        try:
+            want = O.OracleTree(p, f, 3).brute_counts(p, f, 3, radii, nthreads=4)
+            for mode in (N.KD_MODE_MIXED, N.KD_MODE_FP64):
+                assert np.array_equal(N.count_radii(t, t, radii, mode=mode), want), mode
+            pq, fq = np.ascontiguousarray(p[::2]), np.ascontiguousarray(f[::2])
+            q = N.build_tree(pq, fq, 3)
+            try:
+                want = O.OracleTree(p, f, 3).brute_counts(pq, fq, 3, radii, nthreads=4)
+                assert np.array_equal(N.count_radii(t, q, radii), want)
+            finally:
+                N.destroy(q)
+        finally:
+            N.destroy(t)
