@@ -94,7 +94,7 @@ static double now_ms(void)
 static void *alloc_nodes(size_t nb)
 {
     void *mem = NULL;
-    if (nb >= ((size_t)64 << 20)) {
+    if (nb >= ((size_t)8 << 20)) {
         if (posix_memalign(&mem, (size_t)2 << 20, nb) != 0) mem = NULL;
         if (mem) madvise(mem, nb, MADV_HUGEPAGE);
     } else {

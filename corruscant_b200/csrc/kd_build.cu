@@ -48,6 +48,10 @@
 #include <thread>
 #include <vector>
 
+#if defined(__x86_64__)
+#include <immintrin.h>
+#endif
+
 #include "kd_cuda_util.cuh"
 #include "kd_sort.cuh"
 
@@ -2094,16 +2098,172 @@ struct Curve {
     }
 };
 
-static void copy_to_pageable(void *dst, const void *src, size_t bytes);
+// Device -> pageable host copy of the node array returned by tree_construct
+// (1.3 GB at 20M points), one queued item at a time.  A plain cudaMemcpy into
+// pageable memory goes through the driver's own staging, one copy at a time
+// for the whole process, and at the speed of the page faults of its one
+// copying thread; it also makes every other pageable transfer of the process
+// (the build's own small reads of device scalars) queue behind it.  Here the
+// data goes through two pinned staging chunks (the next chunk's DMA overlaps
+// the current one's host copy) and each chunk is copied into the destination
+// by several threads, which take the destination's first-touch page faults in
+// parallel.
+namespace {
+struct Staging {
+    static constexpr size_t kChunk = size_t(32) << 20;
+    void *pin[2] = {nullptr, nullptr};
+};
+// pinned staging pairs kept for the life of the process (allocating pinned
+// memory per copy costs more than the copy): one per copy running at once,
+// at most kMaxStaging (a batch of many small deferred builds would otherwise
+// pin 64 MB per build); a copy that finds them all in use waits for one
+constexpr int kMaxStaging = 4;
+std::mutex g_stage_mu;
+std::condition_variable g_stage_cv;
+std::vector<Staging *> g_stage_free;
+int g_stage_made = 0;
+struct StagingLease {
+    Staging *st = nullptr;
+    StagingLease()
+    {
+        {
+            std::unique_lock<std::mutex> g(g_stage_mu);
+            g_stage_cv.wait(g, [] { return !g_stage_free.empty() || g_stage_made < kMaxStaging; });
+            if (!g_stage_free.empty()) {
+                st = g_stage_free.back();
+                g_stage_free.pop_back();
+                return;
+            }
+            g_stage_made++;  // this thread makes the next pair
+        }
+        std::unique_ptr<Staging> n(new Staging);
+        for (int i = 0; i < 2; i++)
+            if (cudaHostAlloc(&n->pin[i], Staging::kChunk, cudaHostAllocPortable) != cudaSuccess) {
+                cudaGetLastError();
+                for (int j = 0; j < i; j++) cudaFreeHost(n->pin[j]);
+                {
+                    std::lock_guard<std::mutex> g(g_stage_mu);
+                    g_stage_made--;
+                }
+                g_stage_cv.notify_one();
+                raise(KD_ENOMEM, "out of pinned host memory for the node array copy");
+            }
+        st = n.release();
+    }
+    ~StagingLease()
+    {
+        {
+            std::lock_guard<std::mutex> g(g_stage_mu);
+            g_stage_free.push_back(st);
+        }
+        g_stage_cv.notify_one();
+    }
+};
+// Host copies of a transfer's chunks fanned out over a pool of threads made
+// once for the whole transfer (a 32 MB chunk takes ~1 ms; creating threads
+// per chunk would cost a good part of that).  Transfers under 4 MB are
+// copied by the calling thread alone.
+// Copy to or from a staging chunk without leaving its lines in this core's
+// cache: a DMA that meets lines of a core gone idle runs at 6 GB/s instead of
+// 50.  The chunk's side is aligned to 64 bytes.
+static void copy_uncached(char *d, const char *f, size_t n, bool to_staging)
+{
+    size_t i = 0;
+#if defined(__x86_64__)
+    for (; i + 64 <= n; i += 64) {
+        __m128i v[4];
+        if (!to_staging) _mm_prefetch(f + i + 1024, _MM_HINT_NTA);
+        for (int k = 0; k < 4; k++) v[k] = _mm_loadu_si128((const __m128i *)(f + i) + k);
+        for (int k = 0; k < 4; k++)
+            if (to_staging) _mm_stream_si128((__m128i *)(d + i) + k, v[k]);
+            else _mm_storeu_si128((__m128i *)(d + i) + k, v[k]);
+    }
+    if (to_staging) _mm_sfence();
+#endif
+    std::memcpy(d + i, f + i, n - i);
+}
+struct FanOut {
+    int nthr = 1;
+    std::vector<std::thread> th;
+    std::mutex mu;
+    std::condition_variable go, done;
+    size_t gen = 0;
+    int pending = 0;
+    bool stop = false;
+    char *to = nullptr;
+    const char *from = nullptr;
+    size_t len = 0;
+    bool to_staging;
+    explicit FanOut(size_t bytes, bool to_staging_) : to_staging(to_staging_)
+    {
+        const unsigned hw = std::thread::hardware_concurrency();
+        nthr = (int)std::max<size_t>(1, std::min<size_t>({16, hw ? hw : 1, bytes >> 20}));
+        try {
+            for (int t = 1; t < nthr; t++) th.emplace_back(&FanOut::worker, this, t);
+        } catch (const std::exception &) {  // fewer threads: the rest is copied by this one
+        }
+    }
+    void slice(int t, char *d, const char *f, size_t n)
+    {
+        const size_t a = n * t / nthr & ~(size_t)63, b = t == nthr - 1 ? n : n * (t + 1) / nthr & ~(size_t)63;
+        copy_uncached(d + a, f + a, b - a, to_staging);
+    }
+    void worker(int t)
+    {
+        size_t seen = 0;
+        std::unique_lock<std::mutex> g(mu);
+        for (;;) {
+            go.wait(g, [&] { return stop || gen != seen; });
+            if (stop) return;
+            seen = gen;
+            char *d = to;
+            const char *f = from;
+            const size_t n = len;
+            g.unlock();
+            slice(t, d, f, n);
+            g.lock();
+            if (--pending == 0) done.notify_one();
+        }
+    }
+    void copy(char *d, const char *f, size_t n)
+    {
+        {
+            std::lock_guard<std::mutex> g(mu);
+            to = d;
+            from = f;
+            len = n;
+            pending = (int)th.size();
+            gen++;
+        }
+        go.notify_all();
+        // slices of the threads that could not be started are done here
+        for (int t = (int)th.size() + 1; t < nthr; t++) slice(t, d, f, n);
+        slice(0, d, f, n);
+        std::unique_lock<std::mutex> g(mu);
+        done.wait(g, [&] { return pending == 0; });
+    }
+    ~FanOut()
+    {
+        {
+            std::lock_guard<std::mutex> g(mu);
+            stop = true;
+        }
+        go.notify_all();
+        for (auto &x : th) x.join();
+    }
+};
+}  // namespace
+
+static void copy_to_pageable(void *dst, const void *src, size_t bytes, FanOut &fan);
 static void copy_from_host(void *dst, const void *src, size_t bytes, cudaStream_t s);
 
-// Touch one byte of every 4 KiB page of [p, p + bytes), split over up to 16
-// threads, so that the pages are resident before they are copied into.
+// Touch one byte of every 4 KiB page of [p, p + bytes), on a thread per 4 MB
+// and up to 16, so that the pages are resident before they are copied into (a
+// fresh page takes about 1 us, more than its copy).
 static void prefault(void *p, size_t bytes)
 {
-    if (bytes < ((size_t)64 << 20)) return;
     const unsigned hw = std::thread::hardware_concurrency();
-    const int nthr = (int)std::max(1u, std::min(16u, hw ? hw : 1u));
+    const int nthr = (int)std::max<size_t>(1, std::min<size_t>({16, hw ? hw : 1, bytes >> 22}));
     auto touch = [p, bytes, nthr](int t) {
         volatile char *c = (volatile char *)p;
         const size_t a = bytes * t / nthr, b = bytes * (t + 1) / nthr;
@@ -2179,7 +2339,7 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
     init_device();
     Stream st;
     cudaStream_t s = st.s;
-    Pool pool(s);     // temporaries
+    Pool pool(s, true);  // temporaries
     Pool keep(s);     // catalog arrays (released to the catalog on success)
     // phase boundaries: start, dedup, argsorts, levels, layout, end
     cudaEvent_t ph[6] = {};
@@ -2398,6 +2558,7 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
                 // resident pages instead of taking a page fault (and the
                 // kernel's zeroing of a fresh page) at every page
                 prefault(ncp->host, node_bytes);
+                FanOut fan(node_bytes, false);  // (its threads start before the first level is done)
                 for (;;) {
                     NodeCopy::Item it;
                     {
@@ -2407,7 +2568,7 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
                         it = ncp->items[ncp->next++];
                     }
                     check(cudaEventSynchronize(it.ev), "node copy wait");
-                    copy_to_pageable((char *)ncp->host + it.off, src + it.off, it.len);
+                    copy_to_pageable((char *)ncp->host + it.off, src + it.off, it.len, fan);
                 }
             } catch (const Error &e) {
                 ncp->code = e.code;
@@ -2497,9 +2658,10 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
     queue_nodes(node_bytes);
     nc.close();
     if (!nc.th.joinable()) {  // no copier thread: copy here
+        FanOut fan(node_bytes, false);
         for (auto &it : nc.items) {
             check(cudaEventSynchronize(it.ev), "node copy wait");
-            copy_to_pageable((char *)nc.host + it.off, (const char *)to.nodes + it.off, it.len);
+            copy_to_pageable((char *)nc.host + it.off, (const char *)to.nodes + it.off, it.len, fan);
         }
     }
     // ---- counting layout
@@ -2715,7 +2877,7 @@ static void build_query(const double *h_xyz, const int *h_fields, int n, int num
     init_device();
     Stream st;
     cudaStream_t s = st.s;
-    Pool pool(s), keep(s);
+    Pool pool(s, true), keep(s);
     double *xyz = pool.alloc<double>(3 * (size_t)n);
     copy_from_host(xyz, h_xyz, sizeof(double) * 3 * (size_t)n, s);
     int *fin = nullptr;
@@ -2834,153 +2996,18 @@ struct OnDevice {
 
 namespace kd {
 
-// Device -> pageable host copy of the node array returned by tree_construct
-// (1.3 GB at 20M points), one queued item at a time.  A plain cudaMemcpy into
-// pageable memory goes through the driver's own staging, one copy at a time
-// for the whole process, and at the speed of the page faults of its one
-// copying thread; it also makes every other pageable transfer of the process
-// (the build's own small reads of device scalars) queue behind it.  Here the
-// data goes through two pinned staging chunks (the next chunk's DMA overlaps
-// the current one's host copy) and each chunk is copied into the destination
-// by several threads, which take the destination's first-touch page faults in
-// parallel.
-namespace {
-struct Staging {
-    static constexpr size_t kChunk = size_t(32) << 20;
-    void *pin[2] = {nullptr, nullptr};
-};
-// pinned staging pairs kept for the life of the process (allocating pinned
-// memory per copy costs more than the copy): one per copy running at once,
-// at most kMaxStaging (a batch of many small deferred builds would otherwise
-// pin 64 MB per build); a copy that finds them all in use waits for one
-constexpr int kMaxStaging = 4;
-std::mutex g_stage_mu;
-std::condition_variable g_stage_cv;
-std::vector<Staging *> g_stage_free;
-int g_stage_made = 0;
-struct StagingLease {
-    Staging *st = nullptr;
-    StagingLease()
-    {
-        {
-            std::unique_lock<std::mutex> g(g_stage_mu);
-            g_stage_cv.wait(g, [] { return !g_stage_free.empty() || g_stage_made < kMaxStaging; });
-            if (!g_stage_free.empty()) {
-                st = g_stage_free.back();
-                g_stage_free.pop_back();
-                return;
-            }
-            g_stage_made++;  // this thread makes the next pair
-        }
-        std::unique_ptr<Staging> n(new Staging);
-        for (int i = 0; i < 2; i++)
-            if (cudaHostAlloc(&n->pin[i], Staging::kChunk, cudaHostAllocPortable) != cudaSuccess) {
-                cudaGetLastError();
-                for (int j = 0; j < i; j++) cudaFreeHost(n->pin[j]);
-                {
-                    std::lock_guard<std::mutex> g(g_stage_mu);
-                    g_stage_made--;
-                }
-                g_stage_cv.notify_one();
-                raise(KD_ENOMEM, "out of pinned host memory for the node array copy");
-            }
-        st = n.release();
-    }
-    ~StagingLease()
-    {
-        {
-            std::lock_guard<std::mutex> g(g_stage_mu);
-            g_stage_free.push_back(st);
-        }
-        g_stage_cv.notify_one();
-    }
-};
-// Host copies of a transfer's chunks fanned out over a pool of threads made
-// once for the whole transfer (a 32 MB chunk takes ~1 ms; creating threads
-// per chunk would cost a good part of that).  Transfers under 4 MB are
-// copied by the calling thread alone.
-struct FanOut {
-    int nthr = 1;
-    std::vector<std::thread> th;
-    std::mutex mu;
-    std::condition_variable go, done;
-    size_t gen = 0;
-    int pending = 0;
-    bool stop = false;
-    char *to = nullptr;
-    const char *from = nullptr;
-    size_t len = 0;
-    explicit FanOut(size_t bytes)
-    {
-        const unsigned hw = std::thread::hardware_concurrency();
-        nthr = bytes < (size_t(4) << 20) ? 1 : (int)std::max(1u, std::min(16u, hw ? hw : 1u));
-        try {
-            for (int t = 1; t < nthr; t++) th.emplace_back(&FanOut::worker, this, t);
-        } catch (const std::exception &) {  // fewer threads: the rest is copied by this one
-        }
-    }
-    void slice(int t, char *d, const char *f, size_t n)
-    {
-        const size_t a = n * t / nthr, b = n * (t + 1) / nthr;
-        std::memcpy(d + a, f + a, b - a);
-    }
-    void worker(int t)
-    {
-        size_t seen = 0;
-        std::unique_lock<std::mutex> g(mu);
-        for (;;) {
-            go.wait(g, [&] { return stop || gen != seen; });
-            if (stop) return;
-            seen = gen;
-            char *d = to;
-            const char *f = from;
-            const size_t n = len;
-            g.unlock();
-            slice(t, d, f, n);
-            g.lock();
-            if (--pending == 0) done.notify_one();
-        }
-    }
-    void copy(char *d, const char *f, size_t n)
-    {
-        {
-            std::lock_guard<std::mutex> g(mu);
-            to = d;
-            from = f;
-            len = n;
-            pending = (int)th.size();
-            gen++;
-        }
-        go.notify_all();
-        // slices of the threads that could not be started are done here
-        for (int t = (int)th.size() + 1; t < nthr; t++) slice(t, d, f, n);
-        slice(0, d, f, n);
-        std::unique_lock<std::mutex> g(mu);
-        done.wait(g, [&] { return pending == 0; });
-    }
-    ~FanOut()
-    {
-        {
-            std::lock_guard<std::mutex> g(mu);
-            stop = true;
-        }
-        go.notify_all();
-        for (auto &x : th) x.join();
-    }
-};
-}  // namespace
-
 // Host -> device copy of a build's input on stream s.  Pinned (or managed)
-// memory, and anything under 32 MB (where starting the copying threads
-// costs more than it saves), is one cudaMemcpyAsync.  Pageable memory
-// otherwise takes the driver's own staging path at about 10 GB/s (50 ms for
-// the 560 MB of a 20M-point catalog); here several threads copy each 32 MB
-// chunk into a pinned staging buffer while the previous chunk's DMA runs.
-// Returns once the last DMA has finished (the staging pair is then free).
+// memory, and anything under 4 MB (where starting the copying threads costs
+// more than it saves), is one cudaMemcpyAsync.  Pageable memory otherwise
+// takes the driver's own staging path at 10 to 20 GB/s (50 ms for the 560 MB of
+// a 20M-point catalog, 2.0 ms for the 24 MB of 1M points); here several threads
+// copy each chunk into a pinned staging buffer while the previous chunk's DMA
+// runs (1M points 1.0 ms).  Returns once the last DMA has finished (the staging
+// pair is then free).
 static void copy_from_host(void *dst, const void *src, size_t bytes, cudaStream_t s)
 {
     if (bytes == 0) return;
-    bool plain = bytes < (size_t(32) << 20);
+    bool plain = bytes < (size_t(4) << 20);
     if (!plain) {
         cudaPointerAttributes at;
         if (cudaPointerGetAttributes(&at, src) == cudaSuccess)
@@ -2992,7 +3019,7 @@ static void copy_from_host(void *dst, const void *src, size_t bytes, cudaStream_
         check(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s), "H2D");
         return;
     }
-    const size_t chunk = Staging::kChunk;
+    const size_t chunk = size_t(8) << 20;  // (the first chunk's copy has no DMA to overlap)
     StagingLease lease;
     void *const *pin = lease.st->pin;
     cudaEvent_t done[2] = {nullptr, nullptr};
@@ -3009,7 +3036,7 @@ static void copy_from_host(void *dst, const void *src, size_t bytes, cudaStream_
     } rel{done};
     for (int i = 0; i < 2; i++)
         check(cudaEventCreateWithFlags(&done[i], cudaEventDisableTiming), "cudaEventCreate");
-    FanOut fan(bytes);
+    FanOut fan(bytes, true);
     const size_t nch = (bytes + chunk - 1) / chunk;
     for (size_t c = 0; c < nch; c++) {
         const int b = (int)(c & 1);
@@ -3022,7 +3049,7 @@ static void copy_from_host(void *dst, const void *src, size_t bytes, cudaStream_
     for (int b = 0; b < 2; b++) check(cudaEventSynchronize(done[b]), "H2D wait");
 }
 
-static void copy_to_pageable(void *dst, const void *src, size_t bytes)
+static void copy_to_pageable(void *dst, const void *src, size_t bytes, FanOut &fan)
 {
     const size_t chunk = Staging::kChunk;
     if (bytes == 0) return;
@@ -3047,8 +3074,6 @@ static void copy_to_pageable(void *dst, const void *src, size_t bytes)
               "D2H");
         check(cudaEventRecord(done[c & 1], st.s), "event");
     };
-    FanOut fan(bytes);
-
     issue(0);
     for (size_t c = 0; c < nch; c++) {
         check(cudaEventSynchronize(done[c & 1]), "D2H wait");

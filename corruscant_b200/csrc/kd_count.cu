@@ -1162,7 +1162,7 @@ static void count_batch_impl(const kd_catalog *const *tcs, const kd_catalog *con
     init_device();
     Stream st;
     cudaStream_t s = st.s;
-    Pool pool(s);
+    Pool pool(s, true);
     Events ev;
     int launches = 0, tile_launches = 0;
 
@@ -1250,31 +1250,41 @@ static void count_batch_impl(const kd_catalog *const *tcs, const kd_catalog *con
         total += hcnt[i];
         maxblk = std::max<long long>(maxblk, hcnt[i]);
     }
+    // (asked for only where it can matter: not below 2^20 records, nor where
+    // the record pool's idle memory holds them all.  The driver answers in
+    // milliseconds, at times tens of them, on a machine whose other GPUs keep
+    // it busy: a count of 4k / 80k points took 0.7 ms, and now and then 16 or 89)
     // free memory: the driver's, plus what the record pool and the default
     // pool hold cached (reusable without asking the driver)
     const cudaMemPool_t rpool = side_pool(kPoolRecords);
-    size_t freeb = 0, totb = 0;
-    cudaMemGetInfo(&freeb, &totb);
-    freeb += pool_idle_bytes(rpool);
-    {
-        cudaMemPool_t dpool = nullptr;
-        if (cudaDeviceGetDefaultMemPool(&dpool, device) == cudaSuccess && dpool != rpool)
-            freeb += pool_idle_bytes(dpool);
-        cudaGetLastError();
-    }
-    long long cap = std::max<long long>(
-        1 << 20, std::min<long long>(1LL << 30, (long long)(freeb / 4 / sizeof(uint4))));
+    long long cap = 1LL << 30;
+    uint4 *rec = nullptr;
     // KD_TILE_RECORD_CAP (records, > 0) lowers the batch size: it exercises
     // the multi-batch path on small counts
-    if (const char *env = getenv("KD_TILE_RECORD_CAP")) {
-        const long long v = atoll(env);
-        if (v > 0) cap = v;
+    const char *const env = getenv("KD_TILE_RECORD_CAP");
+    const long long set = env ? atoll(env) : 0;
+    if (set <= 0 && total > 1 << 20 && total <= cap && (size_t)total * sizeof(uint4) <= pool_idle_bytes(rpool))
+        rec = pool.try_alloc_from<uint4>(rpool, total);
+    if (rec) {
+        cap = total;
+    } else {
+        if (total > 1 << 20) {
+            size_t freeb = 0, totb = 0;
+            cudaMemGetInfo(&freeb, &totb);
+            freeb += pool_idle_bytes(rpool);
+            cudaMemPool_t dpool = nullptr;
+            if (cudaDeviceGetDefaultMemPool(&dpool, device) == cudaSuccess && dpool != rpool)
+                freeb += pool_idle_bytes(dpool);
+            cudaGetLastError();
+            cap = std::max<long long>(1 << 20, std::min<long long>(cap, (long long)(freeb / 4 / sizeof(uint4))));
+        }
+        if (set > 0) cap = set;
+        // every batch holds at least one whole block: the buffer must take the
+        // largest block's records (a failed allocation is reported, not overrun)
+        cap = std::max(cap, maxblk);
+        cap = std::min<long long>(cap, std::max<long long>(total, 1));
+        rec = pool.alloc_from<uint4>(rpool, cap);
     }
-    // every batch holds at least one whole block: the buffer must take the
-    // largest block's records (a failed allocation is reported, not overrun)
-    cap = std::max(cap, maxblk);
-    cap = std::min<long long>(cap, std::max<long long>(total, 1));
-    uint4 *rec = pool.alloc_from<uint4>(rpool, cap);
     long long *off = pool.alloc<long long>(nb + 1);
     std::vector<long long> hoffs(nb + 1);
 

@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <vector>
 
 #include "kd_internal.h"
@@ -92,13 +93,33 @@ inline size_t pool_idle_bytes(cudaMemPool_t p)
 }
 
 // Stream-ordered allocations owned by one call; anything not released to a
-// longer-lived owner is freed when the call ends.
+// longer-lived owner is freed when the call ends.  A pool of temporaries only
+// (nothing of it is kept) takes its small arrays from shared pieces of 1 MB: a
+// build of a few thousand points asks for about sixty, at 2 us each with the
+// release.
 struct Pool {
+    static constexpr size_t kPiece = (size_t)1 << 20, kSmall = kPiece / 16;
     cudaStream_t s;
+    bool pieces;
     std::vector<void *> ptrs;
     size_t bytes = 0;
-    explicit Pool(cudaStream_t st) : s(st) {}
+    char *piece = nullptr;
+    size_t left = 0;
+    explicit Pool(cudaStream_t st, bool temporaries = false) : s(st), pieces(temporaries) {}
     template <class T> T *alloc(size_t n)
+    {
+        const size_t want = ((n ? n : 1) * sizeof(T) + 255) & ~(size_t)255;
+        if (!pieces || want > kSmall) return take<T>(n);
+        if (want > left) {
+            piece = take<char>(kPiece);
+            left = kPiece;
+        }
+        char *const p = piece;
+        piece += want;
+        left -= want;
+        return (T *)p;
+    }
+    template <class T> T *take(size_t n)
     {
         void *p = nullptr;
         size_t b = (n ? n : 1) * sizeof(T);
@@ -111,19 +132,27 @@ struct Pool {
         bytes += b;
         return (T *)p;
     }
-    // n elements from a given memory pool (stream-ordered like alloc)
-    template <class T> T *alloc_from(cudaMemPool_t mp, size_t n)
+    // n elements from a given memory pool (stream-ordered like alloc), or null
+    template <class T> T *try_alloc_from(cudaMemPool_t mp, size_t n, cudaError_t *why = nullptr)
     {
         void *p = nullptr;
         size_t b = (n ? n : 1) * sizeof(T);
         cudaError_t e = cudaMallocFromPoolAsync(&p, b, mp, s);
+        if (why) *why = e;
         if (e != cudaSuccess) {
             cudaGetLastError();
-            raise(KD_ENOMEM, "device allocation failed", e);
+            return nullptr;
         }
         ptrs.push_back(p);
         bytes += b;
         return (T *)p;
+    }
+    template <class T> T *alloc_from(cudaMemPool_t mp, size_t n)
+    {
+        cudaError_t e;
+        T *const p = try_alloc_from<T>(mp, n, &e);
+        if (!p) raise(KD_ENOMEM, "device allocation failed", e);
+        return p;
     }
     // hand ownership of p to the caller (it will not be freed by ~Pool)
     template <class T> T *keep(T *p)
@@ -140,17 +169,54 @@ struct Pool {
 };
 
 // One non-blocking stream per API call: calls on different threads do not
-// serialise on each other's work.
+// serialise on each other's work.  Up to kIdle streams per device wait, with
+// nothing in flight, for a later call: to make and destroy one takes 92 us, and
+// tens of ms now and then on a machine whose other GPUs keep the driver busy.
 struct Stream {
+    static constexpr size_t kIdle = 8;
+    struct Idle {
+        std::mutex mu;
+        std::vector<cudaStream_t> dev[64];
+    };
+    static Idle &idle()
+    {
+        static Idle *i = new Idle;  // outlives every thread's calls
+        return *i;
+    }
     cudaStream_t s = nullptr;
-    Stream() { check(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "cudaStreamCreate"); }
+    int dev = 0;
+    Stream()
+    {
+        check(cudaGetDevice(&dev), "cudaGetDevice");
+        if (dev < 64) {
+            std::lock_guard<std::mutex> g(idle().mu);
+            auto &v = idle().dev[dev];
+            if (!v.empty()) {
+                s = v.back();
+                v.pop_back();
+                return;
+            }
+        }
+        check(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "cudaStreamCreate");
+    }
     ~Stream()
     {
-        if (s) {
-            cudaStreamSynchronize(s);
-            cudaStreamDestroy(s);
+        if (!s) return;
+        if (cudaStreamSynchronize(s) == cudaSuccess && dev < 64) {
+            std::lock_guard<std::mutex> g(idle().mu);
+            auto &v = idle().dev[dev];
+            if (v.size() < kIdle) {
+                try {
+                    v.push_back(s);
+                    return;
+                } catch (const std::bad_alloc &) {
+                }
+            }
         }
+        cudaStreamDestroy(s);
     }
+    Stream(const Stream &) = delete;
+    Stream &operator=(const Stream &) = delete;
     void sync() { check(cudaStreamSynchronize(s), "kernel execution"); }
 };
 

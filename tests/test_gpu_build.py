@@ -156,3 +156,12 @@ def test_counting_order(n, kind):
                 N.destroy(q)
         finally:
             N.destroy(t)
+
+
+@pytest.mark.parametrize("n", [174_762, 174_763, 349_525, 349_526, 700_001])
+def test_transfer_sizes(n):
+    """Inputs and node arrays one short of, at and past the sizes at which
+    their copies are staged and cut (4 MB, 8 MB, several pieces)."""
+    rs = np.random.RandomState(n)
+    p = rs.rand(n, 3)
+    _check(p, (p[:, 1] * 5).astype(np.int32), 5)
