@@ -323,8 +323,11 @@ __global__ void __launch_bounds__(32 * kTravWarps) k_traverse(const JobDesc *__r
 // error is 0.59 to 1.09 u (sqrt(d2) + Rq)^2 RMS (u = 2^-24) at radii of 2 to 10
 // block radii Rq and 0.25 at half a block radius, where the FP32 FMA chain it
 // replaces has 0.59 to 1.16 and 0.23.
-// FP64 mode: two query tiles at a time, a query per lane, every distance in
-// the reference's operation order.
+// FP64 mode: a query tile at a time, each half of the warp with half of the
+// run's points, every distance in the reference's operation order, up to six
+// edges per distance (two tiles at a time, with one window for both, and four
+// edges: 7% and 4% slower; compares as integers, on the ALU: 4%).  Bound by
+// the issue slots, then the FP64 pipe (73% and 64% used).
 //
 // Bound: the FP32 pipe, by the binning (a ramp, a count and a check per pair
 // and edge: 15 clocks per 128 pairs and edge in isolation, 20 here), then the
@@ -441,17 +444,18 @@ __device__ __forceinline__ uint32_t split_halves(float v)
     return (uint32_t)__half_as_ushort(hi) | ((uint32_t)__half_as_ushort(lo) << 16);
 }
 
-// FP64 mode: a query's pairs with a staged run (np pairs of points; a missing
-// one is at 1e300) below K (<= 4) edges
+// FP64 mode: a query's pairs with np pairs of staged points (a missing one is at
+// 1e300) below the ne first edges of R (ne <= K <= kFpEdges)
+constexpr int kFpEdges = 6;
 template <int K>
 __device__ __forceinline__ void fp64_run(const double2 *__restrict__ tx,
                                          const double2 *__restrict__ ty,
                                          const double2 *__restrict__ tz, int np, double qx, double qy,
-                                         double qz, const double *R, unsigned (&cnt)[4])
+                                         double qz, const double *R, int ne, unsigned (&cnt)[kFpEdges])
 {
     double r[K];
 #pragma unroll
-    for (int k = 0; k < K; k++) r[k] = R[k];
+    for (int k = 0; k < K; k++) r[k] = k < ne ? R[k] : 0.0;  // (no distance is below zero)
 #pragma unroll 4
     for (int j = 0; j < np; j++) {
         const double2 x = tx[j], y = ty[j], z = tz[j];
@@ -882,14 +886,6 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                         }
                     }
                     const int mval = max(0, min(kMT, s.qlen - kMT * wm));  // queries of tile wm
-                    if constexpr (MODE == KD_MODE_FP64) {  // one window for two query tiles
-                        const int p0 = __shfl_xor_sync(FULL, k0, 1), p1 = __shfl_xor_sync(FULL, k1, 1);
-                        const bool pv = __shfl_xor_sync(FULL, mval, 1) != 0;
-                        if (pv && (k1 > k0 || p1 > p0)) {
-                            k0 = min(k0, p0);
-                            k1 = max(k1, p1);
-                        }
-                    }
                     const int K = have && mval ? k1 - k0 : 0;
                     const unsigned win = (unsigned)k0 | ((unsigned)K << 8);
                     const unsigned actm = __ballot_sync(FULL, K != 0), okm = __ballot_sync(FULL, ok);
@@ -989,7 +985,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
 #pragma unroll
                                 for (int h = 0; h < 2; h++) {
                                     const int j = lane + 32 * h;
-                                    if (j < ((n + 1) & ~1)) {
+                                    if (j < ((n + 3) & ~3)) {
                                         s.pt[w][0][j] = j < n ? px[h] : 1e300;
                                         s.pt[w][1][j] = j < n ? py[h] : 1e300;
                                         s.pt[w][2][j] = j < n ? pz[h] : 1e300;
@@ -1001,27 +997,31 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                             const double2 *X = reinterpret_cast<const double2 *>(s.pt[w][0]),
                                           *Y = reinterpret_cast<const double2 *>(s.pt[w][1]),
                                           *Z = reinterpret_cast<const double2 *>(s.pt[w][2]);
-                            for (int p = 0; p < kMTiles / 2; p++) {
-                                // (a tile without queries has no window: take the other's)
-                                const unsigned two = (act >> (2 * p)) & 3u;
-                                if (!two) continue;
-                                const unsigned wv = __shfl_sync(FULL, win, src + 2 * p + (two == 2u));
-                                const int q = 32 * p + lane;
+                            // a query tile at a time, each half of the warp
+                            // with half of the points (two and two)
+                            const int np = (n + 3) / 4, at = (lane >> 4) * np;
+                            for (; act; act &= act - 1) {
+                                const int m = __ffs(act) - 1, q = kMT * m + (lane & (kMT - 1));
+                                const unsigned wv = __shfl_sync(FULL, win, src + m);
                                 const bool v = q < s.qlen;
                                 const double qx = v ? s.job.Q.x[s.qs + q] : s.o[0],
                                              qy = v ? s.job.Q.y[s.qs + q] : s.o[1],
                                              qz = v ? s.job.Q.z[s.qs + q] : s.o[2];
-                                for (int kk = wv & 0xFF, left = wv >> 8; left > 0; left -= 4, kk += 4) {
-                                    unsigned cnt[4] = {0u, 0u, 0u, 0u};
-                                    switch (min(left, 4)) {
-                                    case 1: fp64_run<1>(X, Y, Z, (n + 1) / 2, qx, qy, qz, s.R + kk, cnt); break;
-                                    case 2: fp64_run<2>(X, Y, Z, (n + 1) / 2, qx, qy, qz, s.R + kk, cnt); break;
-                                    case 3: fp64_run<3>(X, Y, Z, (n + 1) / 2, qx, qy, qz, s.R + kk, cnt); break;
-                                    default: fp64_run<4>(X, Y, Z, (n + 1) / 2, qx, qy, qz, s.R + kk, cnt); break;
+                                for (int kk = wv & 0xFF, left = wv >> 8; left > 0; left -= kFpEdges, kk += kFpEdges) {
+                                    unsigned cnt[kFpEdges] = {};
+                                    switch (left) {
+                                    case 1: fp64_run<1>(X + at, Y + at, Z + at, np, qx, qy, qz, s.R + kk, 1, cnt); break;
+                                    case 2: fp64_run<2>(X + at, Y + at, Z + at, np, qx, qy, qz, s.R + kk, 2, cnt); break;
+                                    case 3: fp64_run<3>(X + at, Y + at, Z + at, np, qx, qy, qz, s.R + kk, 3, cnt); break;
+                                    case 4: fp64_run<4>(X + at, Y + at, Z + at, np, qx, qy, qz, s.R + kk, 4, cnt); break;
+                                    default: fp64_run<kFpEdges>(X + at, Y + at, Z + at, np, qx, qy, qz, s.R + kk, left, cnt); break;
                                     }
 #pragma unroll
-                                    for (int k = 0; k < 4; k++)
-                                        if (k < left) atomicAdd(&P[(kk + k) * kPStride + q], cnt[k]);
+                                    for (int k = 0; k < kFpEdges; k++)
+                                        if (k < left) {
+                                            const unsigned c = cnt[k] + __shfl_xor_sync(FULL, cnt[k], kMT);
+                                            if (lane < kMT) atomicAdd(&P[(kk + k) * kPStride + q], c);
+                                        }
                                 }
                             }
                         }
