@@ -342,27 +342,37 @@ struct LevelBufs {
     unsigned char *big, *fallback;
     double *acc;      // per big segment: S0 S1 S2 A0 A1 A2 V0 V1 V2
     int cap_big;
-    int *rank;        // exclusive scan of "has children"
-    int *haskids;
 };
 
-__global__ void k_seg_setup(Segs sg, int ub, LevelBufs lb)
+__global__ void k_first_seg(Segs sg, int n_u)
+{
+    sg.count[0] = sg.p[0] = 1;
+    sg.l[0] = 0;
+    sg.r[0] = n_u - 1;
+}
+
+// One level's buffers cleared, and the next level's segments (every segment of
+// the level loop is larger than kSubCap, so it splits).
+__global__ void k_seg_setup(Segs sg, int ub, LevelBufs lb, Segs nxt)
 {
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= ub) return;
-    int ns = *sg.count;
-    if (s >= ns) {
-        lb.haskids[s] = 0;
-        return;
-    }
-    int size = sg.r[s] - sg.l[s] + 1;
-    int big = size > kSmallSeg && s < lb.cap_big;
+    const int ns = *sg.count;
+    if (s == 0) *nxt.count = 2 * ns;
+    if (s >= ns) return;
+    const int p = sg.p[s], l = sg.l[s], r = sg.r[s], med = (l + r + 1) / 2;
+    int big = r - l + 1 > kSmallSeg && s < lb.cap_big;
     lb.big[s] = (unsigned char)big;
     lb.fallback[s] = 0;
     lb.tdim[s] = 0;
-    lb.haskids[s] = size >= 4;
     if (big)
         for (int k = 0; k < 9; k++) lb.acc[9 * (size_t)s + k] = 0.0;
+    nxt.p[2 * s] = 2 * p;
+    nxt.l[2 * s] = l;
+    nxt.r[2 * s] = med - 1;
+    nxt.p[2 * s + 1] = 2 * p + 1;
+    nxt.l[2 * s + 1] = med + 1;
+    nxt.r[2 * s + 1] = r;
 }
 
 // Parallel sums for big segments: pass 0 accumulates S_j = sum v_j and
@@ -638,23 +648,9 @@ __global__ void k_level_nodes(Segs sg, int ub, LevelBufs lb, const int *__restri
 {
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= ub || s >= *sg.count) return;
-    int p = sg.p[s], l = sg.l[s], r = sg.r[s];
-    int size = r - l + 1;
-    if (size >= 4) {
-        int med = (l + r + 1) / 2;
-        int d = lb.tdim[s];
-        const int *ad = d == 0 ? a0 : (d == 1 ? a1 : a2);
-        put_node(t, u, p, ad[med], d, 1, 1, med, err);
-    } else if (size == 3) {
-        put_node(t, u, p, a0[l + 1], 0, 1, 1, l + 1, err);
-        put_node(t, u, 2 * p, a0[l], 0, 0, 0, l, err);
-        put_node(t, u, 2 * p + 1, a0[r], 0, 0, 0, r, err);
-    } else if (size == 2) {
-        put_node(t, u, p, a0[r], 0, 1, 0, r, err);
-        put_node(t, u, 2 * p, a0[l], 0, 0, 0, l, err);
-    } else if (size == 1) {
-        put_node(t, u, p, a0[l], 0, 0, 0, l, err);
-    }
+    const int med = (sg.l[s] + sg.r[s] + 1) / 2, d = lb.tdim[s];
+    const int *ad = d == 0 ? a0 : (d == 1 ? a1 : a2);
+    put_node(t, u, sg.p[s], ad[med], d, 1, 1, med, err);
 }
 
 // side of every point of a splitting segment: 0 left, 1 right, 2 median
@@ -675,19 +671,27 @@ __global__ void k_mark(int n_u, const int *__restrict__ pos_seg, Segs sg, LevelB
 }
 
 // ---- Stable three-way partition of the three superkey orders, one level.
-// Within every splitting segment [l, r] (at least four points, median
-// position med = (l + r + 1) / 2), the points of each order d go, in their
-// order, to [l, med) when k_mark put them left of the median (side 0), to
-// (med, r] when right (side 1), the median point itself to med; positions
-// outside splitting segments stay.  The destination of a point is its
-// segment's start plus the number of same-side points before it in the
-// segment: a segmented prefix count, computed in three launches over tiles of
-// kPtTile positions that handle all three orders at once (per-tile counts, one
-// block scanning the tile counts, then the move), with no waiting between
-// blocks.  Counts inside a tile fit 16 bits: left | right << 16 in a word.
+// Within every segment [l, r], median position med = (l + r + 1) / 2, the
+// points of each order d go, in their order, to [l, med) when k_mark put them
+// left of the median (side 0), to (med, r] when right (side 1), the median
+// point itself to med; positions outside segments stay.  The destination of a
+// point is its segment's start plus the number of same-side points before it
+// in the segment.  Three launches over tiles of kPtTile positions handle all
+// three orders at once, with no waiting between blocks: per 32 positions, a
+// bit mask of each order's left and right points, and the tile's counts from
+// its last segment start on; one block scans those; the move counts bits
+// below a position, in the tile and back to its segment's start or the tile's
+// carry.  Lanes hold neighbouring positions, so that loads are whole lines and
+// a warp's stores two runs.  Bound by memory: with eight consecutive positions
+// per thread, whose stores met a line once per position, the move of 5M points
+// took 150 us a level (and 20 for the next level's segments, written here),
+// now 83; the counts 57, now 47.
 constexpr int kPtThreads = 256;
-constexpr int kPtItems = 8;  // consecutive positions per thread
-constexpr int kPtTile = kPtThreads * kPtItems;
+constexpr int kPtWarps = kPtThreads / 32;
+constexpr int kPtRounds = 8;                      // positions per thread
+constexpr int kPtTile = kPtThreads * kPtRounds;
+constexpr int kPtWords = kPtTile / 32;            // words of 32 positions per tile
+constexpr int kPtMasks = 6;                       // per word: order 0 left, right, order 1 left, ...
 
 struct PartIO {
     const int *a[3];     // superkey orders (point ids by position)
@@ -695,44 +699,6 @@ struct PartIO {
     const double *c[3];  // coordinate d of the point at each position of order d
     double *co[3];       // the same, partitioned
 };
-
-// kPtItems consecutive ints from p + base (vector loads when all are in range)
-__device__ __forceinline__ void load8(const int *__restrict__ p, int base, int n, int (&x)[kPtItems])
-{
-    static_assert(kPtItems == 8, "two int4 loads per thread");
-    if (base + kPtItems <= n) {
-        const int4 u = __ldg(reinterpret_cast<const int4 *>(p + base));
-        const int4 w = __ldg(reinterpret_cast<const int4 *>(p + base) + 1);
-        x[0] = u.x, x[1] = u.y, x[2] = u.z, x[3] = u.w;
-        x[4] = w.x, x[5] = w.y, x[6] = w.z, x[7] = w.w;
-    } else {
-#pragma unroll
-        for (int k = 0; k < kPtItems; k++) x[k] = base + k < n ? p[base + k] : -1;
-    }
-}
-
-// the splitting segment of each of a thread's positions (-1: none) and the
-// positions that start one
-__device__ __forceinline__ unsigned split_segs(int base, int n_u, const int *__restrict__ pos_seg,
-                                               Segs sg, int (&sgi)[kPtItems])
-{
-    load8(pos_seg, base, n_u, sgi);
-    unsigned headmask = 0;
-#pragma unroll
-    for (int k = 0; k < kPtItems; k++) {
-        const int s = sgi[k];
-        if (s < 0) continue;
-        const int l = sg.l[s], r = sg.r[s];
-        if (r - l + 1 < 4) sgi[k] = -1;
-        else if (base + k == l) headmask |= 1u << k;
-    }
-    return headmask;
-}
-
-__device__ __forceinline__ unsigned side_count(int sd)
-{
-    return sd == 0 ? 1u : (sd == 1 ? 0x10000u : 0u);
-}
 
 // inclusive segmented scan over the lanes of a warp: a lane's value restarts
 // at a lane holding a head (f = 1)
@@ -754,75 +720,73 @@ __device__ __forceinline__ void warp_seg_scan(unsigned &f, unsigned (&v)[NV], in
     }
 }
 
-// Per tile: (a head in the tile?, the three orders' packed side counts from
-// the tile's last head, or from its start when it has none).  Also stores
-// the three sides of every position, sd_pos[i] = side0 | side1 << 8 |
-// side2 << 16 (3: not in a splitting segment), so that the move reads them
-// in order instead of gathering side[] by point again.
+// masks[tile][word][kPtMasks], and per tile (a segment start in the tile?, the
+// three orders' left | right << 16 counts from its last one, or from the
+// tile's start when it has none).
 __global__ void __launch_bounds__(kPtThreads) k_part_count(int n_u, const int *__restrict__ pos_seg,
                                                            Segs sg, const int *__restrict__ a0,
                                                            const int *__restrict__ a1,
                                                            const int *__restrict__ a2,
                                                            const unsigned char *__restrict__ side,
-                                                           unsigned *sd_pos, uint4 *tagg)
+                                                           unsigned *masks, uint4 *tagg)
 {
-    constexpr int NW = kPtThreads / 32;
-    __shared__ unsigned wf[NW], wv[NW][3];
+    constexpr unsigned FULL = 0xffffffffu;
+    static_assert(kPtWords == 64 && kPtWarps >= kPtMasks, "two words per lane, a warp per mask");
+    __shared__ unsigned sm[kPtWords][kPtMasks], heads[kPtWords], tot[kPtMasks + 1];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int base = blockIdx.x * kPtTile + threadIdx.x * kPtItems;
-    int sgi[kPtItems];
-    const unsigned headmask = split_segs(base, n_u, pos_seg, sg, sgi);
-    unsigned sdw[kPtItems];
+    const int base = blockIdx.x * kPtTile;
+    int sd[kPtRounds][3];
+    bool in[kPtRounds];
 #pragma unroll
-    for (int k = 0; k < kPtItems; k++) sdw[k] = 0x030303u;
-    {
-        const int *ad[3] = {a0, a1, a2};
+    for (int k = 0; k < kPtRounds; k++) {
+        const int wd = w * kPtRounds + k, i = base + 32 * wd + lane;
+        const int seg = i < n_u ? pos_seg[i] : -1;
+        in[k] = seg >= 0;
+        const unsigned h = __ballot_sync(FULL, in[k] && sg.l[in[k] ? seg : 0] == i);
+        if (lane == 0) heads[wd] = h;
 #pragma unroll
         for (int d = 0; d < 3; d++) {
-            int pt[kPtItems];
-            load8(ad[d], base, n_u, pt);
-#pragma unroll
-            for (int k = 0; k < kPtItems; k++)
-                if (sgi[k] >= 0)
-                    sdw[k] = (sdw[k] & ~(0xffu << (8 * d))) | ((unsigned)side[pt[k]] << (8 * d));
+            sd[k][d] = 3;
+            if (in[k]) sd[k][d] = side[(d == 0 ? a0 : (d == 1 ? a1 : a2))[i]];
         }
     }
-    unsigned f = 0, v[3] = {0u, 0u, 0u};
 #pragma unroll
-    for (int k = 0; k < kPtItems; k++) {
-        if (headmask >> k & 1) {
-            f = 1;
-            v[0] = v[1] = v[2] = 0;
+    for (int k = 0; k < kPtRounds; k++)
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            const unsigned l = __ballot_sync(FULL, sd[k][d] == 0), r = __ballot_sync(FULL, sd[k][d] == 1);
+            if (lane == 0) {
+                sm[w * kPtRounds + k][2 * d] = l;
+                sm[w * kPtRounds + k][2 * d + 1] = r;
+            }
         }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kPtWords * kPtMasks; i += kPtThreads)
+        masks[(size_t)blockIdx.x * (kPtWords * kPtMasks) + i] = (&sm[0][0])[i];
+    if (w < kPtMasks) {
+        // the last start: its word, then its bit
+        const unsigned h0 = heads[lane], h1 = heads[lane + 32];
+        const unsigned b0 = __ballot_sync(FULL, h0 != 0), b1 = __ballot_sync(FULL, h1 != 0);
+        const int hw = b1 ? 63 - __clz(b1) : (b0 ? 31 - __clz(b0) : -1);
+        const int bit = hw >= 0 ? 31 - __clz(heads[hw]) : 0;
+        unsigned c = 0;
 #pragma unroll
-        for (int d = 0; d < 3; d++) v[d] += side_count((sdw[k] >> (8 * d)) & 0xff);
-    }
-    if (base + kPtItems <= n_u) {
-        reinterpret_cast<uint4 *>(sd_pos + base)[0] = make_uint4(sdw[0], sdw[1], sdw[2], sdw[3]);
-        reinterpret_cast<uint4 *>(sd_pos + base)[1] = make_uint4(sdw[4], sdw[5], sdw[6], sdw[7]);
-    } else {
-#pragma unroll
-        for (int k = 0; k < kPtItems; k++)
-            if (base + k < n_u) sd_pos[base + k] = sdw[k];
-    }
-    warp_seg_scan<3>(f, v, lane);
-    if (lane == 31) {
-        wf[w] = f;
-        wv[w][0] = v[0];
-        wv[w][1] = v[1];
-        wv[w][2] = v[2];
+        for (int q = 0; q < 2; q++) {
+            const int wd = lane + 32 * q;
+            unsigned m = sm[wd][w];
+            if (wd < hw) m = 0;
+            if (wd == hw) m &= FULL << bit;
+            c += __popc(m);
+        }
+        c = __reduce_add_sync(FULL, c);
+        if (lane == 0) tot[w] = c;
+        if (w == 0 && lane == 0) tot[kPtMasks] = hw >= 0;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned F = 0, V[3] = {0u, 0u, 0u};
-        for (int q = 0; q < NW; q++) {
-            for (int k = 0; k < 3; k++) V[k] = wf[q] ? wv[q][k] : V[k] + wv[q][k];
-            F |= wf[q];
-        }
-        tagg[blockIdx.x] = make_uint4(F, V[0], V[1], V[2]);
-    }
+    if (threadIdx.x == 0)
+        tagg[blockIdx.x] = make_uint4(tot[kPtMasks], tot[0] | tot[1] << 16, tot[2] | tot[3] << 16,
+                                      tot[4] | tot[5] << 16);
 }
-
 
 __device__ __forceinline__ void unpack_counts(const uint4 &g, unsigned (&x)[6])
 {
@@ -883,141 +847,75 @@ __global__ void __launch_bounds__(1024) k_part_carry(int ntiles, const uint4 *__
 }
 
 // The move: every position's point id and carried coordinate, in each of the
-// three orders, to its place (see above).
-__global__ void __launch_bounds__(kPtThreads, 3) k_part_move(int n_u, const int *__restrict__ pos_seg,
-                                                             Segs sg, PartIO io,
-                                                             const unsigned *__restrict__ sd_pos,
-                                                             const uint4 *__restrict__ carry,
-                                                             int *err)
+// three orders, to its place, and the next level's segment of every position.
+__global__ void __launch_bounds__(kPtThreads) k_part_move(int n_u, const int *__restrict__ pos_seg, Segs sg,
+                                                          PartIO io, const unsigned *__restrict__ masks,
+                                                          const uint4 *__restrict__ carry, int *pos_next,
+                                                          int *err)
 {
-    constexpr int NW = kPtThreads / 32;
-    __shared__ unsigned wf[NW], wv[NW];
+    constexpr unsigned FULL = 0xffffffffu;
+    __shared__ unsigned sm[kPtWords][kPtMasks];
+    __shared__ int pre[kPtMasks][kPtWords], car[kPtMasks];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int base = blockIdx.x * kPtTile + threadIdx.x * kPtItems;
-    const bool full = base + kPtItems <= n_u;
-    int sgi[kPtItems], sdp[kPtItems];
-    const unsigned headmask = split_segs(base, n_u, pos_seg, sg, sgi);
-    load8(reinterpret_cast<const int *>(sd_pos), base, n_u, sdp);
-    const uint4 c0 = carry[2 * (size_t)blockIdx.x], c1 = carry[2 * (size_t)blockIdx.x + 1];
-#pragma unroll 1
-    for (int d = 0; d < 3; d++) {
-        // (selects rather than indexing io and the carry by d, which would
-        // put them in local memory)
-        const int *__restrict__ ain = d == 0 ? io.a[0] : (d == 1 ? io.a[1] : io.a[2]);
-        int *__restrict__ aout = d == 0 ? io.ao[0] : (d == 1 ? io.ao[1] : io.ao[2]);
-        const double *__restrict__ cin = d == 0 ? io.c[0] : (d == 1 ? io.c[1] : io.c[2]);
-        double *__restrict__ cout = d == 0 ? io.co[0] : (d == 1 ? io.co[1] : io.co[2]);
-        const unsigned crl = d == 0 ? c0.x : (d == 1 ? c0.z : c1.x);
-        const unsigned crr = d == 0 ? c0.y : (d == 1 ? c0.w : c1.y);
-        int sd[kPtItems];
-        unsigned f = 0, v = 0;
+    const int base = blockIdx.x * kPtTile;
+    for (int i = threadIdx.x; i < kPtWords * kPtMasks; i += kPtThreads)
+        (&sm[0][0])[i] = masks[(size_t)blockIdx.x * (kPtWords * kPtMasks) + i];
+    if (threadIdx.x < kPtMasks)
+        car[threadIdx.x] = (int)reinterpret_cast<const unsigned *>(carry + 2 * (size_t)blockIdx.x)[threadIdx.x];
+    __syncthreads();
+    if (w < kPtMasks) {  // points of the tile before each word
+        const int c0 = __popc(sm[2 * lane][w]), c1 = __popc(sm[2 * lane + 1][w]);
+        int inc = c0 + c1;
 #pragma unroll
-        for (int k = 0; k < kPtItems; k++) {
-            sd[k] = ((unsigned)sdp[k] >> (8 * d)) & 0xffu;
-            if (headmask >> k & 1) {
-                f = 1;
-                v = 0;
-            }
-            v += side_count(sd[k]);
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(FULL, inc, o);
+            if (lane >= o) inc += v;
         }
-        unsigned vi[1] = {v};
-        unsigned fi = f;
-        warp_seg_scan<1>(fi, vi, lane);
-        if (lane == 31) {
-            wf[w] = fi;
-            wv[w] = vi[0];
-        }
-        __syncthreads();
-        unsigned pf = 0, pv = 0;
-        for (int q = 0; q < w; q++) {
-            pv = wf[q] ? wv[q] : pv + wv[q];
-            pf |= wf[q];
-        }
-        unsigned ef = __shfl_up_sync(0xffffffffu, fi, 1);
-        unsigned ev = __shfl_up_sync(0xffffffffu, vi[0], 1);
-        if (lane == 0) ef = ev = 0;
-        // the tile's counts before this thread's first position
-        unsigned runf = pf | ef, runv = ef ? ev : pv + ev;
-        __syncthreads();  // wf / wv are written again for the next order
-        int pt[kPtItems];
-        double cv[kPtItems];
-        load8(ain, base, n_u, pt);
-        if (full) {
-            const double2 *cp = reinterpret_cast<const double2 *>(cin + base);
+        pre[w][2 * lane] = inc - c0 - c1;
+        pre[w][2 * lane + 1] = inc - c1;
+    }
+    __syncthreads();
+#pragma unroll 2
+    for (int k = 0; k < kPtRounds; k++) {
+        const int wd = w * kPtRounds + k, i = base + 32 * wd + lane;
+        if (i >= n_u) break;
+        const int s = pos_seg[i];
+        int pt[3];
+        double cv[3];
 #pragma unroll
-            for (int k = 0; k < kPtItems / 2; k++) {
-                const double2 t = __ldg(cp + k);
-                cv[2 * k] = t.x;
-                cv[2 * k + 1] = t.y;
-            }
-        } else {
-#pragma unroll
-            for (int k = 0; k < kPtItems; k++) cv[k] = base + k < n_u ? cin[base + k] : 0.0;
+        for (int d = 0; d < 3; d++) {
+            pt[d] = io.a[d][i];
+            cv[d] = io.c[d][i];
         }
+        int l = i, r = i, med = i, next = -1, at = 0;
+        if (s >= 0) {
+            l = sg.l[s];
+            r = sg.r[s];
+            med = (l + r + 1) / 2;
+            if (i != med) next = 2 * s + (i > med);
+            at = l - base;  // the segment's start in the tile, or before it
+        }
+        pos_next[i] = next;
 #pragma unroll
-        for (int k = 0; k < kPtItems; k++) {
-            const int i = base + k;
-            if (i >= n_u) break;
+        for (int d = 0; d < 3; d++) {
             int dst = i;
-            if (sgi[k] >= 0) {
-                if (headmask >> k & 1) {
-                    runf = 1;
-                    runv = 0;
+            if (s >= 0) {
+                const int sd = (sm[wd][2 * d] >> lane & 1u) ? 0 : ((sm[wd][2 * d + 1] >> lane & 1u) ? 1 : 2), q = 2 * d + sd;
+                dst = med;
+                if (sd < 2) {
+                    int c = pre[q][wd] + __popc(sm[wd][q] & ((1u << lane) - 1u));
+                    if (at >= 0) c -= pre[q][at >> 5] + __popc(sm[at >> 5][q] & ((1u << (at & 31)) - 1u));
+                    else c += car[q];
+                    dst = (sd == 0 ? l : med + 1) + c;
                 }
-                unsigned L = runv & 0xffffu, R = runv >> 16;
-                if (!runf) {  // the segment began in an earlier tile
-                    L += crl;
-                    R += crr;
-                }
-                const int s = sgi[k], l = sg.l[s], r = sg.r[s], med = (l + r + 1) / 2;
-                dst = sd[k] == 0 ? l + (int)L : (sd[k] == 1 ? med + 1 + (int)R : med);
                 if (dst < l || dst > r) {
                     set_err(err, KD_EINTERNAL);
-                    dst = -1;
+                    continue;
                 }
-                runv += side_count(sd[k]);
             }
-            if (dst >= 0) {
-                aout[dst] = pt[k];
-                cout[dst] = cv[k];
-            }
+            io.ao[d][dst] = pt[d];
+            io.co[d][dst] = cv[d];
         }
-    }
-}
-
-__global__ void k_children(Segs cur, int ub, LevelBufs lb, Segs nxt, int cap, int *err)
-{
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= ub) return;
-    int ns = *cur.count;
-    if (s == 0) *nxt.count = ns > 0 ? 2 * (lb.rank[ns - 1] + lb.haskids[ns - 1]) : 0;
-    if (s >= ns || !lb.haskids[s]) return;
-    int p = cur.p[s], l = cur.l[s], r = cur.r[s];
-    int med = (l + r + 1) / 2;
-    int c = 2 * lb.rank[s];
-    if (c + 1 >= cap) {
-        set_err(err, KD_EINTERNAL);
-        return;
-    }
-    nxt.p[c] = 2 * p;
-    nxt.l[c] = l;
-    nxt.r[c] = med - 1;
-    nxt.p[c + 1] = 2 * p + 1;
-    nxt.l[c + 1] = med + 1;
-    nxt.r[c + 1] = r;
-}
-
-__global__ void k_next_pos(int n_u, const int *__restrict__ pos_seg, Segs sg, LevelBufs lb,
-                           int *pos_next)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_u; i += gridDim.x * blockDim.x) {
-        int s = pos_seg[i];
-        int v = -1;
-        if (s >= 0 && lb.haskids[s]) {
-            int med = (sg.l[s] + sg.r[s] + 1) / 2;
-            if (i != med) v = 2 * lb.rank[s] + (i > med);
-        }
-        pos_next[i] = v;
     }
 }
 
@@ -2488,7 +2386,7 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
     to.inorder_rep = keep.alloc<int>(n_u);
     check(cudaMemsetAsync(to.nodes, 0, sizeof(NodeRec) * (size_t)memsize, s), "memset");
 
-    int cap = n_u / 2 + 16;
+    const int cap = n_u / (kSubCap / 4) + 16;  // segments of the level loop, and those it leaves
     Segs sg[2];
     for (int k = 0; k < 2; k++) {
         sg[k].p = pool.alloc<int>(cap);
@@ -2502,21 +2400,15 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
     lb.big = pool.alloc<unsigned char>(cap);
     lb.fallback = pool.alloc<unsigned char>(cap);
     lb.acc = pool.alloc<double>(9 * (size_t)lb.cap_big);
-    lb.rank = pool.alloc<int>(cap);
-    lb.haskids = pool.alloc<int>(cap);
-    int *pos[2] = {pool.alloc<int>(n_u), pool.alloc<int>(n_u)};
+    int *pos[2] = {pool.alloc<int>(n_u), pool.alloc<int>(n_u)}, *place = pool.alloc<int>(n_u);
     unsigned char *side = pool.alloc<unsigned char>(n_u);
     const int ntiles = (int)((n_u + (long long)kPtTile - 1) / kPtTile);
+    unsigned *masks = pool.alloc<unsigned>((size_t)ntiles * (kPtWords * kPtMasks));
     uint4 *tagg = pool.alloc<uint4>(ntiles), *tcarry = pool.alloc<uint4>(2 * (size_t)ntiles);
-    unsigned *sd_pos = pool.alloc<unsigned>(n_u);
     {
-        int one = 1, zero = 0, last = n_u - 1;
-        check(cudaMemcpyAsync(sg[0].count, &one, sizeof(int), cudaMemcpyHostToDevice, s), "H2D");
-        check(cudaMemcpyAsync(sg[0].p, &one, sizeof(int), cudaMemcpyHostToDevice, s), "H2D");
-        check(cudaMemcpyAsync(sg[0].l, &zero, sizeof(int), cudaMemcpyHostToDevice, s), "H2D");
-        check(cudaMemcpyAsync(sg[0].r, &last, sizeof(int), cudaMemcpyHostToDevice, s), "H2D");
         check(cudaMemsetAsync(pos[0], 0, sizeof(int) * (size_t)n_u, s), "memset");
-        st.sync();  // the host scalars above go out of scope
+        k_first_seg<<<1, 1, 0, s>>>(sg[0], n_u);
+        KD_LAUNCH_CHECK("k_first_seg");
     }
     // The node array goes to the caller's host array level by level while
     // the tree is built: iteration lev of the loop below writes the heap
@@ -2586,16 +2478,6 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
         }
     }
 
-    // the partition kernels read and write these with 16-byte vector
-    // accesses at multiples of 8 elements: stream-ordered allocations are
-    // aligned far beyond that, which is checked here rather than assumed
-    {
-        const void *vec[] = {pos[0], pos[1], A[0], A[1], A[2], B[0], B[1], B[2],
-                             C[0],   C[1],   C[2], CB[0], CB[1], CB[2], sd_pos};
-        for (const void *p : vec)
-            if ((reinterpret_cast<uintptr_t>(p) & 15) != 0)
-                raise(KD_EINTERNAL, "build array not 16-byte aligned");
-    }
     check(cudaFuncSetAttribute(k_subtrees, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)sizeof(SubSmem)), "smem attribute");
     int cur = 0, nlevels = 0;
@@ -2608,12 +2490,11 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
         long long maxsize = (long long)n_u >> lev;
         if (maxsize <= kSubCap) {  // the rest of the tree, a CTA per segment
             while ((n_u >> (nlevels - 1)) >= 4) nlevels++;
-            k_subtrees<<<ub, kSubThreads, sizeof(SubSmem), s>>>(S, A[0], A[1], A[2], u, to,
-                                                                reinterpret_cast<int *>(sd_pos), err);
+            k_subtrees<<<ub, kSubThreads, sizeof(SubSmem), s>>>(S, A[0], A[1], A[2], u, to, place, err);
             KD_LAUNCH_CHECK("k_subtrees");
             break;
         }
-        k_seg_setup<<<gs, TPB, 0, s>>>(S, ub, lb);
+        k_seg_setup<<<gs, TPB, 0, s>>>(S, ub, lb, N);
         if (maxsize > kSmallSeg) {
             unsigned gv = blocks_for(n_u, kVarChunk);
             k_var_par<0><<<gv, kVarThreads, 0, s>>>(n_u, pos[cur], S, lb, C[0], C[1], C[2]);
@@ -2632,7 +2513,7 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
         k_mark<<<grid_for(n_u), TPB, 0, s>>>(n_u, pos[cur], S, lb, A[0], A[1], A[2], side);
         {
             k_part_count<<<ntiles, kPtThreads, 0, s>>>(n_u, pos[cur], S, A[0], A[1], A[2], side,
-                                                       sd_pos, tagg);
+                                                       masks, tagg);
             k_part_carry<<<1, 1024, 0, s>>>(ntiles, tagg, tcarry);
             PartIO io;
             for (int d = 0; d < 3; d++) {
@@ -2641,15 +2522,13 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
                 io.c[d] = C[d];
                 io.co[d] = CB[d];
             }
-            k_part_move<<<ntiles, kPtThreads, 0, s>>>(n_u, pos[cur], S, io, sd_pos, tcarry, err);
+            k_part_move<<<ntiles, kPtThreads, 0, s>>>(n_u, pos[cur], S, io, masks, tcarry,
+                                                      pos[cur ^ 1], err);
             for (int d = 0; d < 3; d++) {
                 std::swap(A[d], B[d]);
                 std::swap(C[d], CB[d]);
             }
         }
-        excl_sum(pool, s, lb.haskids, lb.rank, ub);
-        k_children<<<gs, TPB, 0, s>>>(S, ub, lb, N, cap, err);
-        k_next_pos<<<grid_for(n_u), TPB, 0, s>>>(n_u, pos[cur], S, lb, pos[cur ^ 1]);
         KD_LAUNCH_CHECK("partition kernels");
         cur ^= 1;
     }
