@@ -68,14 +68,11 @@ static_assert(sizeof(NodeRec) == 40, "node_t is 40 bytes");
 
 static const int TPB = 256;
 
-// Segments up to this size get the exact sequential variance directly;
-// larger ones first try the parallel sums with a rigorous interval (one
-// thread walking thousands of gathered points is slow: ~1 us per point).
-constexpr int kSmallSeg = 256;
-// Positions per block in the parallel variance kernels (<= kSmallSeg + 1 so a
-// block touches at most two segments).
-constexpr int kVarChunk = 256;   // positions per k_var_par block
-constexpr int kVarThreads = 64;  // threads per k_var_par block (4 positions each)
+// Positions and threads per block in the parallel variance kernels.  Fewer
+// than the smallest segment of the level loop, so that a block meets at most
+// two of them.
+constexpr int kVarChunk = 512;
+constexpr int kVarThreads = 128;
 
 // Once per device (any thread may get here first; doing it twice is harmless):
 // keep freed stream-ordered allocations in the device's pool instead of
@@ -252,12 +249,14 @@ __global__ void k_gather_u64(const uint64_t *__restrict__ src, const int *__rest
         dst[i] = src[idx[i]];
 }
 
-__global__ void k_heads(const int *__restrict__ p, const uint64_t *kx, const uint64_t *ky,
-                        const uint64_t *kz, int n, int *head)
+// first: points sorted by 32-bit keys of x, where two equal points share one
+// (null: not sorted so); spares most gathers (0.13 ms at 5M points, so 0.02)
+__global__ void k_heads(const int *__restrict__ p, const unsigned *__restrict__ first, const uint64_t *kx,
+                        const uint64_t *ky, const uint64_t *kz, int n, int *head)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         int h = 1;
-        if (i > 0) {
+        if (i > 0 && (!first || first[i] == first[i - 1])) {
             int a = p[i], b = p[i - 1];
             h = (kx[a] != kx[b]) | (ky[a] != ky[b]) | (kz[a] != kz[b]);
         }
@@ -268,27 +267,26 @@ __global__ void k_heads(const int *__restrict__ p, const uint64_t *kx, const uin
 struct UniqueArrays {
     double *ux, *uy, *uz;
     int *ufield, *uw, *urep, *uhead;
-    uint64_t *ukx, *uky, *ukz;
+    uint64_t *uky, *ukz;
 };
 
 // cls[i] = 1-based class number of dedup-sorted position i
 __global__ void k_unique(const int *__restrict__ p, const int *__restrict__ head,
                          const int *__restrict__ cls, int n, const double *__restrict__ xyz,
-                         const int *__restrict__ fin, const uint64_t *kx, const uint64_t *ky,
-                         const uint64_t *kz, UniqueArrays u, int n_u)
+                         const int *__restrict__ fin, UniqueArrays u, int n_u)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         if (!head[i]) continue;
         int c = cls[i] - 1, r = p[i];
-        u.ux[c] = xyz[3 * (size_t)r];
-        u.uy[c] = xyz[3 * (size_t)r + 1];
-        u.uz[c] = xyz[3 * (size_t)r + 2];
+        const double x = xyz[3 * (size_t)r], y = xyz[3 * (size_t)r + 1], z = xyz[3 * (size_t)r + 2];
+        u.ux[c] = x;
+        u.uy[c] = y;
+        u.uz[c] = z;
         u.ufield[c] = fin ? (fin[r] & 0xFF) : 0;
         u.urep[c] = r;
         u.uhead[c] = i;
-        u.ukx[c] = kx[r];
-        u.uky[c] = ky[r];
-        u.ukz[c] = kz[r];
+        u.uky[c] = okey(y);  // (gathered, like that of x: 0.41 ms at 5M points, so 0.16)
+        u.ukz[c] = okey(z);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) u.uhead[n_u] = n;
 }
@@ -338,10 +336,10 @@ struct Segs {
 };
 
 struct LevelBufs {
-    int *tdim;
-    unsigned char *big, *fallback;
-    double *acc;      // per big segment: S0 S1 S2 A0 A1 A2 V0 V1 V2
-    int cap_big;
+    int *tdim;                  // split dimension
+    double *acc;                // S0 S1 S2 A0 A1 A2 V0 V1 V2
+    int *mid;                   // the median point's rank in the split order
+    const int *rank1, *rank2;   // ranks of the points in orders 1 and 2
 };
 
 __global__ void k_first_seg(Segs sg, int n_u)
@@ -361,12 +359,7 @@ __global__ void k_seg_setup(Segs sg, int ub, LevelBufs lb, Segs nxt)
     if (s == 0) *nxt.count = 2 * ns;
     if (s >= ns) return;
     const int p = sg.p[s], l = sg.l[s], r = sg.r[s], med = (l + r + 1) / 2;
-    int big = r - l + 1 > kSmallSeg && s < lb.cap_big;
-    lb.big[s] = (unsigned char)big;
-    lb.fallback[s] = 0;
-    lb.tdim[s] = 0;
-    if (big)
-        for (int k = 0; k < 9; k++) lb.acc[9 * (size_t)s + k] = 0.0;
+    for (int k = 0; k < 9; k++) lb.acc[9 * (size_t)s + k] = 0.0;
     nxt.p[2 * s] = 2 * p;
     nxt.l[2 * s] = l;
     nxt.r[2 * s] = med - 1;
@@ -375,8 +368,10 @@ __global__ void k_seg_setup(Segs sg, int ub, LevelBufs lb, Segs nxt)
     nxt.r[2 * s + 1] = r;
 }
 
-// Parallel sums for big segments: pass 0 accumulates S_j = sum v_j and
-// A_j = sum |v_j|; pass 1 accumulates V_j = sum (v_j - S_j/n)^2.
+// Parallel sums per segment: pass 0 accumulates S_j = sum v_j and
+// A_j = sum |v_j|; pass 1 accumulates V_j = sum (v_j - S_j/n)^2.  Bound by
+// memory: 5M points in 30 us and 34 (with 256 positions per block and each
+// load behind its position's segment 47 and 53).
 // c0, c1, c2: the x of the point at each position of superkey order 0, the
 // y along order 1, the z along order 2 (carried through the partitions), so
 // a segment's coordinates are read contiguously; the parallel sums do not
@@ -398,19 +393,19 @@ __global__ void __launch_bounds__(kVarThreads) k_var_par(int n_u, const int *__r
     const int base = blockIdx.x * kVarChunk;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int seg[PER];
+    double x[PER][3];
     int smin = 0x7fffffff;
 #pragma unroll
-    for (int k = 0; k < PER; k++) {
-        const int i = base + threadIdx.x + kVarThreads * k;
-        seg[k] = -1;
-        if (i < n_u) {
-            const int s = pos_seg[i];
-            if (s >= 0 && lb.big[s]) {
-                seg[k] = s;
-                smin = min(smin, s);
-            }
-        }
+    for (int k = 0; k < PER; k++) {  // (every load before the first use)
+        const int i = base + threadIdx.x + kVarThreads * k, j = min(i, n_u - 1);
+        seg[k] = i < n_u ? pos_seg[j] : -1;
+        x[k][0] = c0[j];
+        x[k][1] = c1[j];
+        x[k][2] = c2[j];
     }
+#pragma unroll
+    for (int k = 0; k < PER; k++)
+        if (seg[k] >= 0) smin = min(smin, seg[k]);
     smin = __reduce_min_sync(0xffffffffu, smin);
     if (lane == 0) wmin[w] = smin;
     __syncthreads();
@@ -437,8 +432,7 @@ __global__ void __launch_bounds__(kVarThreads) k_var_par(int n_u, const int *__r
     for (int k = 0; k < PER; k++) {
         const int s = seg[k];
         if (s < 0) continue;
-        const int i = base + threadIdx.x + kVarThreads * k;
-        const double v[3] = {c0[i], c1[i], c2[i]};
+        const double *const v = x[k];
         double c[NV];
         const int slot = s - s0;
         if (PASS == 0) {
@@ -491,7 +485,7 @@ __global__ void __launch_bounds__(kVarThreads) k_var_par(int n_u, const int *__r
         double v = wsum[0][q][j];
 #pragma unroll
         for (int x = 1; x < NW; x++) v += wsum[x][q][j];
-        if (v != 0.0 && s < *sg.count && lb.big[s])
+        if (v != 0.0 && s < *sg.count)
             atomicAdd(&lb.acc[9 * (size_t)s + (PASS == 0 ? 0 : 6) + j], v);
     }
 }
@@ -531,32 +525,16 @@ __device__ __forceinline__ int decide_dim(double n, const double *a)
     return ok ? c : -1;
 }
 
-// Decide the split dimension of a big segment, or mark it for the sequential
-// fallback.
-__global__ void k_var_decide(Segs sg, int ub, LevelBufs lb)
-{
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= ub || s >= *sg.count || !lb.big[s]) return;
-    const int c = decide_dim((double)(sg.r[s] - sg.l[s] + 1), lb.acc + 9 * (size_t)s);
-    if (c >= 0) lb.tdim[s] = c;
-    else lb.fallback[s] = 1;
-}
-
 // max_variance_dim exactly as the reference evaluates it (kdbuild.c:308-351),
 // one thread per segment; the three dimensions' chains are independent and
 // are interleaved for latency hiding without changing any chain's order.
 // c0, c1, c2 as for k_var_par: c_j[i] is coordinate j of the point at
 // position i of superkey order j, so the sums below run over exactly the
 // values, in exactly the order, of the reference's loops over args[j]
-__global__ void k_var_seq(Segs sg, int ub, LevelBufs lb, const double *__restrict__ c0,
-                          const double *__restrict__ c1, const double *__restrict__ c2)
+__device__ __noinline__ int seq_dim(int l, int r, const double *__restrict__ c0, const double *__restrict__ c1,
+                                    const double *__restrict__ c2)
 {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= ub || s >= *sg.count) return;
-    int l = sg.l[s], r = sg.r[s];
-    int size = r - l + 1;
-    if (size < 4) return;
-    if (lb.big[s] && !lb.fallback[s]) return;
+    const int size = r - l + 1;
     double m0 = 0.0, m1 = 0.0, m2 = 0.0;
     int i = l;
     for (; i + 4 <= r + 1; i += 4) {
@@ -614,7 +592,7 @@ __global__ void k_var_seq(Segs sg, int ub, LevelBufs lb, const double *__restric
         dim = 1;
     }
     if (q2 > mx) dim = 2;
-    lb.tdim[s] = dim;
+    return dim;
 }
 
 struct TreeOut {
@@ -642,39 +620,39 @@ __device__ __forceinline__ void put_node(TreeOut t, const UniqueArrays &u, int h
     t.inorder_rep[pos] = u.urep[pt];
 }
 
+// A level's split dimensions, nodes and median ranks, one thread per segment.
 __global__ void k_level_nodes(Segs sg, int ub, LevelBufs lb, const int *__restrict__ a0,
                               const int *__restrict__ a1, const int *__restrict__ a2,
-                              UniqueArrays u, TreeOut t, int *err)
+                              const double *__restrict__ c0, const double *__restrict__ c1,
+                              const double *__restrict__ c2, UniqueArrays u, TreeOut t, int *err)
 {
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= ub || s >= *sg.count) return;
-    const int med = (sg.l[s] + sg.r[s] + 1) / 2, d = lb.tdim[s];
-    const int *ad = d == 0 ? a0 : (d == 1 ? a1 : a2);
-    put_node(t, u, sg.p[s], ad[med], d, 1, 1, med, err);
+    const int l = sg.l[s], r = sg.r[s], med = (l + r + 1) / 2;
+    int d = decide_dim((double)(r - l + 1), lb.acc + 9 * (size_t)s);
+    if (d < 0) d = seq_dim(l, r, c0, c1, c2);
+    const int pt = (d == 0 ? a0 : (d == 1 ? a1 : a2))[med];
+    put_node(t, u, sg.p[s], pt, d, 1, 1, med, err);
+    lb.tdim[s] = d;
+    lb.mid[s] = d == 0 ? pt : (d == 1 ? lb.rank1 : lb.rank2)[pt];
 }
 
-// side of every point of a splitting segment: 0 left, 1 right, 2 median
-__global__ void k_mark(int n_u, const int *__restrict__ pos_seg, Segs sg, LevelBufs lb,
-                       const int *__restrict__ a0, const int *__restrict__ a1,
-                       const int *__restrict__ a2, unsigned char *side)
+__global__ void k_ranks(int n, const int *__restrict__ a1, const int *__restrict__ a2, int *rank1, int *rank2)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_u; i += gridDim.x * blockDim.x) {
-        int s = pos_seg[i];
-        if (s < 0) continue;
-        int l = sg.l[s], r = sg.r[s];
-        if (r - l + 1 < 4) continue;
-        int med = (l + r + 1) / 2;
-        int d = lb.tdim[s];
-        const int *ad = d == 0 ? a0 : (d == 1 ? a1 : a2);
-        side[ad[i]] = i < med ? 0 : (i == med ? 2 : 1);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        rank1[a1[i]] = i;
+        rank2[a2[i]] = i;
     }
 }
 
+// side of every point of a splitting segment: 0 left, 1 right, 2 median
 // ---- Stable three-way partition of the three superkey orders, one level.
 // Within every segment [l, r], median position med = (l + r + 1) / 2, the
-// points of each order d go, in their order, to [l, med) when k_mark put them
-// left of the median (side 0), to (med, r] when right (side 1), the median
-// point itself to med; positions outside segments stay.  The destination of a
+// points of each order d go, in their order, to [l, med) when they stand before
+// the median point in the order of the split dimension (side 0), to (med, r]
+// when behind it (side 1), the median point itself to med; positions outside
+// segments stay.  The side follows from the ranks that the points have in the
+// whole sorted orders (a point's id is its rank in order 0).  The destination of a
 // point is its segment's start plus the number of same-side points before it
 // in the segment.  Three launches over tiles of kPtTile positions handle all
 // three orders at once, with no waiting between blocks: per 32 positions, a
@@ -685,7 +663,8 @@ __global__ void k_mark(int n_u, const int *__restrict__ pos_seg, Segs sg, LevelB
 // a warp's stores two runs.  Bound by memory: with eight consecutive positions
 // per thread, whose stores met a line once per position, the move of 5M points
 // took 150 us a level (and 20 for the next level's segments, written here),
-// now 83; the counts 57, now 47.
+// now 83; the counts 57 after 45 for a kernel that marked each point's side, which
+// the ranks spare, now 62.
 constexpr int kPtThreads = 256;
 constexpr int kPtWarps = kPtThreads / 32;
 constexpr int kPtRounds = 8;                      // positions per thread
@@ -726,8 +705,7 @@ __device__ __forceinline__ void warp_seg_scan(unsigned &f, unsigned (&v)[NV], in
 __global__ void __launch_bounds__(kPtThreads) k_part_count(int n_u, const int *__restrict__ pos_seg,
                                                            Segs sg, const int *__restrict__ a0,
                                                            const int *__restrict__ a1,
-                                                           const int *__restrict__ a2,
-                                                           const unsigned char *__restrict__ side,
+                                                           const int *__restrict__ a2, LevelBufs lb,
                                                            unsigned *masks, uint4 *tagg)
 {
     constexpr unsigned FULL = 0xffffffffu;
@@ -736,18 +714,26 @@ __global__ void __launch_bounds__(kPtThreads) k_part_count(int n_u, const int *_
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int base = blockIdx.x * kPtTile;
     int sd[kPtRounds][3];
-    bool in[kPtRounds];
 #pragma unroll
     for (int k = 0; k < kPtRounds; k++) {
         const int wd = w * kPtRounds + k, i = base + 32 * wd + lane;
         const int seg = i < n_u ? pos_seg[i] : -1;
-        in[k] = seg >= 0;
-        const unsigned h = __ballot_sync(FULL, in[k] && sg.l[in[k] ? seg : 0] == i);
+        const bool in = seg >= 0;
+        const int l = in ? sg.l[seg] : 0, r = in ? sg.r[seg] : 0, dim = in ? lb.tdim[seg] : 0,
+                  mid = in ? lb.mid[seg] : 0, med = (l + r + 1) / 2;
+        const unsigned h = __ballot_sync(FULL, in && l == i);
         if (lane == 0) heads[wd] = h;
 #pragma unroll
         for (int d = 0; d < 3; d++) {
             sd[k][d] = 3;
-            if (in[k]) sd[k][d] = side[(d == 0 ? a0 : (d == 1 ? a1 : a2))[i]];
+            if (!in) continue;
+            int at = i, than = med;  // the split order itself: by place
+            if (d != dim) {
+                const int pt = (d == 0 ? a0 : (d == 1 ? a1 : a2))[i];
+                at = dim == 0 ? pt : (dim == 1 ? lb.rank1 : lb.rank2)[pt];
+                than = mid;
+            }
+            sd[k][d] = at < than ? 0 : (at > than ? 1 : 2);
         }
     }
 #pragma unroll
@@ -927,7 +913,7 @@ __global__ void __launch_bounds__(kPtThreads) k_part_move(int n_u, const int *__
 // together, with the points as 16-bit places in the segment's order 0.  Every
 // point is read once and every node written once, where the level loop reads
 // and writes ~180 bytes per point and level in twelve launches: the last ten
-// levels of a 5M-point build took 3.7 ms there and take 1.8 ms here, all levels
+// levels of a 5M-point build took 3.7 ms there and take 1.6 ms here, all levels
 // of a 4000-point build 0.93 and 0.39 ms.  What bounds it is the latency of its
 // shared-memory gathers and the barriers between its steps (a third of the
 // issue slots are used, with four blocks per SM).  1024 points: a larger cap
@@ -938,7 +924,8 @@ constexpr int kSubSeq = 48;  // segments up to this size: one thread, sequential
 
 struct SubSmem {
     double v[3][kSubCap];               // coordinates by place
-    int gid[kSubCap];                   // unique-point ids by place
+    uint32_t fw[kSubCap];               // field | weight << 8 by place
+    int rep[kSubCap];                   // input indices by place
     unsigned short o[2][3][kSubCap];    // the three orders: places by position
     short seg[2][kSubCap];              // position -> segment of the level, -1: none
     short l[2][kSubCap / 2 + 1], r[2][kSubCap / 2 + 1];  // segments: positions [l, r]
@@ -995,7 +982,8 @@ __global__ void __launch_bounds__(kSubThreads) k_subtrees(Segs sg, const int *__
     // places: positions in order 0; the other orders through the point's place
     for (int i = tid; i < m; i += kSubThreads) {
         const int pt = a0[base + i];
-        s.gid[i] = pt;
+        s.fw[i] = (uint32_t)u.ufield[pt] | ((uint32_t)u.uw[pt] << 8);
+        s.rep[i] = u.urep[pt];
         s.o[0][0][i] = (unsigned short)i;
         place[pt] = i;
         s.v[0][i] = u.ux[pt];
@@ -1016,6 +1004,22 @@ __global__ void __launch_bounds__(kSubThreads) k_subtrees(Segs sg, const int *__
     }
     __syncthreads();
     const int words = (m + 31) / 32;
+    auto node = [&](int hp, int pl, int dim, int hl, int hr, int pos) {
+        if (hp >= t.memsize) {
+            set_err(err, KD_EINTERNAL);
+            return;
+        }
+        NodeRec rec;
+        rec.v[0] = s.v[0][pl];
+        rec.v[1] = s.v[1][pl];
+        rec.v[2] = s.v[2][pl];
+        rec.fw = s.fw[pl];
+        rec.pad0 = 0;
+        rec.flags = (uint32_t)hl | ((uint32_t)hr << 1) | ((uint32_t)dim << 2);
+        rec.pad1 = 0;
+        t.nodes[hp] = rec;
+        t.inorder_rep[base + pos] = s.rep[pl];
+    };
     int cur = 0;
     for (int lev = 0;; lev++) {
         const int nseg = 1 << lev;
@@ -1062,22 +1066,24 @@ __global__ void __launch_bounds__(kSubThreads) k_subtrees(Segs sg, const int *__
             if (n >= 4 && n <= kSubSeq) s.tdim[g] = (unsigned char)sub_var_seq(s, o, l, r);
         }
         __syncthreads();
-        // ---- the level's nodes (k_level_nodes)
+        // ---- the level's nodes, from shared memory (with their points gathered
+        // here, by the few threads that hold a segment, the kernel took a third
+        // more: 1.9 ms at 5M points instead of 1.6)
         for (int g = tid; g < nseg; g += kSubThreads) {
             const int l = L[g], r = R[g], n = r - l + 1;
             const int p = (int)((root << lev) + g);
             if (n >= 4) {
                 const int med = (l + r + 1) / 2, d = s.tdim[g];
-                put_node(t, u, p, s.gid[o[d][med]], d, 1, 1, base + med, err);
+                node(p, o[d][med], d, 1, 1, med);
             } else if (n == 3) {
-                put_node(t, u, p, s.gid[o[0][l + 1]], 0, 1, 1, base + l + 1, err);
-                put_node(t, u, 2 * p, s.gid[o[0][l]], 0, 0, 0, base + l, err);
-                put_node(t, u, 2 * p + 1, s.gid[o[0][r]], 0, 0, 0, base + r, err);
+                node(p, o[0][l + 1], 0, 1, 1, l + 1);
+                node(2 * p, o[0][l], 0, 0, 0, l);
+                node(2 * p + 1, o[0][r], 0, 0, 0, r);
             } else if (n == 2) {
-                put_node(t, u, p, s.gid[o[0][r]], 0, 1, 0, base + r, err);
-                put_node(t, u, 2 * p, s.gid[o[0][l]], 0, 0, 0, base + l, err);
+                node(p, o[0][r], 0, 1, 0, r);
+                node(2 * p, o[0][l], 0, 0, 0, l);
             } else if (n == 1) {
-                put_node(t, u, p, s.gid[o[0][l]], 0, 0, 0, base + l, err);
+                node(p, o[0][l], 0, 0, 0, l);
             }
         }
         if ((m >> lev) < 4) break;  // every segment was a base case
@@ -2312,7 +2318,7 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
 
     // ---- runs of equal points
     int *head = pool.alloc<int>(n), *cls = pool.alloc<int>(n);
-    k_heads<<<grid_for(n), TPB, 0, s>>>(p3, kx, ky, kz, n, head);
+    k_heads<<<grid_for(n), TPB, 0, s>>>(p3, by_all ? nullptr : cs.srt, kx, ky, kz, n, head);
     incl_sum(pool, s, head, cls, n);
     int n_u = read1(cls + (n - 1), s);
 
@@ -2324,10 +2330,9 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
     u.uw = pool.alloc<int>(n_u);
     u.urep = pool.alloc<int>(n_u);
     u.uhead = pool.alloc<int>(n_u + 1);
-    u.ukx = pool.alloc<uint64_t>(n_u);
     u.uky = pool.alloc<uint64_t>(n_u);
     u.ukz = pool.alloc<uint64_t>(n_u);
-    k_unique<<<grid_for(n), TPB, 0, s>>>(p3, head, cls, n, xyz, fin, kx, ky, kz, u, n_u);
+    k_unique<<<grid_for(n), TPB, 0, s>>>(p3, head, cls, n, xyz, fin, u, n_u);
     FieldInfo *fi = pool.alloc<FieldInfo>(1);
     FieldInfo fi0 = {0x7fffffff, -0x7fffffff, 0, 0};
     check(cudaMemcpyAsync(fi, &fi0, sizeof fi0, cudaMemcpyHostToDevice, s), "H2D");
@@ -2395,13 +2400,17 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
         sg[k].count = pool.alloc<int>(1);
     }
     LevelBufs lb;
-    lb.cap_big = n_u / kSmallSeg + 16;
     lb.tdim = pool.alloc<int>(cap);
-    lb.big = pool.alloc<unsigned char>(cap);
-    lb.fallback = pool.alloc<unsigned char>(cap);
-    lb.acc = pool.alloc<double>(9 * (size_t)lb.cap_big);
+    lb.acc = pool.alloc<double>(9 * (size_t)cap);
     int *pos[2] = {pool.alloc<int>(n_u), pool.alloc<int>(n_u)}, *place = pool.alloc<int>(n_u);
-    unsigned char *side = pool.alloc<unsigned char>(n_u);
+    lb.mid = pool.alloc<int>(cap);
+    if (n_u > kSubCap) {
+        int *r1 = pool.alloc<int>(n_u), *r2 = pool.alloc<int>(n_u);
+        k_ranks<<<grid_for(n_u), TPB, 0, s>>>(n_u, A[1], A[2], r1, r2);
+        KD_LAUNCH_CHECK("k_ranks");
+        lb.rank1 = r1;
+        lb.rank2 = r2;
+    }
     const int ntiles = (int)((n_u + (long long)kPtTile - 1) / kPtTile);
     unsigned *masks = pool.alloc<unsigned>((size_t)ntiles * (kPtWords * kPtMasks));
     uint4 *tagg = pool.alloc<uint4>(ntiles), *tcarry = pool.alloc<uint4>(2 * (size_t)ntiles);
@@ -2495,14 +2504,11 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
             break;
         }
         k_seg_setup<<<gs, TPB, 0, s>>>(S, ub, lb, N);
-        if (maxsize > kSmallSeg) {
-            unsigned gv = blocks_for(n_u, kVarChunk);
-            k_var_par<0><<<gv, kVarThreads, 0, s>>>(n_u, pos[cur], S, lb, C[0], C[1], C[2]);
-            k_var_par<1><<<gv, kVarThreads, 0, s>>>(n_u, pos[cur], S, lb, C[0], C[1], C[2]);
-            k_var_decide<<<gs, TPB, 0, s>>>(S, ub, lb);
-        }
-        k_var_seq<<<blocks_for(ub, 64), 64, 0, s>>>(S, ub, lb, C[0], C[1], C[2]);
-        k_level_nodes<<<gs, TPB, 0, s>>>(S, ub, lb, A[0], A[1], A[2], u, to, err);
+        const unsigned gv = blocks_for(n_u, kVarChunk);
+        k_var_par<0><<<gv, kVarThreads, 0, s>>>(n_u, pos[cur], S, lb, C[0], C[1], C[2]);
+        k_var_par<1><<<gv, kVarThreads, 0, s>>>(n_u, pos[cur], S, lb, C[0], C[1], C[2]);
+        k_level_nodes<<<blocks_for(ub, 64), 64, 0, s>>>(S, ub, lb, A[0], A[1], A[2], C[0], C[1], C[2], u, to,
+                                                        err);
         KD_LAUNCH_CHECK("level kernels");
         // levels 0 .. lev are final: copy their slots once they are large
         // enough to be worth a copy of their own
@@ -2510,10 +2516,9 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
             const size_t upto = sizeof(NodeRec) * std::min<size_t>((size_t)2 << lev, memsize);
             if (upto - node_queued >= ((size_t)4 << 20)) queue_nodes(upto);
         }
-        k_mark<<<grid_for(n_u), TPB, 0, s>>>(n_u, pos[cur], S, lb, A[0], A[1], A[2], side);
         {
-            k_part_count<<<ntiles, kPtThreads, 0, s>>>(n_u, pos[cur], S, A[0], A[1], A[2], side,
-                                                       masks, tagg);
+            k_part_count<<<ntiles, kPtThreads, 0, s>>>(n_u, pos[cur], S, A[0], A[1], A[2], lb, masks,
+                                                       tagg);
             k_part_carry<<<1, 1024, 0, s>>>(ntiles, tagg, tcarry);
             PartIO io;
             for (int d = 0; d < 3; d++) {
