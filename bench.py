@@ -601,10 +601,11 @@ def _summary(w, m, steps, peak, peak64, D):
                 "flop_per_pair": FLOP_PER_PAIR}
     if TILE_TRAFFIC_PER_PAIR:
         roofline["traffic_source"] = TILE_TRAFFIC_SOURCE
-    # FP32-pipe model of the binning itself: per pair 3 FMA lane-ops for
-    # the distance and 3 per active edge (ramp, count, band check)
+    # FP32-pipe model of the binning itself: 3 FMA lane-ops per pair and
+    # active edge (ramp, count, band check); the distances are on the tensor
+    # pipe
     kbar = mixed["edge_pairs"] / max(1, mixed["pairs"])
-    ops = 3.0 + 3.0 * kbar
+    ops = 3.0 * kbar
     pipe_bound = 128.0 * nsm * mhz * 1e6 / ops if (nsm and mhz) else None
     tile_rate = launch_pairs / (launch_ms * 1e-3)
     pipe_model = {"active_edges_per_pair": kbar, "fma_lane_ops_per_pair": ops,
@@ -731,13 +732,13 @@ def run_mine(args):
 
 
 # Per-pair DRAM traffic of the tile kernel (dram bytes read + written by one
-# k_tiles launch over the pairs it tested), from the ncu capture of the
-# clustered workload at scale 0.3 summarised in profiles/, scaled to a full
-# launch by its pairs: the traffic is mostly the tile records, whose number
-# grows with the pairs.
-TILE_TRAFFIC_PER_PAIR = (3.271633e9 + 11.673856e6) / 2.02520e11  # bytes per pair tested
+# k_tiles launch over the pairs it tested), from an ncu capture of 1M uniform
+# points with themselves (64 fields, 21 log-spaced edges), scaled to a launch by
+# its pairs: the traffic is mostly the tile records, whose number grows with
+# the pairs.
+TILE_TRAFFIC_PER_PAIR = (1.89379072e8 + 3.620096e6) / 4.5997e10  # bytes per pair tested
 TILE_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of one k_tiles launch, "
-                       "clustered workload at scale 0.3 (2.025e11 pairs), scaled by pairs")
+                       "1M uniform points with themselves (4.6e10 pairs), scaled by pairs")
 
 
 # ------------------------------------------------------- reference (CPU) arm

@@ -27,9 +27,9 @@
 // are processed together.  Positions of the three superkey-ordered index arrays
 // are grouped in contiguous segments, one per subtree.  A level computes every
 // segment's split dimension, writes the level's nodes, then moves every
-// position to its child segment with a stable segmented partition (two global
-// prefix sums packed into one 64-bit scan).  Split dimensions of large
-// segments come from a parallel variance with a rigorous error interval around
+// position to its child segment with a stable segmented partition; segments of
+// up to kSubCap points go through all their remaining levels in one block's
+// shared memory.  Split dimensions of segments of more than kSubSeq points come from a parallel variance with a rigorous error interval around
 // the value the reference's sequential sums produce; only when the intervals of
 // the best and another dimension overlap is the sequential computation run.
 
@@ -2421,12 +2421,11 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
     }
     // The node array goes to the caller's host array level by level while
     // the tree is built: iteration lev of the loop below writes the heap
-    // slots of level lev (and, for segments of at most three points, their
-    // children), so once it has run, every slot below 2^(lev+1) is final.
-    // The build records an event after each iteration and queues that
-    // level's slots; a second host thread waits for each event and copies
-    // the slots (pinned staging, DMA on its own stream) while the build
-    // goes on, then the rest once the loop ends, during the counting layout.
+    // slots of level lev, so once it has run, every slot below 2^(lev+1) is
+    // final; k_subtrees writes all others.  The build records an event where
+    // slots worth a copy are final and queues them; a second host thread waits
+    // for each event and copies the slots (pinned staging, DMA on its own
+    // stream) while the build goes on.
     std::unique_ptr<NodeCopy> ncu(new NodeCopy);
     NodeCopy &nc = *ncu;
     const size_t node_bytes = sizeof(NodeRec) * (size_t)memsize;

@@ -329,19 +329,25 @@ __global__ void __launch_bounds__(32 * kTravWarps) k_traverse(const JobDesc *__r
 // edges: 7% and 4% slower; compares as integers, on the ALU: 4%).  Bound by
 // the issue slots, then the FP64 pipe (73% and 64% used).
 //
-// Bound: the FP32 pipe, by the binning (a ramp, a count and a check per pair
-// and edge: 15 clocks per 128 pairs and edge in isolation, 20 here), then the
-// per-pass work around it.  Seven CTAs per SM: what is uniform over a block
-// lives in shared memory so that 72 registers do (four warps per scheduler and
-// 128 registers: 31.5 ms for 3M uniform points and 21 edges, seven: 23.8; the
-// former kernel, a warp per block with four queries per lane and one window:
-// 36.2.  1 edge: 10.8 against 16.4.  FP64 mode: 37.3 against 51.0).  CTA per
-// block instead of warp per block also gives small counts four times the
-// warps: 0.31 against 1.72 ms for DD + DR + RR of 4k / 80k points.
+// Bound: the issue slots (73% used) and the FP32 pipe (51%), by the binning (a
+// ramp, a count and a check per pair and edge: 15 clocks per 128 pairs and edge
+// in isolation, 20 here) and the per-pass work around it: 289 instructions per
+// 16 queries x 50 points and two edges, 120 of them the binning.  More code is
+// slower (loops unrolled by two or four: 15 to 35%), the instruction cache
+// decides.  Seven CTAs per SM: what is uniform over a block lives in shared
+// memory so that 72 registers do.  In the counting layout of that time, 3M
+// uniform points and 21 edges took 36.2 ms in the former kernel (a warp per
+// block, four queries per lane, one window), 31.5 with four warps per scheduler
+// and 128 registers, 23.8 with seven; 1 edge 10.8 against 16.4; FP64 mode 37.3
+// against 51.0.  CTA per block instead of warp per block also gives small
+// counts four times the warps: 0.31 against 1.72 ms for DD + DR + RR of
+// 4k / 80k points.
 // Measured and left out: tcgen05 with the batch's distances in TMEM (free
 // distances, but 128 queries in step and the same binning: 45.7 ms); items of
 // one query tile and one edge, four at a time, repeating the MMA (39.3); two
-// query tiles per pass where their windows agree on two edges (24.1).
+// query tiles per pass where their windows agree on two edges (24.1); six and
+// eight CTAs per SM (3% and 1% slower); four to sixteen records a fetch (0 to
+// 7% slower).
 
 constexpr int kMT = 16;                       // queries per tile (MMA rows)
 constexpr int kMTiles = KD_BLOCK_MAX / kMT;   // query tiles per block
