@@ -1295,7 +1295,10 @@ struct Cells {
 // CTA per chunk: keys of 20 bits of the coordinate within the segment's box
 // and the point's place, sorted in every segment at once by a bitonic network
 // (registers, then lanes, then shared memory); positions behind the last point
-// sort last.  Bound by the latency of the network's steps and barriers.
+// sort last.  Bound by the latency of the network's steps and barriers.  Chunks
+// (and cells) of 4096 points made the counts of large catalogs 1 to 2% faster
+// (fewer partly filled leaves) and a call with 1000 points 7% slower; of 1024,
+// neither.  5M points: 0.8 ms.
 constexpr int kChunk = 2048;
 constexpr int kCut = 16;
 constexpr int kRefThreads = kChunk / 4;  // thread t: positions 4 t .. 4 t + 3
