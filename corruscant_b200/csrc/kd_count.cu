@@ -1050,14 +1050,17 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                     P[e * kPStride + tid] = 0;
                     const unsigned v = cum - before;
                     before = cum;
+                    const bool wide = __any_sync(FULL, v >> 27);  // 32 of them may pass 2^32
                     unsigned rem = vm;
                     while (rem) {  // one round per distinct own field of the warp
                         const int from = __ffs(rem) - 1;
                         const int f = __shfl_sync(FULL, qf, from);
                         const bool same = qf == f;
-                        const unsigned sum = __reduce_add_sync(FULL, same ? v : 0u);
+                        unsigned long long sum = __reduce_add_sync(FULL, same ? (wide ? v & 0xFFFFu : v) : 0u);
+                        if (wide)
+                            sum += (unsigned long long)__reduce_add_sync(FULL, same ? v >> 16 : 0u) << 16;
                         if (lane == from && sum)
-                            atomicAdd(&Hd[((size_t)e * J.Fqe + f) * J.Fte + tf], (unsigned long long)sum);
+                            atomicAdd(&Hd[((size_t)e * J.Fqe + f) * J.Fte + tf], sum);
                         rem &= ~__ballot_sync(FULL, same);
                     }
                 }
