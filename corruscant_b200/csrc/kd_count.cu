@@ -450,8 +450,9 @@ __device__ __forceinline__ uint32_t split_halves(float v)
     return (uint32_t)__half_as_ushort(hi) | ((uint32_t)__half_as_ushort(lo) << 16);
 }
 
-// FP64 mode: a query's pairs with np pairs of staged points (a missing one is at
-// 1e300) below the ne first edges of R (ne <= K <= kFpEdges)
+// FP64 mode: a query's pairs with np pairs of staged points (a missing one is
+// NaN: its distance is below no edge, while any number could be a query's own
+// place) below the ne first edges of R (ne <= K <= kFpEdges)
 constexpr int kFpEdges = 6;
 template <int K>
 __device__ __forceinline__ void fp64_run(const double2 *__restrict__ tx,
@@ -992,9 +993,9 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                                 for (int h = 0; h < 2; h++) {
                                     const int j = lane + 32 * h;
                                     if (j < ((n + 3) & ~3)) {
-                                        s.pt[w][0][j] = j < n ? px[h] : 1e300;
-                                        s.pt[w][1][j] = j < n ? py[h] : 1e300;
-                                        s.pt[w][2][j] = j < n ? pz[h] : 1e300;
+                                        s.pt[w][0][j] = j < n ? px[h] : NAN;
+                                        s.pt[w][1][j] = j < n ? py[h] : NAN;
+                                        s.pt[w][2][j] = j < n ? pz[h] : NAN;
                                     }
                                 }
                             }
