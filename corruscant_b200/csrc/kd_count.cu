@@ -881,8 +881,10 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                             const float gx = fmaxf(ax - ex, 0.0f), gy = fmaxf(ay - ey, 0.0f),
                                         gz = fmaxf(az - ez, 0.0f);
                             const float sx = ax + ex, sy = ay + ey, sz = az + ez;
-                            const float lo2 = (gx * gx + gy * gy + gz * gz) * (1.0f - 4e-6f);
-                            const float hi2 = (sx * sx + sy * sy + sz * sz) * (1.0f + 4e-6f);
+                            // (squares below FLT_MIN are cut to multiples of
+                            // 2^-149: a few of those steps, within 1e-40)
+                            const float lo2 = fmaf(gx * gx + gy * gy + gz * gz, 1.0f - 4e-6f, -1e-40f);
+                            const float hi2 = fmaf(sx * sx + sy * sy + sz * sz, 1.0f + 4e-6f, 1e-40f);
                             int below = 0, upto = 0;  // edges below / not above the pairs
                             for (int k = rk0; k < rk0 + rK; k++) {
                                 below += s.Rup[k] <= lo2;

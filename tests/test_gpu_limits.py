@@ -1,5 +1,5 @@
-"""Counts where the counters' width and the padding of partly filled runs would
-show (exact: integers, no tolerance)."""
+"""Counts where the counters' width, the padding of partly filled runs and the
+exponent range of the FP32 bounds would show (exact: integers, no tolerance)."""
 import numpy as np
 import pytest
 
@@ -53,3 +53,42 @@ def test_query_at_the_largest_coordinates(nt):
     finally:
         N.destroy(t)
         N.destroy(tq)
+
+
+@pytest.mark.parametrize("seed", [0, 1, 2, 3])
+@pytest.mark.parametrize("extent", [1e-15, 1e-18, 1e-19, 1e-20, 1e-21, 3e-22, 1e-22, 5e-23, 3e-23,
+                                    1e-23, 1e-38, 1e-45, 1e-150])
+def test_squares_below_the_normal_range(extent, seed):
+    """Points so close that FP32 squares of their distances are subnormal or
+    zero, alone and beside points far away."""
+    rs = np.random.RandomState(seed)
+    tp, q = extent * rs.rand(256, 3), extent * rs.rand(256, 3)
+    radii = np.linspace(0.05, 1.7, 12) * extent
+    for far in (0, 40):
+        a = np.concatenate([tp, rs.rand(far, 3)])
+        b = np.concatenate([q, rs.rand(far, 3)])
+        r = np.concatenate([radii, [0.2, 0.6]]) if far else radii
+        want = O.OracleTree(a).brute_counts(b, None, 1, r, nthreads=4)
+        t = N.build_tree(a, None, 1)
+        try:
+            for mode in MODES:
+                assert np.array_equal(N.count_points(t, b, None, 1, r, mode=mode), want), (far, mode)
+        finally:
+            N.destroy(t)
+
+
+@pytest.mark.parametrize("gap,radius", [(2.8e-23, 3e-23), (2.6e-23, 2.7e-23), (3.7e-23, 3.8e-23),
+                                        (4.5e-23, 4.4e-23), (1e-22, 0.999e-22)])
+def test_gaps_of_a_few_subnormal_steps(gap, radius):
+    """Two tight groups whose distance's square is a few steps of 2^-149."""
+    rs = np.random.RandomState(3)
+    a, b = 1e-27 * rs.rand(64, 3), 1e-27 * rs.rand(64, 3)
+    b[:, 0] += gap
+    want = O.OracleTree(a).brute_counts(b, None, 1, [radius], nthreads=4)
+    assert want[0, 0] == (4096 if radius > gap else 0)
+    t = N.build_tree(a, None, 1)
+    try:
+        for mode in MODES:
+            assert np.array_equal(N.count_points(t, b, None, 1, [radius], mode=mode), want), mode
+    finally:
+        N.destroy(t)
