@@ -357,6 +357,11 @@ constexpr int kTileWarps = 4;
 constexpr int kTileThreads = 32 * kTileWarps;
 constexpr int kTilesPerSm = 7;                // CTAs per SM the registers are held to
 constexpr int kPStride = 136;                 // counters per edge (128 queries + bank shift)
+// Own fields of a warp's 32 queries that a flush sums over the warp, a round
+// each; with more, every query adds its own counts.  400k points, symmetric, 21
+// edges, labels at random: 4 fields 2.85 ms by rounds and 4.7 by query, 5 3.45
+// and 3.44, 16 10.2 and 8.2, 64 49.3 and 24.9, 250 142.6 and 49.0.
+constexpr int kFlushRounds = 4;
 static_assert(kMTiles == 8 && kTileThreads == KD_BLOCK_MAX, "lane layouts below");
 
 // FP32 tiles only where every staged value and square stays far inside FP32
@@ -1046,14 +1051,22 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                 const int tf = key & 0xFF, kmin = s.kmin, kmax = s.kmax;
                 const int qf = tid < s.qlen ? J.Q.qf[s.qs + tid] : -1;
                 unsigned run = 0, before = 0;
-                const unsigned vm = __ballot_sync(FULL, qf >= 0);
+                const unsigned vm = __ballot_sync(FULL, qf >= 0), peers = __match_any_sync(FULL, qf);
+                const bool many = __popc(__ballot_sync(FULL, qf >= 0 && lane == __ffs(peers) - 1)) > kFlushRounds;
                 for (int e = kmin; e < min(kmax + 1, ne); e++) {
                     run += s.F[e * kMTiles + tid / kMT];
                     const unsigned cum = run + P[e * kPStride + tid];
                     P[e * kPStride + tid] = 0;
-                    const unsigned v = cum - before;
+                    const unsigned v = qf >= 0 ? cum - before : 0u;
                     before = cum;
-                    const bool wide = __any_sync(FULL, v >> 27);  // 32 of them may pass 2^32
+                    const unsigned top = __reduce_max_sync(FULL, v);
+                    if (!top) continue;
+                    unsigned long long *const row = Hd + (size_t)e * J.Fqe * J.Fte + tf;
+                    if (many) {
+                        if (v) atomicAdd(&row[(size_t)qf * J.Fte], (unsigned long long)v);
+                        continue;
+                    }
+                    const bool wide = top >> 27;  // 32 of them may pass 2^32
                     unsigned rem = vm;
                     while (rem) {  // one round per distinct own field of the warp
                         const int from = __ffs(rem) - 1;
@@ -1062,8 +1075,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                         unsigned long long sum = __reduce_add_sync(FULL, same ? (wide ? v & 0xFFFFu : v) : 0u);
                         if (wide)
                             sum += (unsigned long long)__reduce_add_sync(FULL, same ? v >> 16 : 0u) << 16;
-                        if (lane == from && sum)
-                            atomicAdd(&Hd[((size_t)e * J.Fqe + f) * J.Fte + tf], sum);
+                        if (lane == from && sum) atomicAdd(&row[(size_t)f * J.Fte], sum);
                         rem &= ~__ballot_sync(FULL, same);
                     }
                 }
