@@ -1763,10 +1763,11 @@ __global__ void k_tree_fields(int n, const int *__restrict__ p, const int *__res
         tf[p[i]] = ufield[cls[i] - 1];
 }
 
-// one CTA of KD_BLOCK_MAX threads per query block: box and single own field
+// one CTA of KD_BLOCK_MAX threads per query block: box and single own field;
+// many, if given: warps with more than KD_FEW_FIELDS own fields
 __global__ void __launch_bounds__(KD_BLOCK_MAX) k_block_boxes(int nblocks, const int *bstart,
                                                              const int *blen, RawOut o,
-                                                             double *bbox, int *bqf)
+                                                             double *bbox, int *bqf, int *many)
 {
     constexpr int W = KD_BLOCK_MAX / 32;
     __shared__ double sw[W][6];
@@ -1785,6 +1786,11 @@ __global__ void __launch_bounds__(KD_BLOCK_MAX) k_block_boxes(int nblocks, const
     }
     int q0 = __shfl_sync(0xffffffffu, qf, 0);
     int mixed = valid && qf != q0;
+    if (many) {
+        const unsigned peers = __match_any_sync(0xffffffffu, qf);
+        const unsigned fields = __ballot_sync(0xffffffffu, valid && lane == __ffs(peers) - 1);
+        if (lane == 0 && __popc(fields) > KD_FEW_FIELDS) atomicAdd(many, 1);
+    }
     for (int off = 16; off; off >>= 1)
         for (int d = 0; d < 3; d++) {
             lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], off));
@@ -2689,6 +2695,7 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
     cat->max_qf = h_fields ? hfi.max_qf : 0;
     cat->max_tf = hfi.max_tf;
     cat->fields_split = split;
+    cat->mixed_labels = hfi.max_tf > 0 && 8LL * nruns > n;
     cat->max_abs = maxabs;
     // the host holds the node array; the device copy is freed with the pool,
     // or, while a deferred copy still reads it, once that is done
@@ -2776,7 +2783,7 @@ static void build_query(const double *h_xyz, const int *h_fields, int n, int num
     struct State {
         KeySpan span;
         FieldInfo fi;
-        int full, err;
+        int full, err, many;
     } h, *dstate = pool.alloc<State>(1);
     memset(&h, 0, sizeof h);
     h.fi = {0x7fffffff, -0x7fffffff, 0, 0};
@@ -2799,8 +2806,12 @@ static void build_query(const double *h_xyz, const int *h_fields, int n, int num
         *bqf = keep.alloc<int>(nblocks);
     double *bbox = keep.alloc<double>(6 * (size_t)nblocks);
     k_query_points<<<grid_for(n), TPB, 0, s>>>(xyz, fin, cv.perm, n, ro, nblocks, bstart, blen);
-    k_block_boxes<<<nblocks, KD_BLOCK_MAX, 0, s>>>(nblocks, bstart, blen, ro, bbox, bqf);
+    const bool fields = h.fi.max_qf - h.fi.min_qf >= KD_FEW_FIELDS;
+    k_block_boxes<<<nblocks, KD_BLOCK_MAX, 0, s>>>(nblocks, bstart, blen, ro, bbox, bqf,
+                                                   fields ? &dstate->many : nullptr);
     KD_LAUNCH_CHECK("k_query_points");
+    if (fields)
+        check(cudaMemcpyAsync(&h.many, &dstate->many, sizeof(int), cudaMemcpyDeviceToHost, s), "D2H");
     st.sync();
 
     memset(cat, 0, sizeof *cat);
@@ -2809,6 +2820,7 @@ static void build_query(const double *h_xyz, const int *h_fields, int n, int num
     cat->num_fields = num_fields;
     cat->min_qf = h.fi.min_qf;
     cat->max_qf = h.fi.max_qf;
+    cat->mixed_labels = 2LL * h.many > (n + 31) / 32;
     for (int d = 0; d < 3; d++)
         cat->max_abs = std::max(cat->max_abs, std::max(fabs(okey_value(~h.span.inv_lo[d])),
                                                        fabs(okey_value(h.span.hi[d]))));

@@ -357,11 +357,7 @@ constexpr int kTileWarps = 4;
 constexpr int kTileThreads = 32 * kTileWarps;
 constexpr int kTilesPerSm = 7;                // CTAs per SM the registers are held to
 constexpr int kPStride = 136;                 // counters per edge (128 queries + bank shift)
-// Own fields of a warp's 32 queries that a flush sums over the warp, a round
-// each; with more, every query adds its own counts.  400k points, symmetric, 21
-// edges, labels at random: 4 fields 2.85 ms by rounds and 4.7 by query, 5 3.45
-// and 3.44, 16 10.2 and 8.2, 64 49.3 and 24.9, 250 142.6 and 49.0.
-constexpr int kFlushRounds = 4;
+constexpr unsigned kWideCount = 1u << 27;     // 32 counters below it sum to 32 bits
 static_assert(kMTiles == 8 && kTileThreads == KD_BLOCK_MAX, "lane layouts below");
 
 // FP32 tiles only where every staged value and square stays far inside FP32
@@ -714,7 +710,9 @@ __device__ __forceinline__ void tile_pass(TileSmem<KD_MODE_MIXED> &s, unsigned *
     }
 }
 
-template <int MODE>
+// MANY: what labels that interleave in space, or counters of 2^27 and more, need
+// besides (see tile_kernel)
+template <int MODE, bool MANY>
 __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
 {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -1050,32 +1048,38 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                 unsigned long long *const Hd = (key >> 8) ? J.H2 : J.H;
                 const int tf = key & 0xFF, kmin = s.kmin, kmax = s.kmax;
                 const int qf = tid < s.qlen ? J.Q.qf[s.qs + tid] : -1;
-                unsigned run = 0, before = 0;
-                const unsigned vm = __ballot_sync(FULL, qf >= 0), peers = __match_any_sync(FULL, qf);
-                const bool many = __popc(__ballot_sync(FULL, qf >= 0 && lane == __ffs(peers) - 1)) > kFlushRounds;
+                unsigned run = 0, before = 0, vm = __ballot_sync(FULL, qf >= 0);
+                unsigned alone = 0;  // the bits of its counters that a query adds by itself
+                if constexpr (MANY) {
+                    // Up to KD_FEW_FIELDS own fields are summed over the warp, a
+                    // round each; with more, every query adds its own counts.
+                    // 400k points, symmetric, 21 edges, labels at random: 4
+                    // fields 2.9 ms by rounds and 4.7 by query, 5 3.45 and 3.45,
+                    // 16 10.2 and 8.2, 64 49.3 and 24.7, 250 142.6 and 48.1.
+                    const unsigned peers = __match_any_sync(FULL, qf);
+                    const bool many = __popc(__ballot_sync(FULL, qf >= 0 && lane == __ffs(peers) - 1)) > KD_FEW_FIELDS;
+                    if (qf >= 0) alone = many ? FULL : ~(kWideCount - 1);
+                    if (many) vm = 0;
+                }
                 for (int e = kmin; e < min(kmax + 1, ne); e++) {
                     run += s.F[e * kMTiles + tid / kMT];
                     const unsigned cum = run + P[e * kPStride + tid];
                     P[e * kPStride + tid] = 0;
-                    const unsigned v = qf >= 0 ? cum - before : 0u;
+                    unsigned v = cum - before;
                     before = cum;
-                    const unsigned top = __reduce_max_sync(FULL, v);
-                    if (!top) continue;
-                    unsigned long long *const row = Hd + (size_t)e * J.Fqe * J.Fte + tf;
-                    if (many) {
-                        if (v) atomicAdd(&row[(size_t)qf * J.Fte], (unsigned long long)v);
-                        continue;
+                    if constexpr (MANY) {
+                        if (v & alone)
+                            atomicAdd(&Hd[((size_t)e * J.Fqe + qf) * J.Fte + tf], (unsigned long long)(v & alone));
+                        v &= ~alone;
                     }
-                    const bool wide = top >> 27;  // 32 of them may pass 2^32
                     unsigned rem = vm;
                     while (rem) {  // one round per distinct own field of the warp
                         const int from = __ffs(rem) - 1;
                         const int f = __shfl_sync(FULL, qf, from);
                         const bool same = qf == f;
-                        unsigned long long sum = __reduce_add_sync(FULL, same ? (wide ? v & 0xFFFFu : v) : 0u);
-                        if (wide)
-                            sum += (unsigned long long)__reduce_add_sync(FULL, same ? v >> 16 : 0u) << 16;
-                        if (lane == from && sum) atomicAdd(&row[(size_t)f * J.Fte], sum);
+                        const unsigned sum = __reduce_add_sync(FULL, same ? v : 0u);
+                        if (lane == from && sum)
+                            atomicAdd(&Hd[((size_t)e * J.Fqe + f) * J.Fte + tf], (unsigned long long)sum);
                         rem &= ~__ballot_sync(FULL, same);
                     }
                 }
@@ -1099,6 +1103,19 @@ static size_t tile_smem(int ne, int mode)
     const size_t fixed = mode == KD_MODE_MIXED ? sizeof(TileSmem<KD_MODE_MIXED>)
                                                : sizeof(TileSmem<KD_MODE_FP64>);
     return fixed + sizeof(unsigned) * (size_t)ne * kPStride;
+}
+
+// The kernel for these counts.  Its variant for many labels costs all others
+// 2 to 3% (code: the instruction cache decides), so it is taken only where a
+// tree or query catalog's labels interleave, or where a counter could reach 2^27.
+using TileKernel = void (*)(TileArgs);
+static TileKernel tile_kernel(const kd_catalog *const *tcs, const kd_catalog *const *qcs, int njobs, int mode)
+{
+    bool many = false;
+    for (int j = 0; j < njobs; j++)
+        many = many || tcs[j]->mixed_labels || qcs[j]->mixed_labels || tcs[j]->n_raw >= (int)kWideCount;
+    if (mode == KD_MODE_MIXED) return many ? k_tiles<KD_MODE_MIXED, true> : k_tiles<KD_MODE_MIXED, false>;
+    return many ? k_tiles<KD_MODE_FP64, true> : k_tiles<KD_MODE_FP64, false>;
 }
 
 struct Events {
@@ -1313,7 +1330,7 @@ static void count_batch_impl(const kd_catalog *const *tcs, const kd_catalog *con
     std::vector<long long> hoffs(nb + 1);
 
     const size_t smem = tile_smem(ne, mode);
-    auto kern = mode == KD_MODE_MIXED ? k_tiles<KD_MODE_MIXED> : k_tiles<KD_MODE_FP64>;
+    const TileKernel kern = tile_kernel(tcs, qcs, njobs, mode);
     check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
           "smem attribute");
     int nsm = 148, occ = 1;
@@ -1568,7 +1585,7 @@ static void count_static_impl(const kd_catalog *tc, int Ft, const kd_catalog *qc
           "scan");
 
     const size_t smem = tile_smem(ne, mode);
-    auto kern = mode == KD_MODE_MIXED ? k_tiles<KD_MODE_MIXED> : k_tiles<KD_MODE_FP64>;
+    const TileKernel kern = tile_kernel(&tc, &qc, 1, mode);
     check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
           "smem attribute");
     int nsm = 148, occ = 1;

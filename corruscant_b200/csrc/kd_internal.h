@@ -32,6 +32,7 @@ extern "C" {
 #define KD_RUN_MAX 64      /* points per leaf of the counting tree, so at most per run */
 #define KD_BLOCK_MAX 128   /* query points per block (one warp) */
 #define KD_MAX_EDGES 64    /* distinct finite squared edges per count job */
+#define KD_FEW_FIELDS 4    /* own fields of 32 queries that a count sums field by field */
 
 /* the status codes (KD_OK, KD_EINVAL, ...) and KD_MAX_POINTS are public:
  * include/kdtree.h; the device error words use the same codes */
@@ -53,6 +54,9 @@ typedef struct kd_catalog {
     int max_tf;       /* largest stored tree field id */
     int min_qf;       /* smallest own field id */
     int fields_split; /* 1 when some raw point has qf != tf */
+    int mixed_labels; /* 1 when the labels interleave in space: a tree's runs of one tree field
+                       * are shorter than 8 points on average, or most groups of 32 query
+                       * points hold more than KD_FEW_FIELDS own fields */
     double max_abs;   /* largest |coordinate| */
 
     /* reference-exact tree */
