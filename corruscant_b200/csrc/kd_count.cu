@@ -419,7 +419,7 @@ struct TileArgs {
     int g0, g1;                 // shard-local block indices of this launch
     const int *gmap;            // shard-local index -> global block (NULL: identity)
     const long long *off;       // launch-relative tile offsets
-    const uint4 *rec;
+    uint4 *rec;
     int *work;
     unsigned long long *stats;  // tested, rechecked, accepted, wide, edge-pairs, tiles
 };
@@ -492,6 +492,7 @@ struct TileCommon {
     int ecnt, chunk;
     int qs, qlen;                            // its queries: first, number
     int next, item, kmin, kmax, kfp;
+    int sorted, at;                          // records in order of their keys; the key's first place
     float Rq, hT, S;
 };
 template <int MODE> struct TileSmem;
@@ -546,6 +547,53 @@ __device__ __noinline__ void set_scale(TileSmem<KD_MODE_MIXED> &s, int ne, int t
                                 (float)(0.5 / 1.1 / (band_halfwidth(s.R[k], Rq, hT, S) * S * S)));
 }
 __device__ __forceinline__ void set_scale(TileSmem<KD_MODE_FP64> &, int, int) {}
+
+// A block with many flush keys would read through all its records once for each
+// key.  From kSortKeys keys on its records are ordered by key first: the order
+// is written into the words w of the records themselves, above the bit that is
+// there, so that the record at place i of the order is rec[i].w >> 1.  By the
+// whole CTA; F is clear before and after.  400k points, symmetric, 21 edges,
+// labels at random: 250 of them 48.1 -> 34.9 ms, 64 24.7 -> 20.9, 16 8.4 -> 7.9;
+// with 2, 4 or 16 keys as the line all of these are within 1.5%.
+constexpr int kSortKeys = 8;
+__device__ __noinline__ void order_records(TileCommon &s, uint4 *rec, int tid)
+{
+    static_assert((KD_MAX_EDGES + 1) * kMTiles >= 512 + kTileWarps && kTileThreads * 4 == 512, "keys in F");
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = tid & 31, w = tid >> 5, n = s.ecnt;
+    auto key_of = [&](int i) {  // (not through the read-only cache: w is written here)
+        const uint2 r = __ldcg(reinterpret_cast<const uint2 *>(rec + i) + 1);
+        return ((r.x >> 8) & 0xFF) | (r.y & 1u) << 8;
+    };
+    for (int i = tid; i < n; i += kTileThreads) atomicAdd(&s.F[key_of(i)], 1u);
+    __syncthreads();
+    unsigned c[4], sum = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        c[k] = s.F[4 * tid + k];
+        sum += c[k];
+    }
+    unsigned inc = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(FULL, inc, o);
+        if (lane >= o) inc += y;
+    }
+    if (lane == 31) s.F[512 + w] = inc;
+    __syncthreads();
+    unsigned at = inc - sum;
+    for (int k = 0; k < w; k++) at += s.F[512 + k];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        s.F[4 * tid + k] = at;
+        at += c[k];
+    }
+    __syncthreads();
+    for (int i = tid; i < n; i += kTileThreads)
+        atomicOr(&rec[atomicAdd(&s.F[key_of(i)], 1u)].w, (unsigned)i << 1);
+    __syncthreads();
+    for (int k = tid; k < 512 + kTileWarps; k += kTileThreads) s.F[k] = 0;
+}
 
 // Exact counts of the flagged rows of query tile m (rows: bit per row) over
 // the run [rs, rs + n) for kn (<= 4) edges from kk on, added to their counters
@@ -720,6 +768,8 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
     TileSmem<MODE> &s = *(TileSmem<MODE> *)smem;
     const int ne = A.ne;
     unsigned *const P = (unsigned *)(smem + sizeof(TileSmem<MODE>));
+    // MANY: the records of this warp's chunk
+    int *const place = (int *)(P + ne * kPStride) + (threadIdx.x & ~31);
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     const int wm = lane & (kMTiles - 1), wr = lane / kMTiles;  // this lane's window: tile, record
     for (int k = tid; k < ne; k += kTileThreads) {
@@ -799,14 +849,18 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                 frexpf(Bm, &ex);  // Bm in [2^(ex-1), 2^ex)
                 S = ldexpf(1.0f, max(-60, min(60, 7 - ex)));
             }
+            const int nk = MANY ? __reduce_add_sync(FULL, lane < 16 ? __popc(s.keys[lane]) : 0) : 0;
             if (tid == 0) {
                 s.o[0] = ox;
                 s.o[1] = oy;
                 s.o[2] = oz;
                 s.eoff = eoff;
                 s.ecnt = ecnt;
-                // records a warp takes at a time: a few, where the block has few
-                s.chunk = ecnt >= 1024 ? 32 : (ecnt >= 512 ? 16 : (ecnt >= 128 ? 8 : 4));
+                // records a warp takes at a time: a few, where the pass has few
+                const int cnt = MANY && nk > kSortKeys ? ecnt / nk : ecnt;
+                s.chunk = cnt >= 1024 ? 32 : (cnt >= 512 ? 16 : (cnt >= 128 ? 8 : 4));
+                s.sorted = MANY && nk > kSortKeys;
+                s.at = 0;
                 s.qs = qs;
                 s.qlen = qlen;
                 s.Rq = Rq;
@@ -815,6 +869,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
             }
             __syncthreads();
             if (MODE == KD_MODE_MIXED && S > 0.0f) set_scale(s, ne, tid);
+            if (MANY && nk > kSortKeys) order_records(s, A.rec + eoff, tid);
         }
         // ---- one flush key after the other (tree field | 256 for the
         // once-counted part of a symmetric job)
@@ -826,20 +881,34 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
             }
             key += __ffs(kw) - 1;
             __syncthreads();  // the last key's counters are clear
-            if (tid == 0) s.next = 0;
+            if (tid == 0) s.next = MANY ? s.at : 0;
             __syncthreads();
             while (true) {
                 int c0 = 0;
                 if (lane == 0) c0 = atomicAdd(&s.next, s.chunk);
                 c0 = __shfl_sync(FULL, c0, 0);
                 if (c0 >= s.ecnt) break;
-                const uint4 *const crec = A.rec + s.eoff + c0;
+                const uint4 *const crec = A.rec + s.eoff + (MANY ? 0 : c0);
                 unsigned mine;
                 {
                     uint2 r = make_uint2(0, 0);
                     const bool in = lane < s.chunk && c0 + lane < s.ecnt;
-                    if (in) r = __ldg(reinterpret_cast<const uint2 *>(crec + lane) + 1);
+                    int i = lane;
+                    if constexpr (MANY) {
+                        i = c0 + lane;
+                        if (in && s.sorted) i = (int)(__ldcg(&crec[i].w) >> 1);
+                        place[lane] = i;
+                    }
+                    if (in) r = __ldg(reinterpret_cast<const uint2 *>(crec + i) + 1);
+                    if constexpr (MANY) r.y &= 1u;
                     mine = __ballot_sync(FULL, in && (((r.x >> 8) & 0xFF) | (r.y << 8)) == (unsigned)key);
+                    if constexpr (MANY) {
+                        if (s.sorted) {
+                            if (!mine) break;  // behind the key's records
+                            if (lane == 0) atomicAdd(&s.at, __popc(mine));
+                        }
+                        __syncwarp();
+                    }
                 }
                 while (mine) {
                     // ---- the next four records: lane (wm, wr) has record wr
@@ -849,7 +918,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                     const int nr = min(kGroup, __popc(mine));
                     mine = m3 & (m3 - 1);
                     const int from = have ? __ffs(sel) - 1 : 0;
-                    const uint4 rec = __ldg(crec + from);
+                    const uint4 rec = __ldg(crec + (MANY ? place[from] : from));
                     const int r_rs = (int)rec.x;
                     const unsigned r_z = have ? rec.z : 0u;
                     const int rl = r_z & 0xFF, rk0 = (r_z >> 16) & 0xFF, rK = r_z >> 24;
@@ -1098,25 +1167,35 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
     }
 }
 
-static size_t tile_smem(int ne, int mode)
+static size_t tile_smem(int ne, int mode, bool many)
 {
     const size_t fixed = mode == KD_MODE_MIXED ? sizeof(TileSmem<KD_MODE_MIXED>)
                                                : sizeof(TileSmem<KD_MODE_FP64>);
-    return fixed + sizeof(unsigned) * (size_t)ne * kPStride;
+    return fixed + sizeof(unsigned) * (size_t)ne * kPStride + (many ? sizeof(int) * kTileThreads : 0);
 }
 
 // The kernel for these counts.  Its variant for many labels costs all others
 // 2 to 3% (code: the instruction cache decides), so it is taken only where a
 // tree or query catalog's labels interleave, or where a counter could reach 2^27.
-using TileKernel = void (*)(TileArgs);
-static TileKernel tile_kernel(const kd_catalog *const *tcs, const kd_catalog *const *qcs, int njobs, int mode)
-{
-    bool many = false;
-    for (int j = 0; j < njobs; j++)
-        many = many || tcs[j]->mixed_labels || qcs[j]->mixed_labels || tcs[j]->n_raw >= (int)kWideCount;
-    if (mode == KD_MODE_MIXED) return many ? k_tiles<KD_MODE_MIXED, true> : k_tiles<KD_MODE_MIXED, false>;
-    return many ? k_tiles<KD_MODE_FP64, true> : k_tiles<KD_MODE_FP64, false>;
-}
+struct TileKernel {
+    void (*run)(TileArgs);
+    size_t smem;
+    int ctas;  // per SM
+
+    TileKernel(const kd_catalog *const *tcs, const kd_catalog *const *qcs, int njobs, int ne, int mode)
+    {
+        bool many = false;
+        for (int j = 0; j < njobs; j++)
+            many = many || tcs[j]->mixed_labels || qcs[j]->mixed_labels || tcs[j]->n_raw >= (int)kWideCount;
+        run = mode == KD_MODE_MIXED ? (many ? k_tiles<KD_MODE_MIXED, true> : k_tiles<KD_MODE_MIXED, false>)
+                                    : (many ? k_tiles<KD_MODE_FP64, true> : k_tiles<KD_MODE_FP64, false>);
+        smem = tile_smem(ne, mode, many);
+        check(cudaFuncSetAttribute(run, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+              "smem attribute");
+        check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, run, kTileThreads, smem), "occupancy");
+        ctas = std::max(ctas, 1);
+    }
+};
 
 struct Events {
     cudaEvent_t e[8];
@@ -1329,15 +1408,9 @@ static void count_batch_impl(const kd_catalog *const *tcs, const kd_catalog *con
     long long *off = pool.alloc<long long>(nb + 1);
     std::vector<long long> hoffs(nb + 1);
 
-    const size_t smem = tile_smem(ne, mode);
-    const TileKernel kern = tile_kernel(tcs, qcs, njobs, mode);
-    check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-          "smem attribute");
-    int nsm = 148, occ = 1;
+    const TileKernel kern(tcs, qcs, njobs, ne, mode);
+    int nsm = 148;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
-    check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kTileThreads, smem),
-          "occupancy");
-    occ = std::max(occ, 1);
 
     float ms_trav = 0, ms_tiles = 0;
     int b0 = 0;  // shard-relative
@@ -1376,8 +1449,8 @@ static void count_batch_impl(const kd_catalog *const *tcs, const kd_catalog *con
         ta.work = work;
         ta.stats = dstats;
         check(cudaMemsetAsync(work, 0, sizeof(int), s), "memset");
-        const int grid = (int)std::min<long long>(b1 - b0, (long long)nsm * occ);
-        kern<<<grid, kTileThreads, smem, s>>>(ta);
+        const int grid = (int)std::min<long long>(b1 - b0, (long long)nsm * kern.ctas);
+        kern.run<<<grid, kTileThreads, kern.smem, s>>>(ta);
         launches++;
         tile_launches++;
         KD_LAUNCH_CHECK("k_tiles");
@@ -1584,15 +1657,9 @@ static void count_static_impl(const kd_catalog *tc, int Ft, const kd_catalog *qc
     check(sort::scan<long long, sort::SumOp, false>(scan_tmp, cnt, off, nb + 1, sort::SumOp(), s),
           "scan");
 
-    const size_t smem = tile_smem(ne, mode);
-    const TileKernel kern = tile_kernel(&tc, &qc, 1, mode);
-    check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-          "smem attribute");
-    int nsm = 148, occ = 1;
+    const TileKernel kern(&tc, &qc, 1, ne, mode);
+    int nsm = 148;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, tc->device);
-    check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kTileThreads, smem),
-          "occupancy");
-    occ = std::max(occ, 1);
     int b0 = 0;
     while (b0 < nb) {
         k_static_batch<<<1, 256, 0, s>>>(off, nb, b0, cap, err + 2, rel, rel_cap);
@@ -1622,8 +1689,8 @@ static void count_static_impl(const kd_catalog *tc, int Ft, const kd_catalog *qc
         ta.work = err + 1;
         ta.stats = misc;
         check(cudaMemsetAsync(err + 1, 0, sizeof(int), s), "memset");
-        const int grid = (int)std::min<long long>(b1 - b0, (long long)nsm * occ);
-        kern<<<grid, kTileThreads, smem, s>>>(ta);
+        const int grid = (int)std::min<long long>(b1 - b0, (long long)nsm * kern.ctas);
+        kern.run<<<grid, kTileThreads, kern.smem, s>>>(ta);
         KD_LAUNCH_CHECK("k_tiles");
         b0 = b1;
     }
