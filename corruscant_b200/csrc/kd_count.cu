@@ -493,7 +493,7 @@ struct TileCommon {
     int qs, qlen;                            // its queries: first, number
     int next, item, kmin, kmax, kfp;
     int sorted, at;                          // records in order of their keys; the key's first place
-    float Rq, hT, S;
+    float Rq, hT, hcap, S;                   // (hcap: half-extents' sum of a leaf within hT)
 };
 template <int MODE> struct TileSmem;
 template <> struct TileSmem<KD_MODE_MIXED> : TileCommon {
@@ -821,7 +821,6 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
             const double ox = 0.5 * (bx[0] + bx[3]), oy = 0.5 * (bx[1] + bx[4]), oz = 0.5 * (bx[2] + bx[5]);
             const double hx = 0.5 * (bx[3] - bx[0]), hy = 0.5 * (bx[4] - bx[1]), hz = 0.5 * (bx[5] - bx[2]);
             const float Rq = __double2float_ru(sqrt(hx * hx + hy * hy + hz * hz) * (1.0 + 1e-12));
-            const float hT = __double2float_ru(J.hT);
             float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
             if (tid < qlen) {
                 lo[0] = hi[0] = (float)(J.Q.x[qs + tid] - ox);
@@ -840,10 +839,18 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                     s.qh[tid / kMT][d] = 0.5f * (hi[d] - lo[d]);
                 }
             }
+            // The leaves' half-diagonal that the error band allows for: the
+            // largest, but no more than a few times what this block and its
+            // edges span.  The FP32 path leaves larger leaves out (a few around
+            // any tight group, and their band would cover all its pairs): 1M
+            // points in 20 groups 1e-6 wide, radii 1e-8 and 1e-7, 3.15 -> 0.43
+            // ms; over twelve decades of |x|, 29 -> 6.6; uniform ones the same.
+            const float far = s.kfp >= 0 ? sqrtf(s.Rup[s.kfp]) * 1.0001f : 0.0f;
+            const float hT = fminf(4.0f * (far + Rq), __double2float_ru(J.hT));
             // every coordinate and edge root of a record with pairs below edge
             // kfp stays below Bm: scaled values below 240, squares below 65504
             float S = 0.0f;
-            const float Bm = (s.kfp >= 0 ? sqrtf(s.Rup[s.kfp]) * 1.0001f : 0.0f) + 2.1f * hT + 4.0f * Rq;
+            const float Bm = far + 2.1f * hT + 4.0f * Rq;
             if (Bm > 0.0f && Bm < (float)kFp32Span) {
                 int ex;
                 frexpf(Bm, &ex);  // Bm in [2^(ex-1), 2^ex)
@@ -865,6 +872,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                 s.qlen = qlen;
                 s.Rq = Rq;
                 s.hT = hT;
+                s.hcap = J.hT <= (double)hT ? INFINITY : hT;
                 s.S = S;
             }
             __syncthreads();
@@ -926,7 +934,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                     // tile wm and the record; every pair lies below the edges
                     // from k1 on
                     int k0 = rk0, k1 = rk0 + rK;
-                    bool ok = have && rK != 0;
+                    bool ok = have && rK != 0, fast_ok = false;  // windows, FP32 distances
                     float dx, dy, dz;
                     {
                         const double2 *geo = reinterpret_cast<const double2 *>(s.job.leaf + rec.y);
@@ -937,11 +945,11 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                         dx = (float)(ga.x - s.o[0]);
                         dy = (float)(ga.y - s.o[1]);
                         dz = (float)(gb.x - s.o[2]);
-                        // B >= |t'| of every point of the leaf and sqrt of
-                        // every edge of the record
+                        // B >= |t'| of every point of a leaf of the FP32 path and
+                        // sqrt of every edge of the record
                         const float B = sqrtf(dx * dx + dy * dy + dz * dz) * 1.0001f + s.hT + 2.0f * s.Rq;
-                        ok = ok && B < (float)kFp32Span && s.R[k1 - 1] < kFp32MaxR &&
-                             (MODE == KD_MODE_FP64 || (s.S > 0.0f && B * s.S <= 240.0f));
+                        ok = ok && B < (float)kFp32Span && s.R[k1 - 1] < kFp32MaxR;
+                        fast_ok = ok && s.S > 0.0f && B * s.S <= 240.0f && hx + hy + hz <= s.hcap;
                         if (ok) {
                             // rounding of the staged coordinates and of the tile box
                             const float mg = 4.8e-7f * (fabsf(dx) + fabsf(dy) + fabsf(dz) + hx + hy + hz +
@@ -969,7 +977,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                     const int mval = max(0, min(kMT, s.qlen - kMT * wm));  // queries of tile wm
                     const int K = have && mval ? k1 - k0 : 0;
                     const unsigned win = (unsigned)k0 | ((unsigned)K << 8);
-                    const unsigned actm = __ballot_sync(FULL, K != 0), okm = __ballot_sync(FULL, ok);
+                    const unsigned actm = __ballot_sync(FULL, K != 0), okm = __ballot_sync(FULL, fast_ok);
                     if (have && mval) atomicAdd(&s.F[k1 * kMTiles + wm], (unsigned)rl);
                     {
                         const unsigned q = K ? (unsigned)(mval * rl) : 0u;

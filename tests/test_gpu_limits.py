@@ -92,3 +92,35 @@ def test_gaps_of_a_few_subnormal_steps(gap, radius):
             assert np.array_equal(N.count_points(t, b, None, 1, [radius], mode=mode), want), mode
     finally:
         N.destroy(t)
+
+
+@pytest.mark.parametrize("kind", ["groups", "groups and outlier", "decades", "infinite"])
+@pytest.mark.parametrize("seed", [0, 1])
+def test_leaves_of_very_different_sizes(kind, seed):
+    """Tight groups beside leaves that span the catalog, with edges at the exact
+    distances of pairs (those on an edge are not below it)."""
+    rs = np.random.RandomState(seed)
+    n = 5000
+    if kind == "decades":
+        p = 10.0 ** (-12 * rs.rand(n, 3)) * np.where(rs.rand(n, 3) < 0.5, -1, 1)
+    else:
+        p = rs.rand(12, 3)[rs.randint(0, 12, n)] + 1e-6 * rs.normal(size=(n, 3))
+        p[::50] = rs.rand(len(p[::50]), 3)
+        if kind == "groups and outlier":
+            p[n // 3] = [1e12, -1e12, 1e12]
+        elif kind == "infinite":
+            p[n // 3, 0], p[n // 2, 2] = np.inf, -np.inf
+    a, b = p[rs.randint(0, n, 4000)], p[rs.randint(0, n, 4000)]
+    with np.errstate(invalid="ignore"):
+        d = np.sqrt(((a - b) ** 2).sum(1))
+    d = np.unique(d[np.isfinite(d) & (d > 0)])
+    radii = np.concatenate([d[np.linspace(0, len(d) - 1, 25).astype(int)], [1e-8, 1e-7, 1e-6]])
+    f = rs.randint(0, 2, n).astype(np.int32)
+    want = O.OracleTree(p, f, 2).brute_counts(p, f, 2, radii, nthreads=4)
+    t = N.build_tree(p, f, 2)
+    try:
+        for mode in MODES:
+            assert np.array_equal(N.count_radii(t, t, radii, mode=mode), want), mode
+            assert np.array_equal(N.count_points(t, p, f, 2, radii, mode=mode), want), mode
+    finally:
+        N.destroy(t)
