@@ -254,30 +254,54 @@ def make_workload(scale=1.0):
 # ----------------------------------------------------------------- helpers
 
 class ClockSampler:
-    """nvidia-smi clocks and throttle reasons sampled every 200 ms."""
+    """nvidia-smi clocks and throttle reasons sampled every 200 ms.  Entering
+    waits for the first row (nvidia-smi takes some hundred ms to it, more than a
+    small timed region lasts) and the summary leaves that row out; leaving waits
+    for a row that came after, at most one period past the region's end."""
 
     QUERY = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
              "clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
              "clocks_event_reasons.sw_thermal_slowdown,clocks_event_reasons.sw_power_cap")
+    WAIT_S = 10.0  # for a row, at the most
 
     def __init__(self, device):
         self.device = device
         self.proc = None
         self.path = None
+        self.before = 0
+
+    def _rows(self):
+        try:
+            with open(self.path) as f:
+                lines = [line for line in f if line.endswith("\n")]
+        except OSError:
+            return []
+        rows = [[x.strip() for x in line.split(",")] for line in lines]
+        return [r for r in rows if len(r) >= 9]
+
+    def _wait_rows(self, n):
+        end = time.monotonic() + self.WAIT_S
+        while self.proc and len(self._rows()) < n and self.proc.poll() is None and time.monotonic() < end:
+            time.sleep(0.01)
 
     def __enter__(self):
         fd, self.path = tempfile.mkstemp(suffix=".csv")
         os.close(fd)
         try:
-            self.proc = subprocess.Popen(
-                ["nvidia-smi", "-i", str(self.device), f"--query-gpu={self.QUERY}",
-                 "--format=csv,noheader,nounits", "-lms", "200"],
-                stdout=open(self.path, "w"), stderr=subprocess.DEVNULL)
+            with open(self.path, "w") as out:
+                self.proc = subprocess.Popen(
+                    ["nvidia-smi", "-i", str(self.device), f"--query-gpu={self.QUERY}",
+                     "--format=csv,noheader,nounits", "-lms", "200"],
+                    stdout=out, stderr=subprocess.DEVNULL)
         except OSError:
             self.proc = None
+        self._wait_rows(1)
+        self.before = len(self._rows())
         return self
 
     def __exit__(self, *exc):
+        if self.before:  # (else there is none to wait for)
+            self._wait_rows(self.before + 1)
         if self.proc:
             self.proc.terminate()
             try:
@@ -286,17 +310,9 @@ class ClockSampler:
                 self.proc.kill()
 
     def summary(self):
-        rows = []
-        try:
-            for line in open(self.path):
-                f = [x.strip() for x in line.split(",")]
-                if len(f) >= 9:
-                    rows.append(f)
-        except OSError:
-            pass
-        finally:
-            if self.path and os.path.exists(self.path):
-                os.unlink(self.path)
+        rows = self._rows()[self.before:]
+        if self.path and os.path.exists(self.path):
+            os.unlink(self.path)
         if not rows:
             return {"sm_mhz": None, "sm_max_mhz": None, "reasons": ["nvidia-smi unavailable"]}
         sm = [float(r[1]) for r in rows if r[1].replace(".", "").isdigit()]
