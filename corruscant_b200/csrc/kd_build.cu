@@ -1666,15 +1666,20 @@ __global__ void __launch_bounds__(TPB) k_leaves(int n, int nleaves, Cells cells,
     }
 }
 
-// one warp per leaf: its runs, one per tree field
+// one warp per leaf: its runs, one per tree field; and the number of leaves
+// below the size hcut
 __global__ void __launch_bounds__(TPB) k_leaf_runs(int nleaves, const int *__restrict__ pos,
                                                    const int *__restrict__ tf,
                                                    const int *__restrict__ leaf_run, int *run_start,
-                                                   int *run_len, int *run_tf)
+                                                   int *run_len, int *run_tf, const kd_leaf *__restrict__ leaf,
+                                                   float hcut, int *small)
 {
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    const int a = w < nleaves ? pos[w] : 0, len = w < nleaves ? pos[w + 1] - a : 0;
+    const bool below = lane == 0 && len > 0 && !(leaf[w].h[0] + leaf[w].h[1] + leaf[w].h[2] >= hcut);
+    const int nb = __syncthreads_count(below);
+    if (threadIdx.x == 0 && nb) atomicAdd(small, nb);
     if (w >= nleaves) return;
-    const int a = pos[w], len = pos[w + 1] - a;
     constexpr int PL = KD_RUN_MAX / 32;
     unsigned long long all = 0;
     int f[PL];
@@ -2656,8 +2661,12 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
     double *bbox = keep.alloc<double>(6 * (size_t)nblocks);
     k_tree_blocks<<<blocks_for(groups, TPB), TPB, 0, s>>>(groups, nleaves, lf.pos, boff, sm.box, lf.qf, bstart,
                                                           blen, bbox, bqf);
-    k_leaf_runs<<<gl, TPB, 0, s>>>(nleaves, lf.pos, ro.tf, leaf_run, run_start, run_len, run_tf);
+    int *small = pool.alloc<int>(1), nsmall;
+    check(cudaMemsetAsync(small, 0, sizeof(int), s), "memset");
+    k_leaf_runs<<<gl, TPB, 0, s>>>(nleaves, lf.pos, ro.tf, leaf_run, run_start, run_len, run_tf, lf.leaf,
+                                   (float)(leaf_hdiag / 64), small);
     KD_LAUNCH_CHECK("summary kernels");
+    check(cudaMemcpyAsync(&nsmall, small, sizeof(int), cudaMemcpyDeviceToHost, s), "D2H");
     check(cudaEventRecord(ph[5], s), "event");
     st.sync();
     kd_build_stats bs;
@@ -2696,6 +2705,7 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
     cat->max_tf = hfi.max_tf;
     cat->fields_split = split;
     cat->mixed_labels = hfi.max_tf > 0 && 8LL * nruns > n;
+    cat->uneven_leaves = 8LL * KD_RUN_MAX * nsmall > n;
     cat->max_abs = maxabs;
     // the host holds the node array; the device copy is freed with the pool,
     // or, while a deferred copy still reads it, once that is done

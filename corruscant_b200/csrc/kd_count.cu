@@ -492,14 +492,16 @@ struct TileCommon {
     int ecnt, chunk;
     int qs, qlen;                            // its queries: first, number
     int next, item, kmin, kmax, kfp;
+    float Rq, hT, S;
+    // of the general variant
+    float hSmall, hcap;                      // half-extents' sum of leaves with the smaller band, with any
     int sorted, at;                          // records in order of their keys; the key's first place
-    float Rq, hT, hcap, S;                   // (hcap: half-extents' sum of a leaf within hT)
 };
 template <int MODE> struct TileSmem;
 template <> struct TileSmem<KD_MODE_MIXED> : TileCommon {
     alignas(16) uint4 qa[kMTiles][32];       // MMA A fragments of the query tiles
     float2 qn[kMTiles][kMT / 2];             // |q|^2 S^2 of rows g and g + 8
-    float2 edge[KD_MAX_EDGES];               // R S^2 and 0.4545 / (E S^2)
+    float2 edge[2 * KD_MAX_EDGES];           // R S^2 and 0.4545 / (E S^2); from KD_MAX_EDGES on, for small leaves
     alignas(16) uint32_t bs[kTileWarps][KD_RUN_MAX / kNT * 32];  // MMA B fragments of the staged runs
 };
 template <> struct TileSmem<KD_MODE_FP64> : TileCommon {
@@ -513,7 +515,7 @@ template <> struct TileSmem<KD_MODE_FP64> : TileCommon {
 // lo) against the same; for t = 3, (1, 1) against the halves of N, and (0, 0).
 __device__ __noinline__ void set_scale(TileSmem<KD_MODE_MIXED> &s, int ne, int tid)
 {
-    const double S = (double)s.S, Rq = (double)s.Rq, hT = (double)s.hT;
+    const double S = (double)s.S, Rq = (double)s.Rq;
     const int qs = s.qs, qlen = s.qlen;
     for (int i = tid; i < kMTiles * 32; i += kTileThreads) {
         const int m = i >> 5, g = (i & 31) >> 2, t = i & 3;
@@ -542,9 +544,11 @@ __device__ __noinline__ void set_scale(TileSmem<KD_MODE_MIXED> &s, int ne, int t
         if (tid % kMT < 8) q.x = (float)n;
         else q.y = (float)n;
     }
-    for (int k = tid; k < ne; k += kTileThreads)
-        s.edge[k] = make_float2((float)(s.R[k] * S * S),
-                                (float)(0.5 / 1.1 / (band_halfwidth(s.R[k], Rq, hT, S) * S * S)));
+    for (int b = 0; b < (s.hSmall < s.hT ? 2 : 1); b++)
+        for (int k = tid; k < ne; k += kTileThreads)
+            s.edge[b * KD_MAX_EDGES + k] = make_float2(
+                (float)(s.R[k] * S * S),
+                (float)(0.5 / 1.1 / (band_halfwidth(s.R[k], Rq, b ? (double)s.hSmall : (double)s.hT, S) * S * S)));
 }
 __device__ __forceinline__ void set_scale(TileSmem<KD_MODE_FP64> &, int, int) {}
 
@@ -645,18 +649,19 @@ __device__ __noinline__ void recount_rows(TileCommon &s, unsigned *P, unsigned r
 // saturating ramp has no packed form.
 template <int K, int M>
 __device__ __forceinline__ void tile_pass(TileSmem<KD_MODE_MIXED> &s, unsigned *P, const int (&mt)[2],
-                                          int kk, int nt, float ref, int rs, int n, int lane,
+                                          int kk, int eb, int nt, float ref, int rs, int n, int lane,
                                           const uint32_t *__restrict__ bs)
 {
     static_assert(K * M <= 4 && M <= 2, "an item per lane of a row");
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int NI = K * M;  // item i: edge kk + i % K of tile mt[i / K]
     const int g = lane >> 2, t = lane & 3;
-    const float e0 = s.edge[kk].x, nsl = -s.edge[kk + K - 1].y;
+    const float2 *const edge = s.edge + eb + kk;
+    const float e0 = edge[0].x, nsl = -edge[K - 1].y;
     float a[K];
     a[0] = 0.5f;
 #pragma unroll
-    for (int k = 1; k < K; k++) a[k] = fmaf(e0 - s.edge[kk + k].x, nsl, 0.5f);
+    for (int k = 1; k < K; k++) a[k] = fmaf(e0 - edge[k].x, nsl, 0.5f);
     uint4 qa[M];
     float c0[M], c1[M];
     float2 acc[M][K], sq[M][2];
@@ -758,9 +763,9 @@ __device__ __forceinline__ void tile_pass(TileSmem<KD_MODE_MIXED> &s, unsigned *
     }
 }
 
-// MANY: what labels that interleave in space, or counters of 2^27 and more, need
-// besides (see tile_kernel)
-template <int MODE, bool MANY>
+// GENERAL: with what labels that interleave in space, counters of 2^27 and more and
+// leaves of very different sizes need besides (see TileKernel)
+template <int MODE, bool GENERAL>
 __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
 {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -768,7 +773,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
     TileSmem<MODE> &s = *(TileSmem<MODE> *)smem;
     const int ne = A.ne;
     unsigned *const P = (unsigned *)(smem + sizeof(TileSmem<MODE>));
-    // MANY: the records of this warp's chunk
+    // GENERAL: the records of this warp's chunk
     int *const place = (int *)(P + ne * kPStride) + (threadIdx.x & ~31);
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     const int wm = lane & (kMTiles - 1), wr = lane / kMTiles;  // this lane's window: tile, record
@@ -839,14 +844,19 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                     s.qh[tid / kMT][d] = 0.5f * (hi[d] - lo[d]);
                 }
             }
-            // The leaves' half-diagonal that the error band allows for: the
-            // largest, but no more than a few times what this block and its
-            // edges span.  The FP32 path leaves larger leaves out (a few around
-            // any tight group, and their band would cover all its pairs): 1M
-            // points in 20 groups 1e-6 wide, radii 1e-8 and 1e-7, 3.15 -> 0.43
-            // ms; over twelve decades of |x|, 29 -> 6.6; uniform ones the same.
             const float far = s.kfp >= 0 ? sqrtf(s.Rup[s.kfp]) * 1.0001f : 0.0f;
-            const float hT = fminf(4.0f * (far + Rq), __double2float_ru(J.hT));
+            float hT = __double2float_ru(J.hT), hSmall = hT;
+            if constexpr (GENERAL) {
+                // The error band allows for the rounding of a point relative to
+                // its leaf's centre, so it grows with the leaf, and beside leaves
+                // that span the catalog (around a far point, between tight groups)
+                // it would cover every pair.  So leaves of no more than a few
+                // times what this block and its edges span have a band of their
+                // own, and leaves with which the scale could not resolve the block
+                // take the exact path.
+                hT = fminf(hT, 16384.0f * (Rq + sqrtf(s.Rup[min(s.kmin, ne - 1)])) + 4.0f * far);
+                hSmall = fminf(hT, 4.0f * (far + Rq));
+            }
             // every coordinate and edge root of a record with pairs below edge
             // kfp stays below Bm: scaled values below 240, squares below 65504
             float S = 0.0f;
@@ -856,7 +866,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                 frexpf(Bm, &ex);  // Bm in [2^(ex-1), 2^ex)
                 S = ldexpf(1.0f, max(-60, min(60, 7 - ex)));
             }
-            const int nk = MANY ? __reduce_add_sync(FULL, lane < 16 ? __popc(s.keys[lane]) : 0) : 0;
+            const int nk = GENERAL ? __reduce_add_sync(FULL, lane < 16 ? __popc(s.keys[lane]) : 0) : 0;
             if (tid == 0) {
                 s.o[0] = ox;
                 s.o[1] = oy;
@@ -864,20 +874,23 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                 s.eoff = eoff;
                 s.ecnt = ecnt;
                 // records a warp takes at a time: a few, where the pass has few
-                const int cnt = MANY && nk > kSortKeys ? ecnt / nk : ecnt;
+                const int cnt = GENERAL && nk > kSortKeys ? ecnt / nk : ecnt;
                 s.chunk = cnt >= 1024 ? 32 : (cnt >= 512 ? 16 : (cnt >= 128 ? 8 : 4));
-                s.sorted = MANY && nk > kSortKeys;
-                s.at = 0;
+                if constexpr (GENERAL) {
+                    s.sorted = nk > kSortKeys;
+                    s.at = 0;
+                }
                 s.qs = qs;
                 s.qlen = qlen;
                 s.Rq = Rq;
                 s.hT = hT;
-                s.hcap = J.hT <= (double)hT ? INFINITY : hT;
+                s.hSmall = hSmall;
+                s.hcap = J.hT <= (double)hT ? INFINITY : hT;  // (J.hT may be NaN)
                 s.S = S;
             }
             __syncthreads();
             if (MODE == KD_MODE_MIXED && S > 0.0f) set_scale(s, ne, tid);
-            if (MANY && nk > kSortKeys) order_records(s, A.rec + eoff, tid);
+            if (GENERAL && nk > kSortKeys) order_records(s, A.rec + eoff, tid);
         }
         // ---- one flush key after the other (tree field | 256 for the
         // once-counted part of a symmetric job)
@@ -889,28 +902,28 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
             }
             key += __ffs(kw) - 1;
             __syncthreads();  // the last key's counters are clear
-            if (tid == 0) s.next = MANY ? s.at : 0;
+            if (tid == 0) s.next = GENERAL ? s.at : 0;
             __syncthreads();
             while (true) {
                 int c0 = 0;
                 if (lane == 0) c0 = atomicAdd(&s.next, s.chunk);
                 c0 = __shfl_sync(FULL, c0, 0);
                 if (c0 >= s.ecnt) break;
-                const uint4 *const crec = A.rec + s.eoff + (MANY ? 0 : c0);
+                const uint4 *const crec = A.rec + s.eoff + (GENERAL ? 0 : c0);
                 unsigned mine;
                 {
                     uint2 r = make_uint2(0, 0);
                     const bool in = lane < s.chunk && c0 + lane < s.ecnt;
                     int i = lane;
-                    if constexpr (MANY) {
+                    if constexpr (GENERAL) {
                         i = c0 + lane;
                         if (in && s.sorted) i = (int)(__ldcg(&crec[i].w) >> 1);
                         place[lane] = i;
                     }
                     if (in) r = __ldg(reinterpret_cast<const uint2 *>(crec + i) + 1);
-                    if constexpr (MANY) r.y &= 1u;
+                    if constexpr (GENERAL) r.y &= 1u;
                     mine = __ballot_sync(FULL, in && (((r.x >> 8) & 0xFF) | (r.y << 8)) == (unsigned)key);
-                    if constexpr (MANY) {
+                    if constexpr (GENERAL) {
                         if (s.sorted) {
                             if (!mine) break;  // behind the key's records
                             if (lane == 0) atomicAdd(&s.at, __popc(mine));
@@ -926,7 +939,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                     const int nr = min(kGroup, __popc(mine));
                     mine = m3 & (m3 - 1);
                     const int from = have ? __ffs(sel) - 1 : 0;
-                    const uint4 rec = __ldg(crec + (MANY ? place[from] : from));
+                    const uint4 rec = __ldg(crec + (GENERAL ? place[from] : from));
                     const int r_rs = (int)rec.x;
                     const unsigned r_z = have ? rec.z : 0u;
                     const int rl = r_z & 0xFF, rk0 = (r_z >> 16) & 0xFF, rK = r_z >> 24;
@@ -934,7 +947,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                     // tile wm and the record; every pair lies below the edges
                     // from k1 on
                     int k0 = rk0, k1 = rk0 + rK;
-                    bool ok = have && rK != 0, fast_ok = false;  // windows, FP32 distances
+                    bool ok = have && rK != 0, fast_ok = false, small = false;  // windows, FP32 distances, band
                     float dx, dy, dz;
                     {
                         const double2 *geo = reinterpret_cast<const double2 *>(s.job.leaf + rec.y);
@@ -949,7 +962,14 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                         // sqrt of every edge of the record
                         const float B = sqrtf(dx * dx + dy * dy + dz * dz) * 1.0001f + s.hT + 2.0f * s.Rq;
                         ok = ok && B < (float)kFp32Span && s.R[k1 - 1] < kFp32MaxR;
-                        fast_ok = ok && s.S > 0.0f && B * s.S <= 240.0f && hx + hy + hz <= s.hcap;
+                        const bool scaled = s.S > 0.0f && B * s.S <= 240.0f;
+                        if constexpr (GENERAL) {  // (a window needs no scale)
+                            const float h = hx + hy + hz;
+                            fast_ok = ok && scaled && h <= s.hcap;
+                            small = h <= s.hSmall && s.hSmall < s.hT;
+                        } else {
+                            ok = fast_ok = ok && (MODE == KD_MODE_FP64 || scaled);
+                        }
                         if (ok) {
                             // rounding of the staged coordinates and of the tile box
                             const float mg = 4.8e-7f * (fabsf(dx) + fabsf(dy) + fabsf(dz) + hx + hy + hz +
@@ -976,7 +996,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                     }
                     const int mval = max(0, min(kMT, s.qlen - kMT * wm));  // queries of tile wm
                     const int K = have && mval ? k1 - k0 : 0;
-                    const unsigned win = (unsigned)k0 | ((unsigned)K << 8);
+                    const unsigned win = (unsigned)k0 | ((unsigned)K << 8) | (GENERAL && small ? KD_MAX_EDGES << 16 : 0);
                     const unsigned actm = __ballot_sync(FULL, K != 0), okm = __ballot_sync(FULL, fast_ok);
                     if (have && mval) atomicAdd(&s.F[k1 * kMTiles + wm], (unsigned)rl);
                     {
@@ -1048,21 +1068,22 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                                 mt[1] = act ? __ffs(act) - 1 : mt[0];
                                 const unsigned wv = __shfl_sync(FULL, win, src + mt[0]),
                                                wv2 = __shfl_sync(FULL, win, src + mt[1]);
-                                int kk = wv & 0xFF, left = wv >> 8;
+                                int kk = wv & 0xFF, left = GENERAL ? (wv >> 8) & 0xFF : wv >> 8;
+                                const int eb = GENERAL ? (int)(wv >> 16) : 0;
                                 if (fast) {
                                     // two tiles with one window go together
                                     if (left == 1 && act && wv2 == wv) {
                                         act &= act - 1;
-                                        tile_pass<1, 2>(s, P, mt, kk, nt, ref, rs, n, lane, bs);
+                                        tile_pass<1, 2>(s, P, mt, kk, eb, nt, ref, rs, n, lane, bs);
                                         continue;
                                     }
                                     for (; left > 4; left -= 4, kk += 4)
-                                        tile_pass<4, 1>(s, P, mt, kk, nt, ref, rs, n, lane, bs);
+                                        tile_pass<4, 1>(s, P, mt, kk, eb, nt, ref, rs, n, lane, bs);
                                     switch (left) {
-                                    case 1: tile_pass<1, 1>(s, P, mt, kk, nt, ref, rs, n, lane, bs); break;
-                                    case 2: tile_pass<2, 1>(s, P, mt, kk, nt, ref, rs, n, lane, bs); break;
-                                    case 3: tile_pass<3, 1>(s, P, mt, kk, nt, ref, rs, n, lane, bs); break;
-                                    default: tile_pass<4, 1>(s, P, mt, kk, nt, ref, rs, n, lane, bs); break;
+                                    case 1: tile_pass<1, 1>(s, P, mt, kk, eb, nt, ref, rs, n, lane, bs); break;
+                                    case 2: tile_pass<2, 1>(s, P, mt, kk, eb, nt, ref, rs, n, lane, bs); break;
+                                    case 3: tile_pass<3, 1>(s, P, mt, kk, eb, nt, ref, rs, n, lane, bs); break;
+                                    default: tile_pass<4, 1>(s, P, mt, kk, eb, nt, ref, rs, n, lane, bs); break;
                                     }
                                 } else {  // out of FP32 range: every row exactly
                                     for (; left > 0; left -= 4, kk += 4)
@@ -1096,7 +1117,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                                 const double qx = v ? s.job.Q.x[s.qs + q] : s.o[0],
                                              qy = v ? s.job.Q.y[s.qs + q] : s.o[1],
                                              qz = v ? s.job.Q.z[s.qs + q] : s.o[2];
-                                for (int kk = wv & 0xFF, left = wv >> 8; left > 0; left -= kFpEdges, kk += kFpEdges) {
+                                for (int kk = wv & 0xFF, left = GENERAL ? (wv >> 8) & 0xFF : wv >> 8; left > 0; left -= kFpEdges, kk += kFpEdges) {
                                     unsigned cnt[kFpEdges] = {};
                                     switch (left) {
                                     case 1: fp64_run<1>(X + at, Y + at, Z + at, np, qx, qy, qz, s.R + kk, 1, cnt); break;
@@ -1127,7 +1148,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                 const int qf = tid < s.qlen ? J.Q.qf[s.qs + tid] : -1;
                 unsigned run = 0, before = 0, vm = __ballot_sync(FULL, qf >= 0);
                 unsigned alone = 0;  // the bits of its counters that a query adds by itself
-                if constexpr (MANY) {
+                if constexpr (GENERAL) {
                     // Up to KD_FEW_FIELDS own fields are summed over the warp, a
                     // round each; with more, every query adds its own counts.
                     // 400k points, symmetric, 21 edges, labels at random: 4
@@ -1144,7 +1165,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                     P[e * kPStride + tid] = 0;
                     unsigned v = cum - before;
                     before = cum;
-                    if constexpr (MANY) {
+                    if constexpr (GENERAL) {
                         if (v & alone)
                             atomicAdd(&Hd[((size_t)e * J.Fqe + qf) * J.Fte + tf], (unsigned long long)(v & alone));
                         v &= ~alone;
@@ -1175,16 +1196,20 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
     }
 }
 
-static size_t tile_smem(int ne, int mode, bool many)
+static size_t tile_smem(int ne, int mode, bool general)
 {
     const size_t fixed = mode == KD_MODE_MIXED ? sizeof(TileSmem<KD_MODE_MIXED>)
                                                : sizeof(TileSmem<KD_MODE_FP64>);
-    return fixed + sizeof(unsigned) * (size_t)ne * kPStride + (many ? sizeof(int) * kTileThreads : 0);
+    return fixed + sizeof(unsigned) * (size_t)ne * kPStride + (general ? sizeof(int) * kTileThreads : 0);
 }
 
-// The kernel for these counts.  Its variant for many labels costs all others
-// 2 to 3% (code: the instruction cache decides), so it is taken only where a
-// tree or query catalog's labels interleave, or where a counter could reach 2^27.
+// The kernel for these counts.  Its general variant costs all others 2 to 3% (the
+// code: 3M uniform points in 21 edges 5.66 and 5.80 ms), so it is taken only where
+// a tree's or query catalog's labels interleave, where a counter could reach
+// 2^27, or where the leaves' sizes differ so much that one error band is too wide.
+// In the last case: 1M points, 20 groups 1e-6 wide, radii 1e-8 and 1e-7, 3.13 -> 0.86
+// ms; one point at 1e12 3.78 -> 2.03, at infinity 3.13 -> 1.27; twelve decades of
+// |x| 29 -> 7.3.
 struct TileKernel {
     void (*run)(TileArgs);
     size_t smem;
@@ -1192,12 +1217,13 @@ struct TileKernel {
 
     TileKernel(const kd_catalog *const *tcs, const kd_catalog *const *qcs, int njobs, int ne, int mode)
     {
-        bool many = false;
+        bool general = false;
         for (int j = 0; j < njobs; j++)
-            many = many || tcs[j]->mixed_labels || qcs[j]->mixed_labels || tcs[j]->n_raw >= (int)kWideCount;
-        run = mode == KD_MODE_MIXED ? (many ? k_tiles<KD_MODE_MIXED, true> : k_tiles<KD_MODE_MIXED, false>)
-                                    : (many ? k_tiles<KD_MODE_FP64, true> : k_tiles<KD_MODE_FP64, false>);
-        smem = tile_smem(ne, mode, many);
+            general = general || tcs[j]->mixed_labels || qcs[j]->mixed_labels || tcs[j]->n_raw >= (int)kWideCount ||
+                      (mode == KD_MODE_MIXED && tcs[j]->uneven_leaves);
+        run = mode == KD_MODE_MIXED ? (general ? k_tiles<KD_MODE_MIXED, true> : k_tiles<KD_MODE_MIXED, false>)
+                                    : (general ? k_tiles<KD_MODE_FP64, true> : k_tiles<KD_MODE_FP64, false>);
+        smem = tile_smem(ne, mode, general);
         check(cudaFuncSetAttribute(run, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
               "smem attribute");
         check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, run, kTileThreads, smem), "occupancy");

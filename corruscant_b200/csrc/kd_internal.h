@@ -57,6 +57,8 @@ typedef struct kd_catalog {
     int mixed_labels; /* 1 when the labels interleave in space: a tree's runs of one tree field
                        * are shorter than 8 points on average, or most groups of 32 query
                        * points hold more than KD_FEW_FIELDS own fields */
+    int uneven_leaves; /* 1 when an eighth of the points or more (at full leaves) lie in leaves
+                        * of less than 1/64 of the largest one's size */
     double max_abs;   /* largest |coordinate| */
 
     /* reference-exact tree */

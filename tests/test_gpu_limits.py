@@ -124,3 +124,23 @@ def test_leaves_of_very_different_sizes(kind, seed):
             assert np.array_equal(N.count_points(t, p, f, 2, radii, mode=mode), want), mode
     finally:
         N.destroy(t)
+
+
+@pytest.mark.parametrize("spread", [1.0, 1e-3, 1e-6])
+def test_sparse_trees_and_dense_queries(spread):
+    """A tree whose every leaf is far larger than the query blocks."""
+    rs = np.random.RandomState(9)
+    for nt in (3, 50, 200):
+        tp = rs.rand(nt, 3)
+        q = 0.5 + spread * (rs.rand(3000, 3) - 0.5)
+        radii = np.logspace(-3, 0, 21)
+        want = O.OracleTree(tp).brute_counts(q, None, 1, radii, nthreads=4)
+        t = N.build_tree(tp, None, 1)
+        try:
+            got, st = N.count_points(t, q, None, 1, radii, with_stats=True)
+            assert np.array_equal(got, want)
+            # few of them need the exact path
+            assert st["pairs_rechecked"] <= st["pairs_tested"] / 2
+            assert np.array_equal(N.count_points(t, q, None, 1, radii, mode=N.KD_MODE_FP64), want)
+        finally:
+            N.destroy(t)
