@@ -1666,20 +1666,15 @@ __global__ void __launch_bounds__(TPB) k_leaves(int n, int nleaves, Cells cells,
     }
 }
 
-// one warp per leaf: its runs, one per tree field; and the number of leaves
-// below the size hcut
+// one warp per leaf: its runs, one per tree field
 __global__ void __launch_bounds__(TPB) k_leaf_runs(int nleaves, const int *__restrict__ pos,
                                                    const int *__restrict__ tf,
                                                    const int *__restrict__ leaf_run, int *run_start,
-                                                   int *run_len, int *run_tf, const kd_leaf *__restrict__ leaf,
-                                                   float hcut, int *small)
+                                                   int *run_len, int *run_tf)
 {
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    const int a = w < nleaves ? pos[w] : 0, len = w < nleaves ? pos[w + 1] - a : 0;
-    const bool below = lane == 0 && len > 0 && !(leaf[w].h[0] + leaf[w].h[1] + leaf[w].h[2] >= hcut);
-    const int nb = __syncthreads_count(below);
-    if (threadIdx.x == 0 && nb) atomicAdd(small, nb);
     if (w >= nleaves) return;
+    const int a = pos[w], len = pos[w + 1] - a;
     constexpr int PL = KD_RUN_MAX / 32;
     unsigned long long all = 0;
     int f[PL];
@@ -1708,10 +1703,22 @@ __global__ void __launch_bounds__(TPB) k_leaf_runs(int nleaves, const int *__res
 
 // Summaries of the levels [max(0, d0 - 8), d0), one CTA per subtree of the
 // lowest of them.  Empty leaves (at the end) leave their parent to its sibling.
-__global__ void __launch_bounds__(TPB) k_internal_summary(int d0, Summ sm)
+// leaf, where d0 is the leaves' level: also the number of leaves below 1/64 of
+// the largest half-diagonal.
+__global__ void __launch_bounds__(TPB) k_internal_summary(int d0, Summ sm, const kd_leaf *__restrict__ leaf,
+                                                          const double *hdiag, int *small)
 {
     const int top = max(0, d0 - 8);
     static_assert(TPB >= 128, "a thread per node of the first level");
+    if (leaf) {  // (every thread one of the CTA's up to 256 leaves)
+        static_assert(TPB >= 256, "a thread per leaf");
+        const int per = 1 << (d0 - top), l = blockIdx.x * per + threadIdx.x;
+        bool below = false;
+        if ((int)threadIdx.x < per && sm.count[((size_t)1 << d0) + l] > 0)
+            below = !(leaf[l].h[0] + leaf[l].h[1] + leaf[l].h[2] >= (float)(*hdiag / 64));
+        const int n = __syncthreads_count(below);
+        if (threadIdx.x == 0 && n) atomicAdd(small, n);
+    }
     for (int d = d0 - 1; d >= top; d--) {
         const int cnt = 1 << (d - top);
         if ((int)threadIdx.x < cnt) {
@@ -2638,20 +2645,24 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
     lf.pos = keep.alloc<int>((size_t)nleaves + 1);
     lf.nruns = pool.alloc<int>((size_t)nleaves + 1);
     lf.blocks = pool.alloc<int>((size_t)groups + 1);
-    lf.hdiag = pool.alloc<unsigned long long>(1);
-    check(cudaMemsetAsync(lf.hdiag, 0, sizeof(unsigned long long), s), "memset");
+    lf.hdiag = pool.alloc<unsigned long long>(2);  // and the number of small leaves
+    check(cudaMemsetAsync(lf.hdiag, 0, 2 * sizeof(unsigned long long), s), "memset");
     const unsigned gl = blocks_for(32 * ((long long)nleaves + 1), TPB);
     k_leaves<<<gl, TPB, 0, s>>>(n, nleaves, cells, perm, xyz, fin, tfin, lf);
     for (int d = D; d > 0; d = std::max(0, d - 8))
-        k_internal_summary<<<1u << std::max(0, d - 8), TPB, 0, s>>>(d, sm);
+        k_internal_summary<<<1u << std::max(0, d - 8), TPB, 0, s>>>(d, sm, d == D ? lf.leaf : nullptr,
+                                                                    (const double *)lf.hdiag, (int *)(lf.hdiag + 1));
     int *leaf_run = keep.alloc<int>((size_t)nleaves + 1);
     excl_sum(pool, s, lf.nruns, leaf_run, nleaves + 1);
     int *boff = pool.alloc<int>((size_t)groups + 1);
     excl_sum(pool, s, lf.blocks, boff, groups + 1);
     KD_LAUNCH_CHECK("layout kernels");
-    double leaf_hdiag;
+    struct {
+        double hdiag;
+        int small, pad;
+    } hl;
     int nblocks;
-    check(cudaMemcpyAsync(&leaf_hdiag, lf.hdiag, sizeof(double), cudaMemcpyDeviceToHost, s), "D2H");
+    check(cudaMemcpyAsync(&hl, lf.hdiag, sizeof hl, cudaMemcpyDeviceToHost, s), "D2H");
     check(cudaMemcpyAsync(&nblocks, boff + groups, sizeof(int), cudaMemcpyDeviceToHost, s), "D2H");
     const int nruns = read1(leaf_run + nleaves, s);
     int *run_start = keep.alloc<int>(nruns), *run_len = keep.alloc<int>(nruns),
@@ -2661,12 +2672,8 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
     double *bbox = keep.alloc<double>(6 * (size_t)nblocks);
     k_tree_blocks<<<blocks_for(groups, TPB), TPB, 0, s>>>(groups, nleaves, lf.pos, boff, sm.box, lf.qf, bstart,
                                                           blen, bbox, bqf);
-    int *small = pool.alloc<int>(1), nsmall;
-    check(cudaMemsetAsync(small, 0, sizeof(int), s), "memset");
-    k_leaf_runs<<<gl, TPB, 0, s>>>(nleaves, lf.pos, ro.tf, leaf_run, run_start, run_len, run_tf, lf.leaf,
-                                   (float)(leaf_hdiag / 64), small);
+    k_leaf_runs<<<gl, TPB, 0, s>>>(nleaves, lf.pos, ro.tf, leaf_run, run_start, run_len, run_tf);
     KD_LAUNCH_CHECK("summary kernels");
-    check(cudaMemcpyAsync(&nsmall, small, sizeof(int), cudaMemcpyDeviceToHost, s), "D2H");
     check(cudaEventRecord(ph[5], s), "event");
     st.sync();
     kd_build_stats bs;
@@ -2704,8 +2711,9 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
     cat->max_qf = h_fields ? hfi.max_qf : 0;
     cat->max_tf = hfi.max_tf;
     cat->fields_split = split;
-    cat->mixed_labels = hfi.max_tf > 0 && 8LL * nruns > n;
-    cat->uneven_leaves = 8LL * KD_RUN_MAX * nsmall > n;
+    cat->short_runs = hfi.max_tf > 0 && 4LL * nruns > n;
+    cat->many_fields = hfi.max_tf > 0 && 8LL * nruns > n;
+    cat->uneven_leaves = 8LL * KD_RUN_MAX * hl.small > n;
     cat->max_abs = maxabs;
     // the host holds the node array; the device copy is freed with the pool,
     // or, while a deferred copy still reads it, once that is done
@@ -2731,7 +2739,7 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
     cat->d_run_tf = keep.keep(run_tf);
     cat->d_t4 = keep.keep(lf.t4);
     cat->d_leaf = keep.keep(lf.leaf);
-    cat->leaf_hdiag = leaf_hdiag;
+    cat->leaf_hdiag = hl.hdiag;
     cat->nblocks = nblocks;
     cat->d_blk_start = keep.keep(bstart);
     cat->d_blk_len = keep.keep(blen);
@@ -2816,7 +2824,7 @@ static void build_query(const double *h_xyz, const int *h_fields, int n, int num
         *bqf = keep.alloc<int>(nblocks);
     double *bbox = keep.alloc<double>(6 * (size_t)nblocks);
     k_query_points<<<grid_for(n), TPB, 0, s>>>(xyz, fin, cv.perm, n, ro, nblocks, bstart, blen);
-    const bool fields = h.fi.max_qf - h.fi.min_qf >= KD_FEW_FIELDS;
+    const bool fields = (long long)h.fi.max_qf - h.fi.min_qf >= KD_FEW_FIELDS;
     k_block_boxes<<<nblocks, KD_BLOCK_MAX, 0, s>>>(nblocks, bstart, blen, ro, bbox, bqf,
                                                    fields ? &dstate->many : nullptr);
     KD_LAUNCH_CHECK("k_query_points");
@@ -2830,7 +2838,7 @@ static void build_query(const double *h_xyz, const int *h_fields, int n, int num
     cat->num_fields = num_fields;
     cat->min_qf = h.fi.min_qf;
     cat->max_qf = h.fi.max_qf;
-    cat->mixed_labels = 2LL * h.many > (n + 31) / 32;
+    cat->many_fields = 2LL * h.many > (n + 31) / 32;
     for (int d = 0; d < 3; d++)
         cat->max_abs = std::max(cat->max_abs, std::max(fabs(okey_value(~h.span.inv_lo[d])),
                                                        fabs(okey_value(h.span.hi[d]))));

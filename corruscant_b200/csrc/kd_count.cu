@@ -419,7 +419,7 @@ struct TileArgs {
     int g0, g1;                 // shard-local block indices of this launch
     const int *gmap;            // shard-local index -> global block (NULL: identity)
     const long long *off;       // launch-relative tile offsets
-    uint4 *rec;
+    const uint4 *rec;
     int *work;
     unsigned long long *stats;  // tested, rechecked, accepted, wide, edge-pairs, tiles
 };
@@ -495,7 +495,7 @@ struct TileCommon {
     float Rq, hT, S;
     // of the general variant
     float hSmall, hcap;                      // half-extents' sum of leaves with the smaller band, with any
-    int sorted, at;                          // records in order of their keys; the key's first place
+    int points, bqf;                         // of the block's runs; its single own field, -1 when mixed
 };
 template <int MODE> struct TileSmem;
 template <> struct TileSmem<KD_MODE_MIXED> : TileCommon {
@@ -552,51 +552,100 @@ __device__ __noinline__ void set_scale(TileSmem<KD_MODE_MIXED> &s, int ne, int t
 }
 __device__ __forceinline__ void set_scale(TileSmem<KD_MODE_FP64> &, int, int) {}
 
-// A block with many flush keys would read through all its records once for each
-// key.  From kSortKeys keys on its records are ordered by key first: the order
-// is written into the words w of the records themselves, above the bit that is
-// there, so that the record at place i of the order is rec[i].w >> 1.  By the
-// whole CTA; F is clear before and after.  400k points, symmetric, 21 edges,
-// labels at random: 250 of them 48.1 -> 34.9 ms, 64 24.7 -> 20.9, 16 8.4 -> 7.9;
-// with 2, 4 or 16 keys as the line all of these are within 1.5%.
-constexpr int kSortKeys = 8;
-__device__ __noinline__ void order_records(TileCommon &s, uint4 *rec, int tid)
+// A whole block whose runs are a point or two each (many labels that interleave
+// in space), by the whole CTA: a warp per record, four queries a lane, every
+// distance in FP64 in the reference's order, and the pairs of each bin straight
+// into the histogram.  A tile pass per (16 queries, point) and a flush per tree
+// field take several times the instructions there, for many fields of few pairs
+// each.  ONE, for a block with one own field, adds a run's pairs at once; the
+// others add every pair, which needs enough pairs of fields to keep the adds
+// apart.  400k points, 21 edges, tile passes -> this: labels of 64 kinds at random
+// with themselves 24.7 -> 6.5 ms, of 250 kinds 48.1 -> 6.4; 8 kinds against 64 (512
+// pairs of fields) 42.7 -> 24.9, 8 against 40 31.9 -> 39.8; 16 kinds with themselves
+// (runs of 4 points) 8.4 -> 24.  No labels against 64 kinds 34.6 -> 11.3, against 20
+// 13.6 -> 10.0, 16 10.9 -> 9.7, 12 (runs of 5) 8.1 -> 9.5.
+constexpr float kDirectRun = 2.5f, kDirectRunOne = 5.0f;  // points per run, on average
+constexpr int kDirectCells = 512;                         // pairs of fields
+template <bool ONE>
+__device__ __noinline__ void count_direct(TileCommon &s, const uint4 *__restrict__ recs, int ne, int tid)
 {
-    static_assert((KD_MAX_EDGES + 1) * kMTiles >= 512 + kTileWarps && kTileThreads * 4 == 512, "keys in F");
     constexpr unsigned FULL = 0xffffffffu;
-    const int lane = tid & 31, w = tid >> 5, n = s.ecnt;
-    auto key_of = [&](int i) {  // (not through the read-only cache: w is written here)
-        const uint2 r = __ldcg(reinterpret_cast<const uint2 *>(rec + i) + 1);
-        return ((r.x >> 8) & 0xFF) | (r.y & 1u) << 8;
-    };
-    for (int i = tid; i < n; i += kTileThreads) atomicAdd(&s.F[key_of(i)], 1u);
-    __syncthreads();
-    unsigned c[4], sum = 0;
+    constexpr int NQ = KD_BLOCK_MAX / 32;
+    const int lane = tid & 31, one = ONE ? s.bqf : 0;
+    const JobDesc &J = s.job;
+    double qx[NQ], qy[NQ], qz[NQ];
+    int qf[NQ];
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        c[k] = s.F[4 * tid + k];
-        sum += c[k];
+    for (int g = 0; g < NQ; g++) {
+        const int q = 32 * g + lane, i = s.qs + min(q, s.qlen - 1);
+        qx[g] = J.Q.x[i];
+        qy[g] = J.Q.y[i];
+        qz[g] = J.Q.z[i];
+        qf[g] = q < s.qlen ? (ONE ? one : J.Q.qf[i]) : -1;
     }
-    unsigned inc = sum;
+    unsigned long long pairs = 0, wide = 0, edges = 0, tiles = 0;
+    while (true) {
+        int c0 = 0;
+        if (lane == 0) c0 = atomicAdd(&s.next, s.chunk);
+        c0 = __shfl_sync(FULL, c0, 0);
+        const int nr = min(s.chunk, s.ecnt - c0);
+        if (nr <= 0) break;
+        const uint4 mine = __ldg(recs + c0 + min(lane, nr - 1));
+        for (int r = 0; r < nr; r++) {
+            const int rs = __shfl_sync(FULL, (int)mine.x, r);
+            const unsigned z = __shfl_sync(FULL, mine.z, r);
+            const int n = z & 0xFF, tf = (z >> 8) & 0xFF, k0 = (z >> 16) & 0xFF, K = z >> 24;
+            unsigned long long *const Hd = (__shfl_sync(FULL, mine.w, r) ? J.H2 : J.H) + tf;
+            auto bin = [&](int e, int f) { return &Hd[((size_t)e * J.Fqe + f) * J.Fte]; };
+            if constexpr (ONE) {
+                // a lane per edge holds the run's pairs below it
+                unsigned below = 0;  // the edge before these 32
+                for (int kb = k0; kb < k0 + K; kb += 32) {
+                    const int kn = min(32, k0 + K - kb);
+                    unsigned cum = 0;
+                    for (int j = 0; j < n; j++) {
+                        const double x = __ldg(J.tx + rs + j), y = __ldg(J.ty + rs + j), zz = __ldg(J.tz + rs + j);
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned y = __shfl_up_sync(FULL, inc, o);
-        if (lane >= o) inc += y;
-    }
-    if (lane == 31) s.F[512 + w] = inc;
-    __syncthreads();
-    unsigned at = inc - sum;
-    for (int k = 0; k < w; k++) at += s.F[512 + k];
+                        for (int g = 0; g < NQ; g++) {
+                            const double d2 = d2_ref(x, y, zz, qx[g], qy[g], qz[g]);
+                            for (int k = 0; k < kn; k++) {
+                                const unsigned c = __popc(__ballot_sync(FULL, d2 < s.R[kb + k] && qf[g] >= 0));
+                                if (lane == k) cum += c;
+                            }
+                        }
+                    }
+                    unsigned prev = __shfl_up_sync(FULL, cum, 1);
+                    if (lane == 0) prev = below;
+                    if (lane < kn && cum != prev) atomicAdd(bin(kb + lane, one), (unsigned long long)(cum - prev));
+                    below = __shfl_sync(FULL, cum, kn - 1);
+                }
+                const unsigned rest = (unsigned)(n * s.qlen) - below;
+                if (lane == 0 && k0 + K < ne && rest) atomicAdd(bin(k0 + K, one), (unsigned long long)rest);
+            } else {
+                for (int j = 0; j < n; j++) {
+                    const double x = __ldg(J.tx + rs + j), y = __ldg(J.ty + rs + j), zz = __ldg(J.tz + rs + j);
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        s.F[4 * tid + k] = at;
-        at += c[k];
+                    for (int g = 0; g < NQ; g++) {
+                        const double d2 = d2_ref(x, y, zz, qx[g], qy[g], qz[g]);
+                        int e = k0;
+                        for (int k = k0; k < k0 + K; k++) e += !(d2 < s.R[k]);
+                        if (qf[g] >= 0 && e < ne) atomicAdd(bin(e, qf[g]), 1ull);
+                    }
+                }
+            }
+            const unsigned np = K ? (unsigned)(n * s.qlen) : 0u;
+            pairs += np;
+            edges += (unsigned long long)np * K;
+            wide += K > 4 ? np : 0u;
+            tiles += K ? (s.qlen + kMT - 1) / kMT : 0;
+        }
     }
-    __syncthreads();
-    for (int i = tid; i < n; i += kTileThreads)
-        atomicOr(&rec[atomicAdd(&s.F[key_of(i)], 1u)].w, (unsigned)i << 1);
-    __syncthreads();
-    for (int k = tid; k < 512 + kTileWarps; k += kTileThreads) s.F[k] = 0;
+    if (lane == 0) {
+        atomicAdd(&s.stats[0], pairs);
+        atomicAdd(&s.stats[2], wide);
+        atomicAdd(&s.stats[3], edges);
+        atomicAdd(&s.stats[4], tiles);
+    }
 }
 
 // Exact counts of the flagged rows of query tile m (rows: bit per row) over
@@ -773,8 +822,6 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
     TileSmem<MODE> &s = *(TileSmem<MODE> *)smem;
     const int ne = A.ne;
     unsigned *const P = (unsigned *)(smem + sizeof(TileSmem<MODE>));
-    // GENERAL: the records of this warp's chunk
-    int *const place = (int *)(P + ne * kPStride) + (threadIdx.x & ~31);
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     const int wm = lane & (kMTiles - 1), wr = lane / kMTiles;  // this lane's window: tile, record
     for (int k = tid; k < ne; k += kTileThreads) {
@@ -792,6 +839,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
         if (tid == 0) s.item = atomicAdd(A.work, 1);
         if (tid < 16) s.keys[tid] = 0;
         if (tid == 0) {
+            if constexpr (GENERAL) s.points = s.next = 0;
             s.kmin = ne;
             s.kmax = 0;
             s.kfp = -1;
@@ -809,6 +857,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
             unsigned long long *dst = (unsigned long long *)&s.job;
             for (int u = tid; u < (int)(sizeof(JobDesc) / 8); u += kTileThreads) dst[u] = src[u];
             // the records' keys and edges
+            int points = 0;
             for (int i = tid; i < ecnt; i += kTileThreads) {
                 const uint4 r = __ldg(A.rec + eoff + i);
                 const unsigned key = ((r.z >> 8) & 0xFF) | (r.w << 8);
@@ -817,6 +866,11 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                 atomicMin(&s.kmin, k0);
                 atomicMax(&s.kmax, k1);
                 if (k1 > k0 && s.R[k1 - 1] < kFp32MaxR) atomicMax(&s.kfp, k1 - 1);
+                if constexpr (GENERAL) points += r.z & 0xFF;
+            }
+            if constexpr (GENERAL) {
+                points = __reduce_add_sync(FULL, points);
+                if (lane == 0) atomicAdd(&s.points, points);
             }
             __syncthreads();
             const JobDesc &J = s.job;
@@ -866,20 +920,15 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                 frexpf(Bm, &ex);  // Bm in [2^(ex-1), 2^ex)
                 S = ldexpf(1.0f, max(-60, min(60, 7 - ex)));
             }
-            const int nk = GENERAL ? __reduce_add_sync(FULL, lane < 16 ? __popc(s.keys[lane]) : 0) : 0;
             if (tid == 0) {
                 s.o[0] = ox;
                 s.o[1] = oy;
                 s.o[2] = oz;
                 s.eoff = eoff;
                 s.ecnt = ecnt;
-                // records a warp takes at a time: a few, where the pass has few
-                const int cnt = GENERAL && nk > kSortKeys ? ecnt / nk : ecnt;
-                s.chunk = cnt >= 1024 ? 32 : (cnt >= 512 ? 16 : (cnt >= 128 ? 8 : 4));
-                if constexpr (GENERAL) {
-                    s.sorted = nk > kSortKeys;
-                    s.at = 0;
-                }
+                // records a warp takes at a time: a few, where the block has few
+                s.chunk = ecnt >= 1024 ? 32 : (ecnt >= 512 ? 16 : (ecnt >= 128 ? 8 : 4));
+                if constexpr (GENERAL) s.bqf = J.Q.blk_qf[b];
                 s.qs = qs;
                 s.qlen = qlen;
                 s.Rq = Rq;
@@ -889,8 +938,15 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                 s.S = S;
             }
             __syncthreads();
+            if constexpr (GENERAL)
+                if (s.bqf >= 0 ? (float)s.points <= kDirectRunOne * (float)ecnt
+                               : (float)s.points <= kDirectRun * (float)ecnt &&
+                                     (long long)J.Fqe * J.Fte >= kDirectCells) {
+                    if (s.bqf >= 0) count_direct<true>(s, A.rec + eoff, ne, tid);
+                    else count_direct<false>(s, A.rec + eoff, ne, tid);
+                    continue;
+                }
             if (MODE == KD_MODE_MIXED && S > 0.0f) set_scale(s, ne, tid);
-            if (GENERAL && nk > kSortKeys) order_records(s, A.rec + eoff, tid);
         }
         // ---- one flush key after the other (tree field | 256 for the
         // once-counted part of a symmetric job)
@@ -902,34 +958,20 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
             }
             key += __ffs(kw) - 1;
             __syncthreads();  // the last key's counters are clear
-            if (tid == 0) s.next = GENERAL ? s.at : 0;
+            if (tid == 0) s.next = 0;
             __syncthreads();
             while (true) {
                 int c0 = 0;
                 if (lane == 0) c0 = atomicAdd(&s.next, s.chunk);
                 c0 = __shfl_sync(FULL, c0, 0);
                 if (c0 >= s.ecnt) break;
-                const uint4 *const crec = A.rec + s.eoff + (GENERAL ? 0 : c0);
+                const uint4 *const crec = A.rec + s.eoff + c0;
                 unsigned mine;
                 {
                     uint2 r = make_uint2(0, 0);
                     const bool in = lane < s.chunk && c0 + lane < s.ecnt;
-                    int i = lane;
-                    if constexpr (GENERAL) {
-                        i = c0 + lane;
-                        if (in && s.sorted) i = (int)(__ldcg(&crec[i].w) >> 1);
-                        place[lane] = i;
-                    }
-                    if (in) r = __ldg(reinterpret_cast<const uint2 *>(crec + i) + 1);
-                    if constexpr (GENERAL) r.y &= 1u;
+                    if (in) r = __ldg(reinterpret_cast<const uint2 *>(crec + lane) + 1);
                     mine = __ballot_sync(FULL, in && (((r.x >> 8) & 0xFF) | (r.y << 8)) == (unsigned)key);
-                    if constexpr (GENERAL) {
-                        if (s.sorted) {
-                            if (!mine) break;  // behind the key's records
-                            if (lane == 0) atomicAdd(&s.at, __popc(mine));
-                        }
-                        __syncwarp();
-                    }
                 }
                 while (mine) {
                     // ---- the next four records: lane (wm, wr) has record wr
@@ -939,7 +981,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                     const int nr = min(kGroup, __popc(mine));
                     mine = m3 & (m3 - 1);
                     const int from = have ? __ffs(sel) - 1 : 0;
-                    const uint4 rec = __ldg(crec + (GENERAL ? place[from] : from));
+                    const uint4 rec = __ldg(crec + from);
                     const int r_rs = (int)rec.x;
                     const unsigned r_z = have ? rec.z : 0u;
                     const int rl = r_z & 0xFF, rk0 = (r_z >> 16) & 0xFF, rK = r_z >> 24;
@@ -1153,7 +1195,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                     // round each; with more, every query adds its own counts.
                     // 400k points, symmetric, 21 edges, labels at random: 4
                     // fields 2.9 ms by rounds and 4.7 by query, 5 3.45 and 3.45,
-                    // 16 10.2 and 8.2, 64 49.3 and 24.7, 250 142.6 and 48.1.
+                    // 16 10.2 and 8.2.
                     const unsigned peers = __match_any_sync(FULL, qf);
                     const bool many = __popc(__ballot_sync(FULL, qf >= 0 && lane == __ffs(peers) - 1)) > KD_FEW_FIELDS;
                     if (qf >= 0) alone = many ? FULL : ~(kWideCount - 1);
@@ -1196,20 +1238,20 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
     }
 }
 
-static size_t tile_smem(int ne, int mode, bool general)
+static size_t tile_smem(int ne, int mode)
 {
     const size_t fixed = mode == KD_MODE_MIXED ? sizeof(TileSmem<KD_MODE_MIXED>)
                                                : sizeof(TileSmem<KD_MODE_FP64>);
-    return fixed + sizeof(unsigned) * (size_t)ne * kPStride + (general ? sizeof(int) * kTileThreads : 0);
+    return fixed + sizeof(unsigned) * (size_t)ne * kPStride;
 }
 
 // The kernel for these counts.  Its general variant costs all others 2 to 3% (the
 // code: 3M uniform points in 21 edges 5.66 and 5.80 ms), so it is taken only where
-// a tree's or query catalog's labels interleave, where a counter could reach
-// 2^27, or where the leaves' sizes differ so much that one error band is too wide.
-// In the last case: 1M points, 20 groups 1e-6 wide, radii 1e-8 and 1e-7, 3.13 -> 0.86
-// ms; one point at 1e12 3.78 -> 2.03, at infinity 3.13 -> 1.27; twelve decades of
-// |x| 29 -> 7.3.
+// labels interleave (a tree's runs are short, or a query warp's own fields many),
+// where a counter could reach 2^27, or where the leaves' sizes differ so much that
+// one error band is too wide.  In the last case: 1M points, 20 groups 1e-6 wide,
+// radii 1e-8 and 1e-7, 3.13 -> 0.86 ms; one point at 1e12 3.78 -> 2.03, at infinity
+// 3.13 -> 1.27; twelve decades of |x| 29 -> 7.3.
 struct TileKernel {
     void (*run)(TileArgs);
     size_t smem;
@@ -1219,11 +1261,11 @@ struct TileKernel {
     {
         bool general = false;
         for (int j = 0; j < njobs; j++)
-            general = general || tcs[j]->mixed_labels || qcs[j]->mixed_labels || tcs[j]->n_raw >= (int)kWideCount ||
+            general = general || tcs[j]->short_runs || qcs[j]->many_fields || tcs[j]->n_raw >= (int)kWideCount ||
                       (mode == KD_MODE_MIXED && tcs[j]->uneven_leaves);
         run = mode == KD_MODE_MIXED ? (general ? k_tiles<KD_MODE_MIXED, true> : k_tiles<KD_MODE_MIXED, false>)
                                     : (general ? k_tiles<KD_MODE_FP64, true> : k_tiles<KD_MODE_FP64, false>);
-        smem = tile_smem(ne, mode, general);
+        smem = tile_smem(ne, mode);
         check(cudaFuncSetAttribute(run, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
               "smem attribute");
         check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, run, kTileThreads, smem), "occupancy");

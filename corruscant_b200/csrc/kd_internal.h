@@ -54,9 +54,10 @@ typedef struct kd_catalog {
     int max_tf;       /* largest stored tree field id */
     int min_qf;       /* smallest own field id */
     int fields_split; /* 1 when some raw point has qf != tf */
-    int mixed_labels; /* 1 when the labels interleave in space: a tree's runs of one tree field
-                       * are shorter than 8 points on average, or most groups of 32 query
-                       * points hold more than KD_FEW_FIELDS own fields */
+    int short_runs;   /* 1 when a tree's runs of one tree field are shorter than 4 points on
+                       * average: its labels interleave in space */
+    int many_fields;  /* 1 when most groups of 32 query points hold more than KD_FEW_FIELDS own
+                       * fields (a tree's by its runs: shorter than 8 points on average) */
     int uneven_leaves; /* 1 when an eighth of the points or more (at full leaves) lie in leaves
                         * of less than 1/64 of the largest one's size */
     double max_abs;   /* largest |coordinate| */
