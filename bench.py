@@ -507,7 +507,7 @@ def _measure(N, D, w, steps, warmup):
             step(mode)
         D.barrier()
         acc = dict(dev_ms=0.0, pairs=0, launches=0, tile_launches=0, tiles_ms=0.0, rechecked=0,
-                   edge_pairs=0, accepted=0, one_bin_multifield=0, trav_ms=0.0)
+                   edge_pairs=0, entries=0, accepted=0, one_bin_multifield=0, trav_ms=0.0)
         res = None
         for _ in range(k):
             res, s = step(mode)
@@ -518,6 +518,7 @@ def _measure(N, D, w, steps, warmup):
             acc["tiles_ms"] += s["ms_tiles"]
             acc["rechecked"] += s["pairs_rechecked"]
             acc["edge_pairs"] += s["edge_pairs"]
+            acc["entries"] += s["entries"]
             acc["accepted"] += s["pairs_accepted"]
             acc["one_bin_multifield"] += s["pairs_one_bin_multifield"]
             acc["trav_ms"] += s["ms_traverse"]
@@ -608,15 +609,15 @@ def _summary(w, m, steps, peak, peak64, D):
     lane32 = nsm * 128 * 2 * mhz * 1e6 / 1e12 if (nsm and mhz) else None
     roofline = {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                 "frac": (achieved / peak) if peak else None,
-                "traffic": TILE_TRAFFIC_PER_PAIR * launch_pairs if TILE_TRAFFIC_PER_PAIR else None,
+                "traffic": (RECORD_BYTES * mixed["entries"] / max(1, mixed["tile_launches"]) +
+                            POINT_BYTES * sum(len(c[0]) for c in w.catalogs.values())),
+                "traffic_source": TILE_TRAFFIC_SOURCE,
                 "kernel": "k_tiles<mixed> (one launch: the step's whole batch)",
                 "peak_source": "measured in this run: cuBLAS SGEMM 8192^3, TF32 off",
                 "lane_peak": lane32,
                 "frac_of_lane_peak": (achieved / lane32) if lane32 else None,
                 "lane_peak_basis": "SMs x 128 FP32 lanes x 2 FLOP x median SM clock",
                 "flop_per_pair": FLOP_PER_PAIR}
-    if TILE_TRAFFIC_PER_PAIR:
-        roofline["traffic_source"] = TILE_TRAFFIC_SOURCE
     # FP32-pipe model of the binning itself: 3 FMA lane-ops per pair and
     # active edge (ramp, count, band check); the distances are on the tensor
     # pipe
@@ -747,14 +748,12 @@ def run_mine(args):
     D.close()
 
 
-# Per-pair DRAM traffic of the tile kernel (dram bytes read + written by one
-# k_tiles launch over the pairs it tested), from an ncu capture of 1M uniform
-# points with themselves (64 fields, 21 log-spaced edges), scaled to a launch by
-# its pairs: the traffic is mostly the tile records, whose number grows with
-# the pairs.
-TILE_TRAFFIC_PER_PAIR = (1.89379072e8 + 3.620096e6) / 4.5997e10  # bytes per pair tested
-TILE_TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of one k_tiles launch, "
-                       "1M uniform points with themselves (4.6e10 pairs), scaled by pairs")
+# DRAM traffic of a k_tiles launch: its records and the catalogs' points, once.
+# An ncu capture of 1M uniform points with themselves (64 fields, 21 log-spaced
+# edges; 8.73M records) read 0.1894 and wrote 0.0036 GB, where this gives 0.1877.
+RECORD_BYTES, POINT_BYTES = 16, 48
+TILE_TRAFFIC_SOURCE = ("from this workload's statistics: 16 bytes per (query block, tree run) record and 48 "
+                       "per catalog point, once each (0.188 GB where an ncu capture measured 0.193)")
 
 
 # ------------------------------------------------------- reference (CPU) arm
