@@ -29,9 +29,10 @@
 // segment's split dimension, writes the level's nodes, then moves every
 // position to its child segment with a stable segmented partition; segments of
 // up to kSubCap points go through all their remaining levels in one block's
-// shared memory.  Split dimensions of segments of more than kSubSeq points come from a parallel variance with a rigorous error interval around
-// the value the reference's sequential sums produce; only when the intervals of
-// the best and another dimension overlap is the sequential computation run.
+// shared memory.  Split dimensions of segments of more than kSubSeq points come
+// from a parallel variance with a rigorous error interval around the value the
+// reference's sequential sums produce; only when the intervals of the best and
+// another dimension overlap is the sequential computation run.
 
 #include <algorithm>
 #include <atomic>
@@ -349,8 +350,9 @@ __global__ void k_first_seg(Segs sg, int n_u)
     sg.r[0] = n_u - 1;
 }
 
-// One level's buffers cleared, and the next level's segments (every segment of
-// the level loop is larger than kSubCap, so it splits).
+// One level's buffers cleared, and the next level's segments (the largest of the
+// level loop holds more than kSubCap points and no other more than one fewer, so
+// all of them split).
 __global__ void k_seg_setup(Segs sg, int ub, LevelBufs lb, Segs nxt)
 {
     int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -645,7 +647,6 @@ __global__ void k_ranks(int n, const int *__restrict__ a1, const int *__restrict
     }
 }
 
-// side of every point of a splitting segment: 0 left, 1 right, 2 median
 // ---- Stable three-way partition of the three superkey orders, one level.
 // Within every segment [l, r], median position med = (l + r + 1) / 2, the
 // points of each order d go, in their order, to [l, med) when they stand before
@@ -2086,10 +2087,6 @@ struct StagingLease {
         g_stage_cv.notify_one();
     }
 };
-// Host copies of a transfer's chunks fanned out over a pool of threads made
-// once for the whole transfer (a 32 MB chunk takes ~1 ms; creating threads
-// per chunk would cost a good part of that).  Transfers under 4 MB are
-// copied by the calling thread alone.
 // Copy to or from a staging chunk without leaving its lines in this core's
 // cache: a DMA that meets lines of a core gone idle runs at 6 GB/s instead of
 // 50.  The chunk's side is aligned to 64 bytes.
@@ -2109,6 +2106,10 @@ static void copy_uncached(char *d, const char *f, size_t n, bool to_staging)
 #endif
     std::memcpy(d + i, f + i, n - i);
 }
+// Host copies of a transfer's chunks fanned out over threads made once for the
+// whole transfer (a 32 MB chunk takes ~1 ms; creating threads per chunk would
+// cost a good part of that): one per MB of the transfer, up to 16, the calling
+// thread among them.
 struct FanOut {
     int nthr = 1;
     std::vector<std::thread> th;
@@ -2442,13 +2443,14 @@ static void build_impl(const double *h_xyz, const int *h_fields, int n, int num_
         k_first_seg<<<1, 1, 0, s>>>(sg[0], n_u);
         KD_LAUNCH_CHECK("k_first_seg");
     }
-    // The node array goes to the caller's host array level by level while
-    // the tree is built: iteration lev of the loop below writes the heap
-    // slots of level lev, so once it has run, every slot below 2^(lev+1) is
-    // final; k_subtrees writes all others.  The build records an event where
-    // slots worth a copy are final and queues them; a second host thread waits
-    // for each event and copies the slots (pinned staging, DMA on its own
-    // stream) while the build goes on.
+    // The node array goes to the caller's host array while the counting layout
+    // is built: k_subtrees writes the slots of the last ten levels, so nearly all
+    // of them, and is the last kernel of the tree.  (Iteration lev of the loop
+    // below writes the heap slots of level lev, so once it has run, every slot
+    // below 2^(lev+1) is final; those go ahead where they are worth a copy, from
+    // about 70M points on.)  The build records an event and queues the slots; a
+    // second host thread, which has touched the host pages meanwhile, waits for
+    // each event and copies them (pinned staging, DMA on its own stream).
     std::unique_ptr<NodeCopy> ncu(new NodeCopy);
     NodeCopy &nc = *ncu;
     const size_t node_bytes = sizeof(NodeRec) * (size_t)memsize;
@@ -2781,10 +2783,8 @@ __global__ void k_query_points(const double *__restrict__ xyz, const int *__rest
 // blocks are better ones, too (no cut at the subtrees' ends, near points next
 // to each other): 3M points, 21 edges, 1.58M instead of 1.80M (block, run)
 // records and 9.4 instead of 12.0 ms in the tile kernel; in Z-order, whose
-// jumps stretch the boxes, 2.37M records and 14.4 ms.  Returns false, with
-// nothing kept, where the cells are too coarse for the points (one in eight
-// shares a cell with another: an outlier far away, or an infinite coordinate):
-// the tree's cuts follow the points at any scale.
+// jumps stretch the boxes, 2.37M records and 14.4 ms.  Where the curve's cells
+// are too coarse for the points, Curve::finish follows them at any scale.
 static void build_query(const double *h_xyz, const int *h_fields, int n, int num_fields, kd_catalog *cat)
 {
     init_device();

@@ -22,13 +22,13 @@
 //                with a run's points only against the edges that its own box
 //                and the leaf's allow.  Mixed mode: FP32 distances relative to
 //                the block centre from the tensor pipe, binned against those
-//                edges with a saturating ramp that is exactly 0 or 1 outside a
-//                rigorous error band; a query with any pair of the run inside
-//                the band is recounted in FP64 with the reference's operation
-//                order.  FP64 mode: every distance in FP64.  Per-query counters
-//                live in shared memory and are reduced per own field into the
-//                global (bin, qfield, tfield) histogram, tree field by tree
-//                field.
+//                edges with a saturating ramp that is exactly 0 or 1 outside an
+//                error band; a query with any pair of the run inside the band is
+//                recounted in FP64 with the reference's operation order.  FP64
+//                mode: every distance in FP64 (boxes decide in FP32 with margins
+//                for every rounding, in both modes).  Per-query counters live in
+//                shared memory and are reduced per own field into the global
+//                (bin, qfield, tfield) histogram, tree field by tree field.
 
 #include <algorithm>
 #include <exception>
@@ -383,11 +383,17 @@ constexpr double kFp32MaxR = 1e30;
 //   cross term   8u Rq P      (2^-23 relative for each split factor)
 //   C, edges     2u (Rq^2 + R) + 3u R
 //   ramp         4u R         (its offset and slope)
-//   accumulation 17 terms, each cut at no more than u of the largest one
-//                (|N|, |C| <= M, |2 q t'| <= 2 Rq P): 17u max(M, 2 Rq P)
+//   accumulation 17u max(M, 2 Rq P), with |N|, |C| <= M, |2 q t'| <= 2 Rq P
 // plus the halves' absolute floor, 2^-25 of the scaled values, and the
-// rounding of the FP64 reference itself; 25% on top.  (Measured: at most 6u
-// (sqrt(d2) + Rq)^2 in all.)  Pairs with d2 > 1.2 R: their error grows with
+// rounding of the FP64 reference itself; 25% on top.
+// All but the accumulation is derived.  How the tensor core aligns, cuts and
+// rounds the 17 terms PTX leaves open, so that term is an assumption.  It rests
+// on a measurement: over 2.5M sums each of eight kinds (spread exponents, equal
+// magnitudes, a large term, cancelling ones) the error was at most 2.1u of the
+// largest term where the sum cancels, and else 2u of the result besides, which
+// here stays below 3 max(M, 2 Rq P): 8u in all, where an FP32 FMA chain had up to
+// 12u where the sum cancels.  (x as a whole: at most 6u (sqrt(d2) + Rq)^2
+// measured, about 70u allowed.)  Pairs with d2 > 1.2 R: their error grows with
 // (sqrt(d2) + Rq)^2 while x - (R - R0) >= d2 / 6, so the sign is right
 // unless d2 is so small beside Rq^2 that E's Rq terms cover the error.
 __device__ __forceinline__ double band_halfwidth(double R, double Rq, double hT, double S)

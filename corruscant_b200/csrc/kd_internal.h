@@ -6,9 +6,12 @@
  *   - the reference-exact k-d tree (node_t array, heap order, root at 1) that
  *     kdbuild.c:451-537 would produce, plus its in-order permutation;
  *   - a counting layout of the RAW input points (duplicates kept, one entry
- *     each) along a Hilbert curve, cut into leaves of KD_RUN_MAX points (grouped
- *     by tree-side field into "runs") and query blocks of KD_BLOCK_MAX, under a
- *     binary tree of bounding boxes, raw counts and single-field summaries.
+ *     each) by cells of the tree's own splits, each split on in the middle, and
+ *     cut into leaves of KD_RUN_MAX points (grouped by tree-side field into
+ *     "runs") and query blocks of KD_BLOCK_MAX, under a binary tree of bounding
+ *     boxes, raw counts and single-field summaries.
+ * A catalog of raw query points has only the points, along a Hilbert curve and
+ * split in the same way, and the blocks.
  *
  * Every raw point carries two field ids: qf, its own field (what the
  * reference's query side reads, kdquery.c:67-70), and tf, the low 8 bits of
@@ -30,7 +33,7 @@ extern "C" {
 #endif
 
 #define KD_RUN_MAX 64      /* points per leaf of the counting tree, so at most per run */
-#define KD_BLOCK_MAX 128   /* query points per block (one warp) */
+#define KD_BLOCK_MAX 128   /* query points per block (a CTA of four warps counts it) */
 #define KD_MAX_EDGES 64    /* distinct finite squared edges per count job */
 #define KD_FEW_FIELDS 4    /* own fields of 32 queries that a count sums field by field */
 
