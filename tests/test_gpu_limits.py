@@ -1,5 +1,6 @@
-"""Counts where the counters' width, the padding of partly filled runs and the
-exponent range of the FP32 bounds would show (exact: integers, no tolerance)."""
+"""Counts where the counters' width, the padding of partly filled runs, the
+exponent range of the FP32 bounds, leaves of very different sizes and often
+repeated points would show (exact: integers, no tolerance)."""
 import numpy as np
 import pytest
 
@@ -144,3 +145,30 @@ def test_sparse_trees_and_dense_queries(spread):
             assert np.array_equal(N.count_points(t, q, None, 1, radii, mode=N.KD_MODE_FP64), want)
         finally:
             N.destroy(t)
+
+
+@pytest.mark.parametrize("kind", ["copies", "zeros", "one place"])
+@pytest.mark.parametrize("n", [4097, 20001])
+def test_repeated_query_points_over_several_chunks(n, kind):
+    """Raw query points repeated more often than a tree accepts, at sizes of
+    several chunks of the counting order."""
+    rs = np.random.RandomState(n)
+    if kind == "copies":
+        q = rs.rand(1 + n // 300, 3)[rs.randint(0, 1 + n // 300, n)]
+    elif kind == "zeros":
+        q = rs.rand(n, 3)
+        q[rs.rand(n) < 0.3] = 0.0
+        q[rs.rand(n, 3) < 0.05] = -0.0
+    else:
+        q = np.tile(rs.rand(1, 3), (n, 1))
+    f = rs.randint(0, 3, n).astype(np.int32)
+    tp = np.unique(np.concatenate([q[:500], rs.rand(3000, 3)]), axis=0)
+    tf = rs.randint(0, 3, len(tp)).astype(np.int32)
+    radii = np.array([0.03, 0.1, 0.4, 1.2])
+    want = O.OracleTree(tp, tf, 3).brute_counts(q, f, 3, radii, nthreads=8)
+    t = N.build_tree(tp, tf, 3)
+    try:
+        for mode in MODES:
+            assert np.array_equal(N.count_points(t, q, f, 3, radii, mode=mode), want), mode
+    finally:
+        N.destroy(t)
