@@ -563,9 +563,10 @@ __device__ __forceinline__ void set_scale(TileSmem<KD_MODE_FP64> &, int, int) {}
 // distance in FP64 in the reference's order, and the pairs of each bin straight
 // into the histogram.  A tile pass per (16 queries, point) and a flush per tree
 // field take several times the instructions there, for many fields of few pairs
-// each.  ONE, for a block with one own field, adds a run's pairs at once; the
-// others add every pair, which needs enough pairs of fields to keep the adds
-// apart.  400k points, 21 edges, tile passes -> this: labels of 64 kinds at random
+// each.  Bound by the issue slots (71% at 64 labels: a compare per pair and edge)
+// and the adds' wavefronts (69%).  ONE, for a block with one own field, adds a
+// run's pairs at once; the others add every pair, which needs enough pairs of
+// fields to keep the adds apart.  400k points, 21 edges, tile passes -> this: labels of 64 kinds at random
 // with themselves 24.7 -> 6.5 ms, of 250 kinds 48.1 -> 6.4; 8 kinds against 64 (512
 // pairs of fields) 42.7 -> 24.9, 8 against 40 31.9 -> 39.8; 16 kinds with themselves
 // (runs of 4 points) 8.4 -> 24.  No labels against 64 kinds 34.6 -> 11.3, against 20
