@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(32 * kTravWarps) k_traverse(const JobDesc *__r
 // run's points, every distance in the reference's operation order, up to six
 // edges per distance (two tiles at a time, with one window for both, and four
 // edges: 7% and 4% slower; compares as integers, on the ALU: 4%).  Bound by
-// the issue slots, then the FP64 pipe (73% and 64% used).
+// the issue slots, then the FP64 pipe (76% and 55% used).
 //
 // Bound: the issue slots (73% used) and the FP32 pipe (51%), by the binning (a
 // ramp, a count and a check per pair and edge: 15 clocks per 128 pairs and edge
@@ -566,11 +566,12 @@ __device__ __forceinline__ void set_scale(TileSmem<KD_MODE_FP64> &, int, int) {}
 // each.  Bound by the issue slots (71% at 64 labels: a compare per pair and edge)
 // and the adds' wavefronts (69%).  ONE, for a block with one own field, adds a
 // run's pairs at once; the others add every pair, which needs enough pairs of
-// fields to keep the adds apart.  400k points, 21 edges, tile passes -> this: labels of 64 kinds at random
-// with themselves 24.7 -> 6.5 ms, of 250 kinds 48.1 -> 6.4; 8 kinds against 64 (512
-// pairs of fields) 42.7 -> 24.9, 8 against 40 31.9 -> 39.8; 16 kinds with themselves
-// (runs of 4 points) 8.4 -> 24.  No labels against 64 kinds 34.6 -> 11.3, against 20
-// 13.6 -> 10.0, 16 10.9 -> 9.7, 12 (runs of 5) 8.1 -> 9.5.
+// fields to keep the adds apart.  400k points, 21 edges, tile passes -> this:
+// labels of 64 kinds at random with themselves 24.7 -> 6.5 ms, of 250 kinds 48.1 ->
+// 6.4; 8 kinds against 64 (512 pairs of fields) 42.7 -> 24.9, 8 against 40 31.9 ->
+// 39.8; 16 kinds with themselves (runs of 4 points) 8.4 -> 24.  No labels against
+// 64 kinds 34.6 -> 11.3, against 20 13.6 -> 10.0, 16 10.9 -> 9.7, 12 (runs of 5)
+// 8.1 -> 9.5.
 constexpr float kDirectRun = 2.5f, kDirectRunOne = 5.0f;  // points per run, on average
 constexpr int kDirectCells = 512;                         // pairs of fields
 template <bool ONE>
