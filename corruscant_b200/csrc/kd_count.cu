@@ -485,6 +485,7 @@ __device__ __forceinline__ void fp64_run(const double2 *__restrict__ tx,
 //     query of tile m
 //   P[e * kPStride + q], behind it: pairs of query q below edge e, over the
 //     records whose window for q's tile holds e
+//   behind P, in the general variant: the edge table of small leaves
 struct TileCommon {
     JobDesc job;  // the job of the block being counted
     double R[KD_MAX_EDGES];
@@ -507,7 +508,7 @@ template <int MODE> struct TileSmem;
 template <> struct TileSmem<KD_MODE_MIXED> : TileCommon {
     alignas(16) uint4 qa[kMTiles][32];       // MMA A fragments of the query tiles
     float2 qn[kMTiles][kMT / 2];             // |q|^2 S^2 of rows g and g + 8
-    float2 edge[2 * KD_MAX_EDGES];           // R S^2 and 0.4545 / (E S^2); from KD_MAX_EDGES on, for small leaves
+    float2 edge[KD_MAX_EDGES];               // R S^2 and 0.4545 / (E S^2)
     alignas(16) uint32_t bs[kTileWarps][KD_RUN_MAX / kNT * 32];  // MMA B fragments of the staged runs
 };
 template <> struct TileSmem<KD_MODE_FP64> : TileCommon {
@@ -519,7 +520,7 @@ template <> struct TileSmem<KD_MODE_FP64> : TileCommon {
 // tile's fragment holds, for t < 3, coordinate t of rows g and g + 8: the
 // halves of v = -2 q_t S as (hi, hi) against the point's (hi, lo), and (lo,
 // lo) against the same; for t = 3, (1, 1) against the halves of N, and (0, 0).
-__device__ __noinline__ void set_scale(TileSmem<KD_MODE_MIXED> &s, int ne, int tid)
+__device__ __noinline__ void set_scale(TileSmem<KD_MODE_MIXED> &s, float2 *small, int ne, int tid)
 {
     const double S = (double)s.S, Rq = (double)s.Rq;
     const int qs = s.qs, qlen = s.qlen;
@@ -550,13 +551,15 @@ __device__ __noinline__ void set_scale(TileSmem<KD_MODE_MIXED> &s, int ne, int t
         if (tid % kMT < 8) q.x = (float)n;
         else q.y = (float)n;
     }
-    for (int b = 0; b < (s.hSmall < s.hT ? 2 : 1); b++)
+    for (int b = 0; b < (small ? 2 : 1); b++) {
+        float2 *const edge = b ? small : s.edge;
         for (int k = tid; k < ne; k += kTileThreads)
-            s.edge[b * KD_MAX_EDGES + k] = make_float2(
+            edge[k] = make_float2(
                 (float)(s.R[k] * S * S),
                 (float)(0.5 / 1.1 / (band_halfwidth(s.R[k], Rq, b ? (double)s.hSmall : (double)s.hT, S) * S * S)));
+    }
 }
-__device__ __forceinline__ void set_scale(TileSmem<KD_MODE_FP64> &, int, int) {}
+__device__ __forceinline__ void set_scale(TileSmem<KD_MODE_FP64> &, float2 *, int, int) {}
 
 // A whole block whose runs are a point or two each (many labels that interleave
 // in space), by the whole CTA: a warp per record, four queries a lane, every
@@ -706,14 +709,14 @@ __device__ __noinline__ void recount_rows(TileCommon &s, unsigned *P, unsigned r
 // saturating ramp has no packed form.
 template <int K, int M>
 __device__ __forceinline__ void tile_pass(TileSmem<KD_MODE_MIXED> &s, unsigned *P, const int (&mt)[2],
-                                          int kk, int eb, int nt, float ref, int rs, int n, int lane,
+                                          int kk, const float2 *edges, int nt, float ref, int rs, int n, int lane,
                                           const uint32_t *__restrict__ bs)
 {
     static_assert(K * M <= 4 && M <= 2, "an item per lane of a row");
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int NI = K * M;  // item i: edge kk + i % K of tile mt[i / K]
     const int g = lane >> 2, t = lane & 3;
-    const float2 *const edge = s.edge + eb + kk;
+    const float2 *const edge = edges + kk;
     const float e0 = edge[0].x, nsl = -edge[K - 1].y;
     float a[K];
     a[0] = 0.5f;
@@ -954,7 +957,8 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                     else count_direct<false>(s, A.rec + eoff, ne, tid);
                     continue;
                 }
-            if (MODE == KD_MODE_MIXED && S > 0.0f) set_scale(s, ne, tid);
+            if (MODE == KD_MODE_MIXED && S > 0.0f)
+                set_scale(s, GENERAL && hSmall < hT ? (float2 *)(P + ne * kPStride) : nullptr, ne, tid);
         }
         // ---- one flush key after the other (tree field | 256 for the
         // once-counted part of a symmetric job)
@@ -1046,7 +1050,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                     }
                     const int mval = max(0, min(kMT, s.qlen - kMT * wm));  // queries of tile wm
                     const int K = have && mval ? k1 - k0 : 0;
-                    const unsigned win = (unsigned)k0 | ((unsigned)K << 8) | (GENERAL && small ? KD_MAX_EDGES << 16 : 0);
+                    const unsigned win = (unsigned)k0 | ((unsigned)K << 8) | (GENERAL && small ? 1u << 16 : 0u);
                     const unsigned actm = __ballot_sync(FULL, K != 0), okm = __ballot_sync(FULL, fast_ok);
                     if (have && mval) atomicAdd(&s.F[k1 * kMTiles + wm], (unsigned)rl);
                     {
@@ -1119,21 +1123,21 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                                 const unsigned wv = __shfl_sync(FULL, win, src + mt[0]),
                                                wv2 = __shfl_sync(FULL, win, src + mt[1]);
                                 int kk = wv & 0xFF, left = GENERAL ? (wv >> 8) & 0xFF : wv >> 8;
-                                const int eb = GENERAL ? (int)(wv >> 16) : 0;
+                                const float2 *const edges = GENERAL && wv >> 16 ? (const float2 *)(P + ne * kPStride) : s.edge;
                                 if (fast) {
                                     // two tiles with one window go together
                                     if (left == 1 && act && wv2 == wv) {
                                         act &= act - 1;
-                                        tile_pass<1, 2>(s, P, mt, kk, eb, nt, ref, rs, n, lane, bs);
+                                        tile_pass<1, 2>(s, P, mt, kk, edges, nt, ref, rs, n, lane, bs);
                                         continue;
                                     }
                                     for (; left > 4; left -= 4, kk += 4)
-                                        tile_pass<4, 1>(s, P, mt, kk, eb, nt, ref, rs, n, lane, bs);
+                                        tile_pass<4, 1>(s, P, mt, kk, edges, nt, ref, rs, n, lane, bs);
                                     switch (left) {
-                                    case 1: tile_pass<1, 1>(s, P, mt, kk, eb, nt, ref, rs, n, lane, bs); break;
-                                    case 2: tile_pass<2, 1>(s, P, mt, kk, eb, nt, ref, rs, n, lane, bs); break;
-                                    case 3: tile_pass<3, 1>(s, P, mt, kk, eb, nt, ref, rs, n, lane, bs); break;
-                                    default: tile_pass<4, 1>(s, P, mt, kk, eb, nt, ref, rs, n, lane, bs); break;
+                                    case 1: tile_pass<1, 1>(s, P, mt, kk, edges, nt, ref, rs, n, lane, bs); break;
+                                    case 2: tile_pass<2, 1>(s, P, mt, kk, edges, nt, ref, rs, n, lane, bs); break;
+                                    case 3: tile_pass<3, 1>(s, P, mt, kk, edges, nt, ref, rs, n, lane, bs); break;
+                                    default: tile_pass<4, 1>(s, P, mt, kk, edges, nt, ref, rs, n, lane, bs); break;
                                     }
                                 } else {  // out of FP32 range: every row exactly
                                     for (; left > 0; left -= 4, kk += 4)
@@ -1246,11 +1250,12 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
     }
 }
 
-static size_t tile_smem(int ne, int mode)
+static size_t tile_smem(int ne, int mode, bool general)
 {
     const size_t fixed = mode == KD_MODE_MIXED ? sizeof(TileSmem<KD_MODE_MIXED>)
                                                : sizeof(TileSmem<KD_MODE_FP64>);
-    return fixed + sizeof(unsigned) * (size_t)ne * kPStride;
+    static_assert(kPStride % 2 == 0 && sizeof(TileSmem<KD_MODE_MIXED>) % 8 == 0, "the table behind P is aligned");
+    return fixed + sizeof(unsigned) * (size_t)ne * kPStride + (general ? sizeof(float2) * (size_t)ne : 0);
 }
 
 // The kernel for these counts.  Its general variant costs all others 2 to 3% (the
@@ -1273,7 +1278,7 @@ struct TileKernel {
                       (mode == KD_MODE_MIXED && tcs[j]->uneven_leaves);
         run = mode == KD_MODE_MIXED ? (general ? k_tiles<KD_MODE_MIXED, true> : k_tiles<KD_MODE_MIXED, false>)
                                     : (general ? k_tiles<KD_MODE_FP64, true> : k_tiles<KD_MODE_FP64, false>);
-        smem = tile_smem(ne, mode);
+        smem = tile_smem(ne, mode, general);
         check(cudaFuncSetAttribute(run, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
               "smem attribute");
         check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, run, kTileThreads, smem), "occupancy");
