@@ -1777,7 +1777,7 @@ __global__ void k_tree_fields(int n, const int *__restrict__ p, const int *__res
 }
 
 // one CTA of KD_BLOCK_MAX threads per query block: box and single own field;
-// many, if given: warps with more than KD_FEW_FIELDS own fields
+// many, if given: warps with more than KD_MANY_FIELDS own fields
 __global__ void __launch_bounds__(KD_BLOCK_MAX) k_block_boxes(int nblocks, const int *bstart,
                                                              const int *blen, RawOut o,
                                                              double *bbox, int *bqf, int *many)
@@ -1802,7 +1802,7 @@ __global__ void __launch_bounds__(KD_BLOCK_MAX) k_block_boxes(int nblocks, const
     if (many) {
         const unsigned peers = __match_any_sync(0xffffffffu, qf);
         const unsigned fields = __ballot_sync(0xffffffffu, valid && lane == __ffs(peers) - 1);
-        if (lane == 0 && __popc(fields) > KD_FEW_FIELDS) atomicAdd(many, 1);
+        if (lane == 0 && __popc(fields) > KD_MANY_FIELDS) atomicAdd(many, 1);
     }
     for (int off = 16; off; off >>= 1)
         for (int d = 0; d < 3; d++) {
@@ -2824,7 +2824,7 @@ static void build_query(const double *h_xyz, const int *h_fields, int n, int num
         *bqf = keep.alloc<int>(nblocks);
     double *bbox = keep.alloc<double>(6 * (size_t)nblocks);
     k_query_points<<<grid_for(n), TPB, 0, s>>>(xyz, fin, cv.perm, n, ro, nblocks, bstart, blen);
-    const bool fields = (long long)h.fi.max_qf - h.fi.min_qf >= KD_FEW_FIELDS;
+    const bool fields = (long long)h.fi.max_qf - h.fi.min_qf >= KD_MANY_FIELDS;
     k_block_boxes<<<nblocks, KD_BLOCK_MAX, 0, s>>>(nblocks, bstart, blen, ro, bbox, bqf,
                                                    fields ? &dstate->many : nullptr);
     KD_LAUNCH_CHECK("k_query_points");

@@ -36,6 +36,9 @@ extern "C" {
 #define KD_BLOCK_MAX 128   /* query points per block (a CTA of four warps counts it) */
 #define KD_MAX_EDGES 64    /* distinct finite squared edges per count job */
 #define KD_FEW_FIELDS 4    /* own fields of 32 queries that a count sums field by field */
+#define KD_MANY_FIELDS 8   /* ... above which the tile kernel's general variant pays: 300k queries of
+                            * 10 random labels 2.22 -> 2.15 ms, of 64 2.42 -> 2.18, but 50k of 5
+                            * 1.24 -> 1.30 */
 
 /* the status codes (KD_OK, KD_EINVAL, ...) and KD_MAX_POINTS are public:
  * include/kdtree.h; the device error words use the same codes */
@@ -59,7 +62,7 @@ typedef struct kd_catalog {
     int fields_split; /* 1 when some raw point has qf != tf */
     int short_runs;   /* 1 when a tree's runs of one tree field are shorter than 4 points on
                        * average: its labels interleave in space */
-    int many_fields;  /* 1 when most groups of 32 query points hold more than KD_FEW_FIELDS own
+    int many_fields;  /* 1 when most groups of 32 query points hold more than KD_MANY_FIELDS own
                        * fields (a tree's by its runs: shorter than 8 points on average) */
     int uneven_leaves; /* 1 when an eighth of the points or more (at full leaves) lie in leaves
                         * of less than 1/64 of the largest one's size */
