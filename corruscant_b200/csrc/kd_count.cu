@@ -520,7 +520,7 @@ template <> struct TileSmem<KD_MODE_FP64> : TileCommon {
 // tile's fragment holds, for t < 3, coordinate t of rows g and g + 8: the
 // halves of v = -2 q_t S as (hi, hi) against the point's (hi, lo), and (lo,
 // lo) against the same; for t = 3, (1, 1) against the halves of N, and (0, 0).
-__device__ __noinline__ void set_scale(TileSmem<KD_MODE_MIXED> &s, float2 *small, int ne, int tid)
+template <bool GENERAL> __device__ __noinline__ void set_scale(TileSmem<KD_MODE_MIXED> &s, float2 *small, int ne, int tid)
 {
     const double S = (double)s.S, Rq = (double)s.Rq;
     const int qs = s.qs, qlen = s.qlen;
@@ -551,7 +551,7 @@ __device__ __noinline__ void set_scale(TileSmem<KD_MODE_MIXED> &s, float2 *small
         if (tid % kMT < 8) q.x = (float)n;
         else q.y = (float)n;
     }
-    for (int b = 0; b < (small ? 2 : 1); b++) {
+    for (int b = 0; b < (GENERAL && small ? 2 : 1); b++) {
         float2 *const edge = b ? small : s.edge;
         for (int k = tid; k < ne; k += kTileThreads)
             edge[k] = make_float2(
@@ -559,7 +559,7 @@ __device__ __noinline__ void set_scale(TileSmem<KD_MODE_MIXED> &s, float2 *small
                 (float)(0.5 / 1.1 / (band_halfwidth(s.R[k], Rq, b ? (double)s.hSmall : (double)s.hT, S) * S * S)));
     }
 }
-__device__ __forceinline__ void set_scale(TileSmem<KD_MODE_FP64> &, float2 *, int, int) {}
+template <bool GENERAL> __device__ __forceinline__ void set_scale(TileSmem<KD_MODE_FP64> &, float2 *, int, int) {}
 
 // A whole block whose runs are a point or two each (many labels that interleave
 // in space), by the whole CTA: a warp per record, four queries a lane, every
@@ -910,7 +910,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                 }
             }
             const float far = s.kfp >= 0 ? sqrtf(s.Rup[s.kfp]) * 1.0001f : 0.0f;
-            float hT = __double2float_ru(J.hT), hSmall = hT;
+            float hT = __double2float_ru(J.hT), hSmall = 0.0f;
             if constexpr (GENERAL) {
                 // The error band allows for the rounding of a point relative to
                 // its leaf's centre, so it grows with the leaf, and beside leaves
@@ -944,8 +944,10 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                 s.qlen = qlen;
                 s.Rq = Rq;
                 s.hT = hT;
-                s.hSmall = hSmall;
-                s.hcap = J.hT <= (double)hT ? INFINITY : hT;  // (J.hT may be NaN)
+                if constexpr (GENERAL) {
+                    s.hSmall = hSmall;
+                    s.hcap = J.hT <= (double)hT ? INFINITY : hT;  // (J.hT may be NaN)
+                }
                 s.S = S;
             }
             __syncthreads();
@@ -958,7 +960,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                     continue;
                 }
             if (MODE == KD_MODE_MIXED && S > 0.0f)
-                set_scale(s, GENERAL && hSmall < hT ? (float2 *)(P + ne * kPStride) : nullptr, ne, tid);
+                set_scale<GENERAL>(s, GENERAL && hSmall < hT ? (float2 *)(P + ne * kPStride) : nullptr, ne, tid);
         }
         // ---- one flush key after the other (tree field | 256 for the
         // once-counted part of a symmetric job)
@@ -1016,13 +1018,12 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                         // sqrt of every edge of the record
                         const float B = sqrtf(dx * dx + dy * dy + dz * dz) * 1.0001f + s.hT + 2.0f * s.Rq;
                         ok = ok && B < (float)kFp32Span && s.R[k1 - 1] < kFp32MaxR;
-                        const bool scaled = s.S > 0.0f && B * s.S <= 240.0f;
                         if constexpr (GENERAL) {  // (a window needs no scale)
                             const float h = hx + hy + hz;
-                            fast_ok = ok && scaled && h <= s.hcap;
+                            fast_ok = ok && s.S > 0.0f && B * s.S <= 240.0f && h <= s.hcap;
                             small = h <= s.hSmall && s.hSmall < s.hT;
                         } else {
-                            ok = fast_ok = ok && (MODE == KD_MODE_FP64 || scaled);
+                            ok = ok && (MODE == KD_MODE_FP64 || (s.S > 0.0f && B * s.S <= 240.0f));
                         }
                         if (ok) {
                             // rounding of the staged coordinates and of the tile box
@@ -1051,7 +1052,7 @@ __global__ void __launch_bounds__(kTileThreads, kTilesPerSm) k_tiles(TileArgs A)
                     const int mval = max(0, min(kMT, s.qlen - kMT * wm));  // queries of tile wm
                     const int K = have && mval ? k1 - k0 : 0;
                     const unsigned win = (unsigned)k0 | ((unsigned)K << 8) | (GENERAL && small ? 1u << 16 : 0u);
-                    const unsigned actm = __ballot_sync(FULL, K != 0), okm = __ballot_sync(FULL, fast_ok);
+                    const unsigned actm = __ballot_sync(FULL, K != 0), okm = __ballot_sync(FULL, GENERAL ? fast_ok : ok);
                     if (have && mval) atomicAdd(&s.F[k1 * kMTiles + wm], (unsigned)rl);
                     {
                         const unsigned q = K ? (unsigned)(mval * rl) : 0u;
